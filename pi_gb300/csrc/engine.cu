@@ -156,31 +156,13 @@ static uint64_t find_rho() {
 }
 
 // ------------------------------------------------------------------ kernels
-// Geometry of the HBM passes.  Pass tiles hold 2^12 words (32 KiB plus
-// padding, so that five CTAs share an SM) and are processed by 256 threads:
-//   first pass (p = 0):   2^R rows x 2^(12-R) columns of the single block
-//   middle passes:        2^(9-R) blocks x 2^R rows x 8 columns
-//   last pass (S = 1):    2^(12-R) contiguous blocks of 2^R words
-// Column tiles read 64-byte (or wider) row segments; first-pass rows hold at
-// least 8 consecutive coefficients, one carry window.
-constexpr int PASS_THREADS = 256;
-constexpr int TILE_LOG = 12;
-// Resident CTAs per SM the pass kernels are register-limited for.
-#ifndef PIMUL_PASS_MIN_CTAS
-#define PIMUL_PASS_MIN_CTAS 5
-#endif
-constexpr int PASS_MIN_CTAS = PIMUL_PASS_MIN_CTAS;
-
-static inline size_t pass_smem_bytes(int tile_log) { return ((size_t)1 << tile_log) * 17 / 16 * 8 + 512 * 8; }
-
-// Load the 512 forward roots w_512^t into shared memory (round twiddles).
-__device__ __forceinline__ void load_tw512(uint64_t* tw, const Roots& R) {
-  for (int t = threadIdx.x; t < 512; t += blockDim.x) tw[t] = __ldg(R.lvl + 512 + t);
-}
-
-// Elements per thread in a pass tile, processed in groups of 8 so that
-// every thread keeps 8 independent global loads in flight.
-constexpr int PER_THREAD = (1 << TILE_LOG) / PASS_THREADS;
+// Geometry of the HBM passes (ntt_kernels.cuh): CTAs of 128 threads,
+//   first and middle passes: 2^R rows x 8 or 16 columns of one block
+//   last pass (S = 1):       four warps, each 32 2^B1 contiguous words
+// First-pass rows hold at least 8 consecutive coefficients, one carry window.
+// Four CTAs per SM leave 128 registers for a thread's radix-32 round (113 to
+// 126 used); 96 (five CTAs) spill, 168 (three) run no faster.
+constexpr int PASS_MIN_CTAS = 4;
 
 // One product of a batch (or the only product of a plain call): operands,
 // output and its scratch.  Kernels take `const Job* jobs, Job one`: with a
@@ -195,7 +177,8 @@ struct Job {
   uint64_t* H;  // high parts of the carry windows
   uint8_t* aux; // carry-scan flags
   uint64_t la, lb;
-  const uint64_t* X;  // spectrum added to the pointwise product (a sum of two products), or null
+  const uint64_t* X;  // spectra of a second product added to the pointwise one (a sum of two products), or null
+  const uint64_t* Y;
   uint64_t nout;      // output limbs (0: la + lb); with JF_COEFF, output coefficients
   uint32_t flags;     // JF_* roles inside a batch (0: a plain product)
   // A wrapped product runs a cyclic transform of length N shorter than its
@@ -208,13 +191,11 @@ struct Job {
 };
 
 // Roles of a product inside a batch.  A spectrum shared by several products
-// with the same operand b is computed once, by its owner (JF_B_FULL); the
-// others point B at it (JF_B_SHARED) and skip b's passes.  With a full
-// spectrum in B, k_mid only multiplies and writes the product to A.  An
-// addend (JF_ADDEND) produces no output: its pointwise product A * B stays
-// in A, where the job it is added to reads it as X.
+// with the same operand b is computed once, by its owner; the others point B
+// at it (JF_B_SHARED) and skip b's passes.  An addend (JF_ADDEND) produces no
+// output: the job it is added to reads its spectra as X and Y.  Every product
+// is formed in A.
 constexpr uint32_t JF_B_SHARED = 1;
-constexpr uint32_t JF_B_FULL = 2;
 constexpr uint32_t JF_ADDEND = 4;
 // The product's canonical coefficients 0 .. nout - 1 go to out (no carry):
 // the low part of a wrapped product.
@@ -224,278 +205,272 @@ __device__ __forceinline__ Job job_of(const Job* jobs, const Job& one) {
   if (jobs) return jobs[blockIdx.y];
   return one;
 }
-__device__ __forceinline__ bool is_square(const Job& J) { return J.a == J.b && J.la == J.lb; }
+__host__ __device__ __forceinline__ bool is_square(const Job& J) { return J.a == J.b && J.la == J.lb; }
 // b's own passes are skipped for a square and for a borrowed spectrum.
 __device__ __forceinline__ bool skips_b(const Job& J) { return is_square(J) || (J.flags & JF_B_SHARED); }
-__device__ __forceinline__ bool b_spectrum(const Job& J) { return (J.flags & (JF_B_SHARED | JF_B_FULL)) != 0; }
 __host__ __device__ __forceinline__ uint64_t job_nout(const Job& J) { return J.nout ? J.nout : J.la + J.lb; }
-// Array a pass works on: 0 = A, 1 = B, 2 = the product array.
-__device__ __forceinline__ uint64_t* job_array(const Job& J, int which) {
-  if (which == 0) return J.A;
-  if (which == 1) return J.B;
-  return is_square(J) || b_spectrum(J) ? J.A : J.B;
-}
 
 // Forward pass 0 with the limb -> 16-bit coefficient split fused in
 // (crates/bignum/src/ntt.rs:640-665): element (i, j) of the tile is
-// coefficient n = i * 2^S + j0 + j, i.e. 16-bit slice n % 4 of limb n / 4;
-// limbs past nl are zero (the reference's zero tail).  which = 0: operand a,
-// 1: operand b (squares skip b).
+// coefficient n = i * 2^S + j0 + j, the n-th 16-bit word of the operand;
+// words past its end are zero (the reference's zero tail).  Operand
+// w0 + blockIdx.z (0: a, 1: b; skips_b drops b).
 // twf: the pass's twiddle table (tw_first), or null to compute the twiddles.
 template <int R>
-__global__ void __launch_bounds__(PASS_THREADS, PASS_MIN_CTAS) k_fwd_first(const Job* jobs, Job one, int which, int L, Roots RT,
+__global__ void __launch_bounds__(PASS_THREADS, PASS_MIN_CTAS) k_fwd_first(const Job* jobs, Job one, int w0, int L, Roots RT,
                                                                            const uint64_t* __restrict__ twf) {
-  constexpr int T = TILE_LOG - R;
+  using G = ColGeom<R>;
+  constexpr int B1 = G::B1, B2 = G::B2, T = G::T;
   const Job J = job_of(jobs, one);
+  const int which = w0 + (int)blockIdx.z;
   if (which == 1 && skips_b(J)) return;
-  const uint64_t* __restrict__ limbs = which ? J.b : J.a;
-  const uint64_t nl = which ? J.lb : J.la;
+  const uint16_t* __restrict__ coef = reinterpret_cast<const uint16_t*>(which ? J.b : J.a);
+  const uint64_t nc = 4 * (which ? J.lb : J.la);
   uint64_t* __restrict__ data = which ? J.B : J.A;
   extern __shared__ uint64_t sm[];
-  uint64_t* tw = sm + spad(1u << TILE_LOG);
   const int tid = threadIdx.x;
   const int S = L - R;
   const uint64_t j0 = (uint64_t)blockIdx.x << T;
-  load_tw512(tw, RT);
-  // an operand of at most 2^(L-3) limbs leaves rows 2^(R-1) and up zero
-  // (coefficients N/2 and up): they are neither written nor read
-  const bool half = 4 * nl <= (1ull << (L - 1));
-  // each thread expands whole limbs: 2^R rows (2^(R-1) if half) x 2^(T-2) limbs
-  const uint32_t nq = half ? 1u << (R + T - 3) : 1u << (R + T - 2);
-  for (uint32_t q = tid; q < nq; q += PASS_THREADS) {
-    uint32_t i = q >> (T - 2), c4 = q & ((1u << (T - 2)) - 1);
-    uint64_t li = (((uint64_t)i << S) + j0) / 4 + c4;
-    uint64_t x = li < nl ? __ldg(limbs + li) : 0;
-    uint32_t base = (i << T) + 4 * c4;
-    sm[spad(base + 0)] = x & 0xFFFF;
-    sm[spad(base + 1)] = (x >> 16) & 0xFFFF;
-    sm[spad(base + 2)] = (x >> 32) & 0xFFFF;
-    sm[spad(base + 3)] = x >> 48;
-  }
-  __syncthreads();
-  if (half)
-    tile_fwd_t<R, T, 0, PASS_THREADS, true>(sm, tw, tid);
-  else
-    tile_fwd_t<R, T, 0, PASS_THREADS>(sm, tw, tid);
-  // element e of this thread: lin = e * 256 + tid, row (e << TL) + (tid >> T),
-  // column tid & (2^T - 1); address and twiddle exponent split into a
-  // per-thread part and a compile-time part
-  constexpr int TL = 8 - T;
-  const uint32_t tlo = tid >> T, jj = tid & ((1u << T) - 1);
-  const uint64_t gbase = ((uint64_t)tlo << S) + j0 + jj;
-  if (twf) {
-    // twiddles laid out like the data: one coalesced load each
-#pragma unroll 2
-    for (int g = 0; g < PER_THREAD; g += 8) {
-      uint64_t t8[8];
+  {
+    const uint64_t n0 = ((uint64_t)(tid >> T) << S) + j0 + (tid & G::TM);
+    const uint64_t step = 1ull << (S + B2);
+    // inputs m < mc exist
+    const uint32_t mc = n0 < nc ? (uint32_t)((nc - n0 + step - 1) >> (S + B2)) : 0;
+    uint64_t v[1 << B1];
+    gl::Lz x[1 << B1];
+    // an operand of at most N/8 limbs leaves the upper half of the rows zero
+    // (coefficients N/2 and up): those inputs are neither read nor added
+    if (nc <= (1ull << (L - 1))) {
 #pragma unroll
-      for (int q = 0; q < 8; q++) t8[q] = __ldg(twf + gbase + ((uint64_t)((g + q) << TL) << S));
+      for (int m = 0; m < (1 << (B1 - 1)); m++) x[m] = gl::Lz{m < mc ? (uint32_t)__ldg(coef + n0 + m * step) : 0u, 0u, 0};
+      x[0] = gl::lz_bias(x[0]);
+      dft_lz<B1, false, true>(x, v);
+    } else {
 #pragma unroll
-      for (int q = 0; q < 8; q++)
-        data[gbase + ((uint64_t)((g + q) << TL) << S)] = gl::mul(sm[spad((g + q) * PASS_THREADS + tid)], t8[q]);
+      for (int m = 0; m < (1 << B1); m++) x[m] = gl::Lz{m < mc ? (uint32_t)__ldg(coef + n0 + m * step) : 0u, 0u, 0};
+      x[0] = gl::lz_bias(x[0]);
+      dft_lz<B1, false>(x, v);
     }
-    return;
+#pragma unroll
+    for (int k = 0; k < (1 << B1); k++) sm[k * G::KS + tid] = v[k];
   }
-  if (L > LVL_MAX) {
-    // w^(f (j0 + jj)) = w^(f j0) w^(f jj): the first factor for the tile's
-    // 2^R frequencies replaces the round twiddles in tw (the rounds are
-    // done), the second (f jj < 4096) comes from the L1-resident near table
+  // Without a table, w^(f (j0 + j)) = w^(f j0) w^(f j) for a long transform: the
+  // first factors of the tile's 2^R frequencies are staged, the second
+  // (f j < 4096) come from the L1-resident near table.
+  uint64_t* tw = sm + G::XWORDS;
+  const bool staged = !twf && L > LVL_MAX;
+  if (staged)
     for (uint32_t f = tid; f < (1u << R); f += PASS_THREADS) tw[f] = root_pow32(RT, L, f * (uint32_t)j0, false);
-    __syncthreads();
-    const uint64_t* __restrict__ nt = near_table(RT, L, false);
-    const uint32_t f0 = row_freq_t<R>(tlo);
-#pragma unroll 2
-    for (int g = 0; g < PER_THREAD; g += 8) {
-      uint64_t t8[8];
+  __syncthreads();
+  const uint64_t* __restrict__ rt = RT.rt + rt_offset(R, false);
+#pragma unroll 1
+  for (int it = 0; it < G::ITERS2; it++) {
+    const uint32_t w = it * PASS_THREADS + tid, j = w & G::TM, k1 = w >> T;
+    uint64_t v[1 << B2];
+    pass_fwd2<R>(sm + k1 * G::KS + j, 1u << T, rt, k1, v);
+    const uint64_t at = ((uint64_t)(k1 << B2) << S) + j0 + j;
+    if (twf) {
+      // twiddles laid out like the data: one coalesced load each
 #pragma unroll
-      for (int q = 0; q < 8; q++) {
-        const uint32_t f = f0 + row_freq_t<R>((g + q) << TL);
-        t8[q] = gl::mul(tw[f], __ldg(nt + f * jj));
+      for (int k = 0; k < (1 << B2); k++) data[at + ((uint64_t)k << S)] = gl::mul(v[k], __ldg(twf + at + ((uint64_t)k << S)));
+    } else if (staged) {
+      const uint64_t* __restrict__ nt = near_table(RT, L, false);
+#pragma unroll
+      for (int k = 0; k < (1 << B2); k++) {
+        const uint32_t f = k1 + (k << B1);
+        data[at + ((uint64_t)k << S)] = gl::mul(v[k], gl::mul(tw[f], __ldg(nt + f * j)));
       }
+    } else {
 #pragma unroll
-      for (int q = 0; q < 8; q++)
-        data[gbase + ((uint64_t)((g + q) << TL) << S)] = gl::mul(sm[spad((g + q) * PASS_THREADS + tid)], t8[q]);
+      for (int k = 0; k < (1 << B2); k++)
+        data[at + ((uint64_t)k << S)] = gl::mul(v[k], root_pow32(RT, L, (k1 + (k << B1)) * (uint32_t)(j0 + j), false));
     }
-    return;
-  }
-  const uint32_t Jc = (uint32_t)(j0 + jj);
-  const uint32_t eJ = row_freq_t<R>(tlo) * Jc;
-#pragma unroll 2
-  for (int g = 0; g < PER_THREAD; g += 8) {
-    uint64_t t8[8];
-#pragma unroll
-    for (int q = 0; q < 8; q++) t8[q] = root_pow32(RT, L, eJ + row_freq_t<R>((g + q) << TL) * Jc, false);
-#pragma unroll
-    for (int q = 0; q < 8; q++)
-      data[gbase + ((uint64_t)((g + q) << TL) << S)] = gl::mul(sm[spad((g + q) * PASS_THREADS + tid)], t8[q]);
   }
 }
 
-// Middle column pass: 2^(9-R) blocks x 2^R rows x 2^T columns; forward pass
-// twiddles w_M^(f*j) after the rounds, inverse ones before.
+// Middle column pass of stride 2^S; forward pass twiddles w_M^(f*j) after the
+// rounds (operand w0 + blockIdx.z), inverse ones before (on the product).
 // twm: the pass's twiddle table (tw_mid), or null to compute the twiddles.
 template <int R, bool FWD>
-__global__ void __launch_bounds__(PASS_THREADS, PASS_MIN_CTAS) k_col_mid(const Job* jobs, Job one, int which, int S, Roots RT,
+__global__ void __launch_bounds__(PASS_THREADS, PASS_MIN_CTAS) k_col_mid(const Job* jobs, Job one, int w0, int S, Roots RT,
                                                                          const uint64_t* __restrict__ twm) {
-  constexpr int T = TILE_LOG - 9, BC = 9 - R;
-  constexpr int TL = 8 - T;  // row bits covered by tid >> T
-  static_assert(R >= TL, "thread index must stay inside one block's rows");
-  constexpr uint32_t TM = (1u << T) - 1, RM = (1u << R) - 1;
+  using G = ColGeom<R>;
+  constexpr int B1 = G::B1, B2 = G::B2, T = G::T;
   const Job J = job_of(jobs, one);
+  const int which = w0 + (int)blockIdx.z;
   if (FWD && which == 1 && skips_b(J)) return;
   if (!FWD && (J.flags & JF_ADDEND)) return;
-  uint64_t* __restrict__ data = job_array(J, which);
   extern __shared__ uint64_t sm[];
-  uint64_t* tw = sm + spad(1u << TILE_LOG);
   const int tid = threadIdx.x;
   const int mlog = R + S;
-  const uint64_t ct = blockIdx.x & ((1u << (S - T)) - 1);
-  const uint64_t b0 = ((uint64_t)blockIdx.x >> (S - T)) << BC;
-  const uint64_t j0 = ct << T;
-  // element q of this thread (lin = q * 256 + tid): block q >> (R - TL), row
-  // ((q << TL) & RM) + (tid >> T), column tid & TM
-  const uint32_t tlo = tid >> T, jj = tid & TM;
-  const uint64_t gbase = (b0 << mlog) + ((uint64_t)tlo << S) + j0 + jj;
-  auto gaddr = [&](int q) {
-    return gbase + ((uint64_t)(q >> (R - TL)) << mlog) + ((uint64_t)((q << TL) & RM) << S);
-  };
+  const uint64_t j0 = (uint64_t)(blockIdx.x & ((1u << (S - T)) - 1)) << T;
+  const uint64_t b0 = (uint64_t)blockIdx.x >> (S - T);
+  uint64_t* __restrict__ data = (FWD && which ? J.B : J.A) + (b0 << mlog) + j0;
+  // element (m, column) of this thread in the round that has m fixed
+  const uint64_t mat = ((uint64_t)(tid >> T) << S) + (tid & G::TM);
+  if constexpr (FWD) {
+    {
+      uint64_t v[1 << B1];
+      gl::Lz x[1 << B1];
 #pragma unroll
-  for (int q = 0; q < PER_THREAD; q++) cp_async8(sm + spad(q * PASS_THREADS + tid), data + gaddr(q));
-  load_tw512(tw, RT);
-  cp_async_wait_all();
-  __syncthreads();
-  const uint32_t Jc = (uint32_t)(j0 + jj);
-  if (FWD) {
-    tile_fwd_t<R, T, BC, PASS_THREADS>(sm, tw, tid);
-    // outgoing pass twiddles w_M^(f*j)
-    const uint32_t eJ = row_freq_t<R>(tlo) * Jc;
-    // table: twm[r 2^S + j] for row r of the block and column j
-    const uint64_t tbase = ((uint64_t)tlo << S) + j0 + jj;
+      for (int m = 0; m < (1 << B1); m++) v[m] = data[mat + ((uint64_t)m << (S + B2))];
+#pragma unroll
+      for (int m = 0; m < (1 << B1); m++) x[m] = gl::lz(v[m]);
+      x[0] = gl::lz_bias(x[0]);
+      dft_lz<B1, false>(x, v);
+#pragma unroll
+      for (int k = 0; k < (1 << B1); k++) sm[k * G::KS + tid] = v[k];
+    }
+    __syncthreads();
+    const uint64_t* __restrict__ rt = RT.rt + rt_offset(R, false);
 #pragma unroll 1
-    for (int g = 0; g < PER_THREAD; g += 8) {
-      uint64_t t8[8];
+    for (int it = 0; it < G::ITERS2; it++) {
+      const uint32_t w = it * PASS_THREADS + tid, j = w & G::TM, k1 = w >> T;
+      uint64_t v[1 << B2];
+      pass_fwd2<R>(sm + k1 * G::KS + j, 1u << T, rt, k1, v);
+      const uint64_t at = ((uint64_t)(k1 << B2) << S) + j;
       if (twm) {
 #pragma unroll
-        for (int q = 0; q < 8; q++) t8[q] = __ldg(twm + tbase + ((uint64_t)(((g + q) << TL) & RM) << S));
+        for (int k = 0; k < (1 << B2); k++)
+          data[at + ((uint64_t)k << S)] = gl::mul(v[k], __ldg(twm + j0 + at + ((uint64_t)k << S)));
       } else {
 #pragma unroll
-        for (int q = 0; q < 8; q++)
-          t8[q] = root_pow32(RT, mlog, eJ + row_freq_t<R>(((g + q) << TL) & RM) * Jc, false);
+        for (int k = 0; k < (1 << B2); k++)
+          data[at + ((uint64_t)k << S)] = gl::mul(v[k], root_pow32(RT, mlog, (k1 + (k << B1)) * (uint32_t)(j0 + j), false));
       }
-#pragma unroll
-      for (int q = 0; q < 8; q++) data[gaddr(g + q)] = gl::mul(sm[spad((g + q) * PASS_THREADS + tid)], t8[q]);
     }
   } else {
-    // incoming pass twiddles w_M^-(f*j), applied by the first inverse round
-    // (tile row row0 + k is row (row0 + k) & RM of its block)
-    auto ptw = [&](uint32_t row0, int k, uint32_t j) {
-      if (twm) return __ldg(twm + ((uint64_t)((row0 & RM) + (uint32_t)k) << S) + j0 + j);
-      const uint32_t f = row_freq_t<R>(row0 & RM) + row_freq_t<R>((uint32_t)k);
-      return root_pow32(RT, mlog, f * (uint32_t)(j0 + j), true);
-    };
-    tile_inv_t<R, T, BC, PASS_THREADS, rp_count(R) - 1>(sm, tw, tid, ptw);
+#pragma unroll 1
+    for (int it = 0; it < G::ITERS2; it++) {
+      const uint32_t w = it * PASS_THREADS + tid, j = w & G::TM, k1 = w >> T;
+      const uint64_t at = ((uint64_t)(k1 << B2) << S) + j;
+      uint64_t v[1 << B2];
+      gl::Lz x[1 << B2];
 #pragma unroll
-    for (int q = 0; q < PER_THREAD; q++) data[gaddr(q)] = sm[spad(q * PASS_THREADS + tid)];
+      for (int k = 0; k < (1 << B2); k++) v[k] = data[at + ((uint64_t)k << S)];
+      if (twm) {
+#pragma unroll
+        for (int k = 0; k < (1 << B2); k++) x[k] = gl::lz_mul(v[k], __ldg(twm + j0 + at + ((uint64_t)k << S)));
+      } else {
+#pragma unroll
+        for (int k = 0; k < (1 << B2); k++)
+          x[k] = gl::lz_mul(v[k], root_pow32(RT, mlog, (k1 + (k << B1)) * (uint32_t)(j0 + j), true));
+      }
+      x[0] = gl::lz_bias(x[0]);
+      dft_lz<B2, true>(x, v);
+#pragma unroll
+      for (int m = 0; m < (1 << B2); m++) sm[k1 * G::KS + (m << T) + j] = v[m];
+    }
+    __syncthreads();
+    uint64_t v[1 << B1];
+    pass_inv2<R>(sm + tid, G::KS, RT.rt + rt_offset(R, true), tid >> T, v);
+#pragma unroll
+    for (int m = 0; m < (1 << B1); m++) data[mat + ((uint64_t)m << (S + B2))] = v[m];
   }
 }
 
-// Last forward pass (stride 1): 2^(13-R) contiguous blocks of 2^R words, of
-// operand a (which = 0) or, for a full spectrum of b (JF_B_FULL), of b.
-// Squares skip it: their last pass is fused into k_mid.
+// Last forward pass (stride 1) of operand w0 + blockIdx.z.  Fused with the
+// pointwise product and the first inverse pass it ran slower (2^25 points:
+// 442 us for both operands' last passes and the inverse's first one, against
+// 113 per operand and 150-170 here): four unrolled rounds overflow the
+// instruction caches, and two tiles per CTA cost a CTA per SM.  A warp's 32 2^B1
+// words hold whole blocks; it leaves its spectrum as rows of 32 words, one
+// per (iteration, k2), the order in which the inverse's first round reads it.
 template <int R>
-__global__ void __launch_bounds__(PASS_THREADS, PASS_MIN_CTAS) k_fwd_last(const Job* jobs, Job one, int which,
-                                                                          Roots RT) {
-  static_assert(R <= 9 && PASS_THREADS == 256 && TILE_LOG == 12, "eight warps, one 512-word chunk each");
+__global__ void __launch_bounds__(PASS_THREADS, PASS_MIN_CTAS) k_fwd_last(const Job* jobs, Job one, int w0, Roots RT) {
+  using G = RowGeom<R>;
+  constexpr int B1 = G::B1, B2 = G::B2;
   const Job J = job_of(jobs, one);
-  if (is_square(J)) return;
-  if (which == 1 && !(J.flags & JF_B_FULL)) return;
+  const int which = w0 + (int)blockIdx.z;
+  if (which == 1 && skips_b(J)) return;
   extern __shared__ uint64_t sm[];
-  uint64_t* tw = sm + spad(1u << TILE_LOG);
-  // warp w owns the tile's 512-word chunk w (whole blocks): after the round
-  // twiddles are staged, only __syncwarp separates its rounds
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  uint64_t* chunk = (which ? J.B : J.A) + ((uint64_t)blockIdx.x << TILE_LOG) + ((uint32_t)warp << 9);
-  uint64_t* smc = sm + spad((uint32_t)warp << 9);
+  uint64_t* __restrict__ chunk = (which ? J.B : J.A) + ((uint64_t)blockIdx.x << G::TILE) + warp * G::WWORDS;
+  uint64_t* sw = sm + warp * G::XWORDS;
+  {
+    const uint32_t m0 = lane & ((1u << B2) - 1), blk = lane >> B2;
+    uint64_t v[1 << B1];
+    gl::Lz x[1 << B1];
 #pragma unroll
-  for (int q = 0; q < 16; q++) cp_async8(smc + spad(q * 32 + lane), chunk + q * 32 + lane);
-  load_tw512(tw, RT);
-  cp_async_wait_all();
-  __syncthreads();
-  chunk_fwd_t<R>(smc, tw, lane);
+    for (int m = 0; m < (1 << B1); m++) v[m] = chunk[(blk << R) + (m << B2) + m0];
 #pragma unroll
-  for (int q = 0; q < 16; q++) chunk[q * 32 + lane] = smc[spad(q * 32 + lane)];
+    for (int m = 0; m < (1 << B1); m++) x[m] = gl::lz(v[m]);
+    x[0] = gl::lz_bias(x[0]);
+    dft_lz<B1, false>(x, v);
+    uint64_t* sx = sw + (blk << B1) * G::KS + blk * G::BPAD + m0;
+#pragma unroll
+    for (int k = 0; k < (1 << B1); k++) sx[k * G::KS] = v[k];
+  }
+  __syncwarp();
+  const uint64_t* __restrict__ rt = RT.rt + rt_offset(R, false);
+#pragma unroll 1
+  for (int it = 0; it < G::ITERS2; it++) {
+    const uint32_t idx = it * 32 + lane, k1 = idx & ((1u << B1) - 1), blk = idx >> B1;
+    uint64_t v[1 << B2];
+    pass_fwd2<R>(sw + idx * G::KS + blk * G::BPAD, 1, rt, k1, v);
+#pragma unroll
+    for (int k = 0; k < (1 << B2); k++) chunk[(((it << B2) + k) << 5) + lane] = v[k];
+  }
 }
 
-// Fused middle of the multiply on one contiguous tile: last forward pass of
-// b, pointwise product with the spectrum of a (plus X for a sum of two
-// products; times N^-1, the inverse's 1/N, crates/bignum/src/ntt.rs:383-390
-// and 845-853), first inverse pass; the result overwrites b's array.  A
-// square transforms and squares a's array in place; with b's full spectrum
-// in B (shared or owned) the last pass is skipped and the result goes to A.
-// EXT = false: plain products only (no shared spectrum, no addend), the
-// form every single product and every batch without those roles uses.
-// ninv = 0: no scaling here (the inverse first pass's twiddle table carries N^-1).
-template <int R, bool EXT>
-__global__ void __launch_bounds__(PASS_THREADS, PASS_MIN_CTAS) k_mid(const Job* jobs, Job one, uint64_t ninv, Roots RT) {
-  static_assert(R <= 9 && PASS_THREADS == 256 && TILE_LOG == 12, "eight warps, one 512-word chunk each");
+// Pointwise product of the two spectra (plus X Y, a second product, for a sum;
+// times N^-1, the inverse's 1/N, crates/bignum/src/ntt.rs:383-390 and
+// 845-853), entering the first inverse pass as lazy products; the result
+// overwrites A.  ninv = 0: no scaling here (the inverse first pass's twiddle
+// table carries N^-1).
+template <int R>
+__global__ void __launch_bounds__(PASS_THREADS, PASS_MIN_CTAS) k_inv_last(const Job* jobs, Job one, uint64_t ninv, Roots RT) {
+  using G = RowGeom<R>;
+  constexpr int B1 = G::B1, B2 = G::B2;
   const Job J = job_of(jobs, one);
-  if (EXT && (J.flags & JF_ADDEND)) return;
-  const bool sq = is_square(J), spec = EXT && b_spectrum(J);
-  const uint64_t* cin = sq ? J.A : J.B;
-  uint64_t* cout = sq || spec ? J.A : J.B;
-  const uint64_t* a = J.A;
-  const uint64_t* __restrict__ X = J.X;
+  if (J.flags & JF_ADDEND) return;
   extern __shared__ uint64_t sm[];
-  uint64_t* tw = sm + spad(1u << TILE_LOG);
-  const int tid = threadIdx.x;
-  const uint64_t off = (uint64_t)blockIdx.x << TILE_LOG;
-  // warp w owns the tile's 512-word chunk w (whole blocks) from load to store
-  const int warp = tid >> 5, lane = tid & 31;
-  const uint64_t coff = off + ((uint32_t)warp << 9);
-  uint64_t* smc = sm + spad((uint32_t)warp << 9);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const uint64_t off = ((uint64_t)blockIdx.x << G::TILE) + warp * G::WWORDS;
+  const bool sq = is_square(J);
+  uint64_t* __restrict__ chunk = J.A + off;
+  const uint64_t* __restrict__ bspec = J.B + off;
+  uint64_t* sw = sm + warp * G::XWORDS;
+#pragma unroll 1
+  for (int it = 0; it < G::ITERS2; it++) {
+    const uint32_t idx = it * 32 + lane, blk = idx >> B1;
+    const uint32_t at = (it << (B2 + 5)) + lane;
+    uint64_t v[1 << B2], y[1 << B2];
+    gl::Lz x[1 << B2];
 #pragma unroll
-  for (int q = 0; q < 16; q++) cp_async8(smc + spad(q * 32 + lane), cin + coff + q * 32 + lane);
-  // a's (and the addend's) tile is read after b's rounds: start it towards
-  // L2 now (tiles are 32 KB at 32 KB offsets of 256-byte aligned arrays)
-  if (tid == 0) {
-    if (!sq) prefetch_l2_bulk(a + off, (8u << TILE_LOG));
-    if (EXT && X) prefetch_l2_bulk(X + off, (8u << TILE_LOG));
-  }
-  load_tw512(tw, RT);
-  cp_async_wait_all();
-  __syncthreads();
-  if (!spec) chunk_fwd_t<R>(smc, tw, lane);
-  if (EXT && X) {
-    // sum of two products: a b + X, then the inverse rounds
-#pragma unroll 4
-    for (int q = 0; q < 16; q++) {
-      const uint32_t lin = q * 32 + lane;
-      uint64_t x = smc[spad(lin)];
-      uint64_t p = gl::add(gl::mul(x, sq ? x : a[coff + lin]), X[coff + lin]);
-      smc[spad(lin)] = ninv ? gl::mul(p, ninv) : p;
+    for (int k = 0; k < (1 << B2); k++) v[k] = chunk[at + (k << 5)];
+    if (sq) {
+#pragma unroll
+      for (int k = 0; k < (1 << B2); k++) y[k] = v[k];
+    } else {
+#pragma unroll
+      for (int k = 0; k < (1 << B2); k++) y[k] = bspec[at + (k << 5)];
     }
-    __syncwarp();
-    chunk_inv_t<R>(smc, tw, lane);
-  } else {
-    // the pointwise product (times N^-1 when the inverse first pass's table
-    // does not carry it) enters the first inverse round as lazy products
-    auto pw = [&](uint32_t row0, int k, uint32_t) {
-      const uint32_t lin = row0 + (uint32_t)k;
-      const uint64_t y = sq ? smc[spad(lin)] : a[coff + lin];
-      return ninv ? gl::mul(y, ninv) : y;
-    };
-    chunk_inv_t<R>(smc, tw, lane, pw);
-  }
+    if (J.X) {
+      // a b + X Y in lazy form (|k| <= 2), folded before the scaling or the DFT
+      const uint64_t* __restrict__ X = J.X + off;
+      const uint64_t* __restrict__ Y = J.Y + off;
 #pragma unroll
-  for (int q = 0; q < 16; q++) cout[coff + q * 32 + lane] = smc[spad(q * 32 + lane)];
-}
-
-// Addends: A <- A * B (spectra, element by element), read later as X.
-__global__ void __launch_bounds__(256) k_pointwise_addend(const Job* jobs, Job one, uint64_t n) {
-  const Job J = job_of(jobs, one);
-  if (!(J.flags & JF_ADDEND)) return;
-  for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x)
-    J.A[i] = gl::mul(J.A[i], J.B[i]);
+      for (int k = 0; k < (1 << B2); k++) {
+        v[k] = gl::add(gl::mul(v[k], y[k]), gl::mul(X[at + (k << 5)], Y[at + (k << 5)]));
+        x[k] = gl::lz(ninv ? gl::mul(v[k], ninv) : v[k]);
+      }
+    } else {
+#pragma unroll
+      for (int k = 0; k < (1 << B2); k++) x[k] = gl::lz_mul(v[k], ninv ? gl::mul(y[k], ninv) : y[k]);
+    }
+    x[0] = gl::lz_bias(x[0]);
+    dft_lz<B2, true>(x, v);
+    uint64_t* sx = sw + idx * G::KS + blk * G::BPAD;
+#pragma unroll
+    for (int m = 0; m < (1 << B2); m++) sx[m] = v[m];
+  }
+  __syncwarp();
+  const uint32_t m0 = lane & ((1u << B2) - 1), blk = lane >> B2;
+  uint64_t v[1 << B1];
+  pass_inv2<R>(sw + (blk << B1) * G::KS + blk * G::BPAD + m0, G::KS, RT.rt + rt_offset(R, true), m0, v);
+#pragma unroll
+  for (int m = 0; m < (1 << B1); m++) chunk[(blk << R) + (m << B2) + m0] = v[m];
 }
 
 // ---- carry normalisation (crates/bignum/src/ntt.rs:676-791) --------------
@@ -571,76 +546,80 @@ __host__ __device__ __forceinline__ uint64_t aux_bytes_for(uint64_t nwin) {
 // row holds 2^T consecutive coefficients = 2^(T-3) windows; every window
 // writes its low 2 limbs to the output and its high part to H.
 // twi: the pass's twiddle table (tw_first, inverse, with N^-1), or null to
-// compute the twiddles (the caller then scales by N^-1 in k_mid).
+// compute the twiddles (the caller then scales by N^-1 in k_inv_last).
+// The rows are handed to the windows through shared memory, one pad word each.
+template <int R>
+constexpr uint32_t INV_FIRST_XWORDS = ColGeom<R>::XWORDS > ((ColGeom<R>::TM + 2) << R) ? ColGeom<R>::XWORDS
+                                                                                      : (ColGeom<R>::TM + 2) << R;
 template <int R>
 __global__ void __launch_bounds__(PASS_THREADS, PASS_MIN_CTAS) k_inv_first_carry(const Job* jobs, Job one, int L, Roots RT,
                                                                                  const uint64_t* __restrict__ twi) {
-  constexpr int T = TILE_LOG - R;
+  using G = ColGeom<R>;
+  constexpr int B1 = G::B1, B2 = G::B2, T = G::T;
   const Job J = job_of(jobs, one);
   if (J.flags & JF_ADDEND) return;
-  const uint64_t* __restrict__ data = job_array(J, 2);
+  const uint64_t* __restrict__ data = J.A;
   uint64_t* __restrict__ out = J.out;
   uint64_t* __restrict__ H = J.H;
   const uint64_t nlimbs = job_nout(J), nwin = n_windows_out(nlimbs);
   extern __shared__ uint64_t sm[];
-  uint64_t* tw = sm + spad(1u << TILE_LOG);
   const int tid = threadIdx.x;
   const int S = L - R;
   const uint64_t j0 = (uint64_t)blockIdx.x << T;
-  constexpr int TL = 8 - T;
-  const uint64_t gbase = ((uint64_t)(tid >> T) << S) + j0 + (tid & ((1u << T) - 1));
-#pragma unroll
-  for (int q = 0; q < PER_THREAD; q++)
-    cp_async8(sm + spad(q * PASS_THREADS + tid), data + gbase + ((uint64_t)(q << TL) << S));
-  if (twi) {
-    load_tw512(tw, RT);
-    cp_async_wait_all();
-    __syncthreads();
-    // inverse pass twiddles (times N^-1) from the table, laid out like the data
-    auto ptw = [&](uint32_t row0, int k, uint32_t j) {
-      return __ldg(twi + ((uint64_t)(row0 + (uint32_t)k) << S) + j0 + j);
-    };
-    tile_inv_t<R, T, 0, PASS_THREADS, rp_count(R) - 1>(sm, tw, tid, ptw);
-  } else if (L > LVL_MAX) {
-    // inverse pass twiddles w^-(f (j0 + j)) = w^-(f j0) w^-(f j): the first
-    // factor for the tile's 2^R frequencies is staged in tw, which the
-    // first inverse round does not need for round twiddles (its sub-problems
-    // are the radix itself); the round twiddles are loaded after it
-    constexpr int QL = rp_count(R) - 1;
-    static_assert(rp_mlog(R, QL) == rp_bits(R, QL), "the first inverse round has no round twiddles");
+  uint64_t* tw = sm + INV_FIRST_XWORDS<R>;
+  const bool staged = !twi && L > LVL_MAX;
+  if (staged) {
+    // w^-(f (j0 + j)) = w^-(f j0) w^-(f j), as in k_fwd_first
     for (uint32_t f = tid; f < (1u << R); f += PASS_THREADS) tw[f] = root_pow32(RT, L, f * (uint32_t)j0, true);
-    cp_async_wait_all();
     __syncthreads();
-    const uint64_t* __restrict__ nt = near_table(RT, L, true);
-    auto ptw = [&](uint32_t row0, int k, uint32_t j) {
-      const uint32_t f = row_freq_t<R>(row0) + row_freq_t<R>((uint32_t)k);
-      return gl::mul(tw[f], __ldg(nt + f * j));
-    };
-    round_inv_t<R, T, 0, rp_bits(R, QL), rp_mlog(R, QL), PASS_THREADS>(sm, tw, tid, ptw);
-    __syncthreads();
-    load_tw512(tw, RT);
-    __syncthreads();
-    tile_inv_t<R, T, 0, PASS_THREADS, QL - 1>(sm, tw, tid);
-  } else {
-    load_tw512(tw, RT);
-    cp_async_wait_all();
-    __syncthreads();
-    // inverse pass twiddles w_N^-(f*j), applied by the first inverse round
-    auto ptw = [&](uint32_t row0, int k, uint32_t j) {
-      const uint32_t f = row_freq_t<R>(row0) + row_freq_t<R>((uint32_t)k);
-      return root_pow32(RT, L, f * (uint32_t)(j0 + j), true);
-    };
-    tile_inv_t<R, T, 0, PASS_THREADS, rp_count(R) - 1>(sm, tw, tid, ptw);
   }
+#pragma unroll 1
+  for (int it = 0; it < G::ITERS2; it++) {
+    const uint32_t w = it * PASS_THREADS + tid, j = w & G::TM, k1 = w >> T;
+    const uint64_t at = ((uint64_t)(k1 << B2) << S) + j0 + j;
+    uint64_t v[1 << B2];
+    gl::Lz x[1 << B2];
+#pragma unroll
+    for (int k = 0; k < (1 << B2); k++) v[k] = data[at + ((uint64_t)k << S)];
+    if (twi) {
+#pragma unroll
+      for (int k = 0; k < (1 << B2); k++) x[k] = gl::lz_mul(v[k], __ldg(twi + at + ((uint64_t)k << S)));
+    } else if (staged) {
+      const uint64_t* __restrict__ nt = near_table(RT, L, true);
+#pragma unroll
+      for (int k = 0; k < (1 << B2); k++) {
+        const uint32_t f = k1 + (k << B1);
+        x[k] = gl::lz_mul(v[k], gl::mul(tw[f], __ldg(nt + f * j)));
+      }
+    } else {
+#pragma unroll
+      for (int k = 0; k < (1 << B2); k++)
+        x[k] = gl::lz_mul(v[k], root_pow32(RT, L, (k1 + (k << B1)) * (uint32_t)(j0 + j), true));
+    }
+    x[0] = gl::lz_bias(x[0]);
+    dft_lz<B2, true>(x, v);
+#pragma unroll
+    for (int m = 0; m < (1 << B2); m++) sm[k1 * G::KS + (m << T) + j] = v[m];
+  }
+  __syncthreads();
+  constexpr uint32_t RS = G::TM + 2;  // row stride of the coefficients
+  {
+    uint64_t v[1 << B1];
+    pass_inv2<R>(sm + tid, G::KS, RT.rt + rt_offset(R, true), tid >> T, v);
+    __syncthreads();
+#pragma unroll
+    for (int m = 0; m < (1 << B1); m++) sm[((tid >> T) + (m << B2)) * RS + (tid & G::TM)] = gl::canon(v[m]);
+  }
+  __syncthreads();
   const bool coeff = (J.flags & JF_COEFF) != 0;
   const uint64_t wtop = (1ull << L) >> 3;  // a wrapped product's windows past the transform: w + wtop
-  for (uint32_t q = tid; q < (1u << (TILE_LOG - 3)); q += PASS_THREADS) {
-    uint32_t i = q >> (T - 3), k = q & ((1u << (T - 3)) - 1);
-    uint64_t w = ((((uint64_t)i << S) + j0) >> 3) + k;
+  for (uint32_t q = tid; q < (1u << (G::TILE - 3)); q += PASS_THREADS) {
+    const uint32_t i = q >> (T - 3), k = q & ((1u << (T - 3)) - 1);
+    const uint64_t w = ((((uint64_t)i << S) + j0) >> 3) + k;
     uint64_t c[8];
-    uint32_t b = (i << T) + 8 * k;
+    const uint64_t* row = sm + i * RS + 8 * k;
 #pragma unroll
-    for (int t = 0; t < 8; t++) c[t] = gl::canon(sm[spad(b + t)]);
+    for (int t = 0; t < 8; t++) c[t] = row[t];
     if (coeff) {
 #pragma unroll
       for (int t = 0; t < 8; t++)
@@ -874,7 +853,7 @@ __device__ __forceinline__ void group_fwd_c(uint64_t* a0, uint64_t* a1, uint64_t
 template <int L, int NT, int Q = rp_count(L) - 1>
 __device__ __forceinline__ void group_inv_c(uint64_t* a0, const uint64_t* tw, int tid, bool act) {
   if constexpr (Q >= 0) {
-    if (act) round_inv_t<L, 0, 0, rp_bits(L, Q), rp_mlog(L, Q), NT, NoPassTw, 12>(a0, tw, tid, NoPassTw());
+    if (act) round_inv_t<L, 0, 0, rp_bits(L, Q), rp_mlog(L, Q), NT, 12>(a0, tw, tid);
     __syncthreads();
     group_inv_c<L, NT, Q - 1>(a0, tw, tid, act);
   }
@@ -1215,7 +1194,7 @@ __global__ void __launch_bounds__(MERGE_THREADS, 2) k_split_merge(MergeLevel M, 
 static int log2_ceil(uint64_t x) { return x <= 1 ? 0 : 64 - __builtin_clzll(x - 1); }
 
 // Host copies of the root tables: lo, hi, w12, level tables (in this order).
-constexpr size_t ROOT_WORDS = 2 * 65536 + 4096 + (2u << LVL_MAX) + (size_t)NEAR_LEVELS * 2 * 4096;
+constexpr size_t ROOT_WORDS = 2 * 65536 + 4096 + (2u << LVL_MAX) + (size_t)NEAR_LEVELS * 2 * 4096 + RT_WORDS;
 
 static void build_roots(uint64_t* t) {
   uint64_t rho = find_rho();
@@ -1249,10 +1228,22 @@ static void build_roots(uint64_t* t) {
         const uint32_t e = dir ? 0u - e0 : e0;
         nt[((size_t)(L - LVL_MAX - 1) * 2 + dir) * 4096 + xx] = hf::mul(lo[e & 0xFFFFu], hi[e >> 16]);
       }
+  // round twiddles of the passes
+  uint64_t* rt = nt + (size_t)NEAR_LEVELS * 2 * 4096;
+  for (int r = 6; r <= 9; r++) {
+    const uint64_t* w = lvl + (1u << r);
+    const uint32_t n1 = 1u << pass_b1(r), n2 = 1u << pass_b2(r), n = 1u << r;
+    for (uint32_t k = 0; k < n1; k++)
+      for (uint32_t m = 0; m < n2; m++) {
+        rt[rt_offset(r, false) + m * n1 + k] = w[k * m];
+        rt[rt_offset(r, true) + k * n2 + m] = w[(n - k * m) & (n - 1)];
+      }
+  }
 }
 
 static Roots roots_at(const uint64_t* d) {
-  return Roots{d, d + 65536, d + 2 * 65536, d + 2 * 65536 + 4096, d + 2 * 65536 + 4096 + (2u << LVL_MAX)};
+  const uint64_t* nt = d + 2 * 65536 + 4096 + (2u << LVL_MAX);
+  return Roots{d, d + 65536, d + 2 * 65536, d + 2 * 65536 + 4096, nt, nt + (size_t)NEAR_LEVELS * 2 * 4096};
 }
 
 struct DeviceState {
@@ -1268,29 +1259,10 @@ static DeviceState g_dev;
 static thread_local cudaStream_t t_stream = nullptr;
 static thread_local int t_stream_dev = -1;
 
-// Opt every pass kernel into its dynamic shared memory.
-template <int R>
-static cudaError_t set_smem_attrs_r() {
-  int bytes = (int)pass_smem_bytes(TILE_LOG);
-  cudaError_t e = cudaSuccess;
-  if (R >= 7) {
-    e = cudaFuncSetAttribute(k_fwd_first<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-    if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(k_inv_first_carry<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-  }
-  if (e == cudaSuccess) e = cudaFuncSetAttribute(k_col_mid<R, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-  if (e == cudaSuccess) e = cudaFuncSetAttribute(k_col_mid<R, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-  if (e == cudaSuccess) e = cudaFuncSetAttribute(k_fwd_last<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-  if (e == cudaSuccess) e = cudaFuncSetAttribute(k_mid<R, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-  if (e == cudaSuccess) e = cudaFuncSetAttribute(k_mid<R, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-  return e;
-}
-
+// Opt the one-CTA kernels into their dynamic shared memory (the pass kernels
+// stay below 48 KB).
 static cudaError_t set_smem_attrs() {
-  cudaError_t e = set_smem_attrs_r<6>();
-  if (e == cudaSuccess) e = set_smem_attrs_r<7>();
-  if (e == cudaSuccess) e = set_smem_attrs_r<8>();
-  if (e == cudaSuccess) e = set_smem_attrs_r<9>();
+  cudaError_t e = cudaSuccess;
   if (e == cudaSuccess)
     e = cudaFuncSetAttribute(k_small_mul, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)small_cta_smem(SMALL_LOG_MAX));
   if (e == cudaSuccess) e = cudaFuncSetAttribute(k_split_merge<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)merge_cta_smem(8));
@@ -1644,54 +1616,22 @@ static bool plan_valid(const Plan& p) {
   return true;
 }
 
-static int plan_rounds(const Plan& p) {
-  int n = 0;
-  for (int i = 0; i < p.np; i++) n += rp_count(p.r[i]);
-  return n;
-}
-
-// np passes for 2^L points: among the valid splits, the one with the fewest
-// radix-8/4 rounds (a pass of 2^6 or 2^9 is all radix-8 rounds, one of 2^7
-// or 2^8 needs radix-4 rounds: 2^21 as 9 + 6 + 6 is 7 rounds, 7 + 7 + 7 is
-// 9), the even split when it ties.  Each round costs every element its
-// round twiddles and a shared-memory round trip.
+// np passes for 2^L points: the even split, longer passes first.  Every pass
+// is two rounds whatever its radix, so only the shifts inside the rounds
+// depend on the split, and they grow faster than the radix: 2^21 as 7 + 7 + 7
+// or 9 + 6 + 6 cost the same, uneven splits never less.
 static Plan split_plan(int L, int np) {
-  Plan even{L, np, {0, 0, 0, 0, 0}};
-  for (int i = 0; i < np; i++) even.r[i] = L / np + (i < L % np ? 1 : 0);
-  Plan best = even;
-  int best_rounds = plan_valid(even) ? plan_rounds(even) : 1 << 30;
-  Plan cur{L, np, {0, 0, 0, 0, 0}};
-  // radices from 9 down, first pass 7..9, the others 6..9
-  std::function<void(int, int)> walk = [&](int i, int left) {
-    if (i == np - 1) {
-      cur.r[i] = left;
-      if (plan_valid(cur) && plan_rounds(cur) < best_rounds) {
-        best = cur;
-        best_rounds = plan_rounds(cur);
-      }
-      return;
-    }
-    for (int r = 9; r >= (i == 0 ? 7 : 6); r--) {
-      cur.r[i] = r;
-      walk(i + 1, left - r);
-    }
-  };
-  if (np >= 2 && np <= 5) walk(0, L);
-  return best;
+  Plan p{L, np, {0, 0, 0, 0, 0}};
+  for (int i = 0; i < np; i++) p.r[i] = L / np + (i < L % np ? 1 : 0);
+  return p;
 }
 
-// Splits are tabulated once for 2^0 .. 2^32 points (the entry points reject
-// longer transforms) and 2 .. 5 passes; any other request gets an invalid
-// plan (np 0, which plan_valid rejects).
+// Any request outside 2^0 .. 2^32 points (the entry points reject longer
+// transforms) and 2 .. 5 passes gets an invalid plan (np 0, which plan_valid
+// rejects).
 static Plan make_plan_np(int L, int np) {
   if (L < 0 || L > 32 || np < 2 || np > 5) return Plan{L, 0, {0, 0, 0, 0, 0}};
-  static Plan table[33][6];
-  static std::once_flag once;
-  std::call_once(once, [] {
-    for (int l = 0; l <= 32; l++)
-      for (int n = 2; n <= 5; n++) table[l][n] = split_plan(l, n);
-  });
-  return table[L][np];
+  return split_plan(L, np);
 }
 
 static Plan make_plan(int L) {
@@ -1743,13 +1683,17 @@ static void carve_scratch(Job& J, uint8_t* base, bool square) {
 }
 
 // Launch helpers (template dispatch on the pass radix).
-#define PIMUL_DISPATCH_R(r, CALL)          \
-  switch (r) {                             \
-    case 6: { constexpr int RR = 6; CALL; } break; \
-    case 7: { constexpr int RR = 7; CALL; } break; \
-    case 8: { constexpr int RR = 8; CALL; } break; \
-    default: { constexpr int RR = 9; CALL; } break; \
+#define PIMUL_DISPATCH_R(r, ...)                        \
+  switch (r) {                                          \
+    case 6: { constexpr int RR = 6; __VA_ARGS__; } break; \
+    case 7: { constexpr int RR = 7; __VA_ARGS__; } break; \
+    case 8: { constexpr int RR = 8; __VA_ARGS__; } break; \
+    default: { constexpr int RR = 9; __VA_ARGS__; } break; \
   }
+
+// Both operands of a transform up to this length (log2) go through each
+// forward pass in one launch.
+constexpr int MERGE_OPERANDS_LOG = 20;
 
 struct Launcher {
   cudaStream_t st;
@@ -1764,7 +1708,7 @@ struct Launcher {
 // multiply, one coalesced load per element, instead of being computed from
 // the root tables (a product of two table entries per element in the first
 // passes, a scattered lookup in a 2^(R+S)-entry level table in the middle
-// ones).  With f_R the digit-reversed row frequency (row_freq_t<R>):
+// ones).  With f_R the digit-reversed row frequency (pass_freq<R>):
 //   first pass of length N = 2^L, radix 2^R, S = L - R:
 //     forward  tw[i 2^S + J] = w_N^(f_R(i) J)
 //     inverse  tw[i 2^S + J] = w_N^-(f_R(i) J) N^-1   (the inverse's 1/N for free)
@@ -1782,7 +1726,7 @@ __global__ void k_tw_first(uint64_t* tw, int L, int inv, uint64_t scale, Roots R
   const uint64_t n = 1ull << L, smask = (1ull << S) - 1;
   for (uint64_t e = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; e < n; e += (uint64_t)gridDim.x * blockDim.x) {
     const uint32_t i = (uint32_t)(e >> S), J = (uint32_t)(e & smask);
-    uint64_t t = root_pow32(RT, L, row_freq_t<R>(i) * J, inv != 0);
+    uint64_t t = root_pow32(RT, L, pass_freq<R>(i) * J, inv != 0);
     if (inv) t = gl::mul(t, scale);
     tw[e] = gl::canon(t);
   }
@@ -1794,7 +1738,7 @@ __global__ void k_tw_mid(uint64_t* tw, int S, int inv, Roots RT) {
   const uint64_t n = 1ull << M, smask = (1ull << S) - 1;
   for (uint64_t e = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; e < n; e += (uint64_t)gridDim.x * blockDim.x) {
     const uint32_t r = (uint32_t)(e >> S), j = (uint32_t)(e & smask);
-    tw[e] = gl::canon(root_pow32(RT, M, row_freq_t<R>(r) * j, inv != 0));
+    tw[e] = gl::canon(root_pow32(RT, M, pass_freq<R>(r) * j, inv != 0));
   }
 }
 
@@ -1887,58 +1831,65 @@ static void tw_release_all() {
 // transform length 2^L: the products come from the device array `jobs`
 // (blockIdx.y) or, for nj == 1 and jobs == nullptr, from `one`.
 // max_chunk: largest carry-chunk count among the products.
-static void run_large(const Launcher& X, const Job* jobs, const Job& one, uint32_t nj, int L, uint64_t max_chunk,
-                      bool any_b_full = false, bool any_addend = false) {
+static void run_large(const Launcher& X, const Job* jobs, const Job& one, uint32_t nj, int L, uint64_t max_chunk) {
   const Plan pl = make_plan(L);
-  const dim3 grid((unsigned)(1ull << (L - TILE_LOG)), nj);
-  const size_t smem = pass_smem_bytes(TILE_LOG);
   const PassTables tw = X.tables ? pass_tables(pl, X.st) : PassTables{};
   // 2^-L (2^192 = 1); 0 when the inverse first pass's table applies it
   const uint64_t ninv = tw.first_inv ? 0 : hf::pow(hf::pow(2, 191), L);
   const int rl = pl.r[pl.np - 1];
-  for (int which = 0; which < 2; which++) {
+  const bool one_operand = !jobs && is_square(one);
+  // both operands' passes in one launch while their arrays fit L2 together;
+  // longer transforms one operand after the other
+  const bool merged = L <= MERGE_OPERANDS_LOG && !X.b_ready && !one_operand;
+  const unsigned nz = merged ? 2 : 1;
+  auto grid = [&](int tile, unsigned z) { return dim3((unsigned)(1ull << (L - tile)), nj, z); };
+  for (int which = 0; which < (merged || one_operand ? 1 : 2); which++) {
     if (which == 1 && X.b_ready) cudaStreamWaitEvent(X.st, X.b_ready, 0);
     {
       KTimer kt(K_PACK, X.st, X.stats);
-      PIMUL_DISPATCH_R(pl.r[0], (k_fwd_first<(RR < 7 ? 7 : RR)><<<grid, PASS_THREADS, smem, X.st>>>(jobs, one, which, L, X.R,
-                                                                                                   tw.first_fwd)));
+      PIMUL_DISPATCH_R(pl.r[0], {
+        constexpr int R = RR < 7 ? 7 : RR;
+        k_fwd_first<R><<<grid(ColGeom<R>::TILE, nz), PASS_THREADS, (ColGeom<R>::XWORDS + (1u << R)) * 8, X.st>>>(
+            jobs, one, which, L, X.R, tw.first_fwd);
+      });
     }
     int consumed = pl.r[0];
     for (int p = 1; p < pl.np - 1; p++) {
       consumed += pl.r[p];
       KTimer kt(K_PASS_FWD, X.st, X.stats);
-      PIMUL_DISPATCH_R(pl.r[p], (k_col_mid<RR, true><<<grid, PASS_THREADS, smem, X.st>>>(jobs, one, which, L - consumed, X.R,
-                                                                                        tw.mid_fwd[p])));
+      PIMUL_DISPATCH_R(pl.r[p], {
+        k_col_mid<RR, true><<<grid(ColGeom<RR>::TILE, nz), PASS_THREADS, ColGeom<RR>::XWORDS * 8, X.st>>>(
+            jobs, one, which, L - consumed, X.R, tw.mid_fwd[p]);
+      });
     }
-    if (which == 0 || any_b_full) {
-      KTimer kt(K_PASS_FWD, X.st, X.stats);
-      PIMUL_DISPATCH_R(rl, (k_fwd_last<RR><<<grid, PASS_THREADS, smem, X.st>>>(jobs, one, which, X.R)));
-    }
-  }
-  if (any_addend) {
-    KTimer kt(K_POINTWISE, X.st, X.stats);
-    const uint64_t n = 1ull << L;
-    k_pointwise_addend<<<dim3((unsigned)std::min<uint64_t>(n / 1024, 4096), nj), 256, 0, X.st>>>(jobs, one, n);
+    KTimer kt(K_PASS_FWD, X.st, X.stats);
+    PIMUL_DISPATCH_R(rl, {
+      k_fwd_last<RR><<<grid(RowGeom<RR>::TILE, nz), PASS_THREADS, 4 * RowGeom<RR>::XWORDS * 8, X.st>>>(jobs, one, which, X.R);
+    });
   }
   {
     KTimer kt(K_POINTWISE, X.st, X.stats);
-    if (any_b_full || any_addend) {
-      PIMUL_DISPATCH_R(rl, (k_mid<RR, true><<<grid, PASS_THREADS, smem, X.st>>>(jobs, one, ninv, X.R)));
-    } else {
-      PIMUL_DISPATCH_R(rl, (k_mid<RR, false><<<grid, PASS_THREADS, smem, X.st>>>(jobs, one, ninv, X.R)));
-    }
+    PIMUL_DISPATCH_R(rl, {
+      k_inv_last<RR><<<grid(RowGeom<RR>::TILE, 1), PASS_THREADS, 4 * RowGeom<RR>::XWORDS * 8, X.st>>>(jobs, one, ninv, X.R);
+    });
   }
   int consumed = L - rl;
   for (int p = pl.np - 2; p >= 1; p--) {
-    int S = L - consumed;
+    const int S = L - consumed;
     consumed -= pl.r[p];
     KTimer kt(K_PASS_INV, X.st, X.stats);
-    PIMUL_DISPATCH_R(pl.r[p], (k_col_mid<RR, false><<<grid, PASS_THREADS, smem, X.st>>>(jobs, one, 2, S, X.R, tw.mid_inv[p])));
+    PIMUL_DISPATCH_R(pl.r[p], {
+      k_col_mid<RR, false><<<grid(ColGeom<RR>::TILE, 1), PASS_THREADS, ColGeom<RR>::XWORDS * 8, X.st>>>(jobs, one, 0, S, X.R,
+                                                                                                      tw.mid_inv[p]);
+    });
   }
   {
     KTimer kt(K_PASS_INV, X.st, X.stats);
-    PIMUL_DISPATCH_R(pl.r[0], (k_inv_first_carry<(RR < 7 ? 7 : RR)><<<grid, PASS_THREADS, smem, X.st>>>(jobs, one, L, X.R,
-                                                                                                         tw.first_inv)));
+    PIMUL_DISPATCH_R(pl.r[0], {
+      constexpr int R = RR < 7 ? 7 : RR;
+      k_inv_first_carry<R><<<grid(ColGeom<R>::TILE, 1), PASS_THREADS, (INV_FIRST_XWORDS<R> + (1u << R)) * 8, X.st>>>(
+          jobs, one, L, X.R, tw.first_inv);
+    });
   }
   {
     KTimer kt(K_CARRY, X.st, X.stats);
@@ -2027,7 +1978,6 @@ struct BatchLayout {
     int L;
     size_t d0, nd;
     uint64_t max_chunk;
-    bool any_b_full, any_addend;
   };
   std::vector<Bucket> large;
   uint64_t arena_bytes = 0;
@@ -2093,7 +2043,7 @@ static int layout_batch(const Unit* units, size_t n, BatchLayout& B, bool share)
     const uint64_t N = 1ull << L;
     size_t s = 0;
     while (s < byL[L].size()) {
-      BatchLayout::Bucket bk{L, B.desc.size(), 0, 0, false, false};
+      BatchLayout::Bucket bk{L, B.desc.size(), 0, 0};
       // the group's units: descriptor count and a scratch bound (no sharing)
       uint64_t bound = 0;
       size_t e = s;
@@ -2128,7 +2078,6 @@ static int layout_batch(const Unit* units, size_t n, BatchLayout& B, bool share)
           const size_t i2 = B.desc.size() - 1;
           B.desc[i1].addend = (int64_t)i2;
           if (share) by_b[u.b2].push_back(i2);
-          bk.any_addend = true;
         }
       }
       for (auto& kv : by_b) {
@@ -2144,17 +2093,14 @@ static int layout_batch(const Unit* units, size_t n, BatchLayout& B, bool share)
           } else {
             B.desc[di].flags |= JF_B_SHARED;
             B.desc[di].owner = (int64_t)it->second;
-            B.desc[it->second].flags |= JF_B_FULL;
           }
         }
       }
-      // an addend needs b's full spectrum; scratch offsets
+      // scratch offsets
       uint64_t off = 0;
       for (size_t di = bk.d0; di < bk.d0 + bk.nd; di++) {
         BatchLayout::Desc& d = B.desc[di];
         const Unit& u = units[d.unit];
-        if ((d.flags & JF_ADDEND) && !(d.flags & JF_B_SHARED)) d.flags |= JF_B_FULL;
-        if (d.flags & JF_B_FULL) bk.any_b_full = true;
         const bool sq = !d.second && u.a == u.b && u.la == u.lb;
         d.off_a = off;
         off += round256(N * 8);
@@ -2217,7 +2163,11 @@ static void fill_descriptors(const Unit* units, const BatchLayout& B, uint8_t* a
       J.B = sq ? nullptr : reinterpret_cast<uint64_t*>(arena + d.off_b);
     J.H = d.second ? nullptr : reinterpret_cast<uint64_t*>(arena + d.off_h);
     J.aux = d.second ? nullptr : arena + d.off_aux;
-    J.X = d.addend >= 0 ? reinterpret_cast<const uint64_t*>(arena + B.desc[d.addend].off_a) : nullptr;
+    if (d.addend >= 0) {
+      const BatchLayout::Desc& x = B.desc[d.addend];
+      J.X = reinterpret_cast<const uint64_t*>(arena + x.off_a);
+      J.Y = reinterpret_cast<const uint64_t*>(arena + (x.flags & JF_B_SHARED ? B.desc[x.owner].off_b : x.off_b));
+    }
     ld[di] = J;
   }
 }
@@ -2235,7 +2185,7 @@ static void launch_batch(const Launcher& X, const BatchLayout& B, const SmallJob
                                                                       (uint32_t)B.chunks.size(), X.R);
   }
   for (const auto& bk : B.large)
-    run_large(X, d_large + bk.d0, Job{}, (uint32_t)bk.nd, bk.L, bk.max_chunk, bk.any_b_full, bk.any_addend);
+    run_large(X, d_large + bk.d0, Job{}, (uint32_t)bk.nd, bk.L, bk.max_chunk);
 }
 
 // The calling thread's buffer for a batch's host descriptor image, kept and

@@ -66,17 +66,14 @@ __device__ __forceinline__ uint64_t canon(uint64_t x) { return x >= P ? x - P : 
 __device__ __forceinline__ uint64_t neg(uint64_t a) { return sub(0, a); }
 
 // 128-bit value (x3 x2 x1 x0) -> weak 64-bit:  (x1:x0) + x2 * (2^32 - 1) - x3.
-// u = x2 * (2^32 - 1) comes from one wide multiply; the sum's net carry
-// k in {-1, 0, 1} is worth k * 2^64 = k * EPS, and adding that cannot carry
-// again (|k * EPS| is far from both ends of the 64-bit range).
+// The multiply-add of x2 (on the FMA pipe) carries at most once; the sum's
+// net carry k in {-1, 0, 1} is worth k * 2^64 = k * EPS, and adding that
+// cannot carry again (|k * EPS| is far from both ends of the 64-bit range).
 __device__ __forceinline__ uint64_t reduce_words(uint32_t r0, uint32_t r1, uint32_t r2, uint32_t r3) {
-  uint64_t u;
-  asm("mul.wide.u32 %0, %1, 0xFFFFFFFF;" : "=l"(u) : "r"(r2));
   uint32_t z0, z1;
-  asm("{\n\t.reg .u32 k, nk, hk, u0, u1;\n\t"
-      "mov.b64 {u0, u1}, %6;\n\t"
-      "add.cc.u32 %0, %2, u0;\n\t"
-      "addc.cc.u32 %1, %3, u1;\n\t"
+  asm("{\n\t.reg .u32 k, nk, hk;\n\t"
+      "mad.lo.cc.u32 %0, %4, 0xFFFFFFFF, %2;\n\t"
+      "madc.hi.cc.u32 %1, %4, 0xFFFFFFFF, %3;\n\t"
       "addc.u32 k, 0, 0;\n\t"
       "sub.cc.u32 %0, %0, %5;\n\t"
       "subc.cc.u32 %1, %1, 0;\n\t"
@@ -87,7 +84,7 @@ __device__ __forceinline__ uint64_t reduce_words(uint32_t r0, uint32_t r1, uint3
       "addc.u32 %1, %1, hk;\n\t"
       "}"
       : "=&r"(z0), "=&r"(z1)
-      : "r"(r0), "r"(r1), "r"(r2), "r"(r3), "l"(u));
+      : "r"(r0), "r"(r1), "r"(r2), "r"(r3));
   return mk64(z0, z1);
 }
 
@@ -143,7 +140,7 @@ __device__ __forceinline__ uint64_t shl(uint64_t x) {
 }
 
 // ------------------------------------------------------------ lazy values
-// Inside the radix-8 / radix-4 butterflies values are carried "lazy": a
+// Inside the butterflies values are carried "lazy": a
 // 64-bit word plus a small signed count k of 2^64 overflows,
 //   value = l + h 2^32 + k 2^64   (= l + h 2^32 + k EPS  mod p).
 // Adding or subtracting two lazy values is one 96-bit add (three carry-chain
@@ -172,29 +169,35 @@ __device__ __forceinline__ Lz lz_sub(Lz x, Lz y) {
   return z;
 }
 
-// (h:l) + w * EPS for a signed |w| < 2^31 -> weak 64-bit.  As a 96-bit
-// signed sum, (h:l) - w + w 2^32 has top word c in {-1, 0, 1}; c * EPS is
-// added back as in reduce_words.
-__device__ __forceinline__ uint64_t fold_words(uint32_t l, uint32_t h, int32_t w) {
-  uint32_t z0, z1;
-  asm("{\n\t.reg .u32 wh, c, nc, hc;\n\t"
-      "shr.s32 wh, %4, 31;\n\t"
-      "sub.cc.u32 %0, %2, %4;\n\t"
-      "subc.cc.u32 %1, %3, wh;\n\t"
-      "subc.u32 c, 0, wh;\n\t"
-      "add.cc.u32 %1, %1, %4;\n\t"
-      "addc.u32 c, c, wh;\n\t"
-      "neg.s32 nc, c;\n\t"
-      "shr.s32 hc, c, 31;\n\t"
-      "add.cc.u32 %0, %0, nc;\n\t"
-      "addc.u32 %1, %1, hc;\n\t"
-      "}"
-      : "=&r"(z0), "=&r"(z1)
-      : "r"(l), "r"(h), "r"(w));
-  return mk64(z0, z1);
+// Lazy value + 2^30 p.  A DFT adds what is added to its first input to every
+// output (and never shifts that input), so one biased input makes all outputs'
+// overflow counts non-negative (|k| < 2^29 before), which is what fold() takes.
+__device__ __forceinline__ Lz lz_bias(Lz x) {
+  Lz z;
+  asm("add.cc.u32 %0, %3, 0x40000000;\n\taddc.cc.u32 %1, %4, 0xC0000000;\n\taddc.u32 %2, %5, 0x3FFFFFFF;"
+      : "=r"(z.l), "=r"(z.h), "=r"(z.k)
+      : "r"(x.l), "r"(x.h), "r"(x.k));
+  return z;
 }
 
-__device__ __forceinline__ uint64_t fold(Lz x) { return fold_words(x.l, x.h, x.k); }
+// Lazy value with a non-negative overflow count -> weak 64-bit word:
+// (h:l) + k EPS is one multiply-add on the FMA pipe; it carries at most once
+// (c), and the c EPS = c 2^32 - c which that is worth cannot carry again (the
+// wrapped sum is below k EPS <= (2^32 - 1)^2).
+__device__ __forceinline__ uint64_t fold(Lz x) {
+  uint32_t z0, z1;
+  asm("{\n\t.reg .u32 c;\n\t"
+      "mad.lo.cc.u32 %0, %4, 0xFFFFFFFF, %2;\n\t"
+      "madc.hi.cc.u32 %1, %4, 0xFFFFFFFF, %3;\n\t"
+      "addc.u32 c, 0, 0;\n\t"
+      "sub.cc.u32 %0, %0, c;\n\t"
+      "subc.u32 %1, %1, 0;\n\t"
+      "add.u32 %1, %1, c;\n\t"
+      "}"
+      : "=&r"(z0), "=&r"(z1)
+      : "r"(x.l), "r"(x.h), "r"((uint32_t)x.k));
+  return mk64(z0, z1);
+}
 
 // a * b as a lazy value with k in {-1, 0}: with u = x2 EPS + (EPS - x3)
 // (which cannot overflow 64 bits), a b = (x1:x0) + u - EPS and -EPS = -2^64.
@@ -210,60 +213,80 @@ __device__ __forceinline__ Lz lz_mul(uint64_t a, uint64_t b) {
   return z;
 }
 
-// Shifts that leave their result lazy (no fold), for the radix-8 / radix-4
-// butterflies.  Derivations, with x = l + h 2^32 + k 2^64:
-//  * x 2^24 = (l << 24) + funnel(l, h, 24) 2^32 + ((h >> 8) + k 2^24) 2^64: the
-//    overflow count grows to |k| < 2^28 (|x.k| < 2^6 in), which lz_add,
-//    lz_sub and fold accept but another shift does not;
-//  * x 2^48 = w1 2^32 + w2 2^64 + w3 2^96 with w1 = l << 16, w2 = funnel(l, h, 16),
-//    w3 = (h >> 16) + k 2^16; with 2^64 = 2^32 - 1 and 2^96 = -1 this is
-//    w2 EPS + w1 2^32 - w3, a 96-bit value with k in {-1 .. 2} (|x.k| < 2^15 in);
-//  * x 2^72 = y 2^64 for y = x 2^8 = y0 + y1 2^32 + y2 2^64 (y0 = l << 8,
-//    y1 = funnel(l, h, 8), y2 = (h >> 24) + k 2^8); with 2^128 = -2^32 this is
-//    y0 EPS - y1 - y2 2^32, k in {-1 .. 1} (|x.k| < 2^23 in).
+// Shifts that leave their result lazy (no fold), for the butterflies: x 2^S
+// for a compile-time 0 < S < 96, S = 32 Q + r.  The 96-bit shift by r gives
+// words v0, v1 and a signed top v2 = funnel(h, k, r) (|k| 2^r < 2^31; r > 28
+// takes one more word), in all (v0 + v1 2^32 + v2 2^64) 2^(32 Q).  With
+// 2^64 = EPS = 2^32 - 1, 2^96 = -1 and 2^128 = -2^32:
+//  * Q = 0: (v1:v0) + v2 2^32 - v2, k in {-1 .. 1};
+//  * Q = 1: v0 2^32 + v1 EPS - v2.  u = v1 EPS + (EPS - v2), v2 taken unsigned,
+//    fits 64 bits; -EPS = -2^64, and a negative v2 counts 2^32 too much, which
+//    enters as a carry (the sign bit of k): k in {-1, 0};
+//  * Q = 2: v0 EPS - v1 - v2 2^32 = u - v2 2^32 - 2^64 for u = v0 EPS + (EPS - v1),
+//    k in {-2 .. 0}.
+template <int S>
+__device__ __forceinline__ Lz lz_shl(Lz x) {
+  static_assert(S > 0 && S < 96, "shift out of range");
+  constexpr int Q = S / 32, r = S % 32;
+  uint32_t v0 = x.l, v1 = x.h, v2 = (uint32_t)x.k;
+  if constexpr (r > 0) {
+    v0 = x.l << r;
+    v1 = __funnelshift_l(x.l, x.h, r);
+    v2 = __funnelshift_l(x.h, (uint32_t)x.k, r);
+  }
+  Lz z;
+  if constexpr (Q == 0 && r > 28) {
+    // v2 unsigned and a fourth word v3 = k >> (32 - r): v3 2^96 = -v3
+    const int32_t v3 = x.k >> (32 - r);
+    asm("{\n\t.reg .u32 c;\n\t"
+        "mad.lo.cc.u32 %0, %5, 0xFFFFFFFF, %3;\n\t"
+        "madc.hi.cc.u32 %1, %5, 0xFFFFFFFF, %4;\n\t"
+        "addc.u32 c, 0, 0;\n\t"
+        "sub.cc.u32 %0, %0, %6;\n\t"
+        "subc.cc.u32 %1, %1, %7;\n\t"
+        "subc.u32 %2, c, %7;\n\t"
+        "}"
+        : "=&r"(z.l), "=&r"(z.h), "=&r"(z.k)
+        : "r"(v0), "r"(v1), "r"(v2), "r"(v3), "r"(v3 >> 31));
+  } else if constexpr (Q == 0) {
+    asm("{\n\t.reg .u32 c;\n\t"
+        "sub.cc.u32 %0, %3, %5;\n\t"
+        "subc.cc.u32 %1, %4, %6;\n\t"
+        "subc.u32 c, 0, %6;\n\t"
+        "add.cc.u32 %1, %1, %5;\n\t"
+        "addc.u32 %2, c, %6;\n\t"
+        "}"
+        : "=&r"(z.l), "=&r"(z.h), "=&r"(z.k)
+        : "r"(v0), "r"(v1), "r"(v2), "r"((int32_t)v2 >> 31));
+  } else if constexpr (Q == 1) {
+    uint64_t u;
+    asm("mad.wide.u32 %0, %1, 0xFFFFFFFF, %2;" : "=l"(u) : "r"(v1), "l"((uint64_t)(~v2)));
+    z.l = lo32(u);
+    asm("{\n\t.reg .u32 t;\n\t"
+        "add.cc.u32 t, %4, %4;\n\t"
+        "addc.cc.u32 %0, %2, %3;\n\t"
+        "addc.u32 %1, 0xFFFFFFFF, 0;\n\t"
+        "}"
+        : "=&r"(z.h), "=r"(z.k)
+        : "r"(hi32(u)), "r"(v0), "r"(x.k));
+  } else {
+    uint64_t u;
+    asm("mad.wide.u32 %0, %1, 0xFFFFFFFF, %2;" : "=l"(u) : "r"(v0), "l"((uint64_t)(~v1)));
+    z.l = lo32(u);
+    asm("sub.cc.u32 %0, %2, %3;\n\tsubc.u32 %1, 0xFFFFFFFF, %4;"
+        : "=r"(z.h), "=r"(z.k)
+        : "r"(hi32(u)), "r"(v2), "r"(x.k >> 31));
+  }
+  return z;
+}
+
+// x 2^24 with the shifted-out word left as the overflow count (|k| < 2^28 for
+// |x.k| < 2^4), which lz_add, lz_sub and fold accept but another shift does not.
 __device__ __forceinline__ Lz lz_shl24_wide(Lz x) {
   Lz z;
   z.l = x.l << 24;
   z.h = __funnelshift_l(x.l, x.h, 24);
-  z.k = (int32_t)(x.h >> 8) + (int32_t)((uint32_t)x.k << 24);
-  return z;
-}
-
-__device__ __forceinline__ Lz lz_shl48_n(Lz x) {
-  const uint32_t w1 = x.l << 16, w2 = __funnelshift_l(x.l, x.h, 16);
-  const int32_t w3 = (int32_t)(x.h >> 16) + (int32_t)((uint32_t)x.k << 16);
-  uint64_t u;
-  asm("mul.wide.u32 %0, %1, 0xFFFFFFFF;" : "=l"(u) : "r"(w2));
-  Lz z;
-  asm("{\n\t.reg .u32 sh, u0, u1;\n\t"
-      "mov.b64 {u0, u1}, %5;\n\t"
-      "shr.s32 sh, %4, 31;\n\t"
-      "sub.cc.u32 %0, u0, %4;\n\t"
-      "subc.cc.u32 %1, u1, sh;\n\t"
-      "subc.u32 %2, 0, sh;\n\t"
-      "add.cc.u32 %1, %1, %3;\n\t"
-      "addc.u32 %2, %2, 0;\n\t"
-      "}"
-      : "=&r"(z.l), "=&r"(z.h), "=&r"(z.k)
-      : "r"(w1), "r"(w3), "l"(u));
-  return z;
-}
-
-__device__ __forceinline__ Lz lz_shl72_n(Lz x) {
-  const uint32_t y0 = x.l << 8, y1 = __funnelshift_l(x.l, x.h, 8);
-  const int32_t y2 = (int32_t)(x.h >> 24) + (int32_t)((uint32_t)x.k << 8);
-  uint64_t u;
-  asm("mul.wide.u32 %0, %1, 0xFFFFFFFF;" : "=l"(u) : "r"(y0));
-  Lz z;
-  asm("{\n\t.reg .u32 sh, u0, u1;\n\t"
-      "mov.b64 {u0, u1}, %5;\n\t"
-      "shr.s32 sh, %4, 31;\n\t"
-      "sub.cc.u32 %0, u0, %3;\n\t"
-      "subc.cc.u32 %1, u1, %4;\n\t"
-      "subc.u32 %2, 0, sh;\n\t"
-      "}"
-      : "=&r"(z.l), "=&r"(z.h), "=&r"(z.k)
-      : "r"(y1), "r"(y2), "l"(u));
+  z.k = (int32_t)__funnelshift_l(x.h, (uint32_t)x.k, 24);
   return z;
 }
 

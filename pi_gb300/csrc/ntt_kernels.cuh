@@ -13,10 +13,11 @@
 // (crates/bignum/src/ntt.rs:905-1105) without the transposes: strided tiles
 // are read as coalesced 64-byte (or wider) row segments.
 //
-// Inside a pass the R_p-point DFT runs in shared memory as rounds of radix
-// 8 (or 4 / 2) held in registers.  2 is a 192nd root of unity mod p, and the
-// root tables are built so that the 8th root of unity is 2^24: the
-// butterflies' internal twiddles are constant shifts.
+// Inside a pass the R_p-point DFT runs as two rounds of radix 8, 16 or 32
+// held in registers (rounds of radix 8, 4 or 2 in shared memory in the
+// one-CTA kernels).  2 is a 192nd root of unity mod p, and the root tables
+// are built so that the 64th root of unity is 2^3: the butterflies' internal
+// twiddles are constant shifts.
 #pragma once
 #include <cstdint>
 #include <type_traits>
@@ -33,6 +34,7 @@ struct Roots {
   const uint64_t* w12;  // w_4096^t = rho^(t * 2^20), t in [0, 4096)
   const uint64_t* lvl;  // per-level tables: w_(2^k)^x at lvl[2^k + x], 1 <= k <= LVL_MAX
   const uint64_t* near; // w_(2^L)^(+-x) for x < 4096, LVL_MAX < L <= 32 (see near_table)
+  const uint64_t* rt;   // round twiddles of the two-round passes (see rt_offset)
 };
 
 constexpr int LVL_MAX = 20;
@@ -91,20 +93,6 @@ __host__ __device__ __forceinline__ constexpr uint32_t spad_step(uint32_t m, int
   return (m << s) + ((m << s) >> 4);
 }
 
-// Asynchronous 8-byte global -> shared copy (no register round trip), and
-// the wait for all of this thread's outstanding copies.
-__device__ __forceinline__ void cp_async8(uint64_t* smem_dst, const uint64_t* gsrc) {
-  const uint32_t s = (uint32_t)__cvta_generic_to_shared(smem_dst);
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(s), "l"(gsrc) : "memory");
-}
-__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
-
-// Bulk prefetch of [src, src + bytes) into L2 (no completion to wait for);
-// src 16-byte aligned, bytes a multiple of 16.
-__device__ __forceinline__ void prefetch_l2_bulk(const void* src, uint32_t bytes) {
-  asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(src), "r"(bytes) : "memory");
-}
-
 // DIF radix-2 butterfly with a constant shift twiddle 2^S (S = 0: none).
 template <int S>
 __device__ __forceinline__ void bfly_dif(uint64_t& a, uint64_t& b) {
@@ -113,27 +101,13 @@ __device__ __forceinline__ void bfly_dif(uint64_t& a, uint64_t& b) {
   b = gl::shl<S>(gl::sub(u, w));
 }
 
-// Forward DFT of 2^B values in registers: v[k] <- sum_m v[m] w^(m k), with
-// w = 2^(192 / 2^B) (the 8th root of unity is 2^24).  Natural-order output.
-// Radix 4 and 8 run on lazy values (see gl.cuh) and fold once per output;
-// the internal twiddles are the lazy shifts of gl.cuh.  Inputs are lazy
-// with |k| <= 1 (e.g. products from lz_mul).
-template <int B>
-__device__ __forceinline__ void dft_fwd_lz(const gl::Lz* x, uint64_t* v) {
+// 8-point DFT (INV: unscaled inverse) of lazy values, folded outputs at
+// v[STEP k]; x[0] carries the bias of lz_bias.  w^-s = -w^(96 - s) turns the
+// inverse's twiddles into shifts with the signs swapped.
+template <bool INV, int STEP>
+__device__ __forceinline__ void dft8_lz(const gl::Lz* x, uint64_t* v) {
   using namespace gl;
-  if constexpr (B == 1) {
-    v[0] = fold(lz_add(x[0], x[1]));
-    v[1] = fold(lz_sub(x[0], x[1]));
-  } else if constexpr (B == 2) {
-    Lz a0 = lz_add(x[0], x[2]), c = lz_sub(x[0], x[2]);
-    Lz a1 = lz_add(x[1], x[3]);
-    Lz d = lz_shl48_n(lz_sub(x[1], x[3]));
-    v[0] = fold(lz_add(a0, a1));
-    v[1] = fold(lz_add(c, d));
-    v[2] = fold(lz_sub(a0, a1));
-    v[3] = fold(lz_sub(c, d));
-  } else {
-    static_assert(B == 3, "radix 2, 4 or 8");
+  if constexpr (!INV) {
     // stage 1: x_m +- x_(m+4); the differences d_m carry the twiddle w^m
     Lz a0 = lz_add(x[0], x[4]), d0 = lz_sub(x[0], x[4]);
     Lz a1 = lz_add(x[1], x[5]), d1 = lz_sub(x[1], x[5]);
@@ -141,45 +115,116 @@ __device__ __forceinline__ void dft_fwd_lz(const gl::Lz* x, uint64_t* v) {
     Lz a3 = lz_add(x[3], x[7]), d3 = lz_sub(x[3], x[7]);
     // even outputs: radix 4 on the sums
     Lz c0 = lz_add(a0, a2), c2 = lz_sub(a0, a2);
-    Lz c1 = lz_add(a1, a3), c3 = lz_shl48_n(lz_sub(a1, a3));
+    Lz c1 = lz_add(a1, a3), c3 = lz_shl<48>(lz_sub(a1, a3));
     v[0] = fold(lz_add(c0, c1));
-    v[4] = fold(lz_sub(c0, c1));
-    v[2] = fold(lz_add(c2, c3));
-    v[6] = fold(lz_sub(c2, c3));
+    v[4 * STEP] = fold(lz_sub(c0, c1));
+    v[2 * STEP] = fold(lz_add(c2, c3));
+    v[6 * STEP] = fold(lz_sub(c2, c3));
     // odd outputs: radix 4 on b_m = w^m d_m.  With g = w^2 d3,
     // b1 + b3 = w (d1 + g) and (b1 - b3) w^2 = w^3 (d1 - g), so every shift
     // acts on a value with a small overflow count and the one by w (24 bits)
     // can stay lazy
-    Lz b2 = lz_shl48_n(d2);
+    Lz b2 = lz_shl<48>(d2);
     Lz e0 = lz_add(d0, b2), e2 = lz_sub(d0, b2);
-    Lz g = lz_shl48_n(d3);
-    Lz e1 = lz_shl24_wide(lz_add(d1, g)), e3 = lz_shl72_n(lz_sub(d1, g));
-    v[1] = fold(lz_add(e0, e1));
-    v[5] = fold(lz_sub(e0, e1));
-    v[3] = fold(lz_add(e2, e3));
-    v[7] = fold(lz_sub(e2, e3));
+    Lz g = lz_shl<48>(d3);
+    Lz e1 = lz_shl24_wide(lz_add(d1, g)), e3 = lz_shl<72>(lz_sub(d1, g));
+    v[1 * STEP] = fold(lz_add(e0, e1));
+    v[5 * STEP] = fold(lz_sub(e0, e1));
+    v[3 * STEP] = fold(lz_add(e2, e3));
+    v[7 * STEP] = fold(lz_sub(e2, e3));
+  } else {
+    // radix 2 on the bit-reversed inputs (x0, x4, x2, x6, x1, x5, x3, x7)
+    Lz s01 = lz_add(x[0], x[4]), d01 = lz_sub(x[0], x[4]);
+    Lz s23 = lz_add(x[2], x[6]), d23 = lz_sub(x[2], x[6]);
+    Lz s45 = lz_add(x[1], x[5]), d45 = lz_sub(x[1], x[5]);
+    Lz s67 = lz_add(x[3], x[7]), d67 = lz_sub(x[3], x[7]);
+    Lz t23 = lz_shl<48>(d23), t67 = lz_shl<48>(d67);
+    Lz v0 = lz_add(s01, s23), v2 = lz_sub(s01, s23);
+    Lz v1 = lz_sub(d01, t23), v3 = lz_add(d01, t23);
+    Lz v4 = lz_add(s45, s67), v6 = lz_sub(s45, s67);
+    Lz v5 = lz_sub(d45, t67), v7 = lz_add(d45, t67);
+    Lz t5 = lz_shl<72>(v5), t6 = lz_shl<48>(v6), t7 = lz_shl24_wide(v7);
+    v[0] = fold(lz_add(v0, v4));
+    v[4 * STEP] = fold(lz_sub(v0, v4));
+    v[1 * STEP] = fold(lz_sub(v1, t5));
+    v[5 * STEP] = fold(lz_add(v1, t5));
+    v[2 * STEP] = fold(lz_sub(v2, t6));
+    v[6 * STEP] = fold(lz_add(v2, t6));
+    v[3 * STEP] = fold(lz_sub(v3, t7));
+    v[7 * STEP] = fold(lz_add(v3, t7));
   }
 }
 
-// dft_fwd_lz<3> for inputs whose upper half x[4..7] is zero: stage 1 is
-// then a_m = d_m = x_m.  A lazy sum or difference with zero leaves the lazy
-// value unchanged, so the outputs are those of dft_fwd_lz<3> bit for bit.
-__device__ __forceinline__ void dft_fwd_lz_half8(const gl::Lz* x, uint64_t* v) {
+// First stage of a 2^B-point decimation in frequency, elements M ..: x_M +
+// x_(M+H) and (x_M - x_(M+H)) w^M, w = 2^(192 / 2^B) (INV: (x_(M+H) - x_M)
+// 2^(96 - s) for w^-M = 2^-s = -2^(96-s)).  UPPER0: x_(M+H) is zero.
+template <int B, bool INV, bool UPPER0 = false, int M = 1>
+__device__ __forceinline__ void dif_stage(gl::Lz* x) {
   using namespace gl;
-  Lz c0 = lz_add(x[0], x[2]), c2 = lz_sub(x[0], x[2]);
-  Lz c1 = lz_add(x[1], x[3]), c3 = lz_shl48_n(lz_sub(x[1], x[3]));
-  v[0] = fold(lz_add(c0, c1));
-  v[4] = fold(lz_sub(c0, c1));
-  v[2] = fold(lz_add(c2, c3));
-  v[6] = fold(lz_sub(c2, c3));
-  Lz b2 = lz_shl48_n(x[2]);
-  Lz e0 = lz_add(x[0], b2), e2 = lz_sub(x[0], b2);
-  Lz g = lz_shl48_n(x[3]);
-  Lz e1 = lz_shl24_wide(lz_add(x[1], g)), e3 = lz_shl72_n(lz_sub(x[1], g));
-  v[1] = fold(lz_add(e0, e1));
-  v[5] = fold(lz_sub(e0, e1));
-  v[3] = fold(lz_add(e2, e3));
-  v[7] = fold(lz_sub(e2, e3));
+  constexpr int H = 1 << (B - 1), W = 192 >> B;
+  if constexpr (M < H) {
+    if constexpr (UPPER0) {
+      static_assert(!INV, "zero upper halves only come in forward");
+      x[M + H] = lz_shl<W * M>(x[M]);
+    } else {
+      const Lz a = lz_add(x[M], x[M + H]);
+      if constexpr (!INV)
+        x[M + H] = lz_shl<W * M>(lz_sub(x[M], x[M + H]));
+      else
+        x[M + H] = lz_shl<96 - W * M>(lz_sub(x[M + H], x[M]));
+      x[M] = a;
+    }
+    dif_stage<B, INV, UPPER0, M + 1>(x);
+  }
+}
+
+// DFT of 2^B lazy values (B = 3, 4, 5; INV: its unscaled inverse) with w =
+// 2^(192 / 2^B), the 2^B-th root of unity: all internal twiddles are constant
+// shifts.  Natural-order folded outputs at v[STEP k].  x[0] carries the bias
+// of lz_bias; |k| <= 1 in the other inputs (e.g. products from lz_mul); x is
+// overwritten.  UPPER0 (forward): inputs 2^(B-1) .. are zero (not read).
+template <int B, bool INV, bool UPPER0 = false, int STEP = 1>
+__device__ __forceinline__ void dft_lz(gl::Lz* x, uint64_t* v) {
+  if constexpr (B == 3) {
+    static_assert(!UPPER0, "a zero upper half needs 16 points or more");
+    dft8_lz<INV, STEP>(x, v);
+  } else {
+    constexpr int H = 1 << (B - 1);
+    if constexpr (UPPER0) {
+      x[H] = x[0];
+    } else {
+      const gl::Lz a = gl::lz_add(x[0], x[H]);
+      x[H] = gl::lz_sub(x[0], x[H]);
+      x[0] = a;
+    }
+    dif_stage<B, INV, UPPER0>(x);
+    dft_lz<B - 1, INV, false, 2 * STEP>(x, v);
+    dft_lz<B - 1, INV, false, 2 * STEP>(x + H, v + STEP);
+  }
+}
+
+// Forward DFT of 2^B values in registers (radix 2, 4, 8), for the rounds of
+// the one-CTA kernels: lazy inputs with |k| <= 1, folded outputs.
+template <int B>
+__device__ __forceinline__ void dft_fwd_lz(const gl::Lz* x, uint64_t* v) {
+  using namespace gl;
+  const Lz x0 = lz_bias(x[0]);
+  if constexpr (B == 1) {
+    v[0] = fold(lz_add(x0, x[1]));
+    v[1] = fold(lz_sub(x0, x[1]));
+  } else if constexpr (B == 2) {
+    Lz a0 = lz_add(x0, x[2]), c = lz_sub(x0, x[2]);
+    Lz a1 = lz_add(x[1], x[3]);
+    Lz d = lz_shl<48>(lz_sub(x[1], x[3]));
+    v[0] = fold(lz_add(a0, a1));
+    v[1] = fold(lz_add(c, d));
+    v[2] = fold(lz_sub(a0, a1));
+    v[3] = fold(lz_sub(c, d));
+  } else {
+    static_assert(B == 3, "radix 2, 4 or 8");
+    const Lz y[8] = {x0, x[1], x[2], x[3], x[4], x[5], x[6], x[7]};
+    dft8_lz<false, 1>(y, v);
+  }
 }
 
 template <int B>
@@ -196,52 +241,27 @@ __device__ __forceinline__ void dft_fwd(uint64_t* v) {
 
 // Unscaled inverse of dft_fwd on lazy inputs (|k| <= 1, e.g. twiddle
 // products from lz_mul): v[m] <- sum_k x[k] w^(-m k)  (= 2^B * original).
-// w^-s = -w^(96 - s): the DIT butterfly u +- w^-s b becomes u -+ 2^(96-s) b.
 template <int B>
 __device__ __forceinline__ void dft_inv_lz(const gl::Lz* x, uint64_t* v) {
   using namespace gl;
+  const Lz x0 = lz_bias(x[0]);
   if constexpr (B == 1) {
-    v[0] = fold(lz_add(x[0], x[1]));
-    v[1] = fold(lz_sub(x[0], x[1]));
+    v[0] = fold(lz_add(x0, x[1]));
+    v[1] = fold(lz_sub(x0, x[1]));
   } else if constexpr (B == 2) {
     // inputs in bit-reversed order (x0, x2, x1, x3)
-    Lz s = lz_add(x[0], x[2]), d = lz_sub(x[0], x[2]);
+    Lz s = lz_add(x0, x[2]), d = lz_sub(x0, x[2]);
     Lz t = lz_add(x[1], x[3]);
-    Lz e = lz_shl48_n(lz_sub(x[1], x[3]));
+    Lz e = lz_shl<48>(lz_sub(x[1], x[3]));
     v[0] = fold(lz_add(s, t));
     v[2] = fold(lz_sub(s, t));
     v[1] = fold(lz_sub(d, e));
     v[3] = fold(lz_add(d, e));
   } else {
     static_assert(B == 3, "radix 2, 4 or 8");
-    // inputs in bit-reversed order (x0, x4, x2, x6, x1, x5, x3, x7)
-    Lz s01 = lz_add(x[0], x[4]), d01 = lz_sub(x[0], x[4]);
-    Lz s23 = lz_add(x[2], x[6]), d23 = lz_sub(x[2], x[6]);
-    Lz s45 = lz_add(x[1], x[5]), d45 = lz_sub(x[1], x[5]);
-    Lz s67 = lz_add(x[3], x[7]), d67 = lz_sub(x[3], x[7]);
-    Lz t23 = lz_shl48_n(d23), t67 = lz_shl48_n(d67);
-    Lz v0 = lz_add(s01, s23), v2 = lz_sub(s01, s23);
-    Lz v1 = lz_sub(d01, t23), v3 = lz_add(d01, t23);
-    Lz v4 = lz_add(s45, s67), v6 = lz_sub(s45, s67);
-    Lz v5 = lz_sub(d45, t67), v7 = lz_add(d45, t67);
-    Lz t5 = lz_shl72_n(v5), t6 = lz_shl48_n(v6), t7 = lz_shl24_wide(v7);
-    v[0] = fold(lz_add(v0, v4));
-    v[4] = fold(lz_sub(v0, v4));
-    v[1] = fold(lz_sub(v1, t5));
-    v[5] = fold(lz_add(v1, t5));
-    v[2] = fold(lz_sub(v2, t6));
-    v[6] = fold(lz_add(v2, t6));
-    v[3] = fold(lz_sub(v3, t7));
-    v[7] = fold(lz_add(v3, t7));
+    const Lz y[8] = {x0, x[1], x[2], x[3], x[4], x[5], x[6], x[7]};
+    dft8_lz<true, 1>(y, v);
   }
-}
-
-template <int B>
-__device__ __forceinline__ void dft_inv(uint64_t* v) {
-  gl::Lz x[1 << B];
-#pragma unroll
-  for (int k = 0; k < (1 << B); k++) x[k] = gl::lz(v[k]);
-  dft_inv_lz<B>(x, v);
 }
 
 // ---------------------------------------------------------------- rounds
@@ -285,14 +305,9 @@ __host__ __device__ constexpr int rp_mlog(int r, int q) {
 // no swap).
 template <int R, int T, int BC, int MLOG>
 __host__ __device__ constexpr int round_swaps() {
-  return (T == 3 && BC == 0 && R == 9 && MLOG == 3)   ? (3 | 4 << 4)
-         : (T == 0 && R == 9 && MLOG == 6)             ? (3 | 4 << 4)
-         : (T == 3 && (R == 8 || R == 7) && MLOG == 2) ? (3 | 5 << 4)
-         : (T == 3 && R == 6 && MLOG == 3)             ? (3 | 4 << 4)
-         : (T == 0 && R == 6 && MLOG == 6)             ? (3 | 4 << 4)
-         : (T == 0 && R == 7 && MLOG == 4)             ? (0 | 4 << 4 | 1 << 8 | 5 << 12)
-         : (T == 0 && R == 8 && MLOG == 5)             ? (0 | 1 << 4 | 1 << 8 | 4 << 12)
-                                                       : 0;
+  return (T == 0 && R == 9 && MLOG == 6)   ? (3 | 4 << 4)
+         : (T == 0 && R == 8 && MLOG == 5) ? (0 | 1 << 4 | 1 << 8 | 4 << 12)
+                                           : 0;
 }
 
 template <int A, int B>
@@ -312,22 +327,18 @@ __device__ __forceinline__ uint32_t round_item(uint32_t w) {
 
 // Tile of 2^BC blocks x 2^R rows x 2^T columns in shared memory; element
 // (row, col) of the flattened (BC+R)-bit row index at spad(row << T | col).
-// One forward round of radix 2^B over sub-problems of 2^MLOG rows.
 // One forward round of radix 2^B over sub-problems of 2^MLOG rows.  The
 // twiddles of the previous round (radix 2^PB over 2^PMLOG rows, PB = 0: none)
 // are applied here, to the inputs, as lazy products that feed the DFT
 // directly: element row r had position jp' = r mod 2^MLOG and output index
 // k' = (r >> MLOG) mod 2^PB there, twiddle w_(2^PMLOG)^(k' jp').
-// tw512 holds the 2^TWLOG roots w^t of one fixed length (512 in the pass
-// kernels, 4096 in the one-CTA merge of whole transforms).  HALF: the first
-// radix-8 round of a tile whose rows 2^(R-1) .. 2^R - 1 are zero (they are
-// not read; every row is written).
-template <int R, int T, int BC, int B, int MLOG, int NT, int PB, int PMLOG, int TWLOG = 9, bool HALF = false>
-__device__ __forceinline__ void round_fwd_t(uint64_t* sm, const uint64_t* tw512, int tid) {
+// tw holds the 2^TWLOG roots w^t of one fixed length (4096 in the one-CTA
+// merge of whole transforms).
+template <int R, int T, int BC, int B, int MLOG, int NT, int PB, int PMLOG, int TWLOG>
+__device__ __forceinline__ void round_fwd_t(uint64_t* sm, const uint64_t* tw, int tid) {
   constexpr int SLOG = MLOG - B;
   constexpr int ITEMS = 1 << (BC + R + T - B);
   static_assert(ITEMS % NT == 0, "tile must split evenly over the threads");
-  static_assert(!HALF || (B == 3 && PB == 0 && MLOG == R && BC == 0), "HALF: the first radix-8 round of one block");
 #pragma unroll 2
   for (int it = 0; it < ITEMS / NT; it++) {
     const uint32_t w = round_item<round_swaps<R, T, BC, MLOG>()>(it * NT + tid);
@@ -338,14 +349,6 @@ __device__ __forceinline__ void round_fwd_t(uint64_t* sm, const uint64_t* tw512,
     const uint32_t sb = spad((row0 << T) | j);  // bits [SLOG+T, MLOG+T) are zero
     uint64_t v[1 << B];
     gl::Lz x[1 << B];
-    if constexpr (HALF) {
-#pragma unroll
-      for (int m = 0; m < 4; m++) x[m] = gl::lz(sm[sb + spad_step(m, SLOG + T)]);
-      dft_fwd_lz_half8(x, v);
-#pragma unroll
-      for (int k = 0; k < 8; k++) sm[sb + spad_step(k, SLOG + T)] = v[k];
-      continue;
-    }
 #pragma unroll
     for (int m = 0; m < (1 << B); m++) v[m] = sm[sb + spad_step(m, SLOG + T)];
     if constexpr (PB > 0) {
@@ -353,7 +356,7 @@ __device__ __forceinline__ void round_fwd_t(uint64_t* sm, const uint64_t* tw512,
       const uint32_t kp = (rest >> SLOG) & ((1u << PB) - 1);
       const uint32_t base = (kp * jp) << (TWLOG - PMLOG), step = (kp << SLOG) << (TWLOG - PMLOG);
 #pragma unroll
-      for (int m = 0; m < (1 << B); m++) x[m] = gl::lz_mul(v[m], tw512[base + m * step]);
+      for (int m = 0; m < (1 << B); m++) x[m] = gl::lz_mul(v[m], tw[base + m * step]);
     } else {
 #pragma unroll
       for (int m = 0; m < (1 << B); m++) x[m] = gl::lz(v[m]);
@@ -364,18 +367,11 @@ __device__ __forceinline__ void round_fwd_t(uint64_t* sm, const uint64_t* tw512,
   }
 }
 
-// Pass twiddle applied by the first inverse round: none.
-struct NoPassTw {};
-
-// One inverse round; the first one executed (SLOG = 0, no round twiddles)
-// multiplies its inputs by the pass twiddles of the tile when a functor is
-// given (ptw(row0, k, col) for tile row row0 + k, row0 a multiple of 2^B),
-// feeding the lazy products straight into the DFT.
-template <int R, int T, int BC, int B, int MLOG, int NT, class F, int TWLOG = 9>
-__device__ __forceinline__ void round_inv_t(uint64_t* sm, const uint64_t* tw512, int tid, const F& ptw) {
+// One inverse round; the first one executed (SLOG = 0) has no twiddles.
+template <int R, int T, int BC, int B, int MLOG, int NT, int TWLOG>
+__device__ __forceinline__ void round_inv_t(uint64_t* sm, const uint64_t* tw, int tid) {
   constexpr int SLOG = MLOG - B;
   constexpr int ITEMS = 1 << (BC + R + T - B);
-  constexpr bool PTW = !std::is_same<F, NoPassTw>::value;
   static_assert(ITEMS % NT == 0, "tile must split evenly over the threads");
 #pragma unroll 2
   for (int it = 0; it < ITEMS / NT; it++) {
@@ -389,20 +385,14 @@ __device__ __forceinline__ void round_inv_t(uint64_t* sm, const uint64_t* tw512,
     gl::Lz x[1 << B];
 #pragma unroll
     for (int k = 0; k < (1 << B); k++) v[k] = sm[sb + spad_step(k, SLOG + T)];
-    if constexpr (SLOG == 0 && PTW) {
-      // rows row0 + k, row0 a multiple of 2^B
+    x[0] = gl::lz(v[0]);
+    const uint32_t jps = jp << (TWLOG - MLOG);
 #pragma unroll
-      for (int k = 0; k < (1 << B); k++) x[k] = gl::lz_mul(v[k], ptw(row0, k, j));
-    } else {
-      x[0] = gl::lz(v[0]);
-      const uint32_t jps = jp << (TWLOG - MLOG);
-#pragma unroll
-      for (int k = 1; k < (1 << B); k++) {
-        if constexpr (SLOG > 0) {
-          x[k] = gl::lz_mul(v[k], tw512[((1u << TWLOG) - k * jps) & ((1u << TWLOG) - 1)]);
-        } else {
-          x[k] = gl::lz(v[k]);
-        }
+    for (int k = 1; k < (1 << B); k++) {
+      if constexpr (SLOG > 0) {
+        x[k] = gl::lz_mul(v[k], tw[((1u << TWLOG) - k * jps) & ((1u << TWLOG) - 1)]);
+      } else {
+        x[k] = gl::lz(v[k]);
       }
     }
     dft_inv_lz<B>(x, v);
@@ -411,69 +401,99 @@ __device__ __forceinline__ void round_inv_t(uint64_t* sm, const uint64_t* tw512,
   }
 }
 
-// HALF: rows 2^(R-1) .. 2^R - 1 of the tile are zero on entry (an operand
-// that fills at most half of its transform); only the first round uses it.
-template <int R, int T, int BC, int NT, bool HALF = false, int Q = 0>
-__device__ __forceinline__ void tile_fwd_t(uint64_t* sm, const uint64_t* tw512, int tid) {
-  if constexpr (Q < rp_count(R)) {
-    round_fwd_t<R, T, BC, rp_bits(R, Q), rp_mlog(R, Q), NT, (Q > 0 ? rp_bits(R, Q - 1) : 0),
-                (Q > 0 ? rp_mlog(R, Q - 1) : 0), 9, HALF && Q == 0>(sm, tw512, tid);
-    __syncthreads();
-    tile_fwd_t<R, T, BC, NT, false, Q + 1>(sm, tw512, tid);
-  }
-}
+// ----------------------------------------------------------- two-round passes
+// An HBM pass of radix 2^R (R = 6 .. 9) is two rounds in registers, radix
+// 2^B1 over rows 2^B2 apart and radix 2^B2 over the 2^B2 rows of each result,
+// with one exchange through shared memory between them: a length-512 DFT
+// costs one general twiddle product per element (w_512^(k1 m)) instead of the
+// two of an 8 x 8 x 8 split, its other twiddles being shifts (the 32nd root
+// of unity is 2^6), and the first round reads and the second one writes HBM
+// directly.  The integer pipes bind (ALU 60 %, IMAD 72 % busy before), so the
+// split that needs the fewest instructions per element is taken; against three
+// shared-memory rounds of radix 8 a 2^25-point pass of radix 2^9 went from 203
+// to 154 us (columns, 3.5 TB/s) and 156 to 114 us (contiguous, 4.7 TB/s), the
+// 2^30 x 2^30-bit product from 7.46 to 5.62 ms.  Forward: output index k1 of
+// round 1 and k2 of round 2 (row k1 2^B2 + k2) hold frequency k1 + 2^B1 k2.
+__host__ __device__ constexpr int pass_b1(int r) { return r <= 6 ? 3 : r <= 8 ? 4 : 5; }
+__host__ __device__ constexpr int pass_b2(int r) { return r - pass_b1(r); }
 
-template <int R, int T, int BC, int NT, int Q = rp_count(R) - 1, class F = NoPassTw>
-__device__ __forceinline__ void tile_inv_t(uint64_t* sm, const uint64_t* tw512, int tid, const F& ptw = F()) {
-  if constexpr (Q >= 0) {
-    round_inv_t<R, T, BC, rp_bits(R, Q), rp_mlog(R, Q), NT>(sm, tw512, tid, ptw);
-    __syncthreads();
-    tile_inv_t<R, T, BC, NT, Q - 1>(sm, tw512, tid);
-  }
-}
-
-// Rounds of a contiguous pass with one warp per 512-word chunk of the tile
-// (2^(9-R) blocks of 2^R words): a chunk's data never leaves its warp, so the
-// rounds synchronise with __syncwarp instead of the whole CTA.  smc is the
-// chunk's base in shared memory (its words at smc + spad(i), i < 512).
-template <int R, int Q = 0>
-__device__ __forceinline__ void chunk_fwd_t(uint64_t* smc, const uint64_t* tw512, int lane) {
-  if constexpr (Q < rp_count(R)) {
-    round_fwd_t<R, 0, 9 - R, rp_bits(R, Q), rp_mlog(R, Q), 32, (Q > 0 ? rp_bits(R, Q - 1) : 0),
-                (Q > 0 ? rp_mlog(R, Q - 1) : 0)>(smc, tw512, lane);
-    __syncwarp();
-    chunk_fwd_t<R, Q + 1>(smc, tw512, lane);
-  }
-}
-
-// ptw: factors multiplied into the first inverse round's inputs as lazy
-// products (ptw(row0, k, 0) for chunk word row0 + k), e.g. a pointwise product.
-template <int R, int Q = rp_count(R) - 1, class F = NoPassTw>
-__device__ __forceinline__ void chunk_inv_t(uint64_t* smc, const uint64_t* tw512, int lane, const F& ptw = F()) {
-  if constexpr (Q >= 0) {
-    round_inv_t<R, 0, 9 - R, rp_bits(R, Q), rp_mlog(R, Q), 32>(smc, tw512, lane, ptw);
-    __syncwarp();
-    chunk_inv_t<R, Q - 1>(smc, tw512, lane);
-  }
-}
-
-// Frequency index held at tile row `row` after the rounds of an R-bit DFT
-// (mixed-radix digit reversal of the row index).
-// (A bit permutation: row_freq_t(a | b) = row_freq_t(a) | row_freq_t(b) for
-// disjoint bit sets, which lets callers split a row into a per-thread part
-// and a compile-time part.)
+// Frequency index held at row `row` after a pass of radix 2^R.  (A bit
+// permutation: pass_freq(a | b) = pass_freq(a) | pass_freq(b) for disjoint
+// bit sets.)
 template <int R>
-__host__ __device__ __forceinline__ constexpr uint32_t row_freq_t(uint32_t row) {
-  uint32_t f = 0;
-  int rem = R, sh = 0;
+__host__ __device__ __forceinline__ constexpr uint32_t pass_freq(uint32_t row) {
+  return (row >> pass_b2(R)) | ((row & ((1u << pass_b2(R)) - 1)) << pass_b1(R));
+}
+
+// Column passes: a CTA of 128 threads takes 2^R rows x 2^T columns, T = 3 for
+// R = 8, 9 and 4 for R = 6, 7 (64- and 128-byte row segments; every thread has
+// one item in the round of radix 2^B1 and one or two in the other).  Exchange
+// element (k1, m, column) at k1 KS + (m << T | column); for T = 3 the eight
+// pad words put the two k1 of a half-warp on different banks.
+constexpr int PASS_THREADS = 128;
+template <int R>
+struct ColGeom {
+  static constexpr int B1 = pass_b1(R), B2 = pass_b2(R);
+  static constexpr int T = R >= 8 ? 3 : 4;
+  static constexpr int TILE = R + T;                          // log2 words per CTA
+  static constexpr uint32_t TM = (1u << T) - 1;
+  static constexpr uint32_t KS = (1u << (B2 + T)) + (T == 3 ? 8 : 0);
+  static constexpr uint32_t XWORDS = (1u << B1) * KS;         // exchange area
+  static constexpr int ITERS2 = (1 << (B1 + T)) / PASS_THREADS;  // items per thread of the (k1, column) round
+  static_assert((1 << (B2 + T)) == PASS_THREADS, "one (m, column) item per thread");
+};
+
+// Contiguous passes: each warp owns 32 2^B1 words (whole blocks of 2^R), so
+// only __syncwarp separates its rounds.  Exchange element (block, k1, m) at
+// (block 2^B1 + k1) (2^B2 + 1) + m, plus 8 words per block for R = 7 (blocks
+// 144 words apart would share banks).
+template <int R>
+struct RowGeom {
+  static constexpr int B1 = pass_b1(R), B2 = pass_b2(R);
+  static constexpr uint32_t WWORDS = 32u << B1;               // words per warp
+  static constexpr int TILE = 7 + B1;                         // log2 words per CTA (four warps)
+  static constexpr uint32_t KS = (1u << B2) + 1;
+  static constexpr uint32_t BPAD = R == 7 ? 8 : 0;
+  static constexpr uint32_t XWORDS = (WWORDS >> B2) * KS + (WWORDS >> R) * BPAD;  // exchange words per warp
+  static constexpr int ITERS2 = (int)(WWORDS >> B2) / 32;
+};
+
+// Round twiddles of a pass, in exchange order: forward w_(2^R)^(k1 m) at
+// [m 2^B1 + k1], inverse w_(2^R)^-(k1 m) at [k1 2^B2 + m] (L1-resident: 4 KB
+// per direction for R = 9).
+constexpr uint32_t RT_WORDS = 2 * ((1u << 10) - (1u << 6));
+__host__ __device__ constexpr uint32_t rt_offset(int r, bool inverse) {
+  return 2 * ((1u << r) - (1u << 6)) + (inverse ? 1u << r : 0);
+}
+
+// Forward round 2 / inverse round 1 share the exchange layout (k1 fixed, m
+// over the inputs); forward round 1 / inverse round 2 have m fixed.
+// Forward round 2's inputs: exchange words times their round twiddles.
+template <int R>
+__device__ __forceinline__ void pass_fwd2(const uint64_t* sx, uint32_t stride, const uint64_t* __restrict__ rt, uint32_t k1,
+                                          uint64_t* v) {
+  constexpr int B1 = pass_b1(R), B2 = pass_b2(R);
+  gl::Lz x[1 << B2];
 #pragma unroll
-  for (int q = 0; q < rp_count(R); q++) {
-    int b = rp_bits(R, q);
-    rem -= b;
-    f |= ((row >> rem) & ((1u << b) - 1)) << sh;
-    sh += b;
-  }
-  return f;
+  for (int m = 0; m < (1 << B2); m++) v[m] = sx[m * stride];
+  x[0] = gl::lz_bias(gl::lz(v[0]));  // w^0 = 1
+#pragma unroll
+  for (int m = 1; m < (1 << B2); m++) x[m] = gl::lz_mul(v[m], __ldg(rt + (m << B1) + k1));
+  dft_lz<B2, false>(x, v);
+}
+
+// Inverse round 2: over k1, inputs times their round twiddles.
+template <int R>
+__device__ __forceinline__ void pass_inv2(const uint64_t* sx, uint32_t stride, const uint64_t* __restrict__ rt, uint32_t m,
+                                          uint64_t* v) {
+  constexpr int B1 = pass_b1(R), B2 = pass_b2(R);
+  gl::Lz x[1 << B1];
+#pragma unroll
+  for (int k = 0; k < (1 << B1); k++) v[k] = sx[k * stride];
+  x[0] = gl::lz_bias(gl::lz(v[0]));
+#pragma unroll
+  for (int k = 1; k < (1 << B1); k++) x[k] = gl::lz_mul(v[k], __ldg(rt + (k << B2) + m));
+  dft_lz<B1, true>(x, v);
 }
 
 // ------------------------------------------------- runtime-geometry rounds
