@@ -161,8 +161,11 @@ static uint64_t find_rho() {
 //   last pass (S = 1):       four warps, each 32 2^B1 contiguous words
 // First-pass rows hold at least 8 consecutive coefficients, one carry window.
 // Four CTAs per SM leave 128 registers for a thread's radix-32 round (113 to
-// 126 used); 96 (five CTAs) spill, 168 (three) run no faster.
-constexpr int PASS_MIN_CTAS = 4;
+// 126 used); 96 (five CTAs) spill, 168 (three) run no faster.  The shorter
+// rounds do with less: a 2^24-point product of R = 8 passes takes 667 us at
+// five CTAs, 684 at four, 672 at seven; R = 6, 7 differ by under 1 % from
+// four to nine.
+constexpr int pass_min_ctas(int r) { return r == 9 ? 4 : r == 8 ? 5 : 6; }
 
 // One product of a batch (or the only product of a plain call): operands,
 // output and its scratch.  Kernels take `const Job* jobs, Job one`: with a
@@ -175,7 +178,8 @@ struct Job {
   uint64_t* A;  // N words: a's spectrum (and the product for a square)
   uint64_t* B;  // N words: b's spectrum and the product (unused for a square)
   uint64_t* H;  // high parts of the carry windows
-  uint8_t* aux; // carry-scan flags
+  uint64_t* W;  // their low parts, two limbs each
+  uint32_t* state;  // carry states of the window chunks
   uint64_t la, lb;
   const uint64_t* X;  // spectra of a second product added to the pointwise one (a sum of two products), or null
   const uint64_t* Y;
@@ -190,6 +194,18 @@ struct Job {
   uint64_t wrap;
 };
 
+// Carry windows of 8 coefficients (2 limbs); see the carry normalisation below.
+constexpr int WIN_COEFFS = 8;
+constexpr int CARRY_THREADS = 256;  // windows per CTA
+
+// Windows of an output of nout limbs (4 nout - 1 coefficients).
+__host__ __device__ __forceinline__ uint64_t n_windows_out(uint64_t nout) {
+  return (4 * nout - 1 + WIN_COEFFS - 1) / WIN_COEFFS;
+}
+__host__ __device__ __forceinline__ uint64_t n_windows(uint64_t la, uint64_t lb) { return n_windows_out(la + lb); }
+__host__ __device__ __forceinline__ uint64_t n_chunks(uint64_t nwin) {
+  return (nwin + CARRY_THREADS - 1) / CARRY_THREADS;
+}
 // Roles of a product inside a batch.  A spectrum shared by several products
 // with the same operand b is computed once, by its owner; the others point B
 // at it (JF_B_SHARED) and skip b's passes.  An addend (JF_ADDEND) produces no
@@ -201,7 +217,15 @@ constexpr uint32_t JF_ADDEND = 4;
 // the low part of a wrapped product.
 constexpr uint32_t JF_COEFF = 8;
 
+// Every kernel of the pipeline starts with these two (see launch_pdl): the next
+// kernel on the stream may be scheduled as this one's CTAs leave, and nothing
+// is read or written before the kernels in front are done.
+__device__ __forceinline__ void pdl_wait() {
+  asm volatile("griddepcontrol.launch_dependents;\n\tgriddepcontrol.wait;" ::: "memory");
+}
+
 __device__ __forceinline__ Job job_of(const Job* jobs, const Job& one) {
+  pdl_wait();
   if (jobs) return jobs[blockIdx.y];
   return one;
 }
@@ -217,7 +241,7 @@ __host__ __device__ __forceinline__ uint64_t job_nout(const Job& J) { return J.n
 // w0 + blockIdx.z (0: a, 1: b; skips_b drops b).
 // twf: the pass's twiddle table (tw_first), or null to compute the twiddles.
 template <int R>
-__global__ void __launch_bounds__(PASS_THREADS, PASS_MIN_CTAS) k_fwd_first(const Job* jobs, Job one, int w0, int L, Roots RT,
+__global__ void __launch_bounds__(PASS_THREADS, pass_min_ctas(R)) k_fwd_first(const Job* jobs, Job one, int w0, int L, Roots RT,
                                                                            const uint64_t* __restrict__ twf) {
   using G = ColGeom<R>;
   constexpr int B1 = G::B1, B2 = G::B2, T = G::T;
@@ -292,7 +316,7 @@ __global__ void __launch_bounds__(PASS_THREADS, PASS_MIN_CTAS) k_fwd_first(const
 // rounds (operand w0 + blockIdx.z), inverse ones before (on the product).
 // twm: the pass's twiddle table (tw_mid), or null to compute the twiddles.
 template <int R, bool FWD>
-__global__ void __launch_bounds__(PASS_THREADS, PASS_MIN_CTAS) k_col_mid(const Job* jobs, Job one, int w0, int S, Roots RT,
+__global__ void __launch_bounds__(PASS_THREADS, pass_min_ctas(R)) k_col_mid(const Job* jobs, Job one, int w0, int S, Roots RT,
                                                                          const uint64_t* __restrict__ twm) {
   using G = ColGeom<R>;
   constexpr int B1 = G::B1, B2 = G::B2, T = G::T;
@@ -377,7 +401,7 @@ __global__ void __launch_bounds__(PASS_THREADS, PASS_MIN_CTAS) k_col_mid(const J
 // words hold whole blocks; it leaves its spectrum as rows of 32 words, one
 // per (iteration, k2), the order in which the inverse's first round reads it.
 template <int R>
-__global__ void __launch_bounds__(PASS_THREADS, PASS_MIN_CTAS) k_fwd_last(const Job* jobs, Job one, int w0, Roots RT) {
+__global__ void __launch_bounds__(PASS_THREADS, pass_min_ctas(R)) k_fwd_last(const Job* jobs, Job one, int w0, Roots RT) {
   using G = RowGeom<R>;
   constexpr int B1 = G::B1, B2 = G::B2;
   const Job J = job_of(jobs, one);
@@ -419,11 +443,16 @@ __global__ void __launch_bounds__(PASS_THREADS, PASS_MIN_CTAS) k_fwd_last(const 
 // overwrites A.  ninv = 0: no scaling here (the inverse first pass's twiddle
 // table carries N^-1).
 template <int R>
-__global__ void __launch_bounds__(PASS_THREADS, PASS_MIN_CTAS) k_inv_last(const Job* jobs, Job one, uint64_t ninv, Roots RT) {
+__global__ void __launch_bounds__(PASS_THREADS, pass_min_ctas(R)) k_inv_last(const Job* jobs, Job one, uint64_t ninv, Roots RT) {
   using G = RowGeom<R>;
   constexpr int B1 = G::B1, B2 = G::B2;
   const Job J = job_of(jobs, one);
   if (J.flags & JF_ADDEND) return;
+  if (!(J.flags & JF_COEFF)) {
+    // no carry state published yet (there are fewer chunks than threads)
+    const uint64_t t = (uint64_t)blockIdx.x * PASS_THREADS + threadIdx.x;
+    if (t < n_chunks(n_windows_out(job_nout(J)))) J.state[t] = 0;
+  }
   extern __shared__ uint64_t sm[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint64_t off = ((uint64_t)blockIdx.x << G::TILE) + warp * G::WWORDS;
@@ -481,8 +510,6 @@ __global__ void __launch_bounds__(PASS_THREADS, PASS_MIN_CTAS) k_inv_last(const 
 // propagates.  Carries are resolved with a carry-lookahead scan over (g, p)
 // bit vectors: with A = g|p and B = g, the carry into each window is bit w of
 // (A + B + cin) ^ A ^ B.
-constexpr int WIN_COEFFS = 8;
-constexpr int WIN_LIMBS = 2;
 
 struct Win2 {
   uint64_t l[2];
@@ -525,26 +552,13 @@ __device__ __forceinline__ Win fold16(const uint64_t* c16, int stride) {
   return r;
 }
 
-constexpr int CARRY_THREADS = 256;  // windows per CTA
-
-// Windows of an output of nout limbs (4 nout - 1 coefficients).
-__host__ __device__ __forceinline__ uint64_t n_windows_out(uint64_t nout) {
-  return (4 * nout - 1 + WIN_COEFFS - 1) / WIN_COEFFS;
-}
-__host__ __device__ __forceinline__ uint64_t n_windows(uint64_t la, uint64_t lb) { return n_windows_out(la + lb); }
-__host__ __device__ __forceinline__ uint64_t n_chunks(uint64_t nwin) {
-  return (nwin + CARRY_THREADS - 1) / CARRY_THREADS;
-}
-// Carry-scan flag layout inside Job::aux: per warp (A, B) masks, then per
-// chunk the (g, p) byte and the carry-in byte.
-__host__ __device__ __forceinline__ uint64_t aux_bytes_for(uint64_t nwin) {
-  uint64_t nc = n_chunks(nwin);
-  return nc * (CARRY_THREADS / 32) * 8 + 2 * nc + 64;
-}
+// Words of the carry scratch of a product with nwin windows: high parts, then
+// the chunk states (the low parts lie in an array of 2 nwin words of their own).
+__host__ __device__ __forceinline__ uint64_t carry_words(uint64_t nwin) { return nwin + (n_chunks(nwin) + 1) / 2; }
 
 // Inverse pass 0 (natural order out) fused with the window fold: each tile
 // row holds 2^T consecutive coefficients = 2^(T-3) windows; every window
-// writes its low 2 limbs to the output and its high part to H.
+// writes its low 2 limbs to W and its high part to H.
 // twi: the pass's twiddle table (tw_first, inverse, with N^-1), or null to
 // compute the twiddles (the caller then scales by N^-1 in k_inv_last).
 // The rows are handed to the windows through shared memory, one pad word each.
@@ -552,15 +566,15 @@ template <int R>
 constexpr uint32_t INV_FIRST_XWORDS = ColGeom<R>::XWORDS > ((ColGeom<R>::TM + 2) << R) ? ColGeom<R>::XWORDS
                                                                                       : (ColGeom<R>::TM + 2) << R;
 template <int R>
-__global__ void __launch_bounds__(PASS_THREADS, PASS_MIN_CTAS) k_inv_first_carry(const Job* jobs, Job one, int L, Roots RT,
+__global__ void __launch_bounds__(PASS_THREADS, pass_min_ctas(R)) k_inv_first_carry(const Job* jobs, Job one, int L, Roots RT,
                                                                                  const uint64_t* __restrict__ twi) {
   using G = ColGeom<R>;
   constexpr int B1 = G::B1, B2 = G::B2, T = G::T;
   const Job J = job_of(jobs, one);
   if (J.flags & JF_ADDEND) return;
   const uint64_t* __restrict__ data = J.A;
-  uint64_t* __restrict__ out = J.out;
   uint64_t* __restrict__ H = J.H;
+  ulonglong2* __restrict__ W = reinterpret_cast<ulonglong2*>(J.W);
   const uint64_t nlimbs = job_nout(J), nwin = n_windows_out(nlimbs);
   extern __shared__ uint64_t sm[];
   const int tid = threadIdx.x;
@@ -623,7 +637,7 @@ __global__ void __launch_bounds__(PASS_THREADS, PASS_MIN_CTAS) k_inv_first_carry
     if (coeff) {
 #pragma unroll
       for (int t = 0; t < 8; t++)
-        if (8 * w + t < nlimbs) out[8 * w + t] = c[t];
+        if (8 * w + t < nlimbs) J.out[8 * w + t] = c[t];
       continue;
     }
     if (w >= nwin) continue;
@@ -640,161 +654,140 @@ __global__ void __launch_bounds__(PASS_THREADS, PASS_MIN_CTAS) k_inv_first_carry
       const uint64_t w2 = w + wtop;
       if (w2 < nwin) {
         const Win2 v2 = fold8(d);
-#pragma unroll
-        for (int t = 0; t < 2; t++)
-          if (2 * w2 + t < nlimbs) out[2 * w2 + t] = v2.l[t];
+        W[w2] = make_ulonglong2(v2.l[0], v2.l[1]);
         H[w2] = v2.hi;
       }
     }
-    Win2 v = fold8(c);
-#pragma unroll
-    for (int t = 0; t < 2; t++)
-      if (2 * w + t < nlimbs) out[2 * w + t] = v.l[t];
+    const Win2 v = fold8(c);
+    W[w] = make_ulonglong2(v.l[0], v.l[1]);
     H[w] = v.hi;
   }
 }
 
-// Carry pass 1 (grid.x = chunk, grid.y = product): s_w = lo_w + hi_(w-1)
-// written back as the output limbs; per window (g, p), per warp the (A, B)
-// masks, per CTA the chunk's carry out for carry in 0 and 1.
-__global__ void __launch_bounds__(CARRY_THREADS) k_carry_local(const Job* jobs, Job one) {
+// Window w after its left neighbour's high part: s_w = lo_w + hi_(w-1), and
+// its (generate, propagate) bits; the windows past the end do neither.
+struct WinSum {
+  uint64_t s0, s1;
+  bool g, p;
+};
+__device__ __forceinline__ WinSum win_sum(const Job& J, uint64_t w, uint64_t nwin) {
+  WinSum r{0, 0, false, false};
+  if (w < nwin) {
+    const ulonglong2 l = reinterpret_cast<const ulonglong2*>(J.W)[w];
+    const uint64_t hprev = w > 0 ? J.H[w - 1] : 0;
+    r.s0 = l.x + hprev;
+    const uint64_t c = r.s0 < hprev;
+    r.s1 = l.y + c;
+    r.g = c && r.s1 == 0;
+    r.p = (r.s0 & r.s1) == ~0ull;
+  }
+  return r;
+}
+
+// Carry function of a run of windows as two bits: bit 0 = carry out for carry
+// in 0, bit 1 = carry out for carry in 1.
+__device__ __forceinline__ uint32_t cf_of_masks(uint32_t A, uint32_t B) {
+  const uint64_t s = (uint64_t)A + B;
+  return (uint32_t)(s >> 32) | (uint32_t)((s + 1) >> 32) << 1;
+}
+// Running `first`, then `then`.
+__device__ __forceinline__ uint32_t cf_then(uint32_t first, uint32_t then) {
+  return ((then >> (first & 1)) & 1) | ((then >> ((first >> 1) & 1)) & 1) << 1;
+}
+
+// Carry function of chunk c from its windows, by one warp.
+__device__ uint32_t chunk_function(const Job& J, uint64_t c, uint64_t nwin, int lane) {
+  uint32_t f = 2;  // identity
+  for (int k = 0; k < CARRY_THREADS / 32; k++) {
+    const WinSum x = win_sum(J, c * CARRY_THREADS + 32 * k + lane, nwin);
+    const uint32_t A = __ballot_sync(0xFFFFFFFFu, x.g || x.p), B = __ballot_sync(0xFFFFFFFFu, x.g);
+    f = cf_then(f, cf_of_masks(A, B));
+  }
+  return f;
+}
+
+// Carry normalisation in one pass (grid.x = chunk of 256 windows, grid.y =
+// product).  A chunk's carry in almost always shows in the 32 windows to its
+// left, which warp 0 sums as well: no chunk waits for another.  Where all 32
+// pass a carry on (each all ones), the chunks' states are read instead: every
+// chunk publishes its carry function as soon as it has it (4 | function; the
+// states were zeroed by k_inv_last), one that passes its carry on replaces it
+// once it knows that carry, and the nearest chunk with a fixed carry out
+// gives the carry in.  A state that stays away for CARRY_POLLS reads (its CTA
+// may not run yet) is not waited for: the warp works the function out from
+// that chunk's windows, which are only read here.  Memory-bound: 24 bytes read
+// and 16 written per window; against three kernels (sums in place, scan,
+// increments) 240 -> 141 us at 2^27 points and two launches less.
+constexpr int CARRY_POLLS = 32;
+
+__global__ void __launch_bounds__(CARRY_THREADS) k_carry(const Job* jobs, Job one) {
   const Job J = job_of(jobs, one);
   if (J.flags & (JF_ADDEND | JF_COEFF)) return;
   const uint64_t nlimbs = job_nout(J), nwin = n_windows_out(nlimbs), nchunk = n_chunks(nwin);
-  if (blockIdx.x >= nchunk) return;  // uniform per CTA
-  uint64_t* __restrict__ out = J.out;
-  const uint64_t* __restrict__ H = J.H;
-  uint32_t* masks = reinterpret_cast<uint32_t*>(J.aux);
-  uint8_t* chunk_gp = J.aux + nchunk * (CARRY_THREADS / 32) * 8;
-  __shared__ uint32_t sA[CARRY_THREADS / 32], sB[CARRY_THREADS / 32];
-  const uint64_t w = (uint64_t)blockIdx.x * CARRY_THREADS + threadIdx.x;
+  const uint64_t chunk = blockIdx.x;
+  if (chunk >= nchunk) return;  // uniform per CTA
+  __shared__ uint32_t sA[CARRY_THREADS / 32], sB[CARRY_THREADS / 32], s_cin;
+  const uint64_t w = chunk * CARRY_THREADS + threadIdx.x;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  bool g = false, p = false;
-  if (w < nwin) {
-    uint64_t base = WIN_LIMBS * w;
-    uint64_t l0 = base + 0 < nlimbs ? out[base + 0] : 0;
-    uint64_t l1 = base + 1 < nlimbs ? out[base + 1] : 0;
-    uint64_t hprev = w > 0 ? H[w - 1] : 0;
-    uint64_t s0 = l0 + hprev;
-    uint64_t c = s0 < hprev;
-    uint64_t s1 = l1 + c;  c = c && s1 == 0;
-    g = c != 0;
-    p = (s0 & s1) == ~0ull;
-    if (base + 0 < nlimbs) out[base + 0] = s0;
-    if (base + 1 < nlimbs) out[base + 1] = s1;
+  const WinSum x = win_sum(J, w, nwin);
+  uint32_t left = 0;  // function of the 32 windows to the left (chunk 0: no carry)
+  if (warp == 0 && chunk > 0) {
+    const WinSum y = win_sum(J, w - 32, nwin);
+    const uint32_t yA = __ballot_sync(0xFFFFFFFFu, y.g || y.p), yB = __ballot_sync(0xFFFFFFFFu, y.g);
+    left = cf_of_masks(yA, yB);
   }
-  uint32_t A = __ballot_sync(0xFFFFFFFFu, g || p);
-  uint32_t Bm = __ballot_sync(0xFFFFFFFFu, g);
+  const uint32_t A = __ballot_sync(0xFFFFFFFFu, x.g || x.p);
+  const uint32_t B = __ballot_sync(0xFFFFFFFFu, x.g);
   if (lane == 0) {
-    uint64_t wi = (uint64_t)blockIdx.x * (CARRY_THREADS / 32) + warp;
-    masks[2 * wi] = A;
-    masks[2 * wi + 1] = Bm;
     sA[warp] = A;
-    sB[warp] = Bm;
+    sB[warp] = B;
   }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    uint32_t cg = 0, cp = 1;  // chunk carry out for carry in 0 / 1
-    for (int k = 0; k < CARRY_THREADS / 32; k++) {
-      uint64_t sg = (uint64_t)sA[k] + sB[k] + cg;
-      uint64_t sp = (uint64_t)sA[k] + sB[k] + cp;
-      cg = (uint32_t)(sg >> 32);
-      cp = (uint32_t)(sp >> 32);
-    }
-    chunk_gp[blockIdx.x] = (uint8_t)(cg | (cp << 1));
-  }
-}
-
-// Carry pass 2 (one CTA per product): carry into every chunk.  Each thread
-// walks a contiguous segment of chunks, the segment results are chained by
-// thread 0.
-constexpr int SCAN_THREADS = 1024;
-// Carry function of a run of chunks as two bits: bit 0 = carry out for carry
-// in 0, bit 1 = carry out for carry in 1 (the chunk's (g, p) byte has the
-// same layout).  Identity: 0b10.  Running `first`, then `then`:
-__device__ __forceinline__ uint32_t cf_then(uint32_t first, uint32_t then) {
-  const uint32_t o0 = (then >> (first & 1)) & 1;
-  const uint32_t o1 = (then >> ((first >> 1) & 1)) & 1;
-  return o0 | (o1 << 1);
-}
-
-// Carry pass 2 (one CTA per product): the carry into every chunk, as an
-// exclusive scan of the chunks' carry functions.  Each thread composes a
-// contiguous run (16-byte loads), the CTA scans the runs with warp shuffles,
-// and each thread writes its run's carries in.
-__global__ void __launch_bounds__(SCAN_THREADS) k_carry_scan(const Job* jobs, Job one) {
-  const Job J = job_of(jobs, one);
-  if (J.flags & (JF_ADDEND | JF_COEFF)) return;
-  const uint64_t nchunk = n_chunks(n_windows_out(job_nout(J)));
-  const uint8_t* chunk_gp = J.aux + nchunk * (CARRY_THREADS / 32) * 8;  // 64-byte aligned
-  uint8_t* chunk_cin = const_cast<uint8_t*>(chunk_gp) + nchunk;
-  __shared__ uint32_t warp_f[SCAN_THREADS / 32];
-  const uint64_t per = ((nchunk + SCAN_THREADS - 1) / SCAN_THREADS + 15) & ~15ull;  // a multiple of 16
-  const uint64_t lo = threadIdx.x * per, hi = lo + per < nchunk ? lo + per : nchunk;
-  uint32_t f = 2;  // identity
-  uint64_t k = lo;
-  for (; k + 16 <= hi; k += 16) {
-    const uint4 v = *reinterpret_cast<const uint4*>(chunk_gp + k);
-    const uint32_t w[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-    for (int q = 0; q < 16; q++) f = cf_then(f, (w[q >> 2] >> (8 * (q & 3))) & 3);
-  }
-  for (; k < hi; k++) f = cf_then(f, chunk_gp[k] & 3);
-  // exclusive scan of the threads' functions
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  uint32_t inc = f;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const uint32_t prev = __shfl_up_sync(0xFFFFFFFFu, inc, o);
-    if (lane >= o) inc = cf_then(prev, inc);
-  }
-  if (lane == 31) warp_f[warp] = inc;
   __syncthreads();
   if (warp == 0) {
-    uint32_t winc = lane < SCAN_THREADS / 32 ? warp_f[lane] : 2;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const uint32_t prev = __shfl_up_sync(0xFFFFFFFFu, winc, o);
-      if (lane >= o) winc = cf_then(prev, winc);
+    uint32_t f = 2;
+    for (int k = 0; k < CARRY_THREADS / 32; k++) f = cf_then(f, cf_of_masks(sA[k], sB[k]));
+    volatile uint32_t* state = J.state;
+    if (lane == 0) state[chunk] = 4 | f;
+    uint32_t cin = left & 1;
+    // chunks chunk - 1 - lane, 32 at a time; left of chunk 0 the carry is 0
+    for (int64_t base = (int64_t)chunk - 1; left == 2; base -= 32) {
+      const int64_t c = base - lane;
+      uint32_t st = c < 0 ? 4 : state[c];
+      for (int poll = 0; poll < CARRY_POLLS && __any_sync(0xFFFFFFFFu, st == 0); poll++) {
+        if (st == 0) st = state[c];
+        // enough once a known chunk with a fixed carry out comes before the first unknown one
+        const uint32_t unknown = __ballot_sync(0xFFFFFFFFu, st == 0);
+        const uint32_t fixed = __ballot_sync(0xFFFFFFFFu, st != 0 && (st & 3) != 2);
+        if (fixed && (!unknown || __ffs(fixed) < __ffs(unknown))) break;
+      }
+      // the nearest chunk whose carry out is fixed (identity passes it on)
+      bool done = false;
+      for (int k = 0; k < 32; k++) {
+        uint32_t sk = __shfl_sync(0xFFFFFFFFu, st, k);
+        if (sk == 0) sk = 4 | chunk_function(J, (uint64_t)(base - k), nwin, lane);
+        if ((sk & 3) != 2) {
+          cin = sk & 1;
+          done = true;
+          break;
+        }
+      }
+      if (done) break;
     }
-    const uint32_t wexc = __shfl_up_sync(0xFFFFFFFFu, winc, 1);
-    __syncwarp();
-    if (lane < SCAN_THREADS / 32) warp_f[lane] = lane ? wexc : 2;
+    if (lane == 0) {
+      s_cin = cin;
+      // a chunk that passes its carry on now has a fixed one: look-backs stop here
+      if (f == 2) state[chunk] = 4 | (cin ? 3 : 0);
+    }
   }
   __syncthreads();
-  const uint32_t in_warp = __shfl_up_sync(0xFFFFFFFFu, inc, 1);
-  const uint32_t before = cf_then(warp_f[warp], lane ? in_warp : 2);
-  uint32_t cin = before & 1;  // carry into this run (the product's carry in is 0)
-  for (k = lo; k < hi; k++) {
-    chunk_cin[k] = (uint8_t)cin;
-    cin = (chunk_gp[k] >> cin) & 1;
-  }
-}
-
-// Carry pass 3: add the incoming carry to every window that receives one.
-__global__ void __launch_bounds__(CARRY_THREADS) k_carry_apply(const Job* jobs, Job one) {
-  const Job J = job_of(jobs, one);
-  if (J.flags & (JF_ADDEND | JF_COEFF)) return;
-  const uint64_t nlimbs = job_nout(J), nwin = n_windows_out(nlimbs), nchunk = n_chunks(nwin);
-  if (blockIdx.x >= nchunk) return;
-  uint64_t* __restrict__ out = J.out;
-  const uint32_t* masks = reinterpret_cast<const uint32_t*>(J.aux);
-  const uint8_t* chunk_cin = J.aux + nchunk * (CARRY_THREADS / 32) * 8 + nchunk;
-  const uint64_t w = (uint64_t)blockIdx.x * CARRY_THREADS + threadIdx.x;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  uint32_t cin = chunk_cin[blockIdx.x];
-  const uint64_t wbase = (uint64_t)blockIdx.x * (CARRY_THREADS / 32);
-  for (int k = 0; k < warp; k++) {
-    uint64_t s = (uint64_t)masks[2 * (wbase + k)] + masks[2 * (wbase + k) + 1] + cin;
-    cin = (uint32_t)(s >> 32);
-  }
-  uint32_t A = masks[2 * (wbase + warp)], Bm = masks[2 * (wbase + warp) + 1];
-  uint32_t carries = (A + Bm + cin) ^ A ^ Bm;
-  if (w < nwin && ((carries >> lane) & 1)) {
-    uint64_t base = WIN_LIMBS * w;
-    for (int k = 0; k < WIN_LIMBS && base + k < nlimbs; k++) {
-      if (++out[base + k] != 0) break;
-    }
+  uint32_t cin = s_cin;
+  for (int k = 0; k < warp; k++) cin = (cf_of_masks(sA[k], sB[k]) >> cin) & 1;
+  const uint32_t carries = (A + B + cin) ^ A ^ B;
+  if (w < nwin) {
+    const uint64_t inc = (carries >> lane) & 1;
+    const uint64_t s0 = x.s0 + inc, s1 = x.s1 + (inc && s0 == 0);
+    if (2 * w < nlimbs) J.out[2 * w] = s0;
+    if (2 * w + 1 < nlimbs) J.out[2 * w + 1] = s1;
   }
 }
 
@@ -1644,7 +1637,7 @@ static Plan make_plan(int L) {
 }
 
 struct Sizes {
-  uint64_t n_out, N, nwin, nchunk, aux_bytes;
+  uint64_t n_out, N, nwin, nchunk;
   int L;
 };
 
@@ -1655,31 +1648,30 @@ static Sizes sizes_for(uint64_t la, uint64_t lb) {
   z.N = 1ull << z.L;
   z.nwin = n_windows(la, lb);
   z.nchunk = n_chunks(z.nwin);
-  z.aux_bytes = aux_bytes_for(z.nwin);
   return z;
 }
 
-// Scratch bytes of one large product (A, B unless square, H, aux), each
-// piece rounded to 256 bytes.
+// Scratch bytes of one large product, each piece rounded to 256 bytes: A, B
+// (whose words hold the windows' low parts once the spectra are multiplied;
+// a square allots just those), and the carry scratch.
 static uint64_t round256(uint64_t x) { return (x + 255) & ~255ull; }
 __host__ __device__ __forceinline__ uint64_t round_up_u64(uint64_t x, uint64_t m) { return (x + m - 1) / m * m; }
 static uint64_t scratch_bytes(uint64_t la, uint64_t lb, bool square) {
   Sizes z = sizes_for(la, lb);
-  return round256(z.N * 8) * (square ? 1 : 2) + round256(z.nwin * 8) + round256(z.aux_bytes);
+  return round256(z.N * 8) + round256(square ? z.nwin * 16 : z.N * 8) + round256(carry_words(z.nwin) * 8);
+}
+static void carve_carry(Job& J, uint64_t* base, uint64_t nwin) {
+  J.H = base;
+  J.state = reinterpret_cast<uint32_t*>(base + nwin);
 }
 static void carve_scratch(Job& J, uint8_t* base, bool square) {
   Sizes z = sizes_for(J.la, J.lb);
   J.A = reinterpret_cast<uint64_t*>(base);
   base += round256(z.N * 8);
-  if (!square) {
-    J.B = reinterpret_cast<uint64_t*>(base);
-    base += round256(z.N * 8);
-  } else {
-    J.B = nullptr;
-  }
-  J.H = reinterpret_cast<uint64_t*>(base);
-  base += round256(z.nwin * 8);
-  J.aux = base;
+  J.W = reinterpret_cast<uint64_t*>(base);
+  J.B = square ? nullptr : J.W;
+  base += round256(square ? z.nwin * 16 : z.N * 8);
+  carve_carry(J, reinterpret_cast<uint64_t*>(base), z.nwin);
 }
 
 // Launch helpers (template dispatch on the pass radix).
@@ -1690,6 +1682,26 @@ static void carve_scratch(Job& J, uint8_t* base, bool square) {
     case 8: { constexpr int RR = 8; __VA_ARGS__; } break; \
     default: { constexpr int RR = 9; __VA_ARGS__; } break; \
   }
+
+// Programmatic dependent launch: the pipeline's kernels may be scheduled while
+// the one before them on the stream drains, and wait for its completion and
+// memory (pdl_wait) before they read or write anything of it.  The gaps and
+// ramps between six to nine short kernels were a third of a mid-size product:
+// 2^16 bits 25.2 -> 17.3 us, 2^24 bits 117 -> 99 us, 2^30 bits 5.47 -> 5.45 ms.
+template <class... P, class... A>
+static void launch_pdl(void (*k)(P...), dim3 grid, int threads, size_t smem, cudaStream_t st, A... args) {
+  cudaLaunchConfig_t c = {};
+  c.gridDim = grid;
+  c.blockDim = dim3(threads);
+  c.dynamicSmemBytes = smem;
+  c.stream = st;
+  cudaLaunchAttribute at;
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  c.attrs = &at;
+  c.numAttrs = 1;
+  cudaLaunchKernelEx(&c, k, (P)args...);
+}
 
 // Both operands of a transform up to this length (log2) go through each
 // forward pass in one launch.
@@ -1849,8 +1861,8 @@ static void run_large(const Launcher& X, const Job* jobs, const Job& one, uint32
       KTimer kt(K_PACK, X.st, X.stats);
       PIMUL_DISPATCH_R(pl.r[0], {
         constexpr int R = RR < 7 ? 7 : RR;
-        k_fwd_first<R><<<grid(ColGeom<R>::TILE, nz), PASS_THREADS, (ColGeom<R>::XWORDS + (1u << R)) * 8, X.st>>>(
-            jobs, one, which, L, X.R, tw.first_fwd);
+        launch_pdl(k_fwd_first<R>, grid(ColGeom<R>::TILE, nz), PASS_THREADS, (ColGeom<R>::XWORDS + (1u << R)) * 8, X.st, jobs,
+                   one, which, L, X.R, tw.first_fwd);
       });
     }
     int consumed = pl.r[0];
@@ -1858,19 +1870,21 @@ static void run_large(const Launcher& X, const Job* jobs, const Job& one, uint32
       consumed += pl.r[p];
       KTimer kt(K_PASS_FWD, X.st, X.stats);
       PIMUL_DISPATCH_R(pl.r[p], {
-        k_col_mid<RR, true><<<grid(ColGeom<RR>::TILE, nz), PASS_THREADS, ColGeom<RR>::XWORDS * 8, X.st>>>(
-            jobs, one, which, L - consumed, X.R, tw.mid_fwd[p]);
+        launch_pdl(k_col_mid<RR, true>, grid(ColGeom<RR>::TILE, nz), PASS_THREADS, ColGeom<RR>::XWORDS * 8, X.st, jobs, one,
+                   which, L - consumed, X.R, tw.mid_fwd[p]);
       });
     }
     KTimer kt(K_PASS_FWD, X.st, X.stats);
     PIMUL_DISPATCH_R(rl, {
-      k_fwd_last<RR><<<grid(RowGeom<RR>::TILE, nz), PASS_THREADS, 4 * RowGeom<RR>::XWORDS * 8, X.st>>>(jobs, one, which, X.R);
+      launch_pdl(k_fwd_last<RR>, grid(RowGeom<RR>::TILE, nz), PASS_THREADS, 4 * RowGeom<RR>::XWORDS * 8, X.st, jobs, one, which,
+                 X.R);
     });
   }
   {
     KTimer kt(K_POINTWISE, X.st, X.stats);
     PIMUL_DISPATCH_R(rl, {
-      k_inv_last<RR><<<grid(RowGeom<RR>::TILE, 1), PASS_THREADS, 4 * RowGeom<RR>::XWORDS * 8, X.st>>>(jobs, one, ninv, X.R);
+      launch_pdl(k_inv_last<RR>, grid(RowGeom<RR>::TILE, 1), PASS_THREADS, 4 * RowGeom<RR>::XWORDS * 8, X.st, jobs, one, ninv,
+                 X.R);
     });
   }
   int consumed = L - rl;
@@ -1879,26 +1893,22 @@ static void run_large(const Launcher& X, const Job* jobs, const Job& one, uint32
     consumed -= pl.r[p];
     KTimer kt(K_PASS_INV, X.st, X.stats);
     PIMUL_DISPATCH_R(pl.r[p], {
-      k_col_mid<RR, false><<<grid(ColGeom<RR>::TILE, 1), PASS_THREADS, ColGeom<RR>::XWORDS * 8, X.st>>>(jobs, one, 0, S, X.R,
-                                                                                                      tw.mid_inv[p]);
+      launch_pdl(k_col_mid<RR, false>, grid(ColGeom<RR>::TILE, 1), PASS_THREADS, ColGeom<RR>::XWORDS * 8, X.st, jobs, one, 0, S,
+                 X.R, tw.mid_inv[p]);
     });
   }
   {
     KTimer kt(K_PASS_INV, X.st, X.stats);
     PIMUL_DISPATCH_R(pl.r[0], {
       constexpr int R = RR < 7 ? 7 : RR;
-      k_inv_first_carry<R><<<grid(ColGeom<R>::TILE, 1), PASS_THREADS, (INV_FIRST_XWORDS<R> + (1u << R)) * 8, X.st>>>(
-          jobs, one, L, X.R, tw.first_inv);
+      launch_pdl(k_inv_first_carry<R>, grid(ColGeom<R>::TILE, 1), PASS_THREADS, (INV_FIRST_XWORDS<R> + (1u << R)) * 8, X.st,
+                 jobs, one, L, X.R, tw.first_inv);
     });
   }
   {
     KTimer kt(K_CARRY, X.st, X.stats);
-    const dim3 cgrid((unsigned)max_chunk, nj);
-    k_carry_local<<<cgrid, CARRY_THREADS, 0, X.st>>>(jobs, one);
-    k_carry_scan<<<dim3(1, nj), SCAN_THREADS, 0, X.st>>>(jobs, one);
-    k_carry_apply<<<cgrid, CARRY_THREADS, 0, X.st>>>(jobs, one);
+    launch_pdl(k_carry, dim3((unsigned)max_chunk, nj), CARRY_THREADS, 0, X.st, jobs, one);
   }
-  if (X.stats) g_launch[K_CARRY].fetch_add(2, std::memory_order_relaxed);
 }
 
 // Device multiply: d_out[0 .. la+lb) = a * b, scratch from the memory pool.
@@ -1925,7 +1935,8 @@ static int mul_device(const uint64_t* d_a, uint64_t la, const uint64_t* d_b, uin
     cudaGetLastError();
     return fail(PIMUL_ENOMEM, std::string("scratch allocation: ") + cudaGetErrorString(e));
   }
-  Job J{d_a, d_b, d_out, nullptr, nullptr, nullptr, nullptr, la, lb};
+  Job J{};
+  J.a = d_a, J.la = la, J.b = d_b, J.lb = lb, J.out = d_out;
   carve_scratch(J, base, square);
   Launcher X{st, true, R, b_ready};
   run_large(X, nullptr, J, 1, z.L, z.nchunk);
@@ -1971,7 +1982,8 @@ struct BatchLayout {
     uint32_t flags;          // JF_*
     int64_t owner = -1;      // descriptor whose B this one borrows
     int64_t addend = -1;     // descriptor whose A holds this one's X
-    uint64_t off_a = 0, off_b = 0, off_h = 0, off_aux = 0;
+    bool lent = false;       // others borrow its B
+    uint64_t off_a = 0, off_b = 0, off_w = 0, off_h = 0;
   };
   std::vector<Desc> desc;  // large descriptors in launch order
   struct Bucket {
@@ -2050,8 +2062,8 @@ static int layout_batch(const Unit* units, size_t n, BatchLayout& B, bool share)
       for (; e < byL[L].size(); e++) {
         const Unit& u = units[byL[L][e]];
         const size_t nd = u.la2 ? 2 : 1;
-        const uint64_t need = round256(N * 8) * 2 * nd + round256(n_windows_out(u.nout) * 8) +
-                              round256(aux_bytes_for(n_windows_out(u.nout)));
+        const uint64_t nwin = n_windows_out(u.nout);
+        const uint64_t need = round256(N * 8) * 2 * nd + round256(nwin * 16) + round256(carry_words(nwin) * 8);
         if (e > s && (bk.nd + nd > 65535 || bound + need > BATCH_ARENA_CAP)) break;
         bk.nd += nd;
         bound += need;
@@ -2093,6 +2105,7 @@ static int layout_batch(const Unit* units, size_t n, BatchLayout& B, bool share)
           } else {
             B.desc[di].flags |= JF_B_SHARED;
             B.desc[di].owner = (int64_t)it->second;
+            B.desc[it->second].lent = true;
           }
         }
       }
@@ -2110,10 +2123,14 @@ static int layout_batch(const Unit* units, size_t n, BatchLayout& B, bool share)
         }
         if (!d.second) {
           const uint64_t nwin = n_windows_out(u.nout);
+          // the windows' low parts go to B where the product has one to itself
+          d.off_w = d.off_b;
+          if (sq || (d.flags & JF_B_SHARED) || d.lent) {
+            d.off_w = off;
+            off += round256(nwin * 16);
+          }
           d.off_h = off;
-          off += round256(nwin * 8);
-          d.off_aux = off;
-          off += round256(aux_bytes_for(nwin));
+          off += round256(carry_words(nwin) * 8);
           bk.max_chunk = std::max<uint64_t>(bk.max_chunk, n_chunks(nwin));
         }
       }
@@ -2161,8 +2178,10 @@ static void fill_descriptors(const Unit* units, const BatchLayout& B, uint8_t* a
       J.B = reinterpret_cast<uint64_t*>(arena + B.desc[d.owner].off_b);
     else
       J.B = sq ? nullptr : reinterpret_cast<uint64_t*>(arena + d.off_b);
-    J.H = d.second ? nullptr : reinterpret_cast<uint64_t*>(arena + d.off_h);
-    J.aux = d.second ? nullptr : arena + d.off_aux;
+    if (!d.second) {
+      J.W = reinterpret_cast<uint64_t*>(arena + d.off_w);
+      carve_carry(J, reinterpret_cast<uint64_t*>(arena + d.off_h), n_windows_out(u.nout));
+    }
     if (d.addend >= 0) {
       const BatchLayout::Desc& x = B.desc[d.addend];
       J.X = reinterpret_cast<const uint64_t*>(arena + x.off_a);
@@ -3834,12 +3853,9 @@ namespace pimul {
 constexpr int NOALLOC_LOG_MAX = 20;
 constexpr uint64_t NOALLOC_N_MAX = 1ull << NOALLOC_LOG_MAX;
 constexpr uint64_t NOALLOC_WIN_MAX = NOALLOC_N_MAX / WIN_COEFFS;
-constexpr uint64_t NOALLOC_CHUNK_MAX = (NOALLOC_WIN_MAX + CARRY_THREADS - 1) / CARRY_THREADS;
-constexpr uint64_t NOALLOC_AUX_WORDS = (NOALLOC_CHUNK_MAX * (CARRY_THREADS / 32) * 8 + 2 * NOALLOC_CHUNK_MAX + 64) / 8 + 1;
-static_assert(NOALLOC_AUX_WORDS * 8 >= NOALLOC_CHUNK_MAX * (CARRY_THREADS / 32) * 8 + 2 * NOALLOC_CHUNK_MAX + 64,
-              "no-alloc carry flags must fit");
+constexpr uint64_t NOALLOC_CARRY_WORDS = NOALLOC_WIN_MAX + (NOALLOC_WIN_MAX / CARRY_THREADS + 2) / 2;
 
-static __device__ __align__(256) uint64_t g_noalloc_scratch[2 * NOALLOC_N_MAX + NOALLOC_WIN_MAX + NOALLOC_AUX_WORDS];
+static __device__ __align__(256) uint64_t g_noalloc_scratch[2 * NOALLOC_N_MAX + NOALLOC_CARRY_WORDS];
 static __device__ __align__(256) uint64_t g_noalloc_roots[ROOT_WORDS];
 
 struct NoAllocDev {
@@ -3897,11 +3913,12 @@ static int mul_device_noalloc(const uint64_t* d_a, uint64_t la, const uint64_t* 
     return PIMUL_OK;
   }
   const bool square = d_a == d_b && la == lb;
-  Job J{d_a, d_b, d_out, nullptr, nullptr, nullptr, nullptr, la, lb};
+  Job J{};
+  J.a = d_a, J.la = la, J.b = d_b, J.lb = lb, J.out = d_out;
   J.A = nd->scratch;
-  J.B = square ? nullptr : nd->scratch + NOALLOC_N_MAX;
-  J.H = nd->scratch + 2 * NOALLOC_N_MAX;
-  J.aux = reinterpret_cast<uint8_t*>(nd->scratch + 2 * NOALLOC_N_MAX + NOALLOC_WIN_MAX);
+  J.W = nd->scratch + NOALLOC_N_MAX;
+  J.B = square ? nullptr : J.W;
+  carve_carry(J, nd->scratch + 2 * NOALLOC_N_MAX, z.nwin);
   Launcher X{st, false, R};  // no statistics hook: its event timing would create CUDA events
   X.tables = false;          // nor the twiddle tables, which are allocated on first use
   run_large(X, nullptr, J, 1, z.L, z.nchunk);
