@@ -192,6 +192,14 @@ struct Job {
   // cyclic value minus low[i].
   const uint64_t* low;
   uint64_t wrap;
+  // A segment of a product of a long a by a short b: its transform covers the
+  // coefficients c0 .. c0 + N - 1 of a (zero outside a), and its cyclic values
+  // from window wlo on are the product's windows w + woff.
+  int64_t c0;
+  int64_t woff;
+  uint32_t wlo;
+  uint32_t segments;  // by value: blockIdx.y selects one of these, each segv coefficients on
+  uint64_t segv;
 };
 
 // Carry windows of 8 coefficients (2 limbs); see the carry normalisation below.
@@ -216,6 +224,8 @@ constexpr uint32_t JF_ADDEND = 4;
 // The product's canonical coefficients 0 .. nout - 1 go to out (no carry):
 // the low part of a wrapped product.
 constexpr uint32_t JF_COEFF = 8;
+// A segment after a product's first one: its windows are carried by that one.
+constexpr uint32_t JF_SEGMENT = 16;
 
 // Every kernel of the pipeline starts with these two (see launch_pdl): the next
 // kernel on the stream may be scheduled as this one's CTAs leave, and nothing
@@ -224,10 +234,20 @@ __device__ __forceinline__ void pdl_wait() {
   asm volatile("griddepcontrol.launch_dependents;\n\tgriddepcontrol.wait;" ::: "memory");
 }
 
-__device__ __forceinline__ Job job_of(const Job* jobs, const Job& one) {
+// Segment s of a segmented product whose first segment is J.
+__host__ __device__ __forceinline__ void to_segment(Job& J, uint32_t s, int L) {
+  J.A += (uint64_t)s << L;
+  J.c0 = (int64_t)(s * J.segv) - 8 * (int64_t)J.wlo;
+  J.woff = (int64_t)(s * (J.segv / 8)) - (int64_t)J.wlo;
+  if (s) J.flags |= JF_SEGMENT | JF_B_SHARED;
+}
+
+__device__ __forceinline__ Job job_of(const Job* jobs, const Job& one, int L) {
   pdl_wait();
   if (jobs) return jobs[blockIdx.y];
-  return one;
+  Job J = one;
+  if (J.segments) to_segment(J, blockIdx.y, L);
+  return J;
 }
 __host__ __device__ __forceinline__ bool is_square(const Job& J) { return J.a == J.b && J.la == J.lb; }
 // b's own passes are skipped for a square and for a borrowed spectrum.
@@ -245,33 +265,35 @@ __global__ void __launch_bounds__(PASS_THREADS, pass_min_ctas(R)) k_fwd_first(co
                                                                            const uint64_t* __restrict__ twf) {
   using G = ColGeom<R>;
   constexpr int B1 = G::B1, B2 = G::B2, T = G::T;
-  const Job J = job_of(jobs, one);
+  const Job J = job_of(jobs, one, L);
   const int which = w0 + (int)blockIdx.z;
   if (which == 1 && skips_b(J)) return;
   const uint16_t* __restrict__ coef = reinterpret_cast<const uint16_t*>(which ? J.b : J.a);
-  const uint64_t nc = 4 * (which ? J.lb : J.la);
+  const int64_t c0 = which ? 0 : J.c0, nc = (int64_t)(4 * (which ? J.lb : J.la));
   uint64_t* __restrict__ data = which ? J.B : J.A;
   extern __shared__ uint64_t sm[];
   const int tid = threadIdx.x;
   const int S = L - R;
   const uint64_t j0 = (uint64_t)blockIdx.x << T;
   {
-    const uint64_t n0 = ((uint64_t)(tid >> T) << S) + j0 + (tid & G::TM);
+    const int64_t n0 = c0 + (int64_t)(((uint64_t)(tid >> T) << S) + j0 + (tid & G::TM));
     const uint64_t step = 1ull << (S + B2);
-    // inputs m < mc exist
-    const uint32_t mc = n0 < nc ? (uint32_t)((nc - n0 + step - 1) >> (S + B2)) : 0;
+    // inputs ml <= m < mc exist (ml > 0: a first segment starts before a does)
+    const uint32_t ml = n0 < 0 ? (uint32_t)((uint64_t)(-n0 + (int64_t)step - 1) >> (S + B2)) : 0;
+    const uint32_t mc = n0 < nc ? (uint32_t)((uint64_t)(nc - n0 + (int64_t)step - 1) >> (S + B2)) - ml : 0;
+    const uint16_t* __restrict__ cn = coef + n0;
     uint64_t v[1 << B1];
     gl::Lz x[1 << B1];
     // an operand of at most N/8 limbs leaves the upper half of the rows zero
     // (coefficients N/2 and up): those inputs are neither read nor added
-    if (nc <= (1ull << (L - 1))) {
+    if (nc - c0 <= (int64_t)(1ull << (L - 1))) {
 #pragma unroll
-      for (int m = 0; m < (1 << (B1 - 1)); m++) x[m] = gl::Lz{m < mc ? (uint32_t)__ldg(coef + n0 + m * step) : 0u, 0u, 0};
+      for (int m = 0; m < (1 << (B1 - 1)); m++) x[m] = gl::Lz{m - ml < mc ? (uint32_t)__ldg(cn + m * step) : 0u, 0u, 0};
       x[0] = gl::lz_bias(x[0]);
       dft_lz<B1, false, true>(x, v);
     } else {
 #pragma unroll
-      for (int m = 0; m < (1 << B1); m++) x[m] = gl::Lz{m < mc ? (uint32_t)__ldg(coef + n0 + m * step) : 0u, 0u, 0};
+      for (int m = 0; m < (1 << B1); m++) x[m] = gl::Lz{m - ml < mc ? (uint32_t)__ldg(cn + m * step) : 0u, 0u, 0};
       x[0] = gl::lz_bias(x[0]);
       dft_lz<B1, false>(x, v);
     }
@@ -316,11 +338,11 @@ __global__ void __launch_bounds__(PASS_THREADS, pass_min_ctas(R)) k_fwd_first(co
 // rounds (operand w0 + blockIdx.z), inverse ones before (on the product).
 // twm: the pass's twiddle table (tw_mid), or null to compute the twiddles.
 template <int R, bool FWD>
-__global__ void __launch_bounds__(PASS_THREADS, pass_min_ctas(R)) k_col_mid(const Job* jobs, Job one, int w0, int S, Roots RT,
-                                                                         const uint64_t* __restrict__ twm) {
+__global__ void __launch_bounds__(PASS_THREADS, pass_min_ctas(R)) k_col_mid(const Job* jobs, Job one, int w0, int L, int S,
+                                                                         Roots RT, const uint64_t* __restrict__ twm) {
   using G = ColGeom<R>;
   constexpr int B1 = G::B1, B2 = G::B2, T = G::T;
-  const Job J = job_of(jobs, one);
+  const Job J = job_of(jobs, one, L);
   const int which = w0 + (int)blockIdx.z;
   if (FWD && which == 1 && skips_b(J)) return;
   if (!FWD && (J.flags & JF_ADDEND)) return;
@@ -401,10 +423,10 @@ __global__ void __launch_bounds__(PASS_THREADS, pass_min_ctas(R)) k_col_mid(cons
 // words hold whole blocks; it leaves its spectrum as rows of 32 words, one
 // per (iteration, k2), the order in which the inverse's first round reads it.
 template <int R>
-__global__ void __launch_bounds__(PASS_THREADS, pass_min_ctas(R)) k_fwd_last(const Job* jobs, Job one, int w0, Roots RT) {
+__global__ void __launch_bounds__(PASS_THREADS, pass_min_ctas(R)) k_fwd_last(const Job* jobs, Job one, int w0, int L, Roots RT) {
   using G = RowGeom<R>;
   constexpr int B1 = G::B1, B2 = G::B2;
-  const Job J = job_of(jobs, one);
+  const Job J = job_of(jobs, one, L);
   const int which = w0 + (int)blockIdx.z;
   if (which == 1 && skips_b(J)) return;
   extern __shared__ uint64_t sm[];
@@ -443,15 +465,16 @@ __global__ void __launch_bounds__(PASS_THREADS, pass_min_ctas(R)) k_fwd_last(con
 // overwrites A.  ninv = 0: no scaling here (the inverse first pass's twiddle
 // table carries N^-1).
 template <int R>
-__global__ void __launch_bounds__(PASS_THREADS, pass_min_ctas(R)) k_inv_last(const Job* jobs, Job one, uint64_t ninv, Roots RT) {
+__global__ void __launch_bounds__(PASS_THREADS, pass_min_ctas(R)) k_inv_last(const Job* jobs, Job one, int L, uint64_t ninv, Roots RT) {
   using G = RowGeom<R>;
   constexpr int B1 = G::B1, B2 = G::B2;
-  const Job J = job_of(jobs, one);
+  const Job J = job_of(jobs, one, L);
   if (J.flags & JF_ADDEND) return;
-  if (!(J.flags & JF_COEFF)) {
-    // no carry state published yet (there are fewer chunks than threads)
-    const uint64_t t = (uint64_t)blockIdx.x * PASS_THREADS + threadIdx.x;
-    if (t < n_chunks(n_windows_out(job_nout(J)))) J.state[t] = 0;
+  if (!(J.flags & (JF_COEFF | JF_SEGMENT))) {
+    // no carry state published yet
+    const uint64_t nchunk = n_chunks(n_windows_out(job_nout(J)));
+    for (uint64_t t = (uint64_t)blockIdx.x * PASS_THREADS + threadIdx.x; t < nchunk; t += (uint64_t)gridDim.x * PASS_THREADS)
+      J.state[t] = 0;
   }
   extern __shared__ uint64_t sm[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -570,7 +593,7 @@ __global__ void __launch_bounds__(PASS_THREADS, pass_min_ctas(R)) k_inv_first_ca
                                                                                  const uint64_t* __restrict__ twi) {
   using G = ColGeom<R>;
   constexpr int B1 = G::B1, B2 = G::B2, T = G::T;
-  const Job J = job_of(jobs, one);
+  const Job J = job_of(jobs, one, L);
   if (J.flags & JF_ADDEND) return;
   const uint64_t* __restrict__ data = J.A;
   uint64_t* __restrict__ H = J.H;
@@ -629,7 +652,9 @@ __global__ void __launch_bounds__(PASS_THREADS, pass_min_ctas(R)) k_inv_first_ca
   const uint64_t wtop = (1ull << L) >> 3;  // a wrapped product's windows past the transform: w + wtop
   for (uint32_t q = tid; q < (1u << (G::TILE - 3)); q += PASS_THREADS) {
     const uint32_t i = q >> (T - 3), k = q & ((1u << (T - 3)) - 1);
-    const uint64_t w = ((((uint64_t)i << S) + j0) >> 3) + k;
+    const uint64_t wl = ((((uint64_t)i << S) + j0) >> 3) + k;
+    if (wl < J.wlo) continue;
+    const uint64_t w = wl + (uint64_t)J.woff;  // window of the whole product
     uint64_t c[8];
     const uint64_t* row = sm + i * RS + 8 * k;
 #pragma unroll
@@ -721,7 +746,7 @@ __device__ uint32_t chunk_function(const Job& J, uint64_t c, uint64_t nwin, int 
 constexpr int CARRY_POLLS = 32;
 
 __global__ void __launch_bounds__(CARRY_THREADS) k_carry(const Job* jobs, Job one) {
-  const Job J = job_of(jobs, one);
+  const Job J = job_of(jobs, one, 0);
   if (J.flags & (JF_ADDEND | JF_COEFF)) return;
   const uint64_t nlimbs = job_nout(J), nwin = n_windows_out(nlimbs), nchunk = n_chunks(nwin);
   const uint64_t chunk = blockIdx.x;
@@ -1651,6 +1676,53 @@ static Sizes sizes_for(uint64_t la, uint64_t lb) {
   return z;
 }
 
+// Products of a long operand by a short one are cut into segments (overlap-save):
+// a transform of N points over N - 8 wlo new coefficients of the long operand
+// and the 8 wlo >= 4 lb - 1 before them gives N - 8 wlo exact coefficients of the
+// product (the first 8 wlo values have wrapped around), and all segments share
+// the short operand's spectrum: 2 S + 1 transforms of a length near the short
+// operand's instead of 3 of a length above the sum.  The cost of a transform
+// is taken as N (30 passes + 5.5 log2 N), from the kernels' times per point
+// (2 passes, 2^18 points: 8.0 us forward and 10.7 us inverse per 2^20 points; 3
+// passes, 2^24 points: 11.7 and 13.5).  Cut only where that saves a tenth.
+struct SegPlan {
+  int L = 0;          // transform length of a segment (0: not cut)
+  uint32_t S = 0;     // segments
+  uint64_t wlo = 0;   // windows of the overlap
+  uint64_t segv = 0;  // new coefficients per segment
+};
+constexpr uint32_t SEG_MAX = 8192;
+
+static double transform_cost(int L) {
+  static const std::vector<double> table = [] {
+    std::vector<double> t(33);
+    for (int l = 0; l <= 32; l++) t[l] = (double)(1ull << l) * (30.0 * default_np(l) + 5.5 * l);
+    return t;
+  }();
+  return table[L];
+}
+
+static SegPlan plan_segments(uint64_t la, uint64_t lb) {
+  SegPlan best;
+  if (la < lb) std::swap(la, lb);
+  const Sizes z = sizes_for(la, lb);
+  if (z.L <= SMALL_LOG_MAX + 1 || la < 2 * lb) return best;
+  double cost = 0.9 * 3 * transform_cost(z.L);
+  const uint64_t wlo = (4 * lb - 1 + WIN_COEFFS - 1) / WIN_COEFFS;
+  for (int L = SMALL_LOG_MAX + 1; L < z.L; L++) {
+    const uint64_t N = 1ull << L;
+    if (2 * WIN_COEFFS * wlo > N) continue;
+    const uint64_t v = N - WIN_COEFFS * wlo, S = (z.n_out + v - 1) / v;
+    if (S > SEG_MAX) continue;
+    const double c = (double)(2 * S + 1) * transform_cost(L);
+    if (c < cost) {
+      cost = c;
+      best.L = L, best.S = (uint32_t)S, best.wlo = wlo, best.segv = v;
+    }
+  }
+  return best;
+}
+
 // Scratch bytes of one large product, each piece rounded to 256 bytes: A, B
 // (whose words hold the windows' low parts once the spectra are multiplied;
 // a square allots just those), and the carry scratch.
@@ -1658,6 +1730,8 @@ static uint64_t round256(uint64_t x) { return (x + 255) & ~255ull; }
 __host__ __device__ __forceinline__ uint64_t round_up_u64(uint64_t x, uint64_t m) { return (x + m - 1) / m * m; }
 static uint64_t scratch_bytes(uint64_t la, uint64_t lb, bool square) {
   Sizes z = sizes_for(la, lb);
+  const SegPlan sg = square ? SegPlan{} : plan_segments(la, lb);
+  if (sg.L) return ((uint64_t)(sg.S + 1) << sg.L) * 8 + round256(z.nwin * 16) + round256(carry_words(z.nwin) * 8);
   return round256(z.N * 8) + round256(square ? z.nwin * 16 : z.N * 8) + round256(carry_words(z.nwin) * 8);
 }
 static void carve_carry(Job& J, uint64_t* base, uint64_t nwin) {
@@ -1667,6 +1741,14 @@ static void carve_carry(Job& J, uint64_t* base, uint64_t nwin) {
 static void carve_scratch(Job& J, uint8_t* base, bool square) {
   Sizes z = sizes_for(J.la, J.lb);
   J.A = reinterpret_cast<uint64_t*>(base);
+  if (J.segments) {
+    const uint64_t N = J.segv + WIN_COEFFS * (uint64_t)J.wlo;
+    J.B = J.A + J.segments * N;
+    base += (J.segments + 1) * N * 8;
+    J.W = reinterpret_cast<uint64_t*>(base);
+    carve_carry(J, reinterpret_cast<uint64_t*>(base + round256(z.nwin * 16)), z.nwin);
+    return;
+  }
   base += round256(z.N * 8);
   J.W = reinterpret_cast<uint64_t*>(base);
   J.B = square ? nullptr : J.W;
@@ -1842,8 +1924,10 @@ static void tw_release_all() {
 // All launches of the large-product pipeline for `nj` products sharing the
 // transform length 2^L: the products come from the device array `jobs`
 // (blockIdx.y) or, for nj == 1 and jobs == nullptr, from `one`.
-// max_chunk: largest carry-chunk count among the products.
-static void run_large(const Launcher& X, const Job* jobs, const Job& one, uint32_t nj, int L, uint64_t max_chunk) {
+// nc: how many of them, from the first, have carries to run (the others are
+// addends and further segments); max_chunk: largest carry-chunk count among
+// those.
+static void run_large(const Launcher& X, const Job* jobs, const Job& one, uint32_t nj, int L, uint32_t nc, uint64_t max_chunk) {
   const Plan pl = make_plan(L);
   const PassTables tw = X.tables ? pass_tables(pl, X.st) : PassTables{};
   // 2^-L (2^192 = 1); 0 when the inverse first pass's table applies it
@@ -1871,20 +1955,20 @@ static void run_large(const Launcher& X, const Job* jobs, const Job& one, uint32
       KTimer kt(K_PASS_FWD, X.st, X.stats);
       PIMUL_DISPATCH_R(pl.r[p], {
         launch_pdl(k_col_mid<RR, true>, grid(ColGeom<RR>::TILE, nz), PASS_THREADS, ColGeom<RR>::XWORDS * 8, X.st, jobs, one,
-                   which, L - consumed, X.R, tw.mid_fwd[p]);
+                   which, L, L - consumed, X.R, tw.mid_fwd[p]);
       });
     }
     KTimer kt(K_PASS_FWD, X.st, X.stats);
     PIMUL_DISPATCH_R(rl, {
       launch_pdl(k_fwd_last<RR>, grid(RowGeom<RR>::TILE, nz), PASS_THREADS, 4 * RowGeom<RR>::XWORDS * 8, X.st, jobs, one, which,
-                 X.R);
+                 L, X.R);
     });
   }
   {
     KTimer kt(K_POINTWISE, X.st, X.stats);
     PIMUL_DISPATCH_R(rl, {
-      launch_pdl(k_inv_last<RR>, grid(RowGeom<RR>::TILE, 1), PASS_THREADS, 4 * RowGeom<RR>::XWORDS * 8, X.st, jobs, one, ninv,
-                 X.R);
+      launch_pdl(k_inv_last<RR>, grid(RowGeom<RR>::TILE, 1), PASS_THREADS, 4 * RowGeom<RR>::XWORDS * 8, X.st, jobs, one, L,
+                 ninv, X.R);
     });
   }
   int consumed = L - rl;
@@ -1893,8 +1977,8 @@ static void run_large(const Launcher& X, const Job* jobs, const Job& one, uint32
     consumed -= pl.r[p];
     KTimer kt(K_PASS_INV, X.st, X.stats);
     PIMUL_DISPATCH_R(pl.r[p], {
-      launch_pdl(k_col_mid<RR, false>, grid(ColGeom<RR>::TILE, 1), PASS_THREADS, ColGeom<RR>::XWORDS * 8, X.st, jobs, one, 0, S,
-                 X.R, tw.mid_inv[p]);
+      launch_pdl(k_col_mid<RR, false>, grid(ColGeom<RR>::TILE, 1), PASS_THREADS, ColGeom<RR>::XWORDS * 8, X.st, jobs, one, 0, L,
+                 S, X.R, tw.mid_inv[p]);
     });
   }
   {
@@ -1907,7 +1991,7 @@ static void run_large(const Launcher& X, const Job* jobs, const Job& one, uint32
   }
   {
     KTimer kt(K_CARRY, X.st, X.stats);
-    launch_pdl(k_carry, dim3((unsigned)max_chunk, nj), CARRY_THREADS, 0, X.st, jobs, one);
+    launch_pdl(k_carry, dim3((unsigned)max_chunk, nc), CARRY_THREADS, 0, X.st, jobs, one);
   }
 }
 
@@ -1937,9 +2021,19 @@ static int mul_device(const uint64_t* d_a, uint64_t la, const uint64_t* d_b, uin
   }
   Job J{};
   J.a = d_a, J.la = la, J.b = d_b, J.lb = lb, J.out = d_out;
+  const SegPlan sg = square ? SegPlan{} : plan_segments(la, lb);
+  if (sg.L) {
+    if (la < lb) {  // the long operand is cut; it must be there before the first pass
+      std::swap(J.a, J.b);
+      std::swap(J.la, J.lb);
+      if (b_ready) cudaStreamWaitEvent(st, b_ready, 0);
+      b_ready = nullptr;
+    }
+    J.segments = sg.S, J.segv = sg.segv, J.wlo = (uint32_t)sg.wlo;
+  }
   carve_scratch(J, base, square);
   Launcher X{st, true, R, b_ready};
-  run_large(X, nullptr, J, 1, z.L, z.nchunk);
+  run_large(X, nullptr, J, std::max(1u, sg.S), sg.L ? sg.L : z.L, 1, z.nchunk);
   cudaError_t le = cudaGetLastError();
   cudaFreeAsync(base, st);
   if (le != cudaSuccess) return fail(PIMUL_ECUDA, std::string("kernel launch: ") + cudaGetErrorString(le));
@@ -1979,6 +2073,7 @@ struct BatchLayout {
   struct Desc {
     uint32_t unit;
     bool second;             // the a2 b2 half of a sum (an addend)
+    uint32_t segment = 0;    // segment of a cut product
     uint32_t flags;          // JF_*
     int64_t owner = -1;      // descriptor whose B this one borrows
     int64_t addend = -1;     // descriptor whose A holds this one's X
@@ -1988,12 +2083,14 @@ struct BatchLayout {
   std::vector<Desc> desc;  // large descriptors in launch order
   struct Bucket {
     int L;
-    size_t d0, nd;
+    size_t d0, nd;    // descriptors
+    size_t nc;        // of which the first nc have carries to run
     uint64_t max_chunk;
   };
   std::vector<Bucket> large;
   uint64_t arena_bytes = 0;
   int small_L = 0;  // largest L among the small jobs
+  std::vector<SegPlan> seg;  // per unit: how a product of a long by a short operand is cut
   std::vector<SmallChunk> chunks;  // the small jobs in same-length chunks
   size_t small_smem = 0;           // dynamic shared memory of their CTAs
 };
@@ -2021,6 +2118,24 @@ static int layout_batch(const Unit* units, size_t n, BatchLayout& B, bool share)
   for (size_t i = 0; i < n; i++) {
     Ls[i] = unit_log_n(units[i]);
     if (Ls[i] > 32) return fail(PIMUL_EINVAL, "transform length above 2^32 in batch");
+  }
+  // uneven products are cut into segments, unless others share their b (a
+  // shared spectrum saves more)
+  B.seg.assign(n, SegPlan{});
+  {
+    std::unordered_map<const uint64_t*, uint32_t> uses;
+    if (share)
+      for (size_t i = 0; i < n; i++)
+        if (Ls[i] > SMALL_LOG_MAX) {
+          uses[units[i].b]++;
+          if (units[i].la2) uses[units[i].b2]++;
+        }
+    for (size_t i = 0; i < n; i++) {
+      const Unit& u = units[i];
+      if (Ls[i] <= SMALL_LOG_MAX || u.la2 || u.coeff || u.forceL || (share && uses[u.b] > 1)) continue;
+      B.seg[i] = plan_segments(u.la, u.lb);
+      if (B.seg[i].L) Ls[i] = B.seg[i].L;
+    }
   }
   std::vector<std::vector<uint32_t>> byL(33);
   for (size_t i = 0; i < n; i++) {
@@ -2055,41 +2170,56 @@ static int layout_batch(const Unit* units, size_t n, BatchLayout& B, bool share)
     const uint64_t N = 1ull << L;
     size_t s = 0;
     while (s < byL[L].size()) {
-      BatchLayout::Bucket bk{L, B.desc.size(), 0, 0};
+      BatchLayout::Bucket bk{L, B.desc.size(), 0, 0, 0};
       // the group's units: descriptor count and a scratch bound (no sharing)
       uint64_t bound = 0;
       size_t e = s;
       for (; e < byL[L].size(); e++) {
         const Unit& u = units[byL[L][e]];
-        const size_t nd = u.la2 ? 2 : 1;
+        const SegPlan& sg = B.seg[byL[L][e]];
+        const size_t nd = u.la2 ? 2 : sg.L ? sg.S : 1;
         const uint64_t nwin = n_windows_out(u.nout);
-        const uint64_t need = round256(N * 8) * 2 * nd + round256(nwin * 16) + round256(carry_words(nwin) * 8);
+        const uint64_t need = round256(N * 8) * (sg.L ? nd + 1 : 2 * nd) + round256(nwin * 16) + round256(carry_words(nwin) * 8);
         if (e > s && (bk.nd + nd > 65535 || bound + need > BATCH_ARENA_CAP)) break;
         bk.nd += nd;
         bound += need;
       }
-      // descriptors; the first of several with the same b owns its spectrum
+      // descriptors, those with carries first; the first of several with the
+      // same b owns its spectrum, a product's first segment that of the others
       std::unordered_map<const uint64_t*, std::vector<size_t>> by_b;
+      bk.nc = e - s;
+      for (size_t k = s; k < e; k++) {
+        const Unit& u = units[byL[L][k]];
+        BatchLayout::Desc d1;
+        d1.unit = byL[L][k];
+        d1.second = false;
+        d1.flags = 0;
+        d1.lent = B.seg[d1.unit].S > 1;
+        const bool sq1 = u.a == u.b && u.la == u.lb;
+        if (share && !sq1 && !B.seg[d1.unit].L) by_b[u.b].push_back(B.desc.size());
+        B.desc.push_back(d1);
+      }
       for (size_t k = s; k < e; k++) {
         const uint32_t ui = byL[L][k];
         const Unit& u = units[ui];
-        BatchLayout::Desc d1;
-        d1.unit = ui;
-        d1.second = false;
-        d1.flags = 0;
-        B.desc.push_back(d1);
-        const size_t i1 = B.desc.size() - 1;
-        const bool sq1 = u.a == u.b && u.la == u.lb;
-        if (share && !sq1) by_b[u.b].push_back(i1);
+        const size_t i1 = bk.d0 + (k - s);
         if (u.la2) {
           BatchLayout::Desc d2;
           d2.unit = ui;
           d2.second = true;
           d2.flags = JF_ADDEND;
+          B.desc[i1].addend = (int64_t)B.desc.size();
+          if (share) by_b[u.b2].push_back(B.desc.size());
           B.desc.push_back(d2);
-          const size_t i2 = B.desc.size() - 1;
-          B.desc[i1].addend = (int64_t)i2;
-          if (share) by_b[u.b2].push_back(i2);
+        }
+        for (uint32_t g = 1; g < B.seg[ui].S; g++) {
+          BatchLayout::Desc d2;
+          d2.unit = ui;
+          d2.second = false;
+          d2.segment = g;
+          d2.flags = JF_SEGMENT | JF_B_SHARED;
+          d2.owner = (int64_t)i1;
+          B.desc.push_back(d2);
         }
       }
       for (auto& kv : by_b) {
@@ -2121,7 +2251,7 @@ static int layout_batch(const Unit* units, size_t n, BatchLayout& B, bool share)
           d.off_b = off;
           off += round256(N * 8);
         }
-        if (!d.second) {
+        if (!d.second && !d.segment) {
           const uint64_t nwin = n_windows_out(u.nout);
           // the windows' low parts go to B where the product has one to itself
           d.off_w = d.off_b;
@@ -2171,6 +2301,15 @@ static void fill_descriptors(const Unit* units, const BatchLayout& B, uint8_t* a
       J.low = u.low;
       J.wrap = u.wrap;
     }
+    const SegPlan& sg = B.seg[d.unit];
+    if (sg.L) {
+      if (u.la < u.lb) {  // the long operand is the one that is cut
+        std::swap(J.a, J.b);
+        std::swap(J.la, J.lb);
+      }
+      J.segv = sg.segv, J.wlo = (uint32_t)sg.wlo;
+      to_segment(J, d.segment, 0);  // (A comes from the arena below)
+    }
     J.flags = d.flags | (!d.second && u.coeff ? JF_COEFF : 0);
     const bool sq = !d.second && u.a == u.b && u.la == u.lb;
     J.A = reinterpret_cast<uint64_t*>(arena + d.off_a);
@@ -2179,8 +2318,9 @@ static void fill_descriptors(const Unit* units, const BatchLayout& B, uint8_t* a
     else
       J.B = sq ? nullptr : reinterpret_cast<uint64_t*>(arena + d.off_b);
     if (!d.second) {
-      J.W = reinterpret_cast<uint64_t*>(arena + d.off_w);
-      carve_carry(J, reinterpret_cast<uint64_t*>(arena + d.off_h), n_windows_out(u.nout));
+      const BatchLayout::Desc& first = d.segment ? B.desc[d.owner] : d;  // a segment writes its product's windows
+      J.W = reinterpret_cast<uint64_t*>(arena + first.off_w);
+      carve_carry(J, reinterpret_cast<uint64_t*>(arena + first.off_h), n_windows_out(u.nout));
     }
     if (d.addend >= 0) {
       const BatchLayout::Desc& x = B.desc[d.addend];
@@ -2204,7 +2344,7 @@ static void launch_batch(const Launcher& X, const BatchLayout& B, const SmallJob
                                                                       (uint32_t)B.chunks.size(), X.R);
   }
   for (const auto& bk : B.large)
-    run_large(X, d_large + bk.d0, Job{}, (uint32_t)bk.nd, bk.L, bk.max_chunk);
+    run_large(X, d_large + bk.d0, Job{}, (uint32_t)bk.nd, bk.L, (uint32_t)bk.nc, bk.max_chunk);
 }
 
 // The calling thread's buffer for a batch's host descriptor image, kept and
@@ -2302,10 +2442,7 @@ static int plan_create(const size_t* la, const size_t* lb, size_t n, BatchPlan**
   if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&cs, cudaStreamNonBlocking);
   if (e == cudaSuccess) {
     // twiddle tables are never built inside a capture: build them first
-    for (size_t i = 0; i < n; i++) {
-      const int L = log2_ceil(4 * (uint64_t)la[i] + 4 * (uint64_t)lb[i] - 1);
-      if (la[i] && lb[i] && L > SMALL_LOG_MAX) pass_tables(make_plan(L), nullptr);
-    }
+    for (const auto& bk : P->B.large) pass_tables(make_plan(bk.L), nullptr);
     uint8_t* desc = P->dev + round256(P->B.arena_bytes);
     e = cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal);
     if (e == cudaSuccess) {
@@ -3921,7 +4058,7 @@ static int mul_device_noalloc(const uint64_t* d_a, uint64_t la, const uint64_t* 
   carve_carry(J, nd->scratch + 2 * NOALLOC_N_MAX, z.nwin);
   Launcher X{st, false, R};  // no statistics hook: its event timing would create CUDA events
   X.tables = false;          // nor the twiddle tables, which are allocated on first use
-  run_large(X, nullptr, J, 1, z.L, z.nchunk);
+  run_large(X, nullptr, J, 1, z.L, 1, z.nchunk);
   CU(cudaGetLastError());
   return PIMUL_OK;
 }
