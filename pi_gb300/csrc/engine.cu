@@ -579,6 +579,43 @@ __device__ __forceinline__ Win fold16(const uint64_t* c16, int stride) {
 // the chunk states (the low parts lie in an array of 2 nwin words of their own).
 __host__ __device__ __forceinline__ uint64_t carry_words(uint64_t nwin) { return nwin + (n_chunks(nwin) + 1) / 2; }
 
+// The eight canonical coefficients c of window wl of a 2^L-point transform: the
+// window's low limbs go to W and its high part to H (coefficients out for
+// JF_COEFF, both windows that fall on it for a wrapped product).
+__device__ __forceinline__ void put_window(const Job& J, int L, uint64_t wl, uint64_t* c) {
+  if (wl < J.wlo) return;
+  const uint64_t nlimbs = job_nout(J), nwin = n_windows_out(nlimbs);
+  const uint64_t w = wl + (uint64_t)J.woff;  // window of the whole product
+  ulonglong2* W = reinterpret_cast<ulonglong2*>(J.W);
+  if (J.flags & JF_COEFF) {
+#pragma unroll
+    for (int t = 0; t < 8; t++)
+      if (8 * w + t < nlimbs) J.out[8 * w + t] = c[t];
+    return;
+  }
+  if (w >= nwin) return;
+  if (J.wrap) {
+    // coefficient 8w + t: low[8w + t] below wrap; N + 8w + t: the rest of the cyclic value
+    uint64_t d[8];
+#pragma unroll
+    for (int t = 0; t < 8; t++) {
+      const uint64_t pos = 8 * w + t;
+      const uint64_t lo = pos < J.wrap ? J.low[pos] : c[t];
+      d[t] = c[t] - lo;
+      c[t] = lo;
+    }
+    const uint64_t w2 = w + ((1ull << L) >> 3);
+    if (w2 < nwin) {
+      const Win2 v2 = fold8(d);
+      W[w2] = make_ulonglong2(v2.l[0], v2.l[1]);
+      J.H[w2] = v2.hi;
+    }
+  }
+  const Win2 v = fold8(c);
+  W[w] = make_ulonglong2(v.l[0], v.l[1]);
+  J.H[w] = v.hi;
+}
+
 // Inverse pass 0 (natural order out) fused with the window fold: each tile
 // row holds 2^T consecutive coefficients = 2^(T-3) windows; every window
 // writes its low 2 limbs to W and its high part to H.
@@ -596,9 +633,6 @@ __global__ void __launch_bounds__(PASS_THREADS, pass_min_ctas(R)) k_inv_first_ca
   const Job J = job_of(jobs, one, L);
   if (J.flags & JF_ADDEND) return;
   const uint64_t* __restrict__ data = J.A;
-  uint64_t* __restrict__ H = J.H;
-  ulonglong2* __restrict__ W = reinterpret_cast<ulonglong2*>(J.W);
-  const uint64_t nlimbs = job_nout(J), nwin = n_windows_out(nlimbs);
   extern __shared__ uint64_t sm[];
   const int tid = threadIdx.x;
   const int S = L - R;
@@ -648,44 +682,13 @@ __global__ void __launch_bounds__(PASS_THREADS, pass_min_ctas(R)) k_inv_first_ca
     for (int m = 0; m < (1 << B1); m++) sm[((tid >> T) + (m << B2)) * RS + (tid & G::TM)] = gl::canon(v[m]);
   }
   __syncthreads();
-  const bool coeff = (J.flags & JF_COEFF) != 0;
-  const uint64_t wtop = (1ull << L) >> 3;  // a wrapped product's windows past the transform: w + wtop
   for (uint32_t q = tid; q < (1u << (G::TILE - 3)); q += PASS_THREADS) {
     const uint32_t i = q >> (T - 3), k = q & ((1u << (T - 3)) - 1);
-    const uint64_t wl = ((((uint64_t)i << S) + j0) >> 3) + k;
-    if (wl < J.wlo) continue;
-    const uint64_t w = wl + (uint64_t)J.woff;  // window of the whole product
     uint64_t c[8];
     const uint64_t* row = sm + i * RS + 8 * k;
 #pragma unroll
     for (int t = 0; t < 8; t++) c[t] = row[t];
-    if (coeff) {
-#pragma unroll
-      for (int t = 0; t < 8; t++)
-        if (8 * w + t < nlimbs) J.out[8 * w + t] = c[t];
-      continue;
-    }
-    if (w >= nwin) continue;
-    if (J.wrap) {
-      // coefficient 8w + t: low[8w + t] below wrap; N + 8w + t: the rest of the cyclic value
-      uint64_t d[8];
-#pragma unroll
-      for (int t = 0; t < 8; t++) {
-        const uint64_t pos = 8 * w + t;
-        const uint64_t lo = pos < J.wrap ? J.low[pos] : c[t];
-        d[t] = c[t] - lo;
-        c[t] = lo;
-      }
-      const uint64_t w2 = w + wtop;
-      if (w2 < nwin) {
-        const Win2 v2 = fold8(d);
-        W[w2] = make_ulonglong2(v2.l[0], v2.l[1]);
-        H[w2] = v2.hi;
-      }
-    }
-    const Win2 v = fold8(c);
-    W[w] = make_ulonglong2(v.l[0], v.l[1]);
-    H[w] = v.hi;
+    put_window(J, L, ((((uint64_t)i << S) + j0) >> 3) + k, c);
   }
 }
 
@@ -817,11 +820,47 @@ __global__ void __launch_bounds__(CARRY_THREADS) k_carry(const Job* jobs, Job on
 }
 
 // ---- whole multiply in one CTA (N <= 2^SMALL_LOG_MAX) --------------------
+// Products of up to 64 limbs in all are schoolbook column sums by one warp
+// (class 7); longer ones take three transforms of 2^c points (class c = 8 ..
+// 12) as two or three rounds of radix 8 or 16 in registers.  A lone product
+// (and class 8, one warp) holds operands a and b side by side in the halves of
+// its threads: one SM is all it has, and a thread's instructions are its time.
+// In a batch a group of G threads transforms one operand after the other, two
+// CTAs per SM, so that no thread idles through the inverse and other groups
+// run while one waits.  Lone products: 10.3 -> 6.2 us at 2^10 bits, 18.0 -> 7.7 at
+// 100 x 100 limbs.
 constexpr int SMALL_THREADS = 256;
 constexpr int SMALL_LOG_MAX = 12;
+constexpr int SMALL_TINY = 7;        // class of the one-warp products
+constexpr uint64_t TINY_LIMBS = 64;  // la + lb
 
-// Dynamic shared memory of the one-CTA multiply for N = 2^L (two padded arrays).
-__host__ __device__ __forceinline__ size_t small_smem_bytes(int L) { return 2 * (((size_t)1 << L) * 17 / 16) * 8; }
+// Radix (log2) of round q of a class-c transform (0: no such round).
+__host__ __device__ constexpr int small_b(int c, int q) {
+  return c == 8 ? (q < 2 ? 4 : 0) : c == 9 ? 3 : c == 10 ? (q == 0 ? 4 : 3) : c == 11 ? (q < 2 ? 4 : 3) : 4;
+}
+// Threads per operand: one radix-16 item (8 for class 9) each; per product.
+__host__ __device__ constexpr int small_op_threads(int c) { return c == 9 ? 64 : (1 << c) / 16; }
+__host__ __device__ constexpr int small_threads(int c, bool split) {
+  return c == SMALL_TINY ? 32 : (split ? 2 : 1) * small_op_threads(c);
+}
+__host__ __device__ constexpr bool small_split(int c) { return c <= 8; }  // in a batch
+// Class of a product of la + lb limbs.
+__host__ __device__ __forceinline__ int small_class(uint64_t la, uint64_t lb) {
+  if (la + lb <= TINY_LIMBS) return SMALL_TINY;
+  const uint32_t n = (uint32_t)(4 * (la + lb) - 1);
+  return n <= 256 ? 8 : n <= 512 ? 9 : n <= 1024 ? 10 : n <= 2048 ? 11 : 12;
+}
+// Dynamic shared memory words of one product: a padded array per operand held
+// at a time, and the windows' high parts (a tiny product: its operands, 64 zero
+// limbs on either side of the longer).
+__host__ __device__ constexpr uint32_t small_words(int c, bool split) {
+  return c == SMALL_TINY ? 256 : split ? 2 * spad(1u << c) : spad(1u << c) + (1u << c) / 16;
+}
+// Products of one class side by side in a batch CTA, and its shared memory.
+__host__ __device__ __forceinline__ uint32_t small_per_cta(int c) { return SMALL_THREADS / small_threads(c, small_split(c)); }
+__host__ __device__ __forceinline__ size_t small_cta_smem(int c) {
+  return (size_t)small_per_cta(c) * small_words(c, small_split(c)) * 8;
+}
 
 struct SmallJob {
   const uint64_t* a;
@@ -830,22 +869,10 @@ struct SmallJob {
   uint32_t la, lb;
 };
 
-// Threads per product: an eighth of the transform length (one radix-8
-// butterfly per thread and round), at least a warp; SMALL_THREADS / G
-// products of one length run side by side in a CTA.
-__host__ __device__ __forceinline__ int small_group_threads(int L) {
-  const int g = (1 << L) / 8;
-  return g < 32 ? 32 : (g > SMALL_THREADS ? SMALL_THREADS : g);
-}
-// Dynamic shared memory of a CTA running products of length 2^L.
-__host__ __device__ __forceinline__ size_t small_cta_smem(int L) {
-  return (size_t)(SMALL_THREADS / small_group_threads(L)) * small_smem_bytes(L);
-}
-
-// count (<= SMALL_THREADS / G(L)) consecutive jobs of length 2^L from first.
+// count (<= small_per_cta) consecutive jobs of class c from first.
 struct SmallChunk {
   uint32_t first, count;
-  int L;
+  int c;
 };
 
 // Forward (or unscaled inverse) transforms of NA arrays of 2^L words by a
@@ -877,82 +904,212 @@ __device__ __forceinline__ void group_inv_c(uint64_t* a0, const uint64_t* tw, in
   }
 }
 
-// One product by the G threads of a group (gtid = thread in the group, gw0
-// = the CTA-wide index of the group's first warp).  Inactive groups run
-// every barrier and ballot with no work, so a CTA's groups stay in step.
-__device__ void small_multiply(const SmallJob& job, bool active, int L, const Roots& R, uint64_t* smA, uint64_t* smB,
-                               int gtid, int G, int gw0) {
-  const int tid = threadIdx.x;
-  const uint32_t la = active ? job.la : 0, lb = active ? job.lb : 0;
-  const uint32_t N = 1u << L;
-  const uint32_t n_out = active ? 4 * la + 4 * lb - 1 : 0;
-  const bool square = active && job.a == job.b && la == lb;
-  // one limb per thread and step -> its four 16-bit coefficients
-  for (uint32_t l = gtid; active && l < N / 4; l += G) {
-    const uint64_t xa = l < la ? job.a[l] : 0;
+// Barrier of a product's T threads (group grp of the CTA).
+template <int T>
+__device__ __forceinline__ void small_sync(int grp) {
+  if constexpr (T == 32)
+    __syncwarp();
+  else
+    asm volatile("bar.sync %0, %1;" ::"r"(grp + 1), "n"(T) : "memory");
+}
+
+// Forward transform of an operand of nc coefficients by G threads (u) of a
+// group of T (all of which pass the barriers; run = false: nothing else).
+// After the rounds of radix 2^B1, 2^B2, 2^B3, element (k1, k2, k3) of the
+// spectrum has index (k1 2^B2 + k2) 2^B3 + k3; thread u ends up with items it G
+// + u of the last round in s.  A round's twiddles w^(k j) enter the next
+// round's inputs as lazy products, from the table of 4096th roots.
+template <int C, int T>
+__device__ __forceinline__ void small_forward(const uint64_t* limbs, uint32_t nc, const Roots& R, uint64_t* sm, int u, int grp,
+                                              bool run, uint64_t* s) {
+  constexpr int B1 = small_b(C, 0), B2 = small_b(C, 1), B3 = small_b(C, 2);
+  constexpr int G = small_op_threads(C);
+  constexpr int S1 = C - B1, S2 = S1 - B2;  // log2 sub-problem sizes after rounds 1 and 2
+  static_assert(S2 == B3, "the rounds make up the transform");
+  if (run) {
+    // round 1: coefficients m 2^S1 + j
+    const uint16_t* coef = reinterpret_cast<const uint16_t*>(limbs);
 #pragma unroll
-    for (int q = 0; q < 4; q++) smA[spad(4 * l + q)] = (xa >> (16 * q)) & 0xFFFF;
-    if (!square) {
-      const uint64_t xb = l < lb ? job.b[l] : 0;
+    for (int it = 0; it < (1 << S1) / G; it++) {
+      const uint32_t j = it * G + u;
+      uint64_t v[1 << B1];
+      gl::Lz x[1 << B1];
 #pragma unroll
-      for (int q = 0; q < 4; q++) smB[spad(4 * l + q)] = (xb >> (16 * q)) & 0xFFFF;
+      for (int m = 0; m < (1 << B1); m++) {
+        const uint32_t n = (m << S1) + j;
+        x[m] = gl::Lz{n < nc ? (uint32_t)coef[n] : 0u, 0u, 0};
+      }
+      x[0] = gl::lz_bias(x[0]);
+      dft_lz<B1, false>(x, v);
+#pragma unroll
+      for (int k = 0; k < (1 << B1); k++) sm[spad((k << S1) + j)] = v[k];
     }
   }
-  __syncthreads();
-  TileGeom g{L, 0, 0};
-  const int rt = active ? gtid : (1 << 30);  // an inactive group's rounds do no work
-  tile_dft_fwd(smA, g, R, rt, G);
-  tile_dft_fwd(smB, g, R, square ? (1 << 30) : rt, G);
-  // times N^-1 = 2^(-L): with 2^96 = -1 and 2^64 = 2^32 - 1 (mod p),
-  // 2^(-L) = -2^(96-L) = p - (2^(64-L) - 2^(32-L)) for 1 <= L <= 32
-  const uint64_t ninv = gl::P - ((1ull << (64 - L)) - (1ull << (32 - L)));
-  for (uint32_t i = gtid; active && i < N; i += G) {
-    uint64_t x = smA[spad(i)];
-    uint64_t y = square ? x : smB[spad(i)];
-    smA[spad(i)] = gl::mul(gl::mul(x, y), ninv);
+  small_sync<T>(grp);
+  constexpr int BL = B3 ? B3 : B2;             // last round
+  constexpr int ITL = (1 << (C - BL)) / G;     // its items per thread
+  if constexpr (B3 > 0) {
+    if (run) {
+      // round 2: (k1, j2), inputs j = m 2^S2 + j2 with twiddles w_N^(k1 j)
+#pragma unroll
+      for (int it = 0; it < (1 << (C - B2)) / G; it++) {
+        const uint32_t w = it * G + u, j2 = w & ((1u << S2) - 1), k1 = w >> S2;
+        const uint32_t base = (k1 << S1) + j2;
+        uint64_t v[1 << B2];
+        gl::Lz x[1 << B2];
+#pragma unroll
+        for (int m = 0; m < (1 << B2); m++)
+          x[m] = gl::lz_mul(sm[spad(base + (m << S2))], __ldg(R.w12 + ((k1 * (j2 + (m << S2))) << (12 - C))));
+        x[0] = gl::lz_bias(x[0]);
+        dft_lz<B2, false>(x, v);
+#pragma unroll
+        for (int k = 0; k < (1 << B2); k++) sm[spad(base + (k << S2))] = v[k];
+      }
+    }
+    small_sync<T>(grp);
   }
-  __syncthreads();
-  tile_dft_inv(smA, g, R, rt, G);
-  // carry: windows of 16 coefficients, one per thread (N/16 <= G)
-  const uint32_t nwin = (n_out + 15) / 16, nl = la + lb;
-  uint64_t* sH = smB;  // reuse: B no longer needed
-  __shared__ uint32_t sA[SMALL_THREADS / 32], sBm[SMALL_THREADS / 32];
+  if (run) {
+    // last round: (k1, k2) with twiddles w_(2^S1)^(k2 m), or k1 with w_N^(k1 m)
+    constexpr int mlog = B3 ? S1 : C;
+    constexpr uint32_t kmask = (1u << (B3 ? B2 : B1)) - 1;
+#pragma unroll
+    for (int it = 0; it < ITL; it++) {
+      const uint32_t w = it * G + u, k = w & kmask;
+      gl::Lz x[1 << BL];
+      x[0] = gl::lz_bias(gl::lz(sm[spad(w << BL)]));
+#pragma unroll
+      for (int m = 1; m < (1 << BL); m++)
+        x[m] = gl::lz_mul(sm[spad((w << BL) + m)], __ldg(R.w12 + ((k * m) << (12 - mlog))));
+      dft_lz<BL, false>(x, s + (it << BL));
+    }
+  }
+}
+
+// One product by its T threads (t = thread in the group, grp = group of the
+// CTA).  SPLIT: threads 0 .. G - 1 hold operand a, the others b.
+template <int C, bool SPLIT>
+__device__ __forceinline__ void small_multiply(const SmallJob& job, const Roots& R, uint64_t* smA, int t, int grp, uint32_t* sA,
+                                               uint32_t* sBm) {
+  constexpr int B1 = small_b(C, 0), B2 = small_b(C, 1), B3 = small_b(C, 2);
+  constexpr int G = small_op_threads(C), T = small_threads(C, SPLIT);
+  constexpr int S1 = C - B1, S2 = S1 - B2, BL = B3 ? B3 : B2, ITL = (1 << (C - BL)) / G;
+  constexpr uint32_t N = 1u << C;
+  uint64_t* smB = smA + spad(N);  // b's array (SPLIT); the windows' high parts
+  const uint32_t la = job.la, lb = job.lb;
+  const bool square = job.a == job.b && la == lb;
+  // times N^-1 = 2^(-C): with 2^96 = -1 and 2^64 = 2^32 - 1 (mod p),
+  // 2^(-C) = -2^(96-C) = p - (2^(64-C) - 2^(32-C))
+  constexpr uint64_t ninv = gl::P - ((1ull << (64 - C)) - (1ull << (32 - C)));
+  uint64_t s[ITL << BL], y[SPLIT ? 1 : ITL << BL];
+  const bool isb = SPLIT && t >= G;
+  if constexpr (SPLIT) {
+    const bool idle = isb && square;
+    uint64_t* sm = isb ? smB : smA;
+    small_forward<C, T>(isb ? job.b : job.a, 4 * (isb ? lb : la), R, sm, isb ? t - G : t, grp, !idle, s);
+    // b's spectrum to the threads that hold a's
+    if (isb && !idle) {
+#pragma unroll
+      for (int it = 0; it < ITL; it++)
+#pragma unroll
+        for (int k = 0; k < (1 << BL); k++) sm[spad(((it * G + t - G) << BL) + k)] = gl::mul(s[(it << BL) + k], ninv);
+    }
+    small_sync<T>(grp);
+  } else {
+    small_forward<C, T>(job.a, 4 * la, R, smA, t, grp, true, s);
+    if (square) {
+#pragma unroll
+      for (int k = 0; k < (ITL << BL); k++) y[k] = s[k];
+    } else {
+      small_sync<T>(grp);
+      small_forward<C, T>(job.b, 4 * lb, R, smA, t, grp, true, y);
+    }
+    // (a thread overwrites below what it alone has read)
+  }
+  if (!isb) {
+#pragma unroll
+    for (int it = 0; it < ITL; it++) {
+      const uint32_t base = (it * G + t) << BL;
+      uint64_t v[1 << BL];
+      gl::Lz x[1 << BL];
+#pragma unroll
+      for (int k = 0; k < (1 << BL); k++) {
+        const int i = (it << BL) + k;
+        const uint64_t z = !SPLIT ? gl::mul(y[SPLIT ? 0 : i], ninv) : square ? gl::mul(s[i], ninv) : smB[spad(base + k)];
+        x[k] = gl::lz_mul(s[i], z);
+      }
+      x[0] = gl::lz_bias(x[0]);
+      dft_lz<BL, true>(x, v);
+#pragma unroll
+      for (int m = 0; m < (1 << BL); m++) smA[spad(base + m)] = v[m];
+    }
+  }
+  small_sync<T>(grp);
+  // the other inverse rounds run on all T threads
+  if constexpr (B3 > 0) {
+    for (uint32_t w = t; w < (1u << (C - B2)); w += T) {
+      const uint32_t j2 = w & ((1u << S2) - 1), k1 = w >> S2, base = (k1 << S1) + j2;
+      uint64_t v[1 << B2];
+      gl::Lz x[1 << B2];
+      x[0] = gl::lz_bias(gl::lz(smA[spad(base)]));
+#pragma unroll
+      for (int k = 1; k < (1 << B2); k++)
+        x[k] = gl::lz_mul(smA[spad(base + (k << S2))], __ldg(R.w12 + ((4096 - ((k * j2) << (12 - S1))) & 4095)));
+      dft_lz<B2, true>(x, v);
+#pragma unroll
+      for (int m = 0; m < (1 << B2); m++) smA[spad(base + (m << S2))] = v[m];
+    }
+    small_sync<T>(grp);
+  }
+  for (uint32_t j = t; j < (1u << S1); j += T) {
+    uint64_t v[1 << B1];
+    gl::Lz x[1 << B1];
+    x[0] = gl::lz_bias(gl::lz(smA[spad(j)]));
+#pragma unroll
+    for (int k = 1; k < (1 << B1); k++)
+      x[k] = gl::lz_mul(smA[spad((k << S1) + j)], __ldg(R.w12 + ((4096 - ((k * j) << (12 - C))) & 4095)));
+    dft_lz<B1, true>(x, v);
+#pragma unroll
+    for (int m = 0; m < (1 << B1); m++) smA[spad((m << S1) + j)] = v[m];
+  }
+  small_sync<T>(grp);
+  // carry: windows of 16 coefficients, one per thread (N/16 <= T)
+  const uint32_t n_out = 4 * la + 4 * lb - 1, nwin = (n_out + 15) / 16, nl = la + lb;
+  uint64_t* sH = smB;  // b's spectrum is no longer needed
   Win v{{0, 0, 0, 0}, 0};
-  const uint32_t w = gtid;
+  const uint32_t w = t;
   if (w < nwin) {
     uint64_t c[16];
 #pragma unroll
-    for (int t = 0; t < 16; t++) {
-      uint32_t idx = 16 * w + t;
-      c[t] = idx < N ? gl::canon(smA[spad(idx)]) : 0;
-    }
+    for (int q = 0; q < 16; q++) c[q] = gl::canon(smA[spad(16 * w + q)]);
     v = fold16(c, 1);
+    sH[w] = v.hi;  // nwin <= N/16 words
   }
-  __syncthreads();
-  if (w < nwin) sH[w] = v.hi;  // nwin <= N/16 words fit in the B region
-  __syncthreads();
-  uint64_t hprev = (w > 0 && w - 1 < nwin) ? sH[w - 1] : 0;
+  small_sync<T>(grp);
+  const uint64_t hprev = (w > 0 && w < nwin) ? sH[w - 1] : 0;
   uint64_t s0 = v.l[0] + hprev;
   uint64_t c = s0 < hprev;
   uint64_t s1 = v.l[1] + c;  c = c && s1 == 0;
   uint64_t s2 = v.l[2] + c;  c = c && s2 == 0;
   uint64_t s3 = v.l[3] + c;  c = c && s3 == 0;
-  bool gg = w < nwin && c;
-  bool pp = w < nwin && (s0 & s1 & s2 & s3) == ~0ull;
-  uint32_t A = __ballot_sync(0xFFFFFFFFu, gg || pp), Bm = __ballot_sync(0xFFFFFFFFu, gg);
-  if ((tid & 31) == 0) { sA[tid >> 5] = A; sBm[tid >> 5] = Bm; }
-  __syncthreads();
+  const bool gg = w < nwin && c;
+  const bool pp = w < nwin && (s0 & s1 & s2 & s3) == ~0ull;
+  const uint32_t A = __ballot_sync(0xFFFFFFFFu, gg || pp), Bm = __ballot_sync(0xFFFFFFFFu, gg);
   uint32_t cin = 0;
-  for (int k = gw0; k < (tid >> 5); k++) {
-    uint64_t s = (uint64_t)sA[k] + sBm[k] + cin;
-    cin = (uint32_t)(s >> 32);
+  if constexpr (T > 32) {
+    const int gw0 = grp * (T / 32), gw = gw0 + (t >> 5);
+    if ((t & 31) == 0) sA[gw] = A, sBm[gw] = Bm;
+    small_sync<T>(grp);
+    for (int k = gw0; k < gw; k++) {
+      const uint64_t x = (uint64_t)sA[k] + sBm[k] + cin;
+      cin = (uint32_t)(x >> 32);
+    }
   }
-  uint32_t carries = (A + Bm + cin) ^ A ^ Bm;
-  if ((carries >> (tid & 31)) & 1) {
+  const uint32_t carries = (A + Bm + cin) ^ A ^ Bm;
+  if ((carries >> (t & 31)) & 1) {
     if (++s0 == 0) if (++s1 == 0) if (++s2 == 0) ++s3;
   }
   if (w < nwin) {
-    uint32_t base = 4 * w;
+    const uint32_t base = 4 * w;
     if (base + 0 < nl) job.out[base + 0] = s0;
     if (base + 1 < nl) job.out[base + 1] = s1;
     if (base + 2 < nl) job.out[base + 2] = s2;
@@ -960,30 +1117,351 @@ __device__ void small_multiply(const SmallJob& job, bool active, int L, const Ro
   }
 }
 
-// Chunks of same-length products; with device lists the CTAs stride over
-// the chunks (a persistent kernel over a size-sorted batch).  jobs ==
-// nullptr: the single product `one`.
-__global__ void __launch_bounds__(SMALL_THREADS, 4) k_small_mul(const SmallJob* jobs, const SmallChunk* chunks,
-                                                               SmallJob one, uint32_t nchunks, Roots R) {
+// (x2 x1 x0) += a * b, 192 bits.
+__device__ __forceinline__ void mac192(uint64_t a, uint64_t b, uint64_t& x0, uint64_t& x1, uint64_t& x2) {
+  const uint64_t lo = a * b, hi = __umul64hi(a, b);
+  asm("add.cc.u64 %0, %0, %3;\n\taddc.cc.u64 %1, %1, %4;\n\taddc.u64 %2, %2, 0;"
+      : "+l"(x0), "+l"(x1), "+l"(x2)
+      : "l"(lo), "l"(hi));
+}
+
+// la + lb <= 64 by one warp: lane w sums the columns 2w and 2w + 1 over the
+// shorter operand's limbs (the longer one lies between zeros in shared memory)
+// and resolves its window's carry with the warp's ballots.
+__device__ void tiny_multiply(const SmallJob& job, uint64_t* sm, int lane) {
+  const bool sw = job.lb > job.la;
+  const uint64_t* a = sw ? job.b : job.a;  // the longer
+  const uint64_t* b = sw ? job.a : job.b;
+  const uint32_t la = sw ? job.lb : job.la, lb = sw ? job.la : job.lb, nl = la + lb;
+  uint64_t* sa = sm + 64;   // 64 zeros, a, zeros up to 192 words
+  uint64_t* sb = sm + 192;  // b: at most 32 words
+#pragma unroll
+  for (int q = 0; q < 6; q++) {
+    const uint32_t i = q * 32 + lane;
+    sm[i] = i >= 64 && i - 64 < la ? a[i - 64] : 0;
+  }
+  if ((uint32_t)lane < lb) sb[lane] = b[lane];
+  __syncwarp();
+  uint64_t e0 = 0, e1 = 0, e2 = 0, o0 = 0, o1 = 0, o2 = 0;
+  const uint64_t* col = sa + 2 * lane;
+  for (uint32_t i = 0; i < lb; i++) {
+    const uint64_t y = sb[i];
+    mac192(col[-(int)i], y, e0, e1, e2);
+    mac192(col[1 - (int)i], y, o0, o1, o2);
+  }
+  // window value e + o 2^64: low 128 bits here, high 128 bits to the next lane
+  const uint64_t l1 = e1 + o0;
+  uint64_t h0 = e2 + (l1 < o0);
+  uint64_t h1 = o2;
+  h0 += o1;
+  h1 += h0 < o1;
+  uint64_t p0 = __shfl_up_sync(0xFFFFFFFFu, h0, 1), p1 = __shfl_up_sync(0xFFFFFFFFu, h1, 1);
+  if (lane == 0) p0 = p1 = 0;
+  uint64_t s0 = e0 + p0;
+  const uint64_t c0 = s0 < p0;
+  uint64_t s1 = l1 + c0;
+  uint64_t g = s1 < c0;
+  s1 += p1;
+  g |= s1 < p1;
+  const uint32_t A = __ballot_sync(0xFFFFFFFFu, g || (s0 & s1) == ~0ull), B = __ballot_sync(0xFFFFFFFFu, g != 0);
+  if ((((A + B) ^ A ^ B) >> lane) & 1)
+    if (++s0 == 0) ++s1;
+  if (2 * (uint32_t)lane < nl) job.out[2 * lane] = s0;
+  if (2 * (uint32_t)lane + 1 < nl) job.out[2 * lane + 1] = s1;
+  __syncwarp();
+}
+
+template <int C>
+__device__ __noinline__ void small_chunk(const SmallJob* jobs, const SmallChunk& ch, const Roots& R, uint64_t* sm,
+                                         uint32_t* sA, uint32_t* sBm) {
+  constexpr int T = small_threads(C, small_split(C));
+  const uint32_t grp = threadIdx.x / T;
+  if (grp >= ch.count) return;
+  const SmallJob job = jobs[ch.first + grp];
+  uint64_t* base = sm + (size_t)grp * small_words(C, small_split(C));
+  if constexpr (C == SMALL_TINY)
+    tiny_multiply(job, base, threadIdx.x & 31);
+  else
+    small_multiply<C, small_split(C)>(job, R, base, (int)(threadIdx.x % T), (int)grp, sA, sBm);
+}
+
+// Chunks of same-class products; the CTAs stride over the chunks (a
+// persistent kernel over a size-sorted batch).
+// Against the former kernel (one radix-8 butterfly per thread and round, runtime
+// geometry): 16384 products of 128 .. 256 limbs 1132 -> 712 us, 4096 of 64 .. 128
+// limbs 154 -> 90.  Three CTAs per SM (80 registers) run no faster.
+__global__ void __launch_bounds__(SMALL_THREADS, 2) k_small_mul(const SmallJob* jobs, const SmallChunk* chunks, uint32_t nchunks,
+                                                               Roots R) {
+  pdl_wait();
   extern __shared__ uint64_t sm[];
+  __shared__ uint32_t sA[SMALL_THREADS / 32], sBm[SMALL_THREADS / 32];
   for (uint32_t k = blockIdx.x; k < nchunks; k += gridDim.x) {
-    SmallChunk ch;
-    if (chunks) {
-      ch = chunks[k];
-    } else {
-      const uint32_t n_out = 4 * one.la + 4 * one.lb - 1;
-      int L = 0;
-      while ((1u << L) < n_out) L++;
-      ch = SmallChunk{0, 1, L};
+    const SmallChunk ch = chunks[k];
+    switch (ch.c) {
+      case SMALL_TINY: small_chunk<SMALL_TINY>(jobs, ch, R, sm, sA, sBm); break;
+      case 8: small_chunk<8>(jobs, ch, R, sm, sA, sBm); break;
+      case 9: small_chunk<9>(jobs, ch, R, sm, sA, sBm); break;
+      case 10: small_chunk<10>(jobs, ch, R, sm, sA, sBm); break;
+      case 11: small_chunk<11>(jobs, ch, R, sm, sA, sBm); break;
+      default: small_chunk<12>(jobs, ch, R, sm, sA, sBm); break;
     }
-    const int G = small_group_threads(ch.L);
-    const uint32_t grp = threadIdx.x / G;
-    const bool active = grp < ch.count;
-    const SmallJob job = active ? (jobs ? jobs[ch.first + grp] : one) : SmallJob{};
-    const uint32_t sp = spad(1u << ch.L);
-    uint64_t* base = sm + (size_t)grp * 2 * sp;
-    small_multiply(job, active, ch.L, R, base, base + sp, (int)(threadIdx.x % G), G, (int)(grp * G / 32));
     __syncthreads();
+  }
+}
+
+// One product (the plain call).
+template <int C>
+__global__ void __launch_bounds__(small_threads(C, true), 1) k_small_one(SmallJob job, Roots R) {
+  pdl_wait();
+  extern __shared__ uint64_t sm[];
+  __shared__ uint32_t sA[SMALL_THREADS / 32], sBm[SMALL_THREADS / 32];
+  if constexpr (C == SMALL_TINY)
+    tiny_multiply(job, sm, threadIdx.x);
+  else
+    small_multiply<C, true>(job, R, sm, threadIdx.x, 0, sA, sBm);
+}
+
+// ---- whole multiply in one cluster (a lone product of 2^11 .. 2^14 points) --
+// One SM takes 10.5 us for a lone product of 2^11 points and 18.7 for 2^12, and
+// the pass pipeline 17 us for 2^13 (five launches of mostly idle grids): eight
+// CTAs take 8.5 us for up to 2^12 points, sixteen 10.5 for 2^13 and 13.6 for
+// 2^14 (eight: 13.3 and 21.5).  Half of them hold each operand: two passes of
+// radix 2^R1 (columns) and 2^R2 (rows) of two register rounds each, with the
+// transposes between them (and the hand-over of b's spectrum, of the inverse's
+// columns and of the coefficients in natural order) as stores into the other
+// CTAs' shared memory.  Below 2^11 points one CTA is as fast.
+constexpr int CLUSTER_LOG_MIN = 11, CLUSTER_LOG_MAX = 14;
+
+template <int L>
+struct ClusterGeom {
+  static constexpr int LOP = L == 12 ? 2 : 3, OP = 1 << LOP;  // CTAs per operand
+  static constexpr int R1 = (L + 1) / 2, R2 = L / 2;
+  static constexpr int B1 = pass_b1(R1), B2 = pass_b2(R1), D1 = pass_b1(R2), D2 = pass_b2(R2);
+  static constexpr int TC = R2 - LOP;                // log2 columns per CTA
+  static constexpr int RC = R1 - LOP;                // log2 rows per CTA
+  static constexpr uint32_t WORDS = 1u << (L - LOP); // of one operand, per CTA
+  static constexpr int NT = WORDS / 8 < 256 ? WORDS / 8 : 256;
+  static constexpr uint32_t CS = (1u << TC) + 1;     // row stride of a CTA's columns
+  static constexpr uint32_t YS = (1u << R2) + 1;     // stride of its rows
+  static constexpr uint32_t XW = CS << R1;           // words: columns, rows (or coefficients), spectrum
+  static constexpr uint32_t YW = (YS << RC) > WORDS + WORDS / 16 ? YS << RC : WORDS + WORDS / 16;
+  static constexpr uint32_t SMEM = (XW + YW + WORDS) * 8;
+};
+
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_barrier() {
+  cluster_arrive();
+  cluster_wait();
+}
+// p's counterpart in the shared memory of CTA `rank` of the cluster.
+__device__ __forceinline__ uint64_t* cluster_ptr(uint64_t* p, uint32_t rank) {
+  uint64_t r;
+  asm("mapa.u64 %0, %1, %2;" : "=l"(r) : "l"(p), "r"(rank));
+  return reinterpret_cast<uint64_t*>(r);
+}
+
+template <int L>
+__global__ void __cluster_dims__(2 * ClusterGeom<L>::OP, 1, 1) __launch_bounds__(ClusterGeom<L>::NT, 1) k_cluster_mul(SmallJob job, Roots R) {
+  using G = ClusterGeom<L>;
+  constexpr int R1 = G::R1, R2 = G::R2, B1 = G::B1, B2 = G::B2, D1 = G::D1, D2 = G::D2, TC = G::TC, RC = G::RC, NT = G::NT;
+  constexpr uint32_t N = 1u << L, CM = (1u << TC) - 1;
+  cluster_arrive();  // waited on before the first store into another CTA: all of them run by then
+  pdl_wait();
+  extern __shared__ uint64_t sm[];
+  uint64_t* X = sm;            // this CTA's columns: [row][column], stride CS
+  uint64_t* Y = X + G::XW;     // its rows: [row][2^R2 words], stride YS; later its coefficients
+  uint64_t* Z = Y + G::YW;     // b's spectrum; later the windows' high parts
+  __shared__ uint32_t sA[NT / 32], sB[NT / 32];
+  __shared__ uint64_t sF[G::OP];
+  const uint32_t rank = blockIdx.x & (G::OP - 1);  // the grid is one cluster
+  const bool isb = blockIdx.x >= G::OP;
+  const uint32_t mine = isb ? G::OP : 0;           // first CTA of this operand
+  const uint32_t la = job.la, lb = job.lb;
+  const bool square = job.a == job.b && la == lb;
+  const int t = threadIdx.x;
+  const uint32_t col0 = rank << TC;
+  constexpr uint64_t ninv = gl::P - ((1ull << (64 - L)) - (1ull << (32 - L)));  // 2^-L
+  if (!(isb && square)) {
+    // pass 1, round 1: coefficients row 2^R2 + column, rows (m << B2) + jp
+    const uint16_t* __restrict__ coef = reinterpret_cast<const uint16_t*>(isb ? job.b : job.a);
+    const uint32_t nc = 4 * (isb ? lb : la);
+#pragma unroll 1
+    for (uint32_t w = t; w < (1u << (B2 + TC)); w += NT) {
+      const uint32_t c = w & CM, jp = w >> TC;
+      uint64_t v[1 << B1];
+      gl::Lz x[1 << B1];
+#pragma unroll
+      for (int m = 0; m < (1 << B1); m++) {
+        const uint32_t n = (((m << B2) + jp) << R2) + col0 + c;
+        x[m] = gl::Lz{n < nc ? (uint32_t)__ldg(coef + n) : 0u, 0u, 0};
+      }
+      x[0] = gl::lz_bias(x[0]);
+      dft_lz<B1, false>(x, v);
+#pragma unroll
+      for (int k = 0; k < (1 << B1); k++) X[((k << B2) + jp) * G::CS + c] = v[k];
+    }
+  }
+  __syncthreads();
+  cluster_wait();
+  if (!(isb && square)) {
+    // round 2, pass twiddles, rows to the CTAs that own them
+#pragma unroll 1
+    for (uint32_t w = t; w < (1u << (B1 + TC)); w += NT) {
+      const uint32_t c = w & CM, k1 = w >> TC, J = col0 + c;
+      uint64_t v[1 << B2];
+      pass_fwd2<R1>(X + (k1 << B2) * G::CS + c, G::CS, R.rt + rt_offset(R1, false), k1, v);
+#pragma unroll
+      for (int k = 0; k < (1 << B2); k++) {
+        const uint32_t row = (k1 << B2) + k, f = k1 + (k << B1);
+        const uint64_t y = gl::mul(v[k], __ldg(R.lvl + N + f * J));
+        cluster_ptr(Y, mine + (row >> (RC)))[(row & ((1u << (RC)) - 1)) * G::YS + J] = y;
+      }
+    }
+  }
+  cluster_barrier();
+  // pass 2 on the rows; the last round's outputs stay in registers
+  constexpr int IT2 = (1 << (RC + D1)) / NT;  // (row, k1) items per thread
+  uint64_t s[IT2 << D2];
+  static_assert((IT2 * NT) == (1 << (RC + D1)), "rows divide evenly");
+  if (!(isb && square)) {
+#pragma unroll 1
+    for (uint32_t w = t; w < (1u << (RC + D2)); w += NT) {
+      const uint32_t jp = w & ((1u << D2) - 1), row = w >> D2;
+      uint64_t* y = Y + row * G::YS + jp;
+      uint64_t v[1 << D1];
+      gl::Lz x[1 << D1];
+#pragma unroll
+      for (int m = 0; m < (1 << D1); m++) x[m] = gl::lz(y[m << D2]);
+      x[0] = gl::lz_bias(x[0]);
+      dft_lz<D1, false>(x, v);
+#pragma unroll
+      for (int k = 0; k < (1 << D1); k++) y[k << D2] = v[k];
+    }
+    __syncthreads();
+#pragma unroll
+    for (int it = 0; it < IT2; it++) {
+      const uint32_t w = it * NT + t, k1 = w & ((1u << D1) - 1), row = w >> D1;
+      pass_fwd2<R2>(Y + row * G::YS + (k1 << D2), 1, R.rt + rt_offset(R2, false), k1, s + (it << D2));
+    }
+    if (isb) {
+      uint64_t* z = cluster_ptr(Z, rank);
+#pragma unroll
+      for (int it = 0; it < IT2; it++)
+#pragma unroll
+        for (int k = 0; k < (1 << D2); k++) z[((it << D2) + k) * NT + t] = gl::mul(s[(it << D2) + k], ninv);
+    }
+  }
+  cluster_barrier();
+  if (!isb) {
+    // pointwise product and the inverse of pass 2
+#pragma unroll
+    for (int it = 0; it < IT2; it++) {
+      const uint32_t w = it * NT + t, k1 = w & ((1u << D1) - 1), row = w >> D1;
+      uint64_t v[1 << D2];
+      gl::Lz x[1 << D2];
+#pragma unroll
+      for (int k = 0; k < (1 << D2); k++) {
+        const uint64_t u = s[(it << D2) + k];
+        x[k] = gl::lz_mul(u, square ? gl::mul(u, ninv) : Z[((it << D2) + k) * NT + t]);
+      }
+      x[0] = gl::lz_bias(x[0]);
+      dft_lz<D2, true>(x, v);
+#pragma unroll
+      for (int m = 0; m < (1 << D2); m++) Y[row * G::YS + (k1 << D2) + m] = v[m];
+    }
+    __syncthreads();
+#pragma unroll 1
+    for (uint32_t w = t; w < (1u << (RC + D2)); w += NT) {
+      const uint32_t jp = w & ((1u << D2) - 1), row = w >> D2;
+      uint64_t v[1 << D1];
+      pass_inv2<R2>(Y + row * G::YS + jp, 1u << D2, R.rt + rt_offset(R2, true), jp, v);
+      // columns to the CTAs that own them
+      const uint32_t grow = (rank << (RC)) + row;
+#pragma unroll
+      for (int m = 0; m < (1 << D1); m++) {
+        const uint32_t J = (m << D2) + jp;
+        cluster_ptr(X, J >> TC)[grow * G::CS + (J & CM)] = v[m];
+      }
+    }
+  }
+  cluster_barrier();
+  if (!isb) {
+    // inverse of pass 1
+#pragma unroll 1
+    for (uint32_t w = t; w < (1u << (B1 + TC)); w += NT) {
+      const uint32_t c = w & CM, k1 = w >> TC, J = col0 + c;
+      uint64_t* xc = X + (k1 << B2) * G::CS + c;
+      uint64_t v[1 << B2];
+      gl::Lz x[1 << B2];
+#pragma unroll
+      for (int k = 0; k < (1 << B2); k++) {
+        const uint32_t e = (k1 + (k << B1)) * J;
+        x[k] = gl::lz_mul(xc[k * G::CS], __ldg(R.lvl + N + ((N - e) & (N - 1))));
+      }
+      x[0] = gl::lz_bias(x[0]);
+      dft_lz<B2, true>(x, v);
+#pragma unroll
+      for (int m = 0; m < (1 << B2); m++) xc[m * G::CS] = v[m];
+    }
+    __syncthreads();
+#pragma unroll 1
+    for (uint32_t w = t; w < (1u << (B2 + TC)); w += NT) {
+      const uint32_t c = w & CM, jp = w >> TC;
+      uint64_t v[1 << B1];
+      pass_inv2<R1>(X + jp * G::CS + c, G::CS << B2, R.rt + rt_offset(R1, true), jp, v);
+      // coefficients in natural order, a quarter per CTA
+#pragma unroll
+      for (int m = 0; m < (1 << B1); m++) {
+        const uint32_t row = (m << B2) + jp;
+        const uint32_t n = (row << R2) + col0 + c;
+        const uint32_t i = n & (G::WORDS - 1);
+        cluster_ptr(Y, n >> (L - G::LOP))[i + (i >> 4)] = gl::canon(v[m]);
+      }
+    }
+  }
+  cluster_barrier();
+  // carry: windows of 16 coefficients (4 limbs), one per thread
+  const uint32_t nl = la + lb, nwin = (4 * nl - 1 + 15) / 16, w = rank * (G::WORDS / 16) + t;
+  const bool have = !isb && t < (int)(G::WORDS / 16) && w < nwin;
+  Win v{{0, 0, 0, 0}, 0};
+  uint64_t hprev = 0;
+  if (have) {
+    v = fold16(Y + 17 * t, 1);
+    Z[t] = v.hi;
+    if (t == 0 && rank > 0) hprev = fold16(cluster_ptr(Y, rank - 1) + 17 * (G::WORDS / 16 - 1), 1).hi;
+  }
+  __syncthreads();
+  if (have && t > 0) hprev = Z[t - 1];
+  uint64_t s0 = v.l[0] + hprev;
+  uint64_t c = s0 < hprev;
+  uint64_t s1 = v.l[1] + c;  c = c && s1 == 0;
+  uint64_t s2 = v.l[2] + c;  c = c && s2 == 0;
+  uint64_t s3 = v.l[3] + c;  c = c && s3 == 0;
+  const bool gg = have && c, pp = have && (s0 & s1 & s2 & s3) == ~0ull;
+  const uint32_t A = __ballot_sync(0xFFFFFFFFu, gg || pp), B = __ballot_sync(0xFFFFFFFFu, gg);
+  if ((t & 31) == 0) sA[t >> 5] = A, sB[t >> 5] = B;
+  __syncthreads();
+  constexpr int WARPS = ((int)(G::WORDS / 16) + 31) / 32;
+  if (!isb && t == 0) {
+    uint32_t f = 2; 
+    for (int k = 0; k < WARPS; k++) f = cf_then(f, cf_of_masks(sA[k], sB[k]));
+    for (uint32_t q = rank + 1; q < G::OP; q++) cluster_ptr(sF, q)[rank] = f;
+  }
+  cluster_barrier();
+  if (have) {
+    uint32_t cin = 0;
+    for (uint32_t q = 0; q < rank; q++) cin = ((uint32_t)sF[q] >> cin) & 1;
+    for (int k = 0; k < (t >> 5); k++) cin = (cf_of_masks(sA[k], sB[k]) >> cin) & 1;
+    const uint32_t carries = (A + B + cin) ^ A ^ B;
+    if ((carries >> (t & 31)) & 1) {
+      if (++s0 == 0) if (++s1 == 0) if (++s2 == 0) ++s3;
+    }
+    const uint32_t base = 4 * w;
+    if (base + 0 < nl) job.out[base + 0] = s0;
+    if (base + 1 < nl) job.out[base + 1] = s1;
+    if (base + 2 < nl) job.out[base + 2] = s2;
+    if (base + 3 < nl) job.out[base + 3] = s3;
   }
 }
 
@@ -1283,6 +1761,11 @@ static cudaError_t set_smem_attrs() {
   cudaError_t e = cudaSuccess;
   if (e == cudaSuccess)
     e = cudaFuncSetAttribute(k_small_mul, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)small_cta_smem(SMALL_LOG_MAX));
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(k_cluster_mul<12>, cudaFuncAttributeMaxDynamicSharedMemorySize, ClusterGeom<12>::SMEM);
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(k_cluster_mul<13>, cudaFuncAttributeMaxDynamicSharedMemorySize, ClusterGeom<13>::SMEM);
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(k_cluster_mul<13>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(k_cluster_mul<14>, cudaFuncAttributeMaxDynamicSharedMemorySize, ClusterGeom<14>::SMEM);
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(k_cluster_mul<14>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
   if (e == cudaSuccess) e = cudaFuncSetAttribute(k_split_merge<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)merge_cta_smem(8));
   if (e == cudaSuccess) e = cudaFuncSetAttribute(k_split_merge<9>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)merge_cta_smem(9));
   if (e == cudaSuccess) e = cudaFuncSetAttribute(k_split_merge<10>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)merge_cta_smem(10));
@@ -1785,6 +2268,30 @@ static void launch_pdl(void (*k)(P...), dim3 grid, int threads, size_t smem, cud
   cudaLaunchKernelEx(&c, k, (P)args...);
 }
 
+template <int C>
+static void launch_small_c(const SmallJob& job, const Roots& R, cudaStream_t st) {
+  launch_pdl(k_small_one<C>, dim3(1), small_threads(C, true), small_words(C, true) * 8, st, job, R);
+}
+// One product within a cluster.
+template <int L>
+static void launch_cluster_c(const SmallJob& job, const Roots& R, cudaStream_t st) {
+  launch_pdl(k_cluster_mul<L>, dim3(2 * ClusterGeom<L>::OP), ClusterGeom<L>::NT, ClusterGeom<L>::SMEM, st, job, R);
+}
+static void launch_cluster(int L, const SmallJob& job, const Roots& R, cudaStream_t st) {
+  if (L <= 12) launch_cluster_c<12>(job, R, st);
+  else if (L == 13) launch_cluster_c<13>(job, R, st);
+  else launch_cluster_c<14>(job, R, st);
+}
+// One product within a CTA.
+static void launch_small(const SmallJob& job, const Roots& R, cudaStream_t st) {
+  switch (small_class(job.la, job.lb)) {
+    case SMALL_TINY: launch_small_c<SMALL_TINY>(job, R, st); break;
+    case 8: launch_small_c<8>(job, R, st); break;
+    case 9: launch_small_c<9>(job, R, st); break;
+    default: launch_small_c<10>(job, R, st); break;  // longer ones: launch_cluster
+  }
+}
+
 // Both operands of a transform up to this length (log2) go through each
 // forward pass in one launch.
 constexpr int MERGE_OPERANDS_LOG = 20;
@@ -2003,12 +2510,13 @@ static int mul_device(const uint64_t* d_a, uint64_t la, const uint64_t* d_b, uin
   if (z.L > 32) return fail(PIMUL_EINVAL, "transform length above 2^32");
   const Roots& R = g_dev.roots;
   const bool square = d_a == d_b && la == lb;
-  if (z.L <= SMALL_LOG_MAX) {
+  if (z.L <= CLUSTER_LOG_MAX) {
     if (b_ready) cudaStreamWaitEvent(st, b_ready, 0);
     SmallJob job{d_a, d_b, d_out, (uint32_t)la, (uint32_t)lb};
     {
       KTimer kt(K_SMALL, st, true);
-      k_small_mul<<<1, SMALL_THREADS, small_cta_smem(z.L), st>>>(nullptr, nullptr, job, 1, R);
+      if (z.L < CLUSTER_LOG_MIN) launch_small(job, R, st);
+      else launch_cluster(z.L, job, R, st);
     }
     CU(cudaGetLastError());
     return PIMUL_OK;
@@ -2089,7 +2597,6 @@ struct BatchLayout {
   };
   std::vector<Bucket> large;
   uint64_t arena_bytes = 0;
-  int small_L = 0;  // largest L among the small jobs
   std::vector<SegPlan> seg;  // per unit: how a product of a long by a short operand is cut
   std::vector<SmallChunk> chunks;  // the small jobs in same-length chunks
   size_t small_smem = 0;           // dynamic shared memory of their CTAs
@@ -2121,8 +2628,8 @@ static int layout_batch(const Unit* units, size_t n, BatchLayout& B, bool share)
   }
   // uneven products are cut into segments, unless others share their b (a
   // shared spectrum saves more)
-  B.seg.assign(n, SegPlan{});
-  {
+  if (std::any_of(Ls.begin(), Ls.end(), [](int L) { return L > SMALL_LOG_MAX; })) {
+    B.seg.assign(n, SegPlan{});
     std::unordered_map<const uint64_t*, uint32_t> uses;
     if (share)
       for (size_t i = 0; i < n; i++)
@@ -2143,7 +2650,6 @@ static int layout_batch(const Unit* units, size_t n, BatchLayout& B, bool share)
     if (Ls[i] <= SMALL_LOG_MAX && units[i].la2) return fail(PIMUL_EINVAL, "a sum of products below 2^13 in the pass pipeline");
     if (Ls[i] <= SMALL_LOG_MAX) {
       B.small.push_back((uint32_t)i);
-      if (Ls[i] > B.small_L) B.small_L = Ls[i];
     } else {
       byL[Ls[i]].push_back((uint32_t)i);
     }
@@ -2151,14 +2657,14 @@ static int layout_batch(const Unit* units, size_t n, BatchLayout& B, bool share)
   // longest transforms first (a bucket pass by length, O(n))
   {
     std::vector<std::vector<uint32_t>> sb(SMALL_LOG_MAX + 1);
-    for (uint32_t i : B.small) sb[Ls[i]].push_back(i);
+    for (uint32_t i : B.small) sb[small_class(units[i].la, units[i].lb)].push_back(i);
     B.small.clear();
-    for (int L = SMALL_LOG_MAX; L >= 0; L--) {
-      const uint32_t per = SMALL_THREADS / small_group_threads(L);
-      for (size_t k = 0; k < sb[L].size(); k += per)
-        B.chunks.push_back(SmallChunk{(uint32_t)(B.small.size() + k), (uint32_t)std::min<size_t>(per, sb[L].size() - k), L});
-      if (!sb[L].empty()) B.small_smem = std::max(B.small_smem, small_cta_smem(L));
-      B.small.insert(B.small.end(), sb[L].begin(), sb[L].end());
+    for (int c = SMALL_LOG_MAX; c >= SMALL_TINY; c--) {
+      const uint32_t per = small_per_cta(c);
+      for (size_t k = 0; k < sb[c].size(); k += per)
+        B.chunks.push_back(SmallChunk{(uint32_t)(B.small.size() + k), (uint32_t)std::min<size_t>(per, sb[c].size() - k), c});
+      if (!sb[c].empty()) B.small_smem = std::max(B.small_smem, small_cta_smem(c));
+      B.small.insert(B.small.end(), sb[c].begin(), sb[c].end());
     }
   }
   // Groups of one length: at most 65535 descriptors (grid.y) whose scratch
@@ -2340,8 +2846,8 @@ static void launch_batch(const Launcher& X, const BatchLayout& B, const SmallJob
     const SmallChunk* d_chunks = reinterpret_cast<const SmallChunk*>(reinterpret_cast<const uint8_t*>(d_small) +
                                                                      round256(B.small.size() * sizeof(SmallJob)));
     KTimer kt(K_SMALL, X.st, X.stats);
-    k_small_mul<<<(unsigned)grid, SMALL_THREADS, B.small_smem, X.st>>>(d_small, d_chunks, SmallJob{},
-                                                                      (uint32_t)B.chunks.size(), X.R);
+    launch_pdl(k_small_mul, dim3((unsigned)grid), SMALL_THREADS, B.small_smem, X.st, d_small, d_chunks,
+               (uint32_t)B.chunks.size(), X.R);
   }
   for (const auto& bk : B.large)
     run_large(X, d_large + bk.d0, Job{}, (uint32_t)bk.nd, bk.L, (uint32_t)bk.nc, bk.max_chunk);
@@ -3897,13 +4403,13 @@ int svc_addsub(const pimul_addsub_job* jobs, size_t n, cudaStream_t st) {
 // queueing such a batch costs a few launches whatever n is.
 
 // Descriptors and chunks of n products (a + i sa) * b -> out + i so, all of
-// one transform length 2^L <= 2^SMALL_LOG_MAX, per products per chunk.
+// one class (transform length up to 2^SMALL_LOG_MAX), per products per chunk.
 __global__ void k_fill_small(SmallJob* jobs, SmallChunk* chunks, SmallJob base, uint64_t sa, uint64_t so, uint32_t n,
-                             uint32_t per, int L) {
+                             uint32_t per, int c) {
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   jobs[i] = SmallJob{base.a + (uint64_t)i * sa, base.b, base.out + (uint64_t)i * so, base.la, base.lb};
-  if (i < ((uint64_t)n + per - 1) / per) chunks[i] = SmallChunk{i * per, per < n - i * per ? per : n - i * per, L};
+  if (i < ((uint64_t)n + per - 1) / per) chunks[i] = SmallChunk{i * per, per < n - i * per ? per : n - i * per, c};
 }
 
 int mul_batch_strided(const uint64_t* a, uint64_t sa, size_t la, const uint64_t* b, size_t lb, uint64_t* out,
@@ -3919,7 +4425,8 @@ int mul_batch_strided(const uint64_t* a, uint64_t sa, size_t la, const uint64_t*
   cudaStream_t own;
   int rc = get_stream(&own);  // initialises the engine on first use
   if (rc) return rc;
-  const uint32_t per = SMALL_THREADS / small_group_threads(L);
+  const int c = small_class(la, lb);
+  const uint32_t per = small_per_cta(c);
   const size_t nch = (n + per - 1) / per;
   const size_t jb = round256(n * sizeof(SmallJob));
   uint8_t* dev = nullptr;
@@ -3931,11 +4438,11 @@ int mul_batch_strided(const uint64_t* a, uint64_t sa, size_t la, const uint64_t*
   SmallJob* dj = reinterpret_cast<SmallJob*>(dev);
   SmallChunk* dc = reinterpret_cast<SmallChunk*>(dev + jb);
   k_fill_small<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(dj, dc, SmallJob{a, b, out, (uint32_t)la, (uint32_t)lb},
-                                                           sa, so, (uint32_t)n, per, L);
+                                                           sa, so, (uint32_t)n, per, c);
   int sms = 152;
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, g_dev.device);
   const uint64_t grid = std::min<uint64_t>((uint64_t)sms * (uint64_t)g_small_ctas_per_sm.load(), nch);
-  k_small_mul<<<(unsigned)grid, SMALL_THREADS, small_cta_smem(L), st>>>(dj, dc, SmallJob{}, (uint32_t)nch, g_dev.roots);
+  launch_pdl(k_small_mul, dim3((unsigned)grid), SMALL_THREADS, small_cta_smem(c), st, dj, dc, (uint32_t)nch, g_dev.roots);
   e = cudaGetLastError();
   cudaFreeAsync(dev, st);
   if (e != cudaSuccess) return fail(PIMUL_ECUDA, std::string("strided batch launch: ") + cudaGetErrorString(e));
@@ -4043,9 +4550,10 @@ static int mul_device_noalloc(const uint64_t* d_a, uint64_t la, const uint64_t* 
   if (rc) return rc;
   const Sizes z = sizes_for(la, lb);
   const Roots& R = nd->roots;
-  if (z.L <= SMALL_LOG_MAX) {  // whole product in one CTA's shared memory: no scratch
+  if (z.L <= CLUSTER_LOG_MAX) {  // whole product in shared memory: no scratch
     SmallJob job{d_a, d_b, d_out, (uint32_t)la, (uint32_t)lb};
-    k_small_mul<<<1, SMALL_THREADS, small_cta_smem(z.L), st>>>(nullptr, nullptr, job, 1, R);
+    if (z.L < CLUSTER_LOG_MIN) launch_small(job, R, st);
+    else launch_cluster(z.L, job, R, st);
     CU(cudaGetLastError());
     return PIMUL_OK;
   }

@@ -15,7 +15,7 @@
 //
 // Inside a pass the R_p-point DFT runs as two rounds of radix 8, 16 or 32
 // held in registers (rounds of radix 8, 4 or 2 in shared memory in the
-// one-CTA kernels).  2 is a 192nd root of unity mod p, and the root tables
+// merged splitting levels).  2 is a 192nd root of unity mod p, and the root tables
 // are built so that the 64th root of unity is 2^3: the butterflies' internal
 // twiddles are constant shifts.
 #pragma once
@@ -75,13 +75,6 @@ __device__ __forceinline__ uint64_t root_pow32(const Roots& R, int mlog, uint32_
   return rho_pow(R, x << (32 - mlog));
 }
 
-// w_(2^mlog)^x for x < 2^mlog <= 4096 from the 4096-entry table (forward or inverse).
-__device__ __forceinline__ uint64_t round_tw(const Roots& R, int mlog, uint32_t x, bool inverse) {
-  uint32_t t = x << (12 - mlog);
-  if (inverse) t = (4096u - t) & 4095u;
-  return __ldg(R.w12 + t);
-}
-
 // Shared-memory index with one pad word per 16 to spread 8-byte banks.
 __host__ __device__ __forceinline__ constexpr uint32_t spad(uint32_t lin) { return lin + (lin >> 4); }
 
@@ -91,14 +84,6 @@ __host__ __device__ __forceinline__ constexpr uint32_t spad(uint32_t lin) { retu
 // offsets of a butterfly group are compile-time constants.
 __host__ __device__ __forceinline__ constexpr uint32_t spad_step(uint32_t m, int s) {
   return (m << s) + ((m << s) >> 4);
-}
-
-// DIF radix-2 butterfly with a constant shift twiddle 2^S (S = 0: none).
-template <int S>
-__device__ __forceinline__ void bfly_dif(uint64_t& a, uint64_t& b) {
-  uint64_t u = a, w = b;
-  a = gl::add(u, w);
-  b = gl::shl<S>(gl::sub(u, w));
 }
 
 // 8-point DFT (INV: unscaled inverse) of lazy values, folded outputs at
@@ -204,7 +189,7 @@ __device__ __forceinline__ void dft_lz(gl::Lz* x, uint64_t* v) {
 }
 
 // Forward DFT of 2^B values in registers (radix 2, 4, 8), for the rounds of
-// the one-CTA kernels: lazy inputs with |k| <= 1, folded outputs.
+// the merged splitting levels: lazy inputs with |k| <= 1, folded outputs.
 template <int B>
 __device__ __forceinline__ void dft_fwd_lz(const gl::Lz* x, uint64_t* v) {
   using namespace gl;
@@ -227,19 +212,7 @@ __device__ __forceinline__ void dft_fwd_lz(const gl::Lz* x, uint64_t* v) {
   }
 }
 
-template <int B>
-__device__ __forceinline__ void dft_fwd(uint64_t* v) {
-  if constexpr (B == 1) {
-    bfly_dif<0>(v[0], v[1]);
-  } else {
-    gl::Lz x[1 << B];
-#pragma unroll
-    for (int k = 0; k < (1 << B); k++) x[k] = gl::lz(v[k]);
-    dft_fwd_lz<B>(x, v);
-  }
-}
-
-// Unscaled inverse of dft_fwd on lazy inputs (|k| <= 1, e.g. twiddle
+// Unscaled inverse of dft_fwd_lz on lazy inputs (|k| <= 1, e.g. twiddle
 // products from lz_mul): v[m] <- sum_k x[k] w^(-m k)  (= 2^B * original).
 template <int B>
 __device__ __forceinline__ void dft_inv_lz(const gl::Lz* x, uint64_t* v) {
@@ -494,94 +467,6 @@ __device__ __forceinline__ void pass_inv2(const uint64_t* sx, uint32_t stride, c
 #pragma unroll
   for (int k = 1; k < (1 << B1); k++) x[k] = gl::lz_mul(v[k], __ldg(rt + (k << B2) + m));
   dft_lz<B1, true>(x, v);
-}
-
-// ------------------------------------------------- runtime-geometry rounds
-// Used by the one-CTA multiply, whose transform length varies per call.
-struct TileGeom {
-  int r, t, bc;
-};
-
-template <int B>
-__device__ __forceinline__ void round_fwd(uint64_t* sm, TileGeom g, int mlog, const Roots& R, int tid,
-                                          int nthreads) {
-  const int slog = mlog - B;
-  const int items_log = g.bc + g.r + g.t - B;
-  const uint32_t tmask = (1u << g.t) - 1, smask = (1u << slog) - 1;
-  for (uint32_t w = tid; w < (1u << items_log); w += nthreads) {
-    uint32_t j = w & tmask;
-    uint32_t rest = w >> g.t;
-    uint32_t jp = rest & smask;
-    uint32_t row0 = ((rest >> slog) << mlog) + jp;
-    uint64_t v[1 << B];
-#pragma unroll
-    for (int m = 0; m < (1 << B); m++) v[m] = sm[spad(((row0 + (m << slog)) << g.t) | j)];
-    dft_fwd<B>(v);
-    if (slog > 0) {
-#pragma unroll
-      for (int k = 1; k < (1 << B); k++) v[k] = gl::mul(v[k], round_tw(R, mlog, k * jp, false));
-    }
-#pragma unroll
-    for (int k = 0; k < (1 << B); k++) sm[spad(((row0 + (k << slog)) << g.t) | j)] = v[k];
-  }
-}
-
-template <int B>
-__device__ __forceinline__ void round_inv(uint64_t* sm, TileGeom g, int mlog, const Roots& R, int tid,
-                                          int nthreads) {
-  const int slog = mlog - B;
-  const int items_log = g.bc + g.r + g.t - B;
-  const uint32_t tmask = (1u << g.t) - 1, smask = (1u << slog) - 1;
-  for (uint32_t w = tid; w < (1u << items_log); w += nthreads) {
-    uint32_t j = w & tmask;
-    uint32_t rest = w >> g.t;
-    uint32_t jp = rest & smask;
-    uint32_t row0 = ((rest >> slog) << mlog) + jp;
-    uint64_t v[1 << B];
-    gl::Lz x[1 << B];
-#pragma unroll
-    for (int k = 0; k < (1 << B); k++) v[k] = sm[spad(((row0 + (k << slog)) << g.t) | j)];
-    x[0] = gl::lz(v[0]);
-#pragma unroll
-    for (int k = 1; k < (1 << B); k++)
-      x[k] = slog > 0 ? gl::lz_mul(v[k], round_tw(R, mlog, k * jp, true)) : gl::lz(v[k]);
-    dft_inv_lz<B>(x, v);
-#pragma unroll
-    for (int m = 0; m < (1 << B); m++) sm[spad(((row0 + (m << slog)) << g.t) | j)] = v[m];
-  }
-}
-
-__device__ __forceinline__ void tile_dft_fwd(uint64_t* sm, TileGeom g, const Roots& R, int tid, int nthreads) {
-  int mlog = g.r, rem = g.r;
-  while (rem > 0) {
-    int b = rem >= 3 ? 3 : rem;
-    if (rem == 4) b = 2;
-    if (b == 3) round_fwd<3>(sm, g, mlog, R, tid, nthreads);
-    else if (b == 2) round_fwd<2>(sm, g, mlog, R, tid, nthreads);
-    else round_fwd<1>(sm, g, mlog, R, tid, nthreads);
-    mlog -= b;
-    rem -= b;
-    __syncthreads();
-  }
-}
-
-__device__ __forceinline__ void tile_dft_inv(uint64_t* sm, TileGeom g, const Roots& R, int tid, int nthreads) {
-  int bits[8], n = 0, rem = g.r;
-  while (rem > 0) {
-    int b = rem >= 3 ? 3 : rem;
-    if (rem == 4) b = 2;
-    bits[n++] = b;
-    rem -= b;
-  }
-  int mlog = 0;
-  for (int q = n - 1; q >= 0; q--) {
-    int b = bits[q];
-    mlog += b;
-    if (b == 3) round_inv<3>(sm, g, mlog, R, tid, nthreads);
-    else if (b == 2) round_inv<2>(sm, g, mlog, R, tid, nthreads);
-    else round_inv<1>(sm, g, mlog, R, tid, nthreads);
-    __syncthreads();
-  }
 }
 
 }  // namespace pimul
