@@ -366,10 +366,10 @@ def handle_size(h: int) -> int:
 def download(h: int) -> np.ndarray:
     """The handle's value (trimmed limbs); waits for its producer."""
     cap = handle_size(h)
-    out = np.zeros(max(cap, 1), dtype=np.uint64)
+    out = np.empty(max(cap, 1), dtype=np.uint64)
     n = _sz(0)
     _check(lib().pimul_download(h, out.ctypes.data_as(_u64p), out.size, ctypes.byref(n)))
-    return out[: n.value].copy()
+    return out[: n.value]
 
 
 def free(h: int):
