@@ -259,6 +259,54 @@ __device__ __forceinline__ uint32_t pow2_mod_odd32(uint64_t E, uint32_t m, uint3
   return mm32<SMALL>(x, 1, m, minv);
 }
 
+// The same for odd 3 <= m < 2^30 (RED) or 2^28 with unreduced values.  With
+// minv = m^-1 mod 2^32 and t = x^2 = (th:tl), u = tl minv, the low words of t
+// and u m are equal and r = th - hi(u m) + m is 2^-32 t mod m without a carry
+// to look for: 1 <= r <= th + m.
+//  * m < 2^28: for x < 4m, th < 16 m^2 / 2^32 < m, so r < 2m and a doubled r is
+//    below 4m < 2^30 again: nothing is ever reduced;
+//  * m < 2^30: for x < 2m, th < m, r < 2m, and min(y, y - 2m) (which wraps when
+//    y < 2m) brings a doubled y < 4m < 2^32 below 2m.
+// A step is one wide and two narrow multiplications, one three-input add and
+// the doubling: 64 positions below 5e7 took 103 ms with the reduced values of
+// mont_mul31 and all 32 bits run, 80 ms so.  x starts as 2^32 - q m for a float underestimate q of
+// 2^32 / m: below m + 2^12 (at most 2m, or a small m whose first steps
+// absorb it).  E's bits run from the top group of four that is not zero.
+// The last product with 1 gives r = m - hi(u m), in [1, m) since m does not
+// divide a power of two.
+template <bool RED>
+__device__ __forceinline__ uint32_t pow2_step(uint32_t x, uint32_t bit, uint32_t m, uint32_t minv) {
+  const uint64_t t = (uint64_t)x * x;
+  const uint32_t u = (uint32_t)t * minv;
+  x = ((uint32_t)(t >> 32) - __umulhi(u, m) + m) << bit;
+  if constexpr (RED) x = min(x, x - 2 * m);
+  return x;
+}
+
+template <bool RED>
+__device__ __forceinline__ uint32_t pow2_mod_lazy(uint64_t E, uint32_t m, uint32_t minv) {
+  const uint32_t q = __float2uint_rz(__fmul_rn(__frcp_rn((float)m), 4294965248.0f));  // 2^32 (1 - 2^-21)
+  uint32_t x = 0u - q * m;
+  uint32_t eh = (uint32_t)(E >> 32), el = (uint32_t)E;
+  int groups = 8;
+  if (eh) {
+    int b = 32 - __clz((int)eh);
+    for (eh <<= 32 - b; b > 0; b--, eh <<= 1) x = pow2_step<RED>(x, eh >> 31, m, minv);
+  } else {
+    groups = (35 - __clz((int)el)) >> 2;
+    el <<= 32 - 4 * groups;
+  }
+#pragma unroll 1
+  for (; groups > 0; groups--) {
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+      x = pow2_step<RED>(x, el >> 31, m, minv);
+      el <<= 1;
+    }
+  }
+  return m - __umulhi(x * minv, m);
+}
+
 // The same for odd 2^32 <= m < 2^34 in 64-bit Montgomery arithmetic.
 __device__ __forceinline__ uint64_t pow2_mod_odd64(uint64_t E, uint64_t m, uint64_t minv) {
   uint64_t x = pow2_64_mod(m, __frcp_rn((float)m));  // R mod m (R = 2^64)
@@ -287,7 +335,9 @@ __device__ __forceinline__ uint64_t bbp_term(uint64_t e, uint64_t d) {
   if (m == 1) return lo;
   const uint64_t E = 4 * e + 64 - (uint64_t)t;
   const uint64_t minv = neg_inv64(m);  // -m^-1 mod 2^64
-  const uint64_t r = m < (1ull << 31)   ? (uint64_t)pow2_mod_odd32<true>(E, (uint32_t)m, (uint32_t)minv)
+  const uint64_t r = m < (1ull << 28)   ? (uint64_t)pow2_mod_lazy<false>(E, (uint32_t)m, 0u - (uint32_t)minv)
+                     : m < (1ull << 30) ? (uint64_t)pow2_mod_lazy<true>(E, (uint32_t)m, 0u - (uint32_t)minv)
+                     : m < (1ull << 31) ? (uint64_t)pow2_mod_odd32<true>(E, (uint32_t)m, (uint32_t)minv)
                      : m < (1ull << 32) ? (uint64_t)pow2_mod_odd32<false>(E, (uint32_t)m, (uint32_t)minv)
                                         : pow2_mod_odd64(E, m, minv);
   return (lo - r) * (0 - minv);
