@@ -284,14 +284,19 @@ __global__ void __launch_bounds__(PASS_THREADS, pass_min_ctas(R)) k_fwd_first(co
     const uint16_t* __restrict__ cn = coef + n0;
     uint64_t v[1 << B1];
     gl::Lz x[1 << B1];
-    // an operand of at most N/8 limbs leaves the upper half of the rows zero
-    // (coefficients N/2 and up): those inputs are neither read nor added
-    if (nc - c0 <= (int64_t)(1ull << (L - 1))) {
+    bool done = false;
+    if constexpr (B1 > 3) {
+      // an operand of at most N/8 limbs leaves the upper half of the rows zero
+      // (coefficients N/2 and up): those inputs are neither read nor added
+      if (nc - c0 <= (int64_t)(1ull << (L - 1))) {
 #pragma unroll
-      for (int m = 0; m < (1 << (B1 - 1)); m++) x[m] = gl::Lz{m - ml < mc ? (uint32_t)__ldg(cn + m * step) : 0u, 0u, 0};
-      x[0] = gl::lz_bias(x[0]);
-      dft_lz<B1, false, true>(x, v);
-    } else {
+        for (int m = 0; m < (1 << (B1 - 1)); m++) x[m] = gl::Lz{m - ml < mc ? (uint32_t)__ldg(cn + m * step) : 0u, 0u, 0};
+        x[0] = gl::lz_bias(x[0]);
+        dft_lz<B1, false, true>(x, v);
+        done = true;
+      }
+    }
+    if (!done) {
 #pragma unroll
       for (int m = 0; m < (1 << B1); m++) x[m] = gl::Lz{m - ml < mc ? (uint32_t)__ldg(cn + m * step) : 0u, 0u, 0};
       x[0] = gl::lz_bias(x[0]);
@@ -1726,7 +1731,7 @@ static void build_roots(uint64_t* t) {
       }
   // round twiddles of the passes
   uint64_t* rt = nt + (size_t)NEAR_LEVELS * 2 * 4096;
-  for (int r = 6; r <= 9; r++) {
+  for (int r = 5; r <= 9; r++) {
     const uint64_t* w = lvl + (1u << r);
     const uint32_t n1 = 1u << pass_b1(r), n2 = 1u << pass_b2(r), n = 1u << r;
     for (uint32_t k = 0; k < n1; k++)
@@ -2120,39 +2125,43 @@ static int default_np(int L) {
   return np < 2 ? 2 : np;
 }
 
-// A plan is valid when every pass radix is 2^6 .. 2^9 and the first one at
-// least 2^7 (the compiled kernels).
-static bool plan_valid(const Plan& p) {
-  if (p.np < 2 || p.np > 5 || p.r[0] < 7) return false;
-  for (int i = 0; i < p.np; i++)
-    if (p.r[i] < 6 || p.r[i] > 9) return false;
-  return true;
-}
+// np passes for 2^L points, radices 2^6 .. 2^9 (a first one of at least 2^7 must
+// be possible: 2^18 in three passes is refused); an invalid plan (np 0) for
+// anything else.
+static bool plan_valid(const Plan& p) { return p.np != 0; }
 
-// np passes for 2^L points: the even split, longer passes first.  Every pass
-// is two rounds whatever its radix, so only the shifts inside the rounds
-// depend on the split, and they grow faster than the radix: 2^21 as 7 + 7 + 7
-// or 9 + 6 + 6 cost the same, uneven splits never less.
-static Plan split_plan(int L, int np) {
-  Plan p{L, np, {0, 0, 0, 0, 0}};
-  for (int i = 0; i < np; i++) p.r[i] = L / np + (i < L % np ? 1 : 0);
+// The splits.  Three passes: measured per length, the short radices first (a
+// lone 2^20-point product takes 49.6 us as 6 + 6 + 8, 52.9 as 7 + 7 + 6; 2^21
+// points 84.8 as 7 + 6 + 8, 87.7 as 7 + 7 + 7, 88.4 as 6 + 6 + 9; 2^25 points
+// 1285 as 8 + 8 + 9, 1301 as 9 + 8 + 8).  Two passes: even, the longer first (16
+// products of 2^15 points: 40.0 us as 8 + 7, 43.5 as 7 + 8, 45.3 as 6 + 9).  Four
+// and five: even, the longer last.
+static Plan make_plan_np(int L, int np) {
+  Plan p{L, 0, {0, 0, 0, 0, 0}};
+  if (np < 2 || np > 5 || L < 6 * np + 1 || L > 9 * np) return p;
+  p.np = np;
+  static const int three[9][3] = {{6, 6, 7}, {6, 6, 8}, {7, 6, 8}, {6, 8, 8}, {7, 8, 8}, {8, 8, 8}, {8, 8, 9}, {8, 9, 9}, {9, 9, 9}};
+  for (int i = 0; i < np; i++) {
+    const int from = np == 2 ? i : np - 1 - i;
+    p.r[i] = np == 3 ? three[L - 19][i] : L / np + (from < L % np ? 1 : 0);
+  }
   return p;
 }
 
-// Any request outside 2^0 .. 2^32 points (the entry points reject longer
-// transforms) and 2 .. 5 passes gets an invalid plan (np 0, which plan_valid
-// rejects).
-static Plan make_plan_np(int L, int np) {
-  if (L < 0 || L > 32 || np < 2 || np > 5) return Plan{L, 0, {0, 0, 0, 0, 0}};
-  return split_plan(L, np);
-}
-
-static Plan make_plan(int L) {
+// The plan for transforms of 2^L points, `points` of them in all: few of 2^17 or
+// 2^18 points run three short passes, whose threads hold 8 elements, where two
+// leave a warp or less per SM sub-partition with 32 elements a thread.  2^18
+// points: a lone product 31.0 us against 45.0, four 59.6 against 65.7, eight 90.8
+// against 82.3; 2^17 points: a lone one 26.7 against 35.9, two 39.1 against 45.3, four
+// 48.5 against 46.9.
+static Plan make_plan(int L, uint64_t points = ~0ull) {
   int np = (L >= 0 && L <= 32) ? g_tuned_np[L].load(std::memory_order_relaxed) : 0;
   if (np) {
     Plan p = make_plan_np(L, np);
     if (plan_valid(p)) return p;
   }
+  if (L == 17 && points <= 1ull << 18) return Plan{L, 3, {6, 6, 5, 0, 0}};
+  if (L == 18 && points <= 1ull << 20) return Plan{L, 3, {6, 6, 6, 0, 0}};
   return make_plan_np(L, default_np(L));
 }
 
@@ -2251,7 +2260,9 @@ static void carve_scratch(Job& J, uint8_t* base, bool square) {
   carve_carry(J, reinterpret_cast<uint64_t*>(base), z.nwin);
 }
 
-// Launch helpers (template dispatch on the pass radix).
+// Launch helpers (template dispatch on the pass radix; a last pass may be 2^5).
+#define PIMUL_DISPATCH_ROW(r, ...)                      \
+  if ((r) == 5) { constexpr int RR = 5; __VA_ARGS__; } else PIMUL_DISPATCH_R(r, __VA_ARGS__)
 #define PIMUL_DISPATCH_R(r, ...)                        \
   switch (r) {                                          \
     case 6: { constexpr int RR = 6; __VA_ARGS__; } break; \
@@ -2304,9 +2315,6 @@ static void launch_small(const SmallJob& job, const Roots& R, cudaStream_t st) {
   }
 }
 
-// Both operands of a transform up to this length (log2) go through each
-// forward pass in one launch.
-constexpr int MERGE_OPERANDS_LOG = 20;
 
 struct Launcher {
   cudaStream_t st;
@@ -2447,15 +2455,16 @@ static void tw_release_all() {
 // addends and further segments); max_chunk: largest carry-chunk count among
 // those.
 static void run_large(const Launcher& X, const Job* jobs, const Job& one, uint32_t nj, int L, uint32_t nc, uint64_t max_chunk) {
-  const Plan pl = make_plan(L);
+  const Plan pl = make_plan(L, (uint64_t)nj << L);
   const PassTables tw = X.tables ? pass_tables(pl, X.st) : PassTables{};
   // 2^-L (2^192 = 1); 0 when the inverse first pass's table applies it
   const uint64_t ninv = tw.first_inv ? 0 : hf::pow(hf::pow(2, 191), L);
   const int rl = pl.r[pl.np - 1];
   const bool one_operand = !jobs && is_square(one);
-  // both operands' passes in one launch while their arrays fit L2 together;
-  // longer transforms one operand after the other
-  const bool merged = L <= MERGE_OPERANDS_LOG && !X.b_ready && !one_operand;
+  // both operands in one launch per pass (unless b is still on its way up):
+  // half the launches and partial waves, 98.5 -> 87.8 us for a lone 2^21-point
+  // product, 5.46 -> 5.43 ms at 2^27, where the arrays are far larger than L2
+  const bool merged = !X.b_ready && !one_operand;
   const unsigned nz = merged ? 2 : 1;
   auto grid = [&](int tile, unsigned z) { return dim3((unsigned)(1ull << (L - tile)), nj, z); };
   for (int which = 0; which < (merged || one_operand ? 1 : 2); which++) {
@@ -2463,7 +2472,7 @@ static void run_large(const Launcher& X, const Job* jobs, const Job& one, uint32
     {
       KTimer kt(K_PACK, X.st, X.stats);
       PIMUL_DISPATCH_R(pl.r[0], {
-        constexpr int R = RR < 7 ? 7 : RR;
+        constexpr int R = RR;
         launch_pdl(k_fwd_first<R>, grid(ColGeom<R>::TILE, nz), PASS_THREADS, (ColGeom<R>::XWORDS + (1u << R)) * 8, X.st, jobs,
                    one, which, L, X.R, tw.first_fwd);
       });
@@ -2478,14 +2487,14 @@ static void run_large(const Launcher& X, const Job* jobs, const Job& one, uint32
       });
     }
     KTimer kt(K_PASS_FWD, X.st, X.stats);
-    PIMUL_DISPATCH_R(rl, {
+    PIMUL_DISPATCH_ROW(rl, {
       launch_pdl(k_fwd_last<RR>, grid(RowGeom<RR>::TILE, nz), PASS_THREADS, 4 * RowGeom<RR>::XWORDS * 8, X.st, jobs, one, which,
                  L, X.R);
     });
   }
   {
     KTimer kt(K_POINTWISE, X.st, X.stats);
-    PIMUL_DISPATCH_R(rl, {
+    PIMUL_DISPATCH_ROW(rl, {
       launch_pdl(k_inv_last<RR>, grid(RowGeom<RR>::TILE, 1), PASS_THREADS, 4 * RowGeom<RR>::XWORDS * 8, X.st, jobs, one, L,
                  ninv, X.R);
     });
@@ -2503,7 +2512,7 @@ static void run_large(const Launcher& X, const Job* jobs, const Job& one, uint32
   {
     KTimer kt(K_PASS_INV, X.st, X.stats);
     PIMUL_DISPATCH_R(pl.r[0], {
-      constexpr int R = RR < 7 ? 7 : RR;
+      constexpr int R = RR;
       launch_pdl(k_inv_first_carry<R>, grid(ColGeom<R>::TILE, 1), PASS_THREADS, (INV_FIRST_XWORDS<R> + (1u << R)) * 8, X.st,
                  jobs, one, L, X.R, tw.first_inv);
     });
@@ -2960,7 +2969,7 @@ static int plan_create(const size_t* la, const size_t* lb, size_t n, BatchPlan**
   if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&cs, cudaStreamNonBlocking);
   if (e == cudaSuccess) {
     // twiddle tables are never built inside a capture: build them first
-    for (const auto& bk : P->B.large) pass_tables(make_plan(bk.L), nullptr);
+    for (const auto& bk : P->B.large) pass_tables(make_plan(bk.L, (uint64_t)bk.nd << bk.L), nullptr);
     uint8_t* desc = P->dev + round256(P->B.arena_bytes);
     e = cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal);
     if (e == cudaSuccess) {

@@ -163,15 +163,24 @@ __device__ __forceinline__ void dif_stage(gl::Lz* x) {
   }
 }
 
-// DFT of 2^B lazy values (B = 3, 4, 5; INV: its unscaled inverse) with w =
+// DFT of 2^B lazy values (B = 2 .. 5; INV: its unscaled inverse) with w =
 // 2^(192 / 2^B), the 2^B-th root of unity: all internal twiddles are constant
 // shifts.  Natural-order folded outputs at v[STEP k].  x[0] carries the bias
 // of lz_bias; |k| <= 1 in the other inputs (e.g. products from lz_mul); x is
 // overwritten.  UPPER0 (forward): inputs 2^(B-1) .. are zero (not read).
 template <int B, bool INV, bool UPPER0 = false, int STEP = 1>
 __device__ __forceinline__ void dft_lz(gl::Lz* x, uint64_t* v) {
-  if constexpr (B == 3) {
-    static_assert(!UPPER0, "a zero upper half needs 16 points or more");
+  static_assert(!UPPER0 || B > 3, "a zero upper half needs 16 points or more");
+  if constexpr (B == 2) {
+    using namespace gl;
+    const Lz a = lz_add(x[0], x[2]), c = lz_sub(x[0], x[2]);
+    const Lz b = lz_add(x[1], x[3]);
+    const Lz d = lz_shl<48>(INV ? lz_sub(x[3], x[1]) : lz_sub(x[1], x[3]));
+    v[0] = fold(lz_add(a, b));
+    v[1 * STEP] = fold(lz_add(c, d));
+    v[2 * STEP] = fold(lz_sub(a, b));
+    v[3 * STEP] = fold(lz_sub(c, d));
+  } else if constexpr (B == 3) {
     dft8_lz<INV, STEP>(x, v);
   } else {
     constexpr int H = 1 << (B - 1);
@@ -375,7 +384,7 @@ __device__ __forceinline__ void round_inv_t(uint64_t* sm, const uint64_t* tw, in
 }
 
 // ----------------------------------------------------------- two-round passes
-// An HBM pass of radix 2^R (R = 6 .. 9) is two rounds in registers, radix
+// An HBM pass of radix 2^R (R = 5 .. 9) is two rounds in registers, radix
 // 2^B1 over rows 2^B2 apart and radix 2^B2 over the 2^B2 rows of each result,
 // with one exchange through shared memory between them: a length-512 DFT
 // costs one general twiddle product per element (w_512^(k1 m)) instead of the
@@ -434,9 +443,9 @@ struct RowGeom {
 // Round twiddles of a pass, in exchange order: forward w_(2^R)^(k1 m) at
 // [m 2^B1 + k1], inverse w_(2^R)^-(k1 m) at [k1 2^B2 + m] (L1-resident: 4 KB
 // per direction for R = 9).
-constexpr uint32_t RT_WORDS = 2 * ((1u << 10) - (1u << 6));
+constexpr uint32_t RT_WORDS = 2 * ((1u << 10) - (1u << 5));
 __host__ __device__ constexpr uint32_t rt_offset(int r, bool inverse) {
-  return 2 * ((1u << r) - (1u << 6)) + (inverse ? 1u << r : 0);
+  return 2 * ((1u << r) - (1u << 5)) + (inverse ? 1u << r : 0);
 }
 
 // Forward round 2 / inverse round 1 share the exchange layout (k1 fixed, m
