@@ -739,7 +739,7 @@ __device__ uint32_t chunk_function(const Job& J, uint64_t c, uint64_t nwin, int 
   return f;
 }
 
-// Carry normalisation in one pass (grid.x = chunk of 256 windows, grid.y =
+// Carry normalisation in one pass (chunks of 256 windows over grid.x, grid.y =
 // product).  A chunk's carry in almost always shows in the 32 windows to its
 // left, which warp 0 sums as well: no chunk waits for another.  Where all 32
 // pass a carry on (each all ones), the chunks' states are read instead: every
@@ -752,75 +752,77 @@ __device__ uint32_t chunk_function(const Job& J, uint64_t c, uint64_t nwin, int 
 // and 16 written per window; against three kernels (sums in place, scan,
 // increments) 240 -> 141 us at 2^27 points and two launches less.
 constexpr int CARRY_POLLS = 32;
+constexpr uint64_t CARRY_CTAS = 8192;  // of a batch (4096 and 16384 within 0.5 %)
 
 __global__ void __launch_bounds__(CARRY_THREADS) k_carry(const Job* jobs, Job one) {
   const Job J = job_of(jobs, one, 0);
   if (J.flags & (JF_ADDEND | JF_COEFF)) return;
   const uint64_t nlimbs = job_nout(J), nwin = n_windows_out(nlimbs), nchunk = n_chunks(nwin);
-  const uint64_t chunk = blockIdx.x;
-  if (chunk >= nchunk) return;  // uniform per CTA
   __shared__ uint32_t sA[CARRY_THREADS / 32], sB[CARRY_THREADS / 32], s_cin;
-  const uint64_t w = chunk * CARRY_THREADS + threadIdx.x;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const WinSum x = win_sum(J, w, nwin);
-  uint32_t left = 0;  // function of the 32 windows to the left (chunk 0: no carry)
-  if (warp == 0 && chunk > 0) {
-    const WinSum y = win_sum(J, w - 32, nwin);
-    const uint32_t yA = __ballot_sync(0xFFFFFFFFu, y.g || y.p), yB = __ballot_sync(0xFFFFFFFFu, y.g);
-    left = cf_of_masks(yA, yB);
-  }
-  const uint32_t A = __ballot_sync(0xFFFFFFFFu, x.g || x.p);
-  const uint32_t B = __ballot_sync(0xFFFFFFFFu, x.g);
-  if (lane == 0) {
-    sA[warp] = A;
-    sB[warp] = B;
-  }
-  __syncthreads();
-  if (warp == 0) {
-    uint32_t f = 2;
-    for (int k = 0; k < CARRY_THREADS / 32; k++) f = cf_then(f, cf_of_masks(sA[k], sB[k]));
-    volatile uint32_t* state = J.state;
-    if (lane == 0) state[chunk] = 4 | f;
-    uint32_t cin = left & 1;
-    // chunks chunk - 1 - lane, 32 at a time; left of chunk 0 the carry is 0
-    for (int64_t base = (int64_t)chunk - 1; left == 2; base -= 32) {
-      const int64_t c = base - lane;
-      uint32_t st = c < 0 ? 4 : state[c];
-      for (int poll = 0; poll < CARRY_POLLS && __any_sync(0xFFFFFFFFu, st == 0); poll++) {
-        if (st == 0) st = state[c];
-        // enough once a known chunk with a fixed carry out comes before the first unknown one
-        const uint32_t unknown = __ballot_sync(0xFFFFFFFFu, st == 0);
-        const uint32_t fixed = __ballot_sync(0xFFFFFFFFu, st != 0 && (st & 3) != 2);
-        if (fixed && (!unknown || __ffs(fixed) < __ffs(unknown))) break;
-      }
-      // the nearest chunk whose carry out is fixed (identity passes it on)
-      bool done = false;
-      for (int k = 0; k < 32; k++) {
-        uint32_t sk = __shfl_sync(0xFFFFFFFFu, st, k);
-        if (sk == 0) sk = 4 | chunk_function(J, (uint64_t)(base - k), nwin, lane);
-        if ((sk & 3) != 2) {
-          cin = sk & 1;
-          done = true;
-          break;
-        }
-      }
-      if (done) break;
+  for (uint64_t chunk = blockIdx.x; chunk < nchunk; chunk += gridDim.x) {  // uniform per CTA
+    const uint64_t w = chunk * CARRY_THREADS + threadIdx.x;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const WinSum x = win_sum(J, w, nwin);
+    uint32_t left = 0;  // function of the 32 windows to the left (chunk 0: no carry)
+    if (warp == 0 && chunk > 0) {
+      const WinSum y = win_sum(J, w - 32, nwin);
+      const uint32_t yA = __ballot_sync(0xFFFFFFFFu, y.g || y.p), yB = __ballot_sync(0xFFFFFFFFu, y.g);
+      left = cf_of_masks(yA, yB);
     }
+    const uint32_t A = __ballot_sync(0xFFFFFFFFu, x.g || x.p);
+    const uint32_t B = __ballot_sync(0xFFFFFFFFu, x.g);
     if (lane == 0) {
-      s_cin = cin;
-      // a chunk that passes its carry on now has a fixed one: look-backs stop here
-      if (f == 2) state[chunk] = 4 | (cin ? 3 : 0);
+      sA[warp] = A;
+      sB[warp] = B;
     }
-  }
-  __syncthreads();
-  uint32_t cin = s_cin;
-  for (int k = 0; k < warp; k++) cin = (cf_of_masks(sA[k], sB[k]) >> cin) & 1;
-  const uint32_t carries = (A + B + cin) ^ A ^ B;
-  if (w < nwin) {
-    const uint64_t inc = (carries >> lane) & 1;
-    const uint64_t s0 = x.s0 + inc, s1 = x.s1 + (inc && s0 == 0);
-    if (2 * w < nlimbs) J.out[2 * w] = s0;
-    if (2 * w + 1 < nlimbs) J.out[2 * w + 1] = s1;
+    __syncthreads();
+    if (warp == 0) {
+      uint32_t f = 2;
+      for (int k = 0; k < CARRY_THREADS / 32; k++) f = cf_then(f, cf_of_masks(sA[k], sB[k]));
+      volatile uint32_t* state = J.state;
+      if (lane == 0) state[chunk] = 4 | f;
+      uint32_t cin = left & 1;
+      // chunks chunk - 1 - lane, 32 at a time; left of chunk 0 the carry is 0
+      for (int64_t base = (int64_t)chunk - 1; left == 2; base -= 32) {
+        const int64_t c = base - lane;
+        uint32_t st = c < 0 ? 4 : state[c];
+        for (int poll = 0; poll < CARRY_POLLS && __any_sync(0xFFFFFFFFu, st == 0); poll++) {
+          if (st == 0) st = state[c];
+          // enough once a known chunk with a fixed carry out comes before the first unknown one
+          const uint32_t unknown = __ballot_sync(0xFFFFFFFFu, st == 0);
+          const uint32_t fixed = __ballot_sync(0xFFFFFFFFu, st != 0 && (st & 3) != 2);
+          if (fixed && (!unknown || __ffs(fixed) < __ffs(unknown))) break;
+        }
+        // the nearest chunk whose carry out is fixed (identity passes it on)
+        bool done = false;
+        for (int k = 0; k < 32; k++) {
+          uint32_t sk = __shfl_sync(0xFFFFFFFFu, st, k);
+          if (sk == 0) sk = 4 | chunk_function(J, (uint64_t)(base - k), nwin, lane);
+          if ((sk & 3) != 2) {
+            cin = sk & 1;
+            done = true;
+            break;
+          }
+        }
+        if (done) break;
+      }
+      if (lane == 0) {
+        s_cin = cin;
+        // a chunk that passes its carry on now has a fixed one: look-backs stop here
+        if (f == 2) state[chunk] = 4 | (cin ? 3 : 0);
+      }
+    }
+    __syncthreads();
+    uint32_t cin = s_cin;
+    for (int k = 0; k < warp; k++) cin = (cf_of_masks(sA[k], sB[k]) >> cin) & 1;
+    const uint32_t carries = (A + B + cin) ^ A ^ B;
+    if (w < nwin) {
+      const uint64_t inc = (carries >> lane) & 1;
+      const uint64_t s0 = x.s0 + inc, s1 = x.s1 + (inc && s0 == 0);
+      if (2 * w < nlimbs) J.out[2 * w] = s0;
+      if (2 * w + 1 < nlimbs) J.out[2 * w + 1] = s1;
+    }
+    __syncthreads();  // the next chunk reuses the shared words
   }
 }
 
@@ -2519,7 +2521,12 @@ static void run_large(const Launcher& X, const Job* jobs, const Job& one, uint32
   }
   {
     KTimer kt(K_CARRY, X.st, X.stats);
-    launch_pdl(k_carry, dim3((unsigned)max_chunk, nc), CARRY_THREADS, 0, X.st, jobs, one);
+    // a CTA per chunk of a lone product; in a batch of uneven lengths the CTAs
+    // of a product stride over its chunks (a CTA per chunk of the longest left
+    // nearly all of them without work: 630 of 7200 us in 4096 uneven products,
+    // 290 so)
+    const uint64_t per = std::min<uint64_t>(max_chunk, nc == 1 ? max_chunk : (CARRY_CTAS + nc - 1) / nc);
+    launch_pdl(k_carry, dim3((unsigned)per, nc), CARRY_THREADS, 0, X.st, jobs, one);
   }
 }
 
