@@ -697,6 +697,103 @@ __global__ void __launch_bounds__(PASS_THREADS, pass_min_ctas(R)) k_inv_first_ca
   }
 }
 
+// First and last pass of a transform of N = 3 2^k points (192 rows of stride
+// 2^S, S = k - 6); w_N = w_(2^k)^a w_3^b with 3 a + 2^k b = 1 mod N.  A product
+// that fills at most three quarters of its power of two takes three quarters
+// of the work.
+__global__ void __launch_bounds__(128, 5) k_fwd_first3(const Job* jobs, Job one, int w0, int S, Roots RT,
+                                                       const uint64_t* __restrict__ twf) {
+  using G = ThreeGeom;
+  const Job J = job_of(jobs, one, 0);
+  const int which = w0 + (int)blockIdx.z;
+  if (which == 1 && skips_b(J)) return;
+  const uint16_t* __restrict__ coef = reinterpret_cast<const uint16_t*>(which ? J.b : J.a);
+  const uint64_t nc = 4 * (which ? J.lb : J.la);
+  uint64_t* __restrict__ data = which ? J.B : J.A;
+  extern __shared__ uint64_t sm[];
+  const int tid = threadIdx.x;
+  const uint64_t j0 = (uint64_t)blockIdx.x << G::T;
+  if (tid < 96) {
+    // round 1: rows (tid >> 3) + 12 m
+    const uint64_t n0 = ((uint64_t)(tid >> 3) << S) + j0 + (tid & 7), step = 12ull << S;
+    uint64_t v[16];
+    gl::Lz x[16];
+    if (nc <= 96ull << S) {  // the upper half of the rows is zero
+#pragma unroll
+      for (int m = 0; m < 8; m++) x[m] = gl::Lz{n0 + m * step < nc ? (uint32_t)__ldg(coef + n0 + m * step) : 0u, 0u, 0};
+      x[0] = gl::lz_bias(x[0]);
+      dft_lz<4, false, true>(x, v);
+    } else {
+#pragma unroll
+      for (int m = 0; m < 16; m++) x[m] = gl::Lz{n0 + m * step < nc ? (uint32_t)__ldg(coef + n0 + m * step) : 0u, 0u, 0};
+      x[0] = gl::lz_bias(x[0]);
+      dft_lz<4, false>(x, v);
+    }
+#pragma unroll
+    for (int k = 0; k < 16; k++) sm[k * G::KS + tid] = v[k];
+  }
+  __syncthreads();
+  const uint64_t* __restrict__ rt = RT.rt + RT_WORDS;
+  const uint32_t j = tid & 7, k1 = tid >> 3;
+  uint64_t v[12];
+  gl::Lz x[12];
+  x[0] = gl::lz_bias(gl::lz(sm[k1 * G::KS + j]));
+#pragma unroll
+  for (int m = 1; m < 12; m++) x[m] = gl::lz_mul(sm[k1 * G::KS + m * 8 + j], __ldg(rt + m * 16 + k1));
+  dft12_lz<false>(x, v);
+  const uint64_t at = ((uint64_t)(k1 * 12) << S) + j0 + j;
+#pragma unroll
+  for (int k = 0; k < 12; k++) data[at + ((uint64_t)k << S)] = gl::mul(v[k], __ldg(twf + at + ((uint64_t)k << S)));
+}
+
+__global__ void __launch_bounds__(128, 5) k_inv_first3_carry(const Job* jobs, Job one, int S, Roots RT,
+                                                             const uint64_t* __restrict__ twi) {
+  using G = ThreeGeom;
+  const Job J = job_of(jobs, one, 0);
+  if (J.flags & JF_ADDEND) return;
+  const uint64_t* __restrict__ data = J.A;
+  extern __shared__ uint64_t sm[];
+  const int tid = threadIdx.x;
+  const uint64_t j0 = (uint64_t)blockIdx.x << G::T;
+  const uint64_t* __restrict__ rt = RT.rt + RT_WORDS + 192;
+  {
+    const uint32_t j = tid & 7, k1 = tid >> 3;
+    const uint64_t at = ((uint64_t)(k1 * 12) << S) + j0 + j;
+    uint64_t v[12];
+    gl::Lz x[12];
+#pragma unroll
+    for (int k = 0; k < 12; k++) v[k] = data[at + ((uint64_t)k << S)];
+#pragma unroll
+    for (int k = 0; k < 12; k++) x[k] = gl::lz_mul(v[k], __ldg(twi + at + ((uint64_t)k << S)));
+    x[0] = gl::lz_bias(x[0]);
+    dft12_lz<true>(x, v);
+#pragma unroll
+    for (int m = 0; m < 12; m++) sm[k1 * G::KS + m * 8 + j] = v[m];
+  }
+  __syncthreads();
+  const uint32_t m0 = tid >> 3;
+  uint64_t v[16];
+  if (tid < 96) {
+    gl::Lz x[16];
+    x[0] = gl::lz_bias(gl::lz(sm[tid]));
+#pragma unroll
+    for (int k = 1; k < 16; k++) x[k] = gl::lz_mul(sm[k * G::KS + tid], __ldg(rt + k * 12 + m0));
+    dft_lz<4, true>(x, v);
+  }
+  __syncthreads();
+  if (tid < 96) {
+#pragma unroll
+    for (int m = 0; m < 16; m++) sm[(m0 + 12 * m) * 9 + (tid & 7)] = gl::canon(v[m]);
+  }
+  __syncthreads();
+  for (uint32_t row = tid; row < G::ROWS; row += 128) {
+    uint64_t c[8];
+#pragma unroll
+    for (int t = 0; t < 8; t++) c[t] = sm[row * 9 + t];
+    put_window(J, 0, (((uint64_t)row << S) + j0) >> 3, c);
+  }
+}
+
 // Window w after its left neighbour's high part: s_w = lo_w + hi_(w-1), and
 // its (generate, propagate) bits; the windows past the end do neither.
 struct WinSum {
@@ -1697,7 +1794,7 @@ __global__ void __launch_bounds__(MERGE_THREADS, 2) k_split_merge(MergeLevel M, 
 static int log2_ceil(uint64_t x) { return x <= 1 ? 0 : 64 - __builtin_clzll(x - 1); }
 
 // Host copies of the root tables: lo, hi, w12, level tables (in this order).
-constexpr size_t ROOT_WORDS = 2 * 65536 + 4096 + (2u << LVL_MAX) + (size_t)NEAR_LEVELS * 2 * 4096 + RT_WORDS;
+constexpr size_t ROOT_WORDS = 2 * 65536 + 4096 + (2u << LVL_MAX) + (size_t)NEAR_LEVELS * 2 * 4096 + RT_WORDS + RT3_WORDS;
 
 static void build_roots(uint64_t* t) {
   uint64_t rho = find_rho();
@@ -1742,6 +1839,12 @@ static void build_roots(uint64_t* t) {
         rt[rt_offset(r, true) + k * n2 + m] = w[(n - k * m) & (n - 1)];
       }
   }
+  uint64_t* rt3 = rt + RT_WORDS;
+  for (uint32_t k = 0; k < 16; k++)
+    for (uint32_t m = 0; m < 12; m++) {
+      rt3[m * 16 + k] = hf::pow(2, k * m);
+      rt3[192 + k * 12 + m] = hf::pow(2, 192 - k * m);
+    }
 }
 
 static Roots roots_at(const uint64_t* d) {
@@ -2114,8 +2217,25 @@ void release_host_staging() {
 struct Plan {
   int L;
   int np;
-  int r[5];
+  int r[5];  // (r[0] unused for a length of 3 2^k points)
 };
+
+// Transform lengths: 2^L as L, 3 2^k as THREE + k (3 2^13 .. 3 2^15 and 3 2^17 ..
+// 3 2^24 points have passes).
+constexpr int THREE = 64;
+constexpr int N_LENGTHS = THREE + 33;
+// Points of 2^L that must be there for a batch to run them at 3 2^(L-2) beside
+// others of 2^L: six to nine launches more against a quarter of the work (2^20
+// .. 2^23: 4096 uneven products within 0.3 %, 512 short ones 616 us at 2^20, 593
+// from 2^22 on; 2^24: 7.17 against 6.99 ms).
+constexpr uint64_t THREE_SPLIT = 1ull << 22;
+static bool is_three(int L) { return L >= THREE; }
+// Whether 3 2^(L-2) points hold n coefficients and have passes.
+static bool three_holds(uint64_t n, int L) {
+  const int k = L - 2;
+  return k >= 13 && k != 16 && k <= 24 && n <= 3ull << k;
+}
+static uint64_t length_words(int L) { return is_three(L) ? 3ull << (L - THREE) : 1ull << L; }
 
 // Pass-count override per L chosen by the autotuner (0 = default).
 static std::atomic<int> g_tuned_np[33];
@@ -2157,6 +2277,13 @@ static Plan make_plan_np(int L, int np) {
 // against 82.3; 2^17 points: a lone one 26.7 against 35.9, two 39.1 against 45.3, four
 // 48.5 against 46.9.
 static Plan make_plan(int L, uint64_t points = ~0ull) {
+  if (is_three(L)) {
+    // 192 rows, then 2^S points in one pass or two, the shorter first
+    const int S = L - THREE - 6;
+    if (S <= 9) return Plan{L, 2, {0, S, 0, 0, 0}};
+    const int r1 = S <= 14 ? 6 : S / 2;
+    return Plan{L, 3, {0, r1, S - r1, 0, 0}};
+  }
   int np = (L >= 0 && L <= 32) ? g_tuned_np[L].load(std::memory_order_relaxed) : 0;
   if (np) {
     Plan p = make_plan_np(L, np);
@@ -2213,7 +2340,7 @@ static SegPlan plan_segments(uint64_t la, uint64_t lb) {
   if (la < lb) std::swap(la, lb);
   const Sizes z = sizes_for(la, lb);
   if (z.L <= SMALL_LOG_MAX + 1 || la < 2 * lb) return best;
-  double cost = 0.9 * 3 * transform_cost(z.L);
+  double cost = 0.9 * 3 * transform_cost(z.L) * (three_holds(z.n_out, z.L) ? 0.8 : 1.0);
   const uint64_t wlo = (4 * lb - 1 + WIN_COEFFS - 1) / WIN_COEFFS;
   for (int L = SMALL_LOG_MAX + 1; L < z.L; L++) {
     const uint64_t N = 1ull << L;
@@ -2355,6 +2482,24 @@ __global__ void k_tw_first(uint64_t* tw, int L, int inv, uint64_t scale, Roots R
   }
 }
 
+// The 192-row first pass of N = 3 2^k points: tw[i 2^S + J] = w_N^(+-f J) with f = i
+// / 12 + 16 (i mod 12) (inverse: times `scale`), w_N^x = w_(2^k)^(x / 3) w_3^(2^k x).
+__global__ void k_tw_first3(uint64_t* tw, int k, int inv, uint64_t scale, Roots RT) {
+  const int S = k - 6;
+  const uint64_t n = 3ull << k, smask = (1ull << S) - 1;
+  for (uint64_t e = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; e < n; e += (uint64_t)gridDim.x * blockDim.x) {
+    const uint32_t i = (uint32_t)(e >> S), J = (uint32_t)(e & smask);
+    const uint32_t x = (i / 12 + 16 * (i % 12)) * J;  // < 192 2^18
+    uint64_t t = root_pow32(RT, k, x * 0xAAAAAAABu, inv != 0);  // 3^-1 mod 2^32
+    uint32_t c = x % 3 * ((k & 1) ? 2 : 1) % 3;                // 2^k = 2^-k mod 3
+    if (inv) c = (3 - c) % 3;
+    if (c == 1) t = gl::mul(t, gl::EPS);                       // w_3 = 2^64
+    if (c == 2) t = gl::mul(t, gl::P - (1ull << 32));          // 2^128 = -2^32
+    if (inv) t = gl::mul(t, scale);
+    tw[e] = gl::canon(t);
+  }
+}
+
 template <int R>
 __global__ void k_tw_mid(uint64_t* tw, int S, int inv, Roots RT) {
   const int M = R + S;
@@ -2377,7 +2522,8 @@ static TwCache& tw_cache() {
   return *c;
 }
 
-// The table of one pass (kind 0: first pass, R + S = L; kind 1: middle pass),
+// The table of one pass (kind 0: first pass, R + S = L; kind 1: middle pass;
+// kind 2: 192-row first pass),
 // built on first use.  Null (compute the twiddles) when the shape is above
 // TW_LOG_MAX or the cap, while `caller` is capturing a graph (a table is
 // never built inside a capture), or when allocating it fails.
@@ -2390,7 +2536,7 @@ static const uint64_t* tw_table(int kind, int R, int S, bool inv, cudaStream_t c
   if (it != c.tables.end()) return it->second;
   cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
   if (caller && (cudaStreamIsCapturing(caller, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone)) return nullptr;
-  const uint64_t words = 1ull << (R + S);
+  const uint64_t words = kind == 2 ? 192ull << S : 1ull << (R + S);
   if (c.bytes + 8 * words > c.cap) return nullptr;
   if (!c.st && cudaStreamCreateWithFlags(&c.st, cudaStreamNonBlocking) != cudaSuccess) {
     cudaGetLastError();
@@ -2407,6 +2553,9 @@ static const uint64_t* tw_table(int kind, int R, int S, bool inv, cudaStream_t c
   if (kind == 0) {
     const uint64_t ninv = hf::pow(hf::pow(2, 191), (uint64_t)(R + S));  // 2^-L (2^192 = 1)
     PIMUL_DISPATCH_R(R, (k_tw_first<RR><<<blocks, 256, 0, c.st>>>(d, R + S, inv ? 1 : 0, ninv, RT)));
+  } else if (kind == 2) {
+    const uint64_t ninv = hf::mul(hf::pow(hf::pow(2, 191), (uint64_t)(S + 6)), hf::pow(3, hf::P - 2));  // 1 / (3 2^k)
+    k_tw_first3<<<blocks, 256, 0, c.st>>>(d, S + 6, inv ? 1 : 0, ninv, RT);
   } else {
     PIMUL_DISPATCH_R(R, (k_tw_mid<RR><<<blocks, 256, 0, c.st>>>(d, S, inv ? 1 : 0, RT)));
   }
@@ -2420,6 +2569,8 @@ static const uint64_t* tw_table(int kind, int R, int S, bool inv, cudaStream_t c
 }
 
 // Pointers of every pass table of a length-2^L plan (null entries: compute).
+// log2 stride of the first pass's rows.
+static int first_stride(const Plan& pl) { return is_three(pl.L) ? pl.L - THREE - 6 : pl.L - pl.r[0]; }
 struct PassTables {
   const uint64_t* first_fwd = nullptr;
   const uint64_t* first_inv = nullptr;  // carries N^-1: k_mid then skips its scaling
@@ -2428,16 +2579,29 @@ struct PassTables {
 };
 static PassTables pass_tables(const Plan& pl, cudaStream_t caller) {
   PassTables t;
-  const int L = pl.L;
-  t.first_fwd = tw_table(0, pl.r[0], L - pl.r[0], false, caller);
-  t.first_inv = tw_table(0, pl.r[0], L - pl.r[0], true, caller);
-  int consumed = pl.r[0];
+  int S = first_stride(pl);
+  const int kind = is_three(pl.L) ? 2 : 0, r0 = is_three(pl.L) ? 0 : pl.r[0];
+  t.first_fwd = tw_table(kind, r0, S, false, caller);
+  t.first_inv = tw_table(kind, r0, S, true, caller);
   for (int p = 1; p < pl.np - 1; p++) {
-    consumed += pl.r[p];
-    t.mid_fwd[p] = tw_table(1, pl.r[p], L - consumed, false, caller);
-    t.mid_inv[p] = tw_table(1, pl.r[p], L - consumed, true, caller);
+    S -= pl.r[p];
+    t.mid_fwd[p] = tw_table(1, pl.r[p], S, false, caller);
+    t.mid_inv[p] = tw_table(1, pl.r[p], S, true, caller);
   }
   return t;
+}
+
+// The length that `count` products of at most n coefficients take, L the power
+// of two at or above n: 3 2^(L-2) points where they hold n, have passes, and
+// have their twiddle tables (which a 192-row pass cannot do without: none above
+// the cache's cap, none built inside a capture).  At 70 % of a power of two:
+// 2.56 -> 2.05 ms (2^26), 158 -> 128.5 us (2^22), 83.1 -> 69.4 (2^21), 21.2 ->
+// 18.8 (2^15).  One or two of 2^17 points are left in their three short passes
+// (make_plan: 27.9 us against 29.8 for 3 2^15 in two passes).
+static int product_length(uint64_t n, int L, uint64_t count, cudaStream_t caller) {
+  if (!three_holds(n, L) || (L == 17 && count <= 2)) return L;
+  const PassTables t = pass_tables(make_plan(THREE + L - 2), caller);
+  return t.first_fwd && t.first_inv ? THREE + L - 2 : L;
 }
 
 static void tw_release_all() {
@@ -2451,16 +2615,18 @@ static void tw_release_all() {
 }
 
 // All launches of the large-product pipeline for `nj` products sharing the
-// transform length 2^L: the products come from the device array `jobs`
+// transform length L (see THREE): the products come from the device array `jobs`
 // (blockIdx.y) or, for nj == 1 and jobs == nullptr, from `one`.
 // nc: how many of them, from the first, have carries to run (the others are
 // addends and further segments); max_chunk: largest carry-chunk count among
 // those.
 static void run_large(const Launcher& X, const Job* jobs, const Job& one, uint32_t nj, int L, uint32_t nc, uint64_t max_chunk) {
-  const Plan pl = make_plan(L, (uint64_t)nj << L);
+  const uint64_t N = length_words(L);
+  const Plan pl = make_plan(L, nj * N);
+  const bool three = is_three(L);
   const PassTables tw = X.tables ? pass_tables(pl, X.st) : PassTables{};
   // 2^-L (2^192 = 1); 0 when the inverse first pass's table applies it
-  const uint64_t ninv = tw.first_inv ? 0 : hf::pow(hf::pow(2, 191), L);
+  const uint64_t ninv = tw.first_inv ? 0 : hf::pow(hf::pow(2, 191), L);  // (a length of 3 2^k points has its tables)
   const int rl = pl.r[pl.np - 1];
   const bool one_operand = !jobs && is_square(one);
   // both operands in one launch per pass (unless b is still on its way up):
@@ -2468,24 +2634,29 @@ static void run_large(const Launcher& X, const Job* jobs, const Job& one, uint32
   // product, 5.46 -> 5.43 ms at 2^27, where the arrays are far larger than L2
   const bool merged = !X.b_ready && !one_operand;
   const unsigned nz = merged ? 2 : 1;
-  auto grid = [&](int tile, unsigned z) { return dim3((unsigned)(1ull << (L - tile)), nj, z); };
+  auto grid = [&](int tile, unsigned z) { return dim3((unsigned)(N >> tile), nj, z); };
+  const int S0 = first_stride(pl);
   for (int which = 0; which < (merged || one_operand ? 1 : 2); which++) {
     if (which == 1 && X.b_ready) cudaStreamWaitEvent(X.st, X.b_ready, 0);
     {
       KTimer kt(K_PACK, X.st, X.stats);
-      PIMUL_DISPATCH_R(pl.r[0], {
+      if (three)
+        launch_pdl(k_fwd_first3, dim3(1u << (S0 - ThreeGeom::T), nj, nz), 128, ThreeGeom::XWORDS * 8, X.st, jobs, one, which, S0,
+                   X.R, tw.first_fwd);
+      else
+        PIMUL_DISPATCH_R(pl.r[0], {
         constexpr int R = RR;
         launch_pdl(k_fwd_first<R>, grid(ColGeom<R>::TILE, nz), PASS_THREADS, (ColGeom<R>::XWORDS + (1u << R)) * 8, X.st, jobs,
                    one, which, L, X.R, tw.first_fwd);
       });
     }
-    int consumed = pl.r[0];
+    int S = S0;
     for (int p = 1; p < pl.np - 1; p++) {
-      consumed += pl.r[p];
+      S -= pl.r[p];
       KTimer kt(K_PASS_FWD, X.st, X.stats);
       PIMUL_DISPATCH_R(pl.r[p], {
         launch_pdl(k_col_mid<RR, true>, grid(ColGeom<RR>::TILE, nz), PASS_THREADS, ColGeom<RR>::XWORDS * 8, X.st, jobs, one,
-                   which, L, L - consumed, X.R, tw.mid_fwd[p]);
+                   which, L, S, X.R, tw.mid_fwd[p]);
       });
     }
     KTimer kt(K_PASS_FWD, X.st, X.stats);
@@ -2501,10 +2672,8 @@ static void run_large(const Launcher& X, const Job* jobs, const Job& one, uint32
                  ninv, X.R);
     });
   }
-  int consumed = L - rl;
-  for (int p = pl.np - 2; p >= 1; p--) {
-    const int S = L - consumed;
-    consumed -= pl.r[p];
+  int S = rl;
+  for (int p = pl.np - 2; p >= 1; S += pl.r[p--]) {
     KTimer kt(K_PASS_INV, X.st, X.stats);
     PIMUL_DISPATCH_R(pl.r[p], {
       launch_pdl(k_col_mid<RR, false>, grid(ColGeom<RR>::TILE, 1), PASS_THREADS, ColGeom<RR>::XWORDS * 8, X.st, jobs, one, 0, L,
@@ -2513,6 +2682,10 @@ static void run_large(const Launcher& X, const Job* jobs, const Job& one, uint32
   }
   {
     KTimer kt(K_PASS_INV, X.st, X.stats);
+    if (three)
+      launch_pdl(k_inv_first3_carry, dim3(1u << (S0 - ThreeGeom::T), nj), 128, ThreeGeom::CWORDS * 8, X.st, jobs, one, S0, X.R,
+                 tw.first_inv);
+    else
     PIMUL_DISPATCH_R(pl.r[0], {
       constexpr int R = RR;
       launch_pdl(k_inv_first_carry<R>, grid(ColGeom<R>::TILE, 1), PASS_THREADS, (INV_FIRST_XWORDS<R> + (1u << R)) * 8, X.st,
@@ -2569,7 +2742,7 @@ static int mul_device(const uint64_t* d_a, uint64_t la, const uint64_t* d_b, uin
   }
   carve_scratch(J, base, square);
   Launcher X{st, true, R, b_ready};
-  run_large(X, nullptr, J, std::max(1u, sg.S), sg.L ? sg.L : z.L, 1, z.nchunk);
+  run_large(X, nullptr, J, std::max(1u, sg.S), sg.L ? sg.L : product_length(z.n_out, z.L, 1, st), 1, z.nchunk);
   cudaError_t le = cudaGetLastError();
   if (!scratch) cudaFreeAsync(base, st);
   if (le != cudaSuccess) return fail(PIMUL_ECUDA, std::string("kernel launch: ") + cudaGetErrorString(le));
@@ -2648,7 +2821,7 @@ static int unit_log_n(const Unit& u) {
 
 // share: let products with the same operand b borrow one spectrum (a batch
 // plan lays out a shape without pointers and never shares).
-static int layout_batch(const Unit* units, size_t n, BatchLayout& B, bool share) {
+static int layout_batch(const Unit* units, size_t n, BatchLayout& B, bool share, cudaStream_t st) {
   std::vector<int> Ls(n);
   for (size_t i = 0; i < n; i++) {
     Ls[i] = unit_log_n(units[i]);
@@ -2671,8 +2844,47 @@ static int layout_batch(const Unit* units, size_t n, BatchLayout& B, bool share)
       B.seg[i] = plan_segments(u.la, u.lb);
       if (B.seg[i].L) Ls[i] = B.seg[i].L;
     }
+    // three quarters of a power of two where that holds the product, and every
+    // other one of that power of two that shares its b (else the spectrum
+    // would be computed twice)
+    std::unordered_map<uint64_t, uint64_t> most;  // coefficients, by b and power of two
+    auto key = [](const uint64_t* b, int L) { return (uint64_t)(uintptr_t)b << 3 | (uint64_t)L; };
+    auto three_ok = [&](size_t i) { return Ls[i] > SMALL_LOG_MAX + 1 && !units[i].coeff && !units[i].forceL && !B.seg[i].L; };
+    if (share)
+      for (size_t i = 0; i < n; i++) {
+        const Unit& u = units[i];
+        if (Ls[i] <= SMALL_LOG_MAX || B.seg[i].L) continue;
+        const uint64_t need = three_ok(i) ? 4 * u.nout - 1 : ~0ull;
+        for (const uint64_t* b : {u.b, u.la2 ? u.b2 : nullptr})
+          if (b) {
+            uint64_t& m = most[key(b, Ls[i])];
+            m = std::max(m, need);
+          }
+      }
+    uint64_t all[33] = {}, fit[33] = {};  // transforms of 2^L, and those that could be shorter
+    std::vector<bool> shorter(n, false);
+    for (size_t i = 0; i < n; i++) {
+      const Unit& u = units[i];
+      const int L = Ls[i];
+      if (L <= SMALL_LOG_MAX) continue;
+      const uint64_t w = u.la2 ? 2 : B.seg[i].L ? B.seg[i].S : 1;
+      all[L] += w;
+      if (!three_ok(i)) continue;
+      uint64_t need = 4 * u.nout - 1;
+      if (share) {
+        need = std::max(need, most[key(u.b, L)]);
+        if (u.la2) need = std::max(need, most[key(u.b2, L)]);
+      }
+      shorter[i] = three_holds(need, L);
+      if (shorter[i]) fit[L] += w;
+    }
+    for (int L = SMALL_LOG_MAX + 1; L <= 32; L++)
+      if (fit[L] && (fit[L] == all[L] || fit[L] << L >= THREE_SPLIT)) fit[L] = (uint64_t)product_length(1, L, fit[L], st);
+      else fit[L] = (uint64_t)L;
+    for (size_t i = 0; i < n; i++)
+      if (shorter[i]) Ls[i] = (int)fit[Ls[i]];
   }
-  std::vector<std::vector<uint32_t>> byL(33);
+  std::vector<std::vector<uint32_t>> byL(N_LENGTHS);
   for (size_t i = 0; i < n; i++) {
     if (Ls[i] < 0) continue;
     if (Ls[i] <= SMALL_LOG_MAX && units[i].la2) return fail(PIMUL_EINVAL, "a sum of products below 2^13 in the pass pipeline");
@@ -2699,9 +2911,10 @@ static int layout_batch(const Unit* units, size_t n, BatchLayout& B, bool share)
   // fits BATCH_ARENA_CAP; groups run one after another on the stream, so
   // they all reuse the same arena.
   uint64_t arena = 0;
-  for (int L = 32; L > SMALL_LOG_MAX; L--) {
+  for (int q = 2 * 32; q > 2 * SMALL_LOG_MAX; q--) {
+    const int L = q % 2 ? THREE + (q + 1) / 2 - 2 : q / 2;  // 2^32, 3 2^30, 2^31, ...
     if (byL[L].empty()) continue;
-    const uint64_t N = 1ull << L;
+    const uint64_t N = length_words(L);
     size_t s = 0;
     while (s < byL[L].size()) {
       BatchLayout::Bucket bk{L, B.desc.size(), 0, 0, 0};
@@ -2897,7 +3110,7 @@ static uint8_t* host_image(size_t bytes) {
 
 static int run_units(const Unit* units, size_t n, cudaStream_t st, bool share) {
   BatchLayout B;
-  int rc = layout_batch(units, n, B, share);
+  int rc = layout_batch(units, n, B, share, st);
   if (rc) return rc;
   const size_t ns = B.small.size(), nl = B.desc.size();
   if (ns + nl == 0) return PIMUL_OK;
@@ -2964,7 +3177,7 @@ static int plan_create(const size_t* la, const size_t* lb, size_t n, BatchPlan**
   std::vector<Unit> shape(n);
   for (size_t i = 0; i < n; i++)
     shape[i] = unit_of(pimul_job{nullptr, la[i], (const uint64_t*)(uintptr_t)(8 + 16 * i), lb[i], nullptr});
-  rc = layout_batch(shape.data(), n, P->B, false);
+  rc = layout_batch(shape.data(), n, P->B, false, nullptr);
   if (rc) { delete P; return rc; }
   P->ns = P->B.small.size();
   P->nl = P->B.desc.size();
@@ -2976,7 +3189,7 @@ static int plan_create(const size_t* la, const size_t* lb, size_t n, BatchPlan**
   if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&cs, cudaStreamNonBlocking);
   if (e == cudaSuccess) {
     // twiddle tables are never built inside a capture: build them first
-    for (const auto& bk : P->B.large) pass_tables(make_plan(bk.L, (uint64_t)bk.nd << bk.L), nullptr);
+    for (const auto& bk : P->B.large) pass_tables(make_plan(bk.L, bk.nd * length_words(bk.L)), nullptr);
     uint8_t* desc = P->dev + round256(P->B.arena_bytes);
     e = cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal);
     if (e == cudaSuccess) {

@@ -197,6 +197,48 @@ __device__ __forceinline__ void dft_lz(gl::Lz* x, uint64_t* v) {
   }
 }
 
+// 3-point DFT (INV: its inverse) with the cube root of unity w = 2^64: with
+// 1 + w + w^2 = 0 both other outputs need only w (x1 - x2).
+template <bool INV>
+__device__ __forceinline__ void dft3_lz(gl::Lz x0, gl::Lz x1, gl::Lz x2, gl::Lz* y) {
+  using namespace gl;
+  const Lz t = lz_shl<64>(lz_sub(x1, x2));
+  y[0] = lz_add(x0, lz_add(x1, x2));
+  y[INV ? 2 : 1] = lz_add(lz_sub(x0, x2), t);
+  y[INV ? 1 : 2] = lz_sub(lz_sub(x0, x1), t);
+}
+
+// 12-point DFT (INV: its unscaled inverse) with w = 2^16: n = 4a + b, k = c +
+// 3d, a 3-point DFT over a, the twiddles w^(b c) = 2^(16 b c), a 4-point DFT
+// over b.  (w^-s = -2^(96 - s); w^6 = 2^96 = -1.)  As dft_lz otherwise.
+template <bool INV>
+__device__ __forceinline__ void dft12_lz(const gl::Lz* x, uint64_t* v) {
+  using namespace gl;
+  Lz y[4][3];
+#pragma unroll
+  for (int b = 0; b < 4; b++) dft3_lz<INV>(x[b], x[4 + b], x[8 + b], y[b]);
+#pragma unroll
+  for (int c = 0; c < 3; c++) {
+    Lz z1 = y[1][c], z2 = y[2][c], z3 = y[3][c];
+    // the inverse's twiddles are those of 96 - s with the sign of z_b turned
+    constexpr bool NEG = INV;
+    if (c == 1) z1 = lz_shl<INV ? 80 : 16>(z1), z2 = lz_shl<INV ? 64 : 32>(z2), z3 = lz_shl<48>(z3);
+    if (c == 2) z1 = lz_shl<INV ? 64 : 32>(z1), z2 = lz_shl<INV ? 32 : 64>(z2);
+    const bool n1 = c > 0 && NEG, n2 = c > 0 && NEG;
+    const bool n3 = c == 2 || (c == 1 && NEG);  // 2^96 = 2^-96 = -1 for c = 2
+    const Lz a = n2 ? lz_sub(y[0][c], z2) : lz_add(y[0][c], z2);
+    const Lz e = n2 ? lz_add(y[0][c], z2) : lz_sub(y[0][c], z2);
+    // b = z1 + z3 and z1 - z3 with their signs
+    const Lz s = n1 == n3 ? lz_add(z1, z3) : lz_sub(z1, z3);
+    const Lz d = n1 == n3 ? lz_sub(z1, z3) : lz_add(z1, z3);
+    const Lz t = lz_shl<48>(d);
+    v[c] = fold(n1 ? lz_sub(a, s) : lz_add(a, s));
+    v[c + 6] = fold(n1 ? lz_add(a, s) : lz_sub(a, s));
+    v[c + 3] = fold((n1 != INV) ? lz_sub(e, t) : lz_add(e, t));
+    v[c + 9] = fold((n1 != INV) ? lz_add(e, t) : lz_sub(e, t));
+  }
+}
+
 // Forward DFT of 2^B values in registers (radix 2, 4, 8), for the rounds of
 // the merged splitting levels: lazy inputs with |k| <= 1, folded outputs.
 template <int B>
@@ -447,6 +489,18 @@ constexpr uint32_t RT_WORDS = 2 * ((1u << 10) - (1u << 5));
 __host__ __device__ constexpr uint32_t rt_offset(int r, bool inverse) {
   return 2 * ((1u << r) - (1u << 5)) + (inverse ? 1u << r : 0);
 }
+
+// First passes of 192 = 16 x 12 rows, for transforms of 3 2^k points: output k1
+// of the radix-16 round and k2 of the radix-12 round (row 12 k1 + k2) hold
+// frequency k1 + 16 k2.  2 is the 192nd root of unity: the round twiddles are
+// 2^(k1 m) at [m 16 + k1] and 2^-(k1 m) at [k1 12 + m], behind the others.
+constexpr uint32_t RT3_WORDS = 2 * 192;
+struct ThreeGeom {
+  static constexpr int T = 3;                       // eight columns
+  static constexpr uint32_t ROWS = 192, KS = 12 * 8 + 8;
+  static constexpr uint32_t XWORDS = 16 * KS;
+  static constexpr uint32_t CWORDS = ROWS * 9;      // coefficients, one pad word per row
+};
 
 // Forward round 2 / inverse round 1 share the exchange layout (k1 fixed, m
 // over the inputs); forward round 1 / inverse round 2 have m fixed.

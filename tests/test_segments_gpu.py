@@ -61,7 +61,9 @@ def test_batches_and_plans_of_uneven_products():
             got = o.cpu().numpy().view(np.uint64)
             assert np.array_equal(got[: w.size], w) and not got[w.size :].any()
             o.fill_(-1)
+        torch.cuda.synchronize()
 
+    torch.cuda.synchronize()
     pm.mul_batch(jobs)
     check()
     plan = pm.BatchPlan([a.size for a, _ in host], [b.size for _, b in host])

@@ -55,6 +55,7 @@ def test_side_by_side_in_a_batch(kind):
         if i % 4 == 3:  # a square
             db, ops[i] = da, (a, a)
         jobs.append((da, db, torch.full((da.numel() + db.numel(),), -1, dtype=torch.int64, device="cuda")))
+    torch.cuda.synchronize()
     pm.mul_batch(jobs)
     torch.cuda.synchronize()
     for (a, b), (_, _, o) in zip(ops, jobs):
