@@ -269,9 +269,11 @@ __device__ __forceinline__ uint32_t pow2_mod_odd32(uint64_t E, uint32_t m, uint3
 //    y < 2m) brings a doubled y < 4m < 2^32 below 2m.
 // A step is one wide and two narrow multiplications, one three-input add and
 // the doubling: 64 positions below 5e7 took 103 ms with the reduced values of
-// mont_mul31 and all 32 bits run, 80 ms so.  x starts as 2^32 - q m for a float underestimate q of
-// 2^32 / m: below m + 2^12 (at most 2m, or a small m whose first steps
-// absorb it).  E's bits run from the top group of four that is not zero.
+// mont_mul31 and all 32 bits run, 80 ms so, 73.6 with the start below.
+// x starts as 2^(32 + g) - q m for the top group of four bits g of E (E < 2^32;
+// g = 0 otherwise, and for m < 2^15, where q would pass 32 bits) and a float
+// underestimate q of 2^(32 + g) / m: below m + 2^(12 + g) (at most 2m for
+// RED; the first steps absorb the rest).  The other groups run from the top.
 // The last product with 1 gives r = m - hi(u m), in [1, m) since m does not
 // divide a power of two.
 template <bool RED>
@@ -285,16 +287,24 @@ __device__ __forceinline__ uint32_t pow2_step(uint32_t x, uint32_t bit, uint32_t
 
 template <bool RED>
 __device__ __forceinline__ uint32_t pow2_mod_lazy(uint64_t E, uint32_t m, uint32_t minv) {
-  const uint32_t q = __float2uint_rz(__fmul_rn(__frcp_rn((float)m), 4294965248.0f));  // 2^32 (1 - 2^-21)
-  uint32_t x = 0u - q * m;
   uint32_t eh = (uint32_t)(E >> 32), el = (uint32_t)E;
   int groups = 8;
+  uint32_t g = 0;
+  if (!eh) {
+    groups = (35 - __clz((int)el)) >> 2;
+    el <<= 32 - 4 * groups;
+    if (m >= 1u << 15) {
+      g = el >> 28;
+      el <<= 4;
+      groups--;
+    }
+  }
+  const float scale = __uint_as_float(0x4F7FFFF8u + (g << 23));  // 2^(32 + g) (1 - 2^-21)
+  const uint32_t q = __float2uint_rz(__fmul_rn(__frcp_rn((float)m), scale));
+  uint32_t x = 0u - q * m;
   if (eh) {
     int b = 32 - __clz((int)eh);
     for (eh <<= 32 - b; b > 0; b--, eh <<= 1) x = pow2_step<RED>(x, eh >> 31, m, minv);
-  } else {
-    groups = (35 - __clz((int)el)) >> 2;
-    el <<= 32 - 4 * groups;
   }
 #pragma unroll 1
   for (; groups > 0; groups--) {
