@@ -63,8 +63,6 @@ __device__ __forceinline__ uint64_t sub(uint64_t a, uint64_t b) {
 // Canonical representative in [0, p).
 __device__ __forceinline__ uint64_t canon(uint64_t x) { return x >= P ? x - P : x; }
 
-__device__ __forceinline__ uint64_t neg(uint64_t a) { return sub(0, a); }
-
 // 128-bit value (x3 x2 x1 x0) -> weak 64-bit:  (x1:x0) + x2 * (2^32 - 1) - x3.
 // The multiply-add of x2 (on the FMA pipe) carries at most once; the sum's
 // net carry k in {-1, 0, 1} is worth k * 2^64 = k * EPS, and adding that
@@ -86,10 +84,6 @@ __device__ __forceinline__ uint64_t reduce_words(uint32_t r0, uint32_t r1, uint3
       : "=&r"(z0), "=&r"(z1)
       : "r"(r0), "r"(r1), "r"(r2), "r"(r3));
   return mk64(z0, z1);
-}
-
-__device__ __forceinline__ uint64_t reduce128(uint64_t lo, uint64_t hi) {
-  return reduce_words(lo32(lo), hi32(lo), lo32(hi), hi32(hi));
 }
 
 // 64x64 -> 128 product from four 32x32 partial products.
@@ -116,27 +110,6 @@ __device__ __forceinline__ uint64_t mul(uint64_t a, uint64_t b) {
   uint32_t r0, r1, r2, r3;
   mul128(a, b, r0, r1, r2, r3);
   return reduce_words(r0, r1, r2, r3);
-}
-
-// x * 2^s mod p for a compile-time 0 <= s < 192 (2^96 = -1, 2^192 = 1).
-template <int S>
-__device__ __forceinline__ uint64_t shl(uint64_t x) {
-  static_assert(S >= 0 && S < 192, "shift out of range");
-  if constexpr (S >= 96) {
-    return neg(shl<S - 96>(x));
-  } else if constexpr (S == 0) {
-    return x;
-  } else if constexpr (S < 64) {
-    uint64_t lo = x << S, hi = x >> (64 - S);
-    return reduce128(lo, hi);
-  } else {
-    // x * 2^S = (x << (S-64)) * 2^64; with y = x << (S-64) = (yh:yl),
-    // y * 2^64 = yl * 2^64 + yh * 2^128 and 2^128 = -2^32 (mod p).
-    constexpr int T = S - 64;
-    uint64_t yl = T ? (x << T) : x;
-    uint64_t yh = T ? (x >> (64 - T)) : 0;  // < 2^32
-    return sub(reduce128(0, yl), yh << 32);
-  }
 }
 
 // ------------------------------------------------------------ lazy values

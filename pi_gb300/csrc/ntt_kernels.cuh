@@ -55,18 +55,8 @@ __device__ __forceinline__ uint64_t rho_pow(const Roots& R, uint32_t e) {
   return h ? gl::mul(a, __ldg(R.hi + h)) : a;
 }
 
-// w_M^x for M = 2^mlog, x in [0, M); inverse gives w_M^(-x).  Levels up
-// to 2^20 read one contiguous table; longer ones combine two table entries.
-__device__ __forceinline__ uint64_t root_pow(const Roots& R, int mlog, uint64_t x, bool inverse) {
-  uint64_t m = 1ull << mlog;
-  x &= m - 1;
-  if (inverse) x = (m - x) & (m - 1);
-  if (mlog <= LVL_MAX) return __ldg(R.lvl + m + x);
-  return rho_pow(R, (uint32_t)(x << (32 - mlog)));
-}
-
-// root_pow for an exponent already reduced mod 2^32 (x is taken mod 2^mlog),
-// with 32-bit index arithmetic.
+// w_M^x for M = 2^mlog and x mod 2^mlog; inverse gives w_M^(-x).  Levels up to
+// 2^20 read one contiguous table; longer ones combine two table entries.
 __device__ __forceinline__ uint64_t root_pow32(const Roots& R, int mlog, uint32_t x, bool inverse) {
   const uint32_t mask = mlog >= 32 ? 0xFFFFFFFFu : (1u << mlog) - 1;
   x &= mask;
