@@ -234,6 +234,8 @@ __device__ __forceinline__ void pdl_wait() {
   asm volatile("griddepcontrol.launch_dependents;\n\tgriddepcontrol.wait;" ::: "memory");
 }
 
+__device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
+
 // Segment s of a segmented product whose first segment is J.
 __host__ __device__ __forceinline__ void to_segment(Job& J, uint32_t s, int L) {
   J.A += (uint64_t)s << L;
@@ -464,13 +466,15 @@ __global__ void __launch_bounds__(PASS_THREADS, pass_min_ctas(R)) k_fwd_last(con
   }
 }
 
-// Pointwise product of the two spectra (plus X Y, a second product, for a sum;
-// times N^-1, the inverse's 1/N, crates/bignum/src/ntt.rs:383-390 and
-// 845-853), entering the first inverse pass as lazy products; the result
-// overwrites A.  ninv = 0: no scaling here (the inverse first pass's twiddle
-// table carries N^-1).
+// Pointwise product of the two spectra (plus X Y, a second product, for a sum),
+// entering the first inverse pass as lazy products; the result overwrites A.
+// (The inverse's 1/N, crates/bignum/src/ntt.rs:383-390 and 845-853, comes with
+// its last pass's twiddles; a scaling here, though skipped where those have a
+// table, cost 0.3 to 1.3 % of a whole product in instruction cache misses.)
+// The second iteration's words are fetched into L2 while the first one runs: a
+// 2^30-bit product 5420 -> 5377 us, shorter ones as before.
 template <int R>
-__global__ void __launch_bounds__(PASS_THREADS, pass_min_ctas(R)) k_inv_last(const Job* jobs, Job one, int L, uint64_t ninv, Roots RT) {
+__global__ void __launch_bounds__(PASS_THREADS, pass_min_ctas(R)) k_inv_last(const Job* jobs, Job one, int L, Roots RT) {
   using G = RowGeom<R>;
   constexpr int B1 = G::B1, B2 = G::B2;
   const Job J = job_of(jobs, one, L);
@@ -488,6 +492,11 @@ __global__ void __launch_bounds__(PASS_THREADS, pass_min_ctas(R)) k_inv_last(con
   uint64_t* __restrict__ chunk = J.A + off;
   const uint64_t* __restrict__ bspec = J.B + off;
   uint64_t* sw = sm + warp * G::XWORDS;
+  constexpr uint32_t LINE = 16;  // words of 128 bytes
+  for (uint32_t t = G::WWORDS / G::ITERS2 + LINE * lane; t < G::WWORDS; t += LINE * 32) {
+    prefetch_l2(chunk + t);
+    if (!sq) prefetch_l2(bspec + t);
+  }
 #pragma unroll 1
   for (int it = 0; it < G::ITERS2; it++) {
     const uint32_t idx = it * 32 + lane, blk = idx >> B1;
@@ -504,17 +513,13 @@ __global__ void __launch_bounds__(PASS_THREADS, pass_min_ctas(R)) k_inv_last(con
       for (int k = 0; k < (1 << B2); k++) y[k] = bspec[at + (k << 5)];
     }
     if (J.X) {
-      // a b + X Y in lazy form (|k| <= 2), folded before the scaling or the DFT
       const uint64_t* __restrict__ X = J.X + off;
       const uint64_t* __restrict__ Y = J.Y + off;
 #pragma unroll
-      for (int k = 0; k < (1 << B2); k++) {
-        v[k] = gl::add(gl::mul(v[k], y[k]), gl::mul(X[at + (k << 5)], Y[at + (k << 5)]));
-        x[k] = gl::lz(ninv ? gl::mul(v[k], ninv) : v[k]);
-      }
+      for (int k = 0; k < (1 << B2); k++) x[k] = gl::lz(gl::add(gl::mul(v[k], y[k]), gl::mul(X[at + (k << 5)], Y[at + (k << 5)])));
     } else {
 #pragma unroll
-      for (int k = 0; k < (1 << B2); k++) x[k] = gl::lz_mul(v[k], ninv ? gl::mul(y[k], ninv) : y[k]);
+      for (int k = 0; k < (1 << B2); k++) x[k] = gl::lz_mul(v[k], y[k]);
     }
     x[0] = gl::lz_bias(x[0]);
     dft_lz<B2, true>(x, v);
@@ -625,14 +630,14 @@ __device__ __forceinline__ void put_window(const Job& J, int L, uint64_t wl, uin
 // row holds 2^T consecutive coefficients = 2^(T-3) windows; every window
 // writes its low 2 limbs to W and its high part to H.
 // twi: the pass's twiddle table (tw_first, inverse, with N^-1), or null to
-// compute the twiddles (the caller then scales by N^-1 in k_inv_last).
+// compute the twiddles, times ninv = N^-1.
 // The rows are handed to the windows through shared memory, one pad word each.
 template <int R>
 constexpr uint32_t INV_FIRST_XWORDS = ColGeom<R>::XWORDS > ((ColGeom<R>::TM + 2) << R) ? ColGeom<R>::XWORDS
                                                                                       : (ColGeom<R>::TM + 2) << R;
 template <int R>
 __global__ void __launch_bounds__(PASS_THREADS, pass_min_ctas(R)) k_inv_first_carry(const Job* jobs, Job one, int L, Roots RT,
-                                                                                 const uint64_t* __restrict__ twi) {
+                                                                                 const uint64_t* __restrict__ twi, uint64_t ninv) {
   using G = ColGeom<R>;
   constexpr int B1 = G::B1, B2 = G::B2, T = G::T;
   const Job J = job_of(jobs, one, L);
@@ -646,7 +651,7 @@ __global__ void __launch_bounds__(PASS_THREADS, pass_min_ctas(R)) k_inv_first_ca
   const bool staged = !twi && L > LVL_MAX;
   if (staged) {
     // w^-(f (j0 + j)) = w^-(f j0) w^-(f j), as in k_fwd_first
-    for (uint32_t f = tid; f < (1u << R); f += PASS_THREADS) tw[f] = root_pow32(RT, L, f * (uint32_t)j0, true);
+    for (uint32_t f = tid; f < (1u << R); f += PASS_THREADS) tw[f] = gl::mul(root_pow32(RT, L, f * (uint32_t)j0, true), ninv);
     __syncthreads();
   }
 #pragma unroll 1
@@ -670,7 +675,7 @@ __global__ void __launch_bounds__(PASS_THREADS, pass_min_ctas(R)) k_inv_first_ca
     } else {
 #pragma unroll
       for (int k = 0; k < (1 << B2); k++)
-        x[k] = gl::lz_mul(v[k], root_pow32(RT, L, (k1 + (k << B1)) * (uint32_t)(j0 + j), true));
+        x[k] = gl::lz_mul(v[k], gl::mul(root_pow32(RT, L, (k1 + (k << B1)) * (uint32_t)(j0 + j), true), ninv));
     }
     x[0] = gl::lz_bias(x[0]);
     dft_lz<B2, true>(x, v);
@@ -2247,9 +2252,6 @@ static int default_np(int L) {
   return np < 2 ? 2 : np;
 }
 
-// np passes for 2^L points, radices 2^6 .. 2^9 (a first one of at least 2^7 must
-// be possible: 2^18 in three passes is refused); an invalid plan (np 0) for
-// anything else.
 static bool plan_valid(const Plan& p) { return p.np != 0; }
 
 // The splits.  Three passes: measured per length, the short radices first (a
@@ -2257,7 +2259,8 @@ static bool plan_valid(const Plan& p) { return p.np != 0; }
 // points 84.8 as 7 + 6 + 8, 87.7 as 7 + 7 + 7, 88.4 as 6 + 6 + 9; 2^25 points
 // 1285 as 8 + 8 + 9, 1301 as 9 + 8 + 8).  Two passes: even, the longer first (16
 // products of 2^15 points: 40.0 us as 8 + 7, 43.5 as 7 + 8, 45.3 as 6 + 9).  Four
-// and five: even, the longer last.
+// and five: even, the longer last.  np passes must leave radices of 2^6 .. 2^9 and
+// one of at least 2^7; an invalid plan (np 0) for anything else.
 static Plan make_plan_np(int L, int np) {
   Plan p{L, 0, {0, 0, 0, 0, 0}};
   if (np < 2 || np > 5 || L < 6 * np + 1 || L > 9 * np) return p;
@@ -2568,12 +2571,12 @@ static const uint64_t* tw_table(int kind, int R, int S, bool inv, cudaStream_t c
   return d;
 }
 
-// Pointers of every pass table of a length-2^L plan (null entries: compute).
 // log2 stride of the first pass's rows.
 static int first_stride(const Plan& pl) { return is_three(pl.L) ? pl.L - THREE - 6 : pl.L - pl.r[0]; }
+// Pointers of every pass table of a plan (null entries: compute).
 struct PassTables {
   const uint64_t* first_fwd = nullptr;
-  const uint64_t* first_inv = nullptr;  // carries N^-1: k_mid then skips its scaling
+  const uint64_t* first_inv = nullptr;  // carries N^-1
   const uint64_t* mid_fwd[5] = {};
   const uint64_t* mid_inv[5] = {};
 };
@@ -2625,8 +2628,8 @@ static void run_large(const Launcher& X, const Job* jobs, const Job& one, uint32
   const Plan pl = make_plan(L, nj * N);
   const bool three = is_three(L);
   const PassTables tw = X.tables ? pass_tables(pl, X.st) : PassTables{};
-  // 2^-L (2^192 = 1); 0 when the inverse first pass's table applies it
-  const uint64_t ninv = tw.first_inv ? 0 : hf::pow(hf::pow(2, 191), L);  // (a length of 3 2^k points has its tables)
+  // 2^-L (2^192 = 1), unless the inverse first pass's table has it (a length of 3 2^k points has its tables)
+  const uint64_t ninv = tw.first_inv ? 0 : hf::pow(hf::pow(2, 191), L);
   const int rl = pl.r[pl.np - 1];
   const bool one_operand = !jobs && is_square(one);
   // both operands in one launch per pass (unless b is still on its way up):
@@ -2645,10 +2648,9 @@ static void run_large(const Launcher& X, const Job* jobs, const Job& one, uint32
                    X.R, tw.first_fwd);
       else
         PIMUL_DISPATCH_R(pl.r[0], {
-        constexpr int R = RR;
-        launch_pdl(k_fwd_first<R>, grid(ColGeom<R>::TILE, nz), PASS_THREADS, (ColGeom<R>::XWORDS + (1u << R)) * 8, X.st, jobs,
-                   one, which, L, X.R, tw.first_fwd);
-      });
+          launch_pdl(k_fwd_first<RR>, grid(ColGeom<RR>::TILE, nz), PASS_THREADS, (ColGeom<RR>::XWORDS + (1u << RR)) * 8, X.st,
+                     jobs, one, which, L, X.R, tw.first_fwd);
+        });
     }
     int S = S0;
     for (int p = 1; p < pl.np - 1; p++) {
@@ -2669,7 +2671,7 @@ static void run_large(const Launcher& X, const Job* jobs, const Job& one, uint32
     KTimer kt(K_POINTWISE, X.st, X.stats);
     PIMUL_DISPATCH_ROW(rl, {
       launch_pdl(k_inv_last<RR>, grid(RowGeom<RR>::TILE, 1), PASS_THREADS, 4 * RowGeom<RR>::XWORDS * 8, X.st, jobs, one, L,
-                 ninv, X.R);
+                 X.R);
     });
   }
   int S = rl;
@@ -2686,11 +2688,10 @@ static void run_large(const Launcher& X, const Job* jobs, const Job& one, uint32
       launch_pdl(k_inv_first3_carry, dim3(1u << (S0 - ThreeGeom::T), nj), 128, ThreeGeom::CWORDS * 8, X.st, jobs, one, S0, X.R,
                  tw.first_inv);
     else
-    PIMUL_DISPATCH_R(pl.r[0], {
-      constexpr int R = RR;
-      launch_pdl(k_inv_first_carry<R>, grid(ColGeom<R>::TILE, 1), PASS_THREADS, (INV_FIRST_XWORDS<R> + (1u << R)) * 8, X.st,
-                 jobs, one, L, X.R, tw.first_inv);
-    });
+      PIMUL_DISPATCH_R(pl.r[0], {
+        launch_pdl(k_inv_first_carry<RR>, grid(ColGeom<RR>::TILE, 1), PASS_THREADS, (INV_FIRST_XWORDS<RR> + (1u << RR)) * 8,
+                   X.st, jobs, one, L, X.R, tw.first_inv, ninv);
+      });
   }
   {
     KTimer kt(K_CARRY, X.st, X.stats);
@@ -3245,7 +3246,7 @@ static void plan_destroy(BatchPlan* P) {
 }
 
 // ------------------------------------------------------------------ autotuner
-// Times the candidate pass splits for each length in [Lmin, Lmax] on a
+// Times the candidate pass counts for each length in [Lmin, Lmax] on a
 // batch of `reps` synthetic products (device-resident), keeps the fastest,
 // and tunes the one-CTA kernel's persistent grid on a batch of small
 // products.  The choice only changes the schedule; products are identical.
