@@ -984,35 +984,6 @@ struct SmallChunk {
   int c;
 };
 
-// Forward (or unscaled inverse) transforms of NA arrays of 2^L words by a
-// group of NT threads: the pass kernels' rounds (radix 8, then 4) with
-// compile-time geometry, each round's twiddles applied as lazy products by
-// the next one, from the 4096-entry table of 4096th roots; one CTA barrier
-// per round.  Bit i of act: array i is transformed (idle groups and skipped
-// arrays pass the barriers only).
-template <int L, int NT, int NA, int Q = 0>
-__device__ __forceinline__ void group_fwd_c(uint64_t* a0, uint64_t* a1, uint64_t* a2, const uint64_t* tw, int tid,
-                                            unsigned act) {
-  if constexpr (Q < rp_count(L)) {
-    constexpr int B = rp_bits(L, Q), MLOG = rp_mlog(L, Q);
-    constexpr int PB = Q > 0 ? rp_bits(L, Q - 1) : 0, PMLOG = Q > 0 ? rp_mlog(L, Q - 1) : 0;
-    if (act & 1) round_fwd_t<L, 0, 0, B, MLOG, NT, PB, PMLOG, 12>(a0, tw, tid);
-    if constexpr (NA > 1) if (act & 2) round_fwd_t<L, 0, 0, B, MLOG, NT, PB, PMLOG, 12>(a1, tw, tid);
-    if constexpr (NA > 2) if (act & 4) round_fwd_t<L, 0, 0, B, MLOG, NT, PB, PMLOG, 12>(a2, tw, tid);
-    __syncthreads();
-    group_fwd_c<L, NT, NA, Q + 1>(a0, a1, a2, tw, tid, act);
-  }
-}
-
-template <int L, int NT, int Q = rp_count(L) - 1>
-__device__ __forceinline__ void group_inv_c(uint64_t* a0, const uint64_t* tw, int tid, bool act) {
-  if constexpr (Q >= 0) {
-    if (act) round_inv_t<L, 0, 0, rp_bits(L, Q), rp_mlog(L, Q), NT, 12>(a0, tw, tid);
-    __syncthreads();
-    group_inv_c<L, NT, Q - 1>(a0, tw, tid, act);
-  }
-}
-
 // Barrier of a product's T threads (group grp of the CTA).
 template <int T>
 __device__ __forceinline__ void small_sync(int grp) {
@@ -1094,6 +1065,42 @@ __device__ __forceinline__ void small_forward(const uint64_t* limbs, uint32_t nc
   }
 }
 
+// The inverse's rounds after its first one, on all T threads of the group:
+// natural order in sm.
+template <int C, int T>
+__device__ __forceinline__ void small_inverse(const Roots& R, uint64_t* sm, int t, int grp) {
+  constexpr int B1 = small_b(C, 0), B2 = small_b(C, 1), B3 = small_b(C, 2);
+  constexpr int S1 = C - B1, S2 = S1 - B2;
+  small_sync<T>(grp);
+  if constexpr (B3 > 0) {
+    for (uint32_t w = t; w < (1u << (C - B2)); w += T) {
+      const uint32_t j2 = w & ((1u << S2) - 1), k1 = w >> S2, base = (k1 << S1) + j2;
+      uint64_t v[1 << B2];
+      gl::Lz x[1 << B2];
+      x[0] = gl::lz_bias(gl::lz(sm[spad(base)]));
+#pragma unroll
+      for (int k = 1; k < (1 << B2); k++)
+        x[k] = gl::lz_mul(sm[spad(base + (k << S2))], __ldg(R.w12 + ((4096 - ((k * j2) << (12 - S1))) & 4095)));
+      dft_lz<B2, true>(x, v);
+#pragma unroll
+      for (int m = 0; m < (1 << B2); m++) sm[spad(base + (m << S2))] = v[m];
+    }
+    small_sync<T>(grp);
+  }
+  for (uint32_t j = t; j < (1u << S1); j += T) {
+    uint64_t v[1 << B1];
+    gl::Lz x[1 << B1];
+    x[0] = gl::lz_bias(gl::lz(sm[spad(j)]));
+#pragma unroll
+    for (int k = 1; k < (1 << B1); k++)
+      x[k] = gl::lz_mul(sm[spad((k << S1) + j)], __ldg(R.w12 + ((4096 - ((k * j) << (12 - C))) & 4095)));
+    dft_lz<B1, true>(x, v);
+#pragma unroll
+    for (int m = 0; m < (1 << B1); m++) sm[spad((m << S1) + j)] = v[m];
+  }
+  small_sync<T>(grp);
+}
+
 // One product by its T threads (t = thread in the group, grp = group of the
 // CTA).  SPLIT: threads 0 .. G - 1 hold operand a, the others b.
 template <int C, bool SPLIT>
@@ -1152,35 +1159,7 @@ __device__ __forceinline__ void small_multiply(const SmallJob& job, const Roots&
       for (int m = 0; m < (1 << BL); m++) smA[spad(base + m)] = v[m];
     }
   }
-  small_sync<T>(grp);
-  // the other inverse rounds run on all T threads
-  if constexpr (B3 > 0) {
-    for (uint32_t w = t; w < (1u << (C - B2)); w += T) {
-      const uint32_t j2 = w & ((1u << S2) - 1), k1 = w >> S2, base = (k1 << S1) + j2;
-      uint64_t v[1 << B2];
-      gl::Lz x[1 << B2];
-      x[0] = gl::lz_bias(gl::lz(smA[spad(base)]));
-#pragma unroll
-      for (int k = 1; k < (1 << B2); k++)
-        x[k] = gl::lz_mul(smA[spad(base + (k << S2))], __ldg(R.w12 + ((4096 - ((k * j2) << (12 - S1))) & 4095)));
-      dft_lz<B2, true>(x, v);
-#pragma unroll
-      for (int m = 0; m < (1 << B2); m++) smA[spad(base + (m << S2))] = v[m];
-    }
-    small_sync<T>(grp);
-  }
-  for (uint32_t j = t; j < (1u << S1); j += T) {
-    uint64_t v[1 << B1];
-    gl::Lz x[1 << B1];
-    x[0] = gl::lz_bias(gl::lz(smA[spad(j)]));
-#pragma unroll
-    for (int k = 1; k < (1 << B1); k++)
-      x[k] = gl::lz_mul(smA[spad((k << S1) + j)], __ldg(R.w12 + ((4096 - ((k * j) << (12 - C))) & 4095)));
-    dft_lz<B1, true>(x, v);
-#pragma unroll
-    for (int m = 0; m < (1 << B1); m++) smA[spad((m << S1) + j)] = v[m];
-  }
-  small_sync<T>(grp);
+  small_inverse<C, T>(R, smA, t, grp);
   // carry: windows of 16 coefficients, one per thread (N/16 <= T)
   const uint32_t n_out = 4 * la + 4 * lb - 1, nwin = (n_out + 15) / 16, nl = la + lb;
   uint64_t* sH = smB;  // b's spectrum is no longer needed
@@ -1577,16 +1556,17 @@ __global__ void __cluster_dims__(2 * ClusterGeom<L>::OP, 1, 1) __launch_bounds__
 // ---- merged binary-splitting levels (one node pair per thread group) ------
 // The lowest levels of a Chudnovsky splitting segment hold hundreds of
 // thousands of node pairs whose products all fit one CTA's shared memory.
-// A group of G = N/8 threads merges one pair (L, R) into
+// A group of T = N/16 threads merges one pair (L, R) into
 //   P = P_L P_R,  Q = Q_L Q_R,  T = T_L Q_R + P_L T_R
 // (magnitudes; crates/pi-core/src/algorithm/chudnovsky.rs:377-413).  The
 // spectra of Q_R and P_L serve two products each and T's two products are
 // added in the transform domain: six forward and three inverse transforms
 // per pair instead of eight and four, no temporaries in HBM and no separate
-// addition.  Three padded arrays per group; every CTA holds 512 threads and
-// 3 * 2^12 padded words whatever the level's length (2^L / 8 threads and
-// 3 * 2^L words per group).
-constexpr int MERGE_THREADS = 512;
+// addition.  Three padded arrays per group, 256 threads and at most 3 * 2^12
+// padded words per CTA, two CTAs per SM.  Bound by the integer pipes; against
+// radix-8 rounds by N/8 threads, three arrays at a time: pi to 10^8 digits 204.9 ->
+// 200.7 ms.
+constexpr int MERGE_THREADS = 256;
 
 struct MergeLevel {
   const uint64_t* in;
@@ -1599,51 +1579,32 @@ struct MergeLevel {
   int* bad;
 };
 
-__host__ __device__ __forceinline__ int merge_group_threads(int L) {
-  const int g = (1 << L) / 8;
-  return g < 32 ? 32 : g;
-}
+// Threads of a node pair: one radix-16 item (8 at 2^9 points) each, a warp or more.
+__host__ __device__ constexpr int merge_group_threads(int L) { return L == 8 ? 32 : small_op_threads(L); }
 __host__ __device__ __forceinline__ size_t merge_cta_smem(int L) {
   return (size_t)(MERGE_THREADS / merge_group_threads(L)) * 3 * spad(1u << L) * 8;
 }
 
-// Limbs x[0..n) -> 16-bit coefficients of an array of 2^Lp words (zero tail).
-__device__ __forceinline__ void group_pack(uint64_t* sm, const uint64_t* x, uint32_t n, int Lp, int tid, int G) {
-  for (uint32_t l = tid; l < (1u << Lp) / 4; l += G) {
-    const uint64_t v = l < n ? x[l] : 0;
-#pragma unroll
-    for (int q = 0; q < 4; q++) sm[spad(4 * l + q)] = (v >> (16 * q)) & 0xFFFF;
-  }
-}
-
 // Carry normalisation of a group's inverse-transformed array (exact
 // convolution values, below 2^45) into nl limbs at out, one 16-coefficient
-// window per thread (nl <= 2^Lp / 4 + 1, so the windows fit G = 2^Lp / 8
-// threads); sH (a free array) holds the windows' high parts.  Returns the
-// trimmed length to every thread of the group.  Same window arithmetic as
-// the one-CTA multiply above.
-__device__ uint32_t group_carry_store(const uint64_t* smX, int Lp, uint32_t nl, uint64_t* out, uint64_t* sH,
-                                      bool active, int gtid, int G, int gw0, uint32_t* sA, uint32_t* sBm,
-                                      uint32_t* sTop) {
-  const int tid = threadIdx.x;
-  const uint32_t N = 1u << Lp;
-  const uint32_t n_out = active && nl ? 4 * nl - 1 : 0;
-  const uint32_t nwin = (n_out + 15) / 16;
-  const uint32_t w = gtid;
+// window per thread: nl <= N/4 + 1, and a limb past the T windows takes the last
+// one's high part and carry.  Returns the trimmed length to every thread of the
+// group.  Same window arithmetic as the one-CTA multiply above.
+template <int C, int T>
+__device__ __forceinline__ uint32_t merge_carry(uint64_t* sm, uint32_t nl, uint64_t* out, int t, int grp, uint32_t* sA,
+                                                uint32_t* sBm, uint32_t* sTop) {
+  const uint32_t nwin = nl ? (4 * nl + 14) / 16 : 0, w = t;
   Win v{{0, 0, 0, 0}, 0};
-  if (w < nwin) {
+  if (w < nwin && w < (1u << C) / 16) {
     uint64_t c[16];
 #pragma unroll
-    for (int t = 0; t < 16; t++) {
-      const uint32_t idx = 16 * w + t;
-      c[t] = idx < N ? gl::canon(smX[spad(idx)]) : 0;
-    }
+    for (int q = 0; q < 16; q++) c[q] = gl::canon(sm[spad(16 * w + q)]);
     v = fold16(c, 1);
   }
-  __syncthreads();
-  if (w < nwin) sH[w] = v.hi;
-  __syncthreads();
-  const uint64_t hprev = (w > 0 && w - 1 < nwin) ? sH[w - 1] : 0;
+  small_sync<T>(grp);
+  sm[w] = v.hi;
+  small_sync<T>(grp);
+  const uint64_t hprev = w > 0 ? sm[w - 1] : 0;
   uint64_t s0 = v.l[0] + hprev;
   uint64_t c = s0 < hprev;
   uint64_t s1 = v.l[1] + c;  c = c && s1 == 0;
@@ -1652,146 +1613,160 @@ __device__ uint32_t group_carry_store(const uint64_t* smX, int Lp, uint32_t nl, 
   const bool gg = w < nwin && c;
   const bool pp = w < nwin && (s0 & s1 & s2 & s3) == ~0ull;
   const uint32_t A = __ballot_sync(0xFFFFFFFFu, gg || pp), Bm = __ballot_sync(0xFFFFFFFFu, gg);
-  if ((tid & 31) == 0) {
-    sA[tid >> 5] = A;
-    sBm[tid >> 5] = Bm;
-  }
-  __syncthreads();
+  const int gw0 = grp * (T / 32), gw = gw0 + (t >> 5);
   uint32_t cin = 0;
-  for (int k = gw0; k < (tid >> 5); k++) {
-    const uint64_t s = (uint64_t)sA[k] + sBm[k] + cin;
-    cin = (uint32_t)(s >> 32);
+  if constexpr (T > 32) {
+    if ((t & 31) == 0) sA[gw] = A, sBm[gw] = Bm;
+    small_sync<T>(grp);
+    for (int k = gw0; k < gw; k++) {
+      const uint64_t x = (uint64_t)sA[k] + sBm[k] + cin;
+      cin = (uint32_t)(x >> 32);
+    }
   }
-  const uint32_t carries = (A + Bm + cin) ^ A ^ Bm;
-  if ((carries >> (tid & 31)) & 1) {
+  const bool in = (((A + Bm + cin) ^ A ^ Bm) >> (t & 31)) & 1;
+  if (in) {
     if (++s0 == 0) if (++s1 == 0) if (++s2 == 0) ++s3;
   }
   uint32_t top = 0;
   if (w < nwin) {
-    const uint32_t base = 4 * w;
     const uint64_t s[4] = {s0, s1, s2, s3};
 #pragma unroll
     for (int q = 0; q < 4; q++)
-      if (base + q < nl) {
-        out[base + q] = s[q];
-        if (s[q]) top = base + q + 1;
+      if (4 * w + q < nl) {
+        out[4 * w + q] = s[q];
+        if (s[q]) top = 4 * w + q + 1;
       }
-  }
-  top = __reduce_max_sync(0xFFFFFFFFu, top);
-  if ((tid & 31) == 0) sTop[tid >> 5] = top;
-  __syncthreads();
-  uint32_t t = 0;
-  for (int k = gw0; k < gw0 + G / 32; k++) t = max(t, sTop[k]);
-  __syncthreads();  // sTop is reused by the next call
-  return t;
-}
-
-// One node pair (pair = true) or the copy of an odd last node (copy = true)
-// by one group of G = 2^L / 8 threads; an idle group passes the same
-// barriers.  Every pair of the level runs transforms of 2^L points (a pair
-// that needs fewer gets a longer transform, which changes nothing).
-template <int L>
-__device__ void merge_item(const MergeLevel& M, const uint64_t* tw, uint32_t item, bool pair, bool copy,
-                           uint64_t* X1, uint64_t* X2, uint64_t* X3, int gtid, int gw0, uint32_t* sA, uint32_t* sBm,
-                           uint32_t* sTop) {
-  constexpr int G = (1 << L) / 8;
-  constexpr uint32_t N = 1u << L;
-  const size_t in_stride = (size_t)M.sp + M.sq + M.st, out_stride = (size_t)M.op + M.oq + M.ot;
-  uint64_t* zp = M.out + (size_t)item * out_stride;
-  uint64_t* zq = zp + M.op;
-  uint64_t* zt = zq + M.oq;
-  if (copy) {
-    const uint32_t i = M.n_in - 1;
-    const uint64_t* p = M.in + (size_t)i * in_stride;
-    const uint32_t pn = M.in_len[3 * i], qn = M.in_len[3 * i + 1], tn = M.in_len[3 * i + 2];
-    for (uint32_t k = gtid; k < pn; k += G) zp[k] = p[k];
-    for (uint32_t k = gtid; k < qn; k += G) zq[k] = p[M.sp + k];
-    for (uint32_t k = gtid; k < tn; k += G) zt[k] = p[M.sp + M.sq + k];
-    if (gtid == 0) {
-      M.out_len[3 * item] = pn;
-      M.out_len[3 * item + 1] = qn;
-      M.out_len[3 * item + 2] = tn;
+    if (w == T - 1 && nwin > T) {
+      const uint64_t last = v.hi + (gg || (pp && in));
+      out[4 * T] = last;
+      if (last) top = 4 * T + 1;
     }
   }
-  uint32_t pl = 0, ql = 0, tl = 0, pr = 0, qr = 0, tr = 0;
-  const uint64_t *PL = nullptr, *QL = nullptr, *TL = nullptr, *PR = nullptr, *QR = nullptr, *TR = nullptr;
-  if (pair) {
-    const uint32_t l = 2 * item, r = l + 1;
-    pl = M.in_len[3 * l], ql = M.in_len[3 * l + 1], tl = M.in_len[3 * l + 2];
-    pr = M.in_len[3 * r], qr = M.in_len[3 * r + 1], tr = M.in_len[3 * r + 2];
-    PL = M.in + (size_t)l * in_stride, QL = PL + M.sp, TL = QL + M.sq;
-    PR = M.in + (size_t)r * in_stride, QR = PR + M.sp, TR = QR + M.sq;
+  top = __reduce_max_sync(0xFFFFFFFFu, top);
+  if constexpr (T > 32) {
+    if ((t & 31) == 0) sTop[gw] = top;
+    small_sync<T>(grp);
+    for (int k = gw0; k < gw0 + T / 32; k++) top = max(top, sTop[k]);
   }
+  small_sync<T>(grp);
+  return top;
+}
+
+// One node pair by a group of T threads.  Every pair of the level runs transforms
+// of 2^L points (a pair that needs fewer gets a longer transform, which changes
+// nothing).  The six operands go through one forward transform in a loop (six
+// copies of it would not fit the instruction caches), a thread's part of the
+// spectrum in registers: Q_R's and P_L's, times N^-1, stay in keep for the
+// products that share them, T_L Q_R waits in acc (both read by the thread that
+// wrote them).
+template <int L>
+__device__ __forceinline__ void merge_pair(const MergeLevel& M, const Roots& R, uint32_t item, uint64_t* work, uint64_t* acc,
+                                           uint64_t* keep, int t, int grp, uint32_t* sA, uint32_t* sBm, uint32_t* sTop) {
+  constexpr int T = merge_group_threads(L), G = small_op_threads(L);
+  constexpr int BL = small_b(L, 2) ? small_b(L, 2) : small_b(L, 1), ITL = (1 << (L - BL)) / G;
+  constexpr uint32_t N = 1u << L;
+  const size_t in_stride = (size_t)M.sp + M.sq + M.st, out_stride = (size_t)M.op + M.oq + M.ot;
+  const uint32_t* len = M.in_len + 6 * (size_t)item;  // P, Q, T of the left node, then the right one
+  const uint64_t* node = M.in + 2 * (size_t)item * in_stride;
+  const uint32_t pl = len[0], ql = len[1], tl = len[2], pr = len[3], qr = len[4], tr = len[5];
   const uint32_t n_p = pl + pr, n_q = ql + qr, n_t = max(tl + qr, pl + tr) + 1;
   // output coefficients of the longest product: 4 len - 1 <= 2^L
   const uint32_t need = max(max(n_p, n_q), max(tl + qr, pl + tr));
-  const bool fits = 4ull * need <= N + 1ull && n_p <= M.op && n_q <= M.oq && n_t <= M.ot;
-  if (pair && !fits && gtid == 0) atomicExch(M.bad, 1);
-  const bool act = pair && fits;
+  if (!(4ull * need <= N + 1ull && n_p <= M.op && n_q <= M.oq && n_t <= M.ot)) {
+    if (t == 0) atomicExch(M.bad, 1);
+    return;
+  }
   // N^-1 = 2^-L = p - (2^(64-L) - 2^(32-L))  (2^96 = -1, 2^64 = 2^32 - 1)
   constexpr uint64_t ninv = gl::P - ((1ull << (64 - L)) - (1ull << (32 - L)));
-
-  // Q_R, T_L, Q_L: X2 <- T_L Q_R, X3 <- Q_L Q_R N^-1
-  if (act) {
-    group_pack(X1, QR, qr, L, gtid, G);
-    group_pack(X2, TL, tl, L, gtid, G);
-    group_pack(X3, QL, ql, L, gtid, G);
-  }
-  __syncthreads();
-  group_fwd_c<L, G, 3>(X1, X2, X3, tw, gtid, act ? 7u : 0u);
-  for (uint32_t i = gtid; act && i < N; i += G) {
-    const uint64_t y = X1[spad(i)];
-    X2[spad(i)] = gl::mul(X2[spad(i)], y);
-    X3[spad(i)] = gl::mul(gl::mul(X3[spad(i)], y), ninv);
-  }
-  __syncthreads();
-  group_inv_c<L, G>(X3, tw, gtid, act);
-  const uint32_t q_len = group_carry_store(X3, L, n_q, zq, X1, act, gtid, G, gw0, sA, sBm, sTop);
-  // P_L, T_R: X2 <- (T_L Q_R + P_L T_R) N^-1, X1 keeps P_L's spectrum
-  if (act) {
-    group_pack(X1, PL, pl, L, gtid, G);
-    group_pack(X3, TR, tr, L, gtid, G);
-  }
-  __syncthreads();
-  group_fwd_c<L, G, 2>(X1, X3, nullptr, tw, gtid, act ? 3u : 0u);
-  for (uint32_t i = gtid; act && i < N; i += G)
-    X2[spad(i)] = gl::mul(gl::add(X2[spad(i)], gl::mul(X1[spad(i)], X3[spad(i)])), ninv);
-  __syncthreads();
-  group_inv_c<L, G>(X2, tw, gtid, act);
-  const uint32_t t_len = group_carry_store(X2, L, n_t, zt, X3, act, gtid, G, gw0, sA, sBm, sTop);
-  // P_R: X2 <- P_L P_R N^-1
-  if (act) group_pack(X2, PR, pr, L, gtid, G);
-  __syncthreads();
-  group_fwd_c<L, G, 1>(X2, nullptr, nullptr, tw, gtid, act ? 1u : 0u);
-  for (uint32_t i = gtid; act && i < N; i += G) X2[spad(i)] = gl::mul(gl::mul(X2[spad(i)], X1[spad(i)]), ninv);
-  __syncthreads();
-  group_inv_c<L, G>(X2, tw, gtid, act);
-  const uint32_t p_len = group_carry_store(X2, L, n_p, zp, X3, act, gtid, G, gw0, sA, sBm, sTop);
-  if (act && gtid == 0) {
-    M.out_len[3 * item] = p_len;
-    M.out_len[3 * item + 1] = q_len;
-    M.out_len[3 * item + 2] = t_len;
+  const bool run = T == G || t < G;
+#pragma unroll 1
+  for (int step = 0; step < 6; step++) {
+    // Q_R, T_L, Q_L, P_L, T_R, P_R
+    const int right = (0x31 >> step) & 1, kind = (0x0219 >> (2 * step)) & 3;
+    const uint64_t* x = node + (right ? in_stride : 0) + (kind > 0 ? M.sp : 0) + (kind > 1 ? M.sq : 0);
+    uint64_t s[ITL << BL];
+    small_forward<L, T>(x, 4 * len[3 * right + kind], R, work, t, grp, run, s);
+    if (step == 0 || step == 3) {
+      if (run) {
+#pragma unroll
+        for (int it = 0; it < ITL; it++)
+#pragma unroll
+          for (int k = 0; k < (1 << BL); k++) keep[spad(((it * G + t) << BL) + k)] = gl::mul(s[(it << BL) + k], ninv);
+      }
+      small_sync<T>(grp);
+      continue;
+    }
+    if (step == 1) {
+      if (run) {
+#pragma unroll
+        for (int it = 0; it < ITL; it++)
+#pragma unroll
+          for (int k = 0; k < (1 << BL); k++) {
+            const uint32_t i = spad(((it * G + t) << BL) + k);
+            acc[i] = gl::mul(s[(it << BL) + k], keep[i]);
+          }
+      }
+      small_sync<T>(grp);
+      continue;
+    }
+    if (run) {
+#pragma unroll
+      for (int it = 0; it < ITL; it++) {
+        const uint32_t base = (it * G + t) << BL;
+        uint64_t v[1 << BL];
+        gl::Lz y[1 << BL];
+#pragma unroll
+        for (int k = 0; k < (1 << BL); k++) v[k] = gl::mul(s[(it << BL) + k], keep[spad(base + k)]);
+        if (step == 4) {
+#pragma unroll
+          for (int k = 0; k < (1 << BL); k++) v[k] = gl::add(v[k], acc[spad(base + k)]);
+        }
+#pragma unroll
+        for (int k = 0; k < (1 << BL); k++) y[k] = gl::lz(v[k]);
+        y[0] = gl::lz_bias(y[0]);
+        dft_lz<BL, true>(y, v);
+#pragma unroll
+        for (int m = 0; m < (1 << BL); m++) work[spad(base + m)] = v[m];
+      }
+    }
+    small_inverse<L, T>(R, work, t, grp);
+    const uint32_t off = step == 2 ? M.op : step == 4 ? M.op + M.oq : 0;
+    const uint32_t n = merge_carry<L, T>(work, step == 2 ? n_q : step == 4 ? n_t : n_p, M.out + item * out_stride + off, t, grp,
+                                         sA, sBm, sTop);
+    if (t == 0) M.out_len[3 * (size_t)item + (step == 2 ? 1 : step == 4 ? 2 : 0)] = n;
   }
 }
 
-// Persistent over the level's items (pairs, then the odd last node): each
-// CTA runs MERGE_THREADS / G groups side by side.  8 <= L <= 12.
+// Persistent over the level's items (pairs, then the odd last node), each by
+// one of the MERGE_THREADS / T groups of a CTA.  8 <= L <= 12.
 template <int L>
 __global__ void __launch_bounds__(MERGE_THREADS, 2) k_split_merge(MergeLevel M, Roots R) {
   extern __shared__ uint64_t sm[];
   __shared__ uint32_t sA[MERGE_THREADS / 32], sBm[MERGE_THREADS / 32], sTop[MERGE_THREADS / 32];
-  constexpr int G = (1 << L) / 8;
-  constexpr uint32_t gpc = MERGE_THREADS / G, words = spad(1u << L);
-  const uint32_t grp = threadIdx.x / G;
-  const int gtid = (int)(threadIdx.x % G);
+  constexpr int T = merge_group_threads(L);
+  constexpr uint32_t gpc = MERGE_THREADS / T, words = spad(1u << L);
+  const uint32_t grp = threadIdx.x / T;
+  const int t = (int)(threadIdx.x % T);
   const uint32_t np = M.n_in / 2, items = np + (M.n_in & 1);
-  const uint32_t nchunks = (items + gpc - 1) / gpc;
-  uint64_t* X1 = sm + (size_t)grp * 3 * words;
-  for (uint32_t k = blockIdx.x; k < nchunks; k += gridDim.x) {
-    const uint32_t item = k * gpc + grp;
-    merge_item<L>(M, R.w12, item, item < np, item == np && (M.n_in & 1), X1, X1 + words, X1 + 2 * words, gtid,
-                  (int)(grp * G / 32), sA, sBm, sTop);
-    __syncthreads();
+  uint64_t* work = sm + (size_t)grp * 3 * words;
+  for (uint32_t item = blockIdx.x * gpc + grp; item < items; item += gridDim.x * gpc) {
+    if (item < np) {
+      merge_pair<L>(M, R, item, work, work + words, work + 2 * words, t, (int)grp, sA, sBm, sTop);
+      continue;
+    }
+    // the odd last node is copied
+    const uint32_t i = M.n_in - 1;
+    const uint64_t* p = M.in + (size_t)i * ((size_t)M.sp + M.sq + M.st);
+    uint64_t* z = M.out + (size_t)item * ((size_t)M.op + M.oq + M.ot);
+    const uint32_t pn = M.in_len[3 * i], qn = M.in_len[3 * i + 1], tn = M.in_len[3 * i + 2];
+    for (uint32_t k = t; k < pn; k += T) z[k] = p[k];
+    for (uint32_t k = t; k < qn; k += T) z[M.op + k] = p[M.sp + k];
+    for (uint32_t k = t; k < tn; k += T) z[M.op + M.oq + k] = p[M.sp + M.sq + k];
+    if (t == 0) {
+      M.out_len[3 * item] = pn;
+      M.out_len[3 * item + 1] = qn;
+      M.out_len[3 * item + 2] = tn;
+    }
   }
 }
 

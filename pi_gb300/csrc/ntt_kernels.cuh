@@ -68,14 +68,6 @@ __device__ __forceinline__ uint64_t root_pow32(const Roots& R, int mlog, uint32_
 // Shared-memory index with one pad word per 16 to spread 8-byte banks.
 __host__ __device__ __forceinline__ constexpr uint32_t spad(uint32_t lin) { return lin + (lin >> 4); }
 
-// spad(base | (m << s)) = spad(base) + spad_step(m, s) whenever base has zero
-// bits where m << s lands (the bits below 4 either come from base alone or
-// the shifted m stays inside one 16-word run): per-element shared-memory
-// offsets of a butterfly group are compile-time constants.
-__host__ __device__ __forceinline__ constexpr uint32_t spad_step(uint32_t m, int s) {
-  return (m << s) + ((m << s) >> 4);
-}
-
 // 8-point DFT (INV: unscaled inverse) of lazy values, folded outputs at
 // v[STEP k]; x[0] carries the bias of lz_bias.  w^-s = -w^(96 - s) turns the
 // inverse's twiddles into shifts with the signs swapped.
@@ -226,192 +218,6 @@ __device__ __forceinline__ void dft12_lz(const gl::Lz* x, uint64_t* v) {
     v[c + 6] = fold(n1 ? lz_add(a, s) : lz_sub(a, s));
     v[c + 3] = fold((n1 != INV) ? lz_sub(e, t) : lz_add(e, t));
     v[c + 9] = fold((n1 != INV) ? lz_add(e, t) : lz_sub(e, t));
-  }
-}
-
-// Forward DFT of 2^B values in registers (radix 2, 4, 8), for the rounds of
-// the merged splitting levels: lazy inputs with |k| <= 1, folded outputs.
-template <int B>
-__device__ __forceinline__ void dft_fwd_lz(const gl::Lz* x, uint64_t* v) {
-  using namespace gl;
-  const Lz x0 = lz_bias(x[0]);
-  if constexpr (B == 1) {
-    v[0] = fold(lz_add(x0, x[1]));
-    v[1] = fold(lz_sub(x0, x[1]));
-  } else if constexpr (B == 2) {
-    Lz a0 = lz_add(x0, x[2]), c = lz_sub(x0, x[2]);
-    Lz a1 = lz_add(x[1], x[3]);
-    Lz d = lz_shl<48>(lz_sub(x[1], x[3]));
-    v[0] = fold(lz_add(a0, a1));
-    v[1] = fold(lz_add(c, d));
-    v[2] = fold(lz_sub(a0, a1));
-    v[3] = fold(lz_sub(c, d));
-  } else {
-    static_assert(B == 3, "radix 2, 4 or 8");
-    const Lz y[8] = {x0, x[1], x[2], x[3], x[4], x[5], x[6], x[7]};
-    dft8_lz<false, 1>(y, v);
-  }
-}
-
-// Unscaled inverse of dft_fwd_lz on lazy inputs (|k| <= 1, e.g. twiddle
-// products from lz_mul): v[m] <- sum_k x[k] w^(-m k)  (= 2^B * original).
-template <int B>
-__device__ __forceinline__ void dft_inv_lz(const gl::Lz* x, uint64_t* v) {
-  using namespace gl;
-  const Lz x0 = lz_bias(x[0]);
-  if constexpr (B == 1) {
-    v[0] = fold(lz_add(x0, x[1]));
-    v[1] = fold(lz_sub(x0, x[1]));
-  } else if constexpr (B == 2) {
-    // inputs in bit-reversed order (x0, x2, x1, x3)
-    Lz s = lz_add(x0, x[2]), d = lz_sub(x0, x[2]);
-    Lz t = lz_add(x[1], x[3]);
-    Lz e = lz_shl<48>(lz_sub(x[1], x[3]));
-    v[0] = fold(lz_add(s, t));
-    v[2] = fold(lz_sub(s, t));
-    v[1] = fold(lz_sub(d, e));
-    v[3] = fold(lz_add(d, e));
-  } else {
-    static_assert(B == 3, "radix 2, 4 or 8");
-    const Lz y[8] = {x0, x[1], x[2], x[3], x[4], x[5], x[6], x[7]};
-    dft8_lz<true, 1>(y, v);
-  }
-}
-
-// ---------------------------------------------------------------- rounds
-// Round split of an r-bit in-tile DFT: radix-8 rounds first, then radix 4
-// or 2 (two radix-4 rounds instead of 8 + 2).
-__host__ __device__ constexpr int rp_count(int r) {
-  int n = 0;
-  while (r > 0) {
-    int b = r >= 3 ? 3 : r;
-    if (r == 4) b = 2;
-    r -= b;
-    n++;
-  }
-  return n;
-}
-
-__host__ __device__ constexpr int rp_bits(int r, int q) {
-  int i = 0;
-  while (r > 0) {
-    int b = r >= 3 ? 3 : r;
-    if (r == 4) b = 2;
-    if (i == q) return b;
-    r -= b;
-    i++;
-  }
-  return 0;
-}
-
-// Sub-problem size (log2) at the start of round q.
-__host__ __device__ constexpr int rp_mlog(int r, int q) {
-  int m = r;
-  for (int i = 0; i < q; i++) m -= rp_bits(r, i);
-  return m;
-}
-
-// Item order of a round: with one pad word per 16, a half-warp of some
-// rounds puts two or four lanes on one 8-byte bank (rows 64 words apart
-// land 4 banks apart).  Up to two swaps of item-number bits, a bijection on
-// the round's items, spread them; the swaps per round come from a model of
-// the padded layout, packed as a1 | b1 << 4 | a2 << 8 | b2 << 12 (a == b:
-// no swap).
-template <int R, int T, int BC, int MLOG>
-__host__ __device__ constexpr int round_swaps() {
-  return (T == 0 && R == 9 && MLOG == 6)   ? (3 | 4 << 4)
-         : (T == 0 && R == 8 && MLOG == 5) ? (0 | 1 << 4 | 1 << 8 | 4 << 12)
-                                           : 0;
-}
-
-template <int A, int B>
-__device__ __forceinline__ uint32_t swap_bits(uint32_t w) {
-  if constexpr (A == B) {
-    return w;
-  } else {
-    const uint32_t d = ((w >> A) ^ (w >> B)) & 1u;
-    return w ^ (d << A) ^ (d << B);
-  }
-}
-
-template <int S>
-__device__ __forceinline__ uint32_t round_item(uint32_t w) {
-  return swap_bits<(S >> 8) & 15, (S >> 12) & 15>(swap_bits<S & 15, (S >> 4) & 15>(w));
-}
-
-// Tile of 2^BC blocks x 2^R rows x 2^T columns in shared memory; element
-// (row, col) of the flattened (BC+R)-bit row index at spad(row << T | col).
-// One forward round of radix 2^B over sub-problems of 2^MLOG rows.  The
-// twiddles of the previous round (radix 2^PB over 2^PMLOG rows, PB = 0: none)
-// are applied here, to the inputs, as lazy products that feed the DFT
-// directly: element row r had position jp' = r mod 2^MLOG and output index
-// k' = (r >> MLOG) mod 2^PB there, twiddle w_(2^PMLOG)^(k' jp').
-// tw holds the 2^TWLOG roots w^t of one fixed length (4096 in the one-CTA
-// merge of whole transforms).
-template <int R, int T, int BC, int B, int MLOG, int NT, int PB, int PMLOG, int TWLOG>
-__device__ __forceinline__ void round_fwd_t(uint64_t* sm, const uint64_t* tw, int tid) {
-  constexpr int SLOG = MLOG - B;
-  constexpr int ITEMS = 1 << (BC + R + T - B);
-  static_assert(ITEMS % NT == 0, "tile must split evenly over the threads");
-#pragma unroll 2
-  for (int it = 0; it < ITEMS / NT; it++) {
-    const uint32_t w = round_item<round_swaps<R, T, BC, MLOG>()>(it * NT + tid);
-    const uint32_t j = w & ((1u << T) - 1);
-    const uint32_t rest = w >> T;
-    const uint32_t jp = rest & ((1u << SLOG) - 1);
-    const uint32_t row0 = ((rest >> SLOG) << MLOG) + jp;
-    const uint32_t sb = spad((row0 << T) | j);  // bits [SLOG+T, MLOG+T) are zero
-    uint64_t v[1 << B];
-    gl::Lz x[1 << B];
-#pragma unroll
-    for (int m = 0; m < (1 << B); m++) v[m] = sm[sb + spad_step(m, SLOG + T)];
-    if constexpr (PB > 0) {
-      static_assert(PMLOG - PB == MLOG, "rounds must nest");
-      const uint32_t kp = (rest >> SLOG) & ((1u << PB) - 1);
-      const uint32_t base = (kp * jp) << (TWLOG - PMLOG), step = (kp << SLOG) << (TWLOG - PMLOG);
-#pragma unroll
-      for (int m = 0; m < (1 << B); m++) x[m] = gl::lz_mul(v[m], tw[base + m * step]);
-    } else {
-#pragma unroll
-      for (int m = 0; m < (1 << B); m++) x[m] = gl::lz(v[m]);
-    }
-    dft_fwd_lz<B>(x, v);
-#pragma unroll
-    for (int k = 0; k < (1 << B); k++) sm[sb + spad_step(k, SLOG + T)] = v[k];
-  }
-}
-
-// One inverse round; the first one executed (SLOG = 0) has no twiddles.
-template <int R, int T, int BC, int B, int MLOG, int NT, int TWLOG>
-__device__ __forceinline__ void round_inv_t(uint64_t* sm, const uint64_t* tw, int tid) {
-  constexpr int SLOG = MLOG - B;
-  constexpr int ITEMS = 1 << (BC + R + T - B);
-  static_assert(ITEMS % NT == 0, "tile must split evenly over the threads");
-#pragma unroll 2
-  for (int it = 0; it < ITEMS / NT; it++) {
-    const uint32_t w = round_item<round_swaps<R, T, BC, MLOG>()>(it * NT + tid);
-    const uint32_t j = w & ((1u << T) - 1);
-    const uint32_t rest = w >> T;
-    const uint32_t jp = rest & ((1u << SLOG) - 1);
-    const uint32_t row0 = ((rest >> SLOG) << MLOG) + jp;
-    const uint32_t sb = spad((row0 << T) | j);  // bits [SLOG+T, MLOG+T) are zero
-    uint64_t v[1 << B];
-    gl::Lz x[1 << B];
-#pragma unroll
-    for (int k = 0; k < (1 << B); k++) v[k] = sm[sb + spad_step(k, SLOG + T)];
-    x[0] = gl::lz(v[0]);
-    const uint32_t jps = jp << (TWLOG - MLOG);
-#pragma unroll
-    for (int k = 1; k < (1 << B); k++) {
-      if constexpr (SLOG > 0) {
-        x[k] = gl::lz_mul(v[k], tw[((1u << TWLOG) - k * jps) & ((1u << TWLOG) - 1)]);
-      } else {
-        x[k] = gl::lz(v[k]);
-      }
-    }
-    dft_inv_lz<B>(x, v);
-#pragma unroll
-    for (int m = 0; m < (1 << B); m++) sm[sb + spad_step(m, SLOG + T)] = v[m];
   }
 }
 
