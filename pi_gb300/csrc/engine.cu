@@ -4065,7 +4065,20 @@ __host__ __device__ __forceinline__ uint64_t as_aux_bytes(uint64_t nout) {
   return round_up_u64(nc * (AS_THREADS / 32) * 8 + 2 * nc + 16, 16);
 }
 
-__global__ void __launch_bounds__(AS_THREADS) k_as_local(const AsJob* jobs) {
+// Carries of a warp's 32 windows for the carry in of its chunk: bit i is
+// window i's carry in.
+__device__ __forceinline__ uint32_t as_carries(const uint32_t* A, const uint32_t* B, int stride, int warp, uint32_t cin) {
+  for (int k = 0; k < warp; k++) cin = (uint32_t)(((uint64_t)A[k * stride] + B[k * stride] + cin) >> 32);
+  const uint32_t a = A[warp * stride], b = B[warp * stride];
+  return (a + b + cin) ^ a ^ b;
+}
+// The top window's carry out (generated, or propagated from its carry in).
+__device__ __forceinline__ bool as_out(uint32_t A, uint32_t B, uint32_t carries, int lane) {
+  return ((B | (A & carries)) >> lane) & 1;
+}
+
+// An array of one chunk is finished here: its carries are known in the CTA.
+__global__ void __launch_bounds__(AS_THREADS) k_as_local(const AsJob* jobs, int* overflow) {
   const AsJob J = jobs[blockIdx.y];
   const uint64_t nwin = as_nwin(J.nout), nchunk = as_nchunk(J.nout);
   if (blockIdx.x >= nchunk) return;
@@ -4074,7 +4087,9 @@ __global__ void __launch_bounds__(AS_THREADS) k_as_local(const AsJob* jobs) {
   __shared__ uint32_t sA[AS_THREADS / 32], sB[AS_THREADS / 32];
   const uint64_t w = (uint64_t)blockIdx.x * AS_THREADS + threadIdx.x;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const bool one = nchunk == 1;
   bool g = false, p = false;
+  uint64_t z[AS_W];
   if (w < nwin) {
     uint64_t c = 0;
     bool all = true;
@@ -4083,21 +4098,20 @@ __global__ void __launch_bounds__(AS_THREADS) k_as_local(const AsJob* jobs) {
       const uint64_t i = AS_W * w + t;
       if (i >= J.nout) break;
       const uint64_t xi = i < J.nx ? J.x[i] : 0, yi = i < J.ny ? J.y[i] : 0;
-      uint64_t z;
       if (J.sub) {
         const uint64_t d = xi - yi;
         const uint64_t b1 = xi < yi, b2 = d < c;
-        z = d - c;
+        z[t] = d - c;
         c = b1 | b2;
-        all = all && z == 0;
+        all = all && z[t] == 0;
       } else {
         const uint64_t s0 = xi + yi;
         const uint64_t c1 = s0 < xi;
-        z = s0 + c;
-        c = c1 | (z < s0);
-        all = all && z == ~0ull;
+        z[t] = s0 + c;
+        c = c1 | (z[t] < s0);
+        all = all && z[t] == ~0ull;
       }
-      J.out[i] = z;
+      if (!one) J.out[i] = z[t];
     }
     g = c != 0;
     p = all;
@@ -4105,13 +4119,33 @@ __global__ void __launch_bounds__(AS_THREADS) k_as_local(const AsJob* jobs) {
   const uint32_t A = __ballot_sync(0xFFFFFFFFu, g || p);
   const uint32_t Bm = __ballot_sync(0xFFFFFFFFu, g);
   if (lane == 0) {
-    const uint64_t wi = (uint64_t)blockIdx.x * (AS_THREADS / 32) + warp;
-    masks[2 * wi] = A;
-    masks[2 * wi + 1] = Bm;
+    if (!one) {
+      const uint64_t wi = (uint64_t)blockIdx.x * (AS_THREADS / 32) + warp;
+      masks[2 * wi] = A;
+      masks[2 * wi + 1] = Bm;
+    }
     sA[warp] = A;
     sB[warp] = Bm;
   }
   __syncthreads();
+  if (one) {
+    const uint32_t carries = as_carries(sA, sB, 1, warp, 0);
+    if (J.check && w + 1 == nwin && as_out(A, Bm, carries, lane)) atomicExch(overflow, 1);
+    if (w < nwin) {
+      bool c = (carries >> lane) & 1;
+#pragma unroll
+      for (int t = 0; t < AS_W; t++) {
+        const uint64_t i = AS_W * w + t;
+        if (i >= J.nout) break;
+        if (c) {
+          c = z[t] == (J.sub ? 0 : ~0ull);
+          z[t] += J.sub ? ~0ull : 1;
+        }
+        J.out[i] = z[t];
+      }
+    }
+    return;
+  }
   if (threadIdx.x == 0) {
     uint32_t cg = 0, cp = 1;  // chunk carry out for carry in 0 / 1
     for (int k = 0; k < AS_THREADS / 32; k++) {
@@ -4124,11 +4158,40 @@ __global__ void __launch_bounds__(AS_THREADS) k_as_local(const AsJob* jobs) {
   }
 }
 
+// Arrays of up to AS_LOOK chunks look left for a chunk's carry in (as_carry_in);
+// longer ones, whose look-back over an all-propagating array would cost more,
+// have it scanned.  The scan takes 14 us whatever the length; a look-back is one
+// byte in general and at most AS_LOOK / 512 steps of about 1 us (pi to 10^5, 10^6,
+// 10^8 digits 7.64 -> 7.34, 11.97 -> 11.67, 205.3 -> 203.1 ms, one-chunk arrays in one
+// kernel included).
+constexpr uint64_t AS_LOOK = 2048;
+
+// Carry into a chunk: that out of the nearest chunk on its left whose carry out
+// does not depend on its carry in (all lanes of the warp call).
+__device__ uint32_t as_carry_in(const uint8_t* chunk_gp, uint64_t chunk, int lane) {
+  if (chunk == 0) return 0;
+  const uint32_t f = chunk_gp[chunk - 1];
+  if (f != 2) return f & 1;
+  for (int64_t base = (int64_t)((chunk - 1) & ~511ull); base >= 0; base -= 512) {
+    uint32_t near = 2;  // of this lane's 16 chunks
+#pragma unroll
+    for (int t = 0; t < 16; t++) {
+      const uint64_t c = (uint64_t)base + 16 * lane + t;
+      const uint32_t v = c < chunk ? chunk_gp[c] : 2;
+      if (v != 2) near = v;
+    }
+    const uint32_t fixed = __ballot_sync(0xFFFFFFFFu, near != 2);
+    if (fixed) return __shfl_sync(0xFFFFFFFFu, near, 31 - __clz((int)fixed)) & 1;
+  }
+  return 0;
+}
+
 // One CTA per job: carry into every chunk (segments of chunks per thread,
 // chained by thread 0).
 __global__ void __launch_bounds__(1024) k_as_scan(const AsJob* jobs) {
   const AsJob J = jobs[blockIdx.x];
   const uint64_t nchunk = as_nchunk(J.nout);
+  if (nchunk <= AS_LOOK) return;
   const uint8_t* chunk_gp = J.aux + nchunk * (AS_THREADS / 32) * 8;
   uint8_t* chunk_cin = J.aux + nchunk * (AS_THREADS / 32) * 8 + nchunk;
   __shared__ uint8_t seg_g[1024], seg_p[1024], seg_cin[1024];
@@ -4167,23 +4230,14 @@ __global__ void __launch_bounds__(1024) k_as_scan(const AsJob* jobs) {
 __global__ void __launch_bounds__(AS_THREADS) k_as_apply(const AsJob* jobs, int* overflow) {
   const AsJob J = jobs[blockIdx.y];
   const uint64_t nwin = as_nwin(J.nout), nchunk = as_nchunk(J.nout);
-  if (blockIdx.x >= nchunk) return;
-  const uint32_t* masks = reinterpret_cast<const uint32_t*>(J.aux);
-  const uint8_t* chunk_cin = J.aux + nchunk * (AS_THREADS / 32) * 8 + nchunk;
+  if (blockIdx.x >= nchunk || nchunk == 1) return;
+  const uint32_t* masks = reinterpret_cast<const uint32_t*>(J.aux) + 2 * (uint64_t)blockIdx.x * (AS_THREADS / 32);
+  const uint8_t* chunk_gp = J.aux + nchunk * (AS_THREADS / 32) * 8;
   const uint64_t w = (uint64_t)blockIdx.x * AS_THREADS + threadIdx.x;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  uint32_t cin = nchunk == 1 ? 0 : chunk_cin[blockIdx.x];  // one chunk: no scan ran
-  const uint64_t wbase = (uint64_t)blockIdx.x * (AS_THREADS / 32);
-  for (int k = 0; k < warp; k++) {
-    uint64_t s = (uint64_t)masks[2 * (wbase + k)] + masks[2 * (wbase + k) + 1] + cin;
-    cin = (uint32_t)(s >> 32);
-  }
-  const uint32_t A = masks[2 * (wbase + warp)], Bm = masks[2 * (wbase + warp) + 1];
-  const uint32_t carries = (A + Bm + cin) ^ A ^ Bm;
-  if (J.check && w + 1 == nwin) {
-    const uint32_t g = (Bm >> lane) & 1, pg = (A >> lane) & 1, c = (carries >> lane) & 1;
-    if (g || (pg && c)) atomicExch(overflow, 1);
-  }
+  const uint32_t cin = nchunk > AS_LOOK ? chunk_gp[nchunk + blockIdx.x] : as_carry_in(chunk_gp, blockIdx.x, lane);
+  const uint32_t carries = as_carries(masks, masks + 1, 2, warp, cin);
+  if (J.check && w + 1 == nwin && as_out(masks[2 * warp], masks[2 * warp + 1], carries, lane)) atomicExch(overflow, 1);
   if (w < nwin && ((carries >> lane) & 1)) {
     for (int t = 0; t < AS_W; t++) {
       const uint64_t i = AS_W * w + t;
@@ -4215,6 +4269,16 @@ __global__ void __launch_bounds__(256) k_top_limb(const uint64_t* const* arrs, c
   if ((threadIdx.x & 31) == 0 && best) atomicMax((unsigned long long*)&len[j], (unsigned long long)best);
 }
 
+static void as_launch(const AsJob* jobs, size_t n, uint64_t max_chunk, cudaStream_t st, int* d_overflow) {
+  for (size_t j0 = 0; j0 < n; j0 += 65535) {
+    const unsigned nj = (unsigned)std::min<size_t>(65535, n - j0);
+    const dim3 grid((unsigned)max_chunk, nj);
+    k_as_local<<<grid, AS_THREADS, 0, st>>>(jobs + j0, d_overflow);
+    if (max_chunk > AS_LOOK) k_as_scan<<<nj, 1024, 0, st>>>(jobs + j0);
+    if (max_chunk > 1) k_as_apply<<<grid, AS_THREADS, 0, st>>>(jobs + j0, d_overflow);
+  }
+}
+
 // Batched add/subtract on `st` (asynchronous); *d_overflow (device int,
 // zeroed by the caller) is set when a carry or borrow leaves a top limb.
 static int addsub_launch(const pimul_addsub_job* jobs, size_t n, cudaStream_t st, int* d_overflow, bool unchecked) {
@@ -4240,13 +4304,7 @@ static int addsub_launch(const pimul_addsub_job* jobs, size_t n, cudaStream_t st
   }
   if (host_to_device(dev, h, n * sizeof(AsJob), st)) e = cudaErrorUnknown;
   if (e == cudaSuccess) {
-    const AsJob* dj = reinterpret_cast<const AsJob*>(dev);
-    for (size_t j0 = 0; j0 < n; j0 += 65535) {
-      const unsigned nj = (unsigned)std::min<size_t>(65535, n - j0);
-      k_as_local<<<dim3((unsigned)max_chunk, nj), AS_THREADS, 0, st>>>(dj + j0);
-      if (max_chunk > 1) k_as_scan<<<nj, 1024, 0, st>>>(dj + j0);
-      k_as_apply<<<dim3((unsigned)max_chunk, nj), AS_THREADS, 0, st>>>(dj + j0, d_overflow);
-    }
+    as_launch(reinterpret_cast<const AsJob*>(dev), n, max_chunk, st, d_overflow);
     e = cudaGetLastError();
   }
   // the host image is pageable: the copy has been staged before return
@@ -4739,12 +4797,7 @@ int addsub_strided(const uint64_t* x, uint64_t sx, size_t nx, const uint64_t* y,
   AsJob* dj = reinterpret_cast<AsJob*>(dev);
   k_fill_as<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(
       dj, AsJob{x, y, out, nx, ny, nout, dev + desc, (uint32_t)(sub != 0), 0u}, sx, sy, so, saux, (uint32_t)n);
-  for (size_t j0 = 0; j0 < n; j0 += 65535) {
-    const unsigned nj = (unsigned)std::min<size_t>(65535, n - j0);
-    k_as_local<<<dim3((unsigned)nchunk, nj), AS_THREADS, 0, st>>>(dj + j0);
-    if (nchunk > 1) k_as_scan<<<nj, 1024, 0, st>>>(dj + j0);
-    k_as_apply<<<dim3((unsigned)nchunk, nj), AS_THREADS, 0, st>>>(dj + j0, nullptr);
-  }
+  as_launch(dj, n, nchunk, st, nullptr);
   e = cudaGetLastError();
   cudaFreeAsync(dev, st);
   if (e != cudaSuccess) return fail(PIMUL_ECUDA, std::string("strided add/subtract launch: ") + cudaGetErrorString(e));
