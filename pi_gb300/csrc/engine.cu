@@ -2795,6 +2795,35 @@ static int unit_log_n(const Unit& u) {
   return log2_ceil(4 * u.nout - 1);
 }
 
+// Open-addressing map from (pointer, number) to a number, for at most n keys: a
+// batch's shared operands (with std::unordered_map the layout of 2500 products took
+// 770 us, longer than their kernels).
+class PairMap {
+ public:
+  explicit PairMap(size_t n) {
+    size_t c = 16;
+    while (c < 2 * n) c *= 2;
+    slots_.resize(c);
+  }
+  // The number of (p, k), `fresh` where there is none yet.
+  uint64_t& at(const void* p, uint64_t k, uint64_t fresh) {
+    const uint64_t h = ((uint64_t)(uintptr_t)p + k * 0x9E3779B97F4A7C15ull) * 0xD6E8FEB86659FD93ull;
+    for (size_t i = (h >> 32) & (slots_.size() - 1);; i = (i + 1) & (slots_.size() - 1)) {
+      Slot& s = slots_[i];
+      if (!s.used) s = Slot{p, k, fresh, true};
+      if (s.p == p && s.k == k) return s.v;
+    }
+  }
+
+ private:
+  struct Slot {
+    const void* p = nullptr;
+    uint64_t k = 0, v = 0;
+    bool used = false;
+  };
+  std::vector<Slot> slots_;
+};
+
 // share: let products with the same operand b borrow one spectrum (a batch
 // plan lays out a shape without pointers and never shares).
 static int layout_batch(const Unit* units, size_t n, BatchLayout& B, bool share, cudaStream_t st) {
@@ -2807,24 +2836,22 @@ static int layout_batch(const Unit* units, size_t n, BatchLayout& B, bool share,
   // shared spectrum saves more)
   if (std::any_of(Ls.begin(), Ls.end(), [](int L) { return L > SMALL_LOG_MAX; })) {
     B.seg.assign(n, SegPlan{});
-    std::unordered_map<const uint64_t*, uint32_t> uses;
+    PairMap uses(share ? 2 * n : 0), most(share ? 2 * n : 0);  // most: coefficients, by b and power of two
     if (share)
       for (size_t i = 0; i < n; i++)
         if (Ls[i] > SMALL_LOG_MAX) {
-          uses[units[i].b]++;
-          if (units[i].la2) uses[units[i].b2]++;
+          uses.at(units[i].b, 0, 0)++;
+          if (units[i].la2) uses.at(units[i].b2, 0, 0)++;
         }
     for (size_t i = 0; i < n; i++) {
       const Unit& u = units[i];
-      if (Ls[i] <= SMALL_LOG_MAX || u.la2 || u.coeff || u.forceL || (share && uses[u.b] > 1)) continue;
+      if (Ls[i] <= SMALL_LOG_MAX || u.la2 || u.coeff || u.forceL || (share && uses.at(u.b, 0, 0) > 1)) continue;
       B.seg[i] = plan_segments(u.la, u.lb);
       if (B.seg[i].L) Ls[i] = B.seg[i].L;
     }
     // three quarters of a power of two where that holds the product, and every
     // other one of that power of two that shares its b (else the spectrum
     // would be computed twice)
-    std::unordered_map<uint64_t, uint64_t> most;  // coefficients, by b and power of two
-    auto key = [](const uint64_t* b, int L) { return (uint64_t)(uintptr_t)b << 3 | (uint64_t)L; };
     auto three_ok = [&](size_t i) { return Ls[i] > SMALL_LOG_MAX + 1 && !units[i].coeff && !units[i].forceL && !B.seg[i].L; };
     if (share)
       for (size_t i = 0; i < n; i++) {
@@ -2833,7 +2860,7 @@ static int layout_batch(const Unit* units, size_t n, BatchLayout& B, bool share,
         const uint64_t need = three_ok(i) ? 4 * u.nout - 1 : ~0ull;
         for (const uint64_t* b : {u.b, u.la2 ? u.b2 : nullptr})
           if (b) {
-            uint64_t& m = most[key(b, Ls[i])];
+            uint64_t& m = most.at(b, (uint64_t)Ls[i], 0);
             m = std::max(m, need);
           }
       }
@@ -2848,8 +2875,8 @@ static int layout_batch(const Unit* units, size_t n, BatchLayout& B, bool share,
       if (!three_ok(i)) continue;
       uint64_t need = 4 * u.nout - 1;
       if (share) {
-        need = std::max(need, most[key(u.b, L)]);
-        if (u.la2) need = std::max(need, most[key(u.b2, L)]);
+        need = std::max(need, most.at(u.b, (uint64_t)L, 0));
+        if (u.la2) need = std::max(need, most.at(u.b2, (uint64_t)L, 0));
       }
       shorter[i] = three_holds(need, L);
       if (shorter[i]) fit[L] += w;
@@ -2861,28 +2888,35 @@ static int layout_batch(const Unit* units, size_t n, BatchLayout& B, bool share,
       if (shorter[i]) Ls[i] = (int)fit[Ls[i]];
   }
   std::vector<std::vector<uint32_t>> byL(N_LENGTHS);
+  size_t count[SMALL_LOG_MAX + 1] = {}, at[SMALL_LOG_MAX + 1] = {};  // of a class of short products: number, place
+  size_t n_large = 0;
   for (size_t i = 0; i < n; i++) {
     if (Ls[i] < 0) continue;
-    if (Ls[i] <= SMALL_LOG_MAX && units[i].la2) return fail(PIMUL_EINVAL, "a sum of products below 2^13 in the pass pipeline");
     if (Ls[i] <= SMALL_LOG_MAX) {
-      B.small.push_back((uint32_t)i);
+      if (units[i].la2) return fail(PIMUL_EINVAL, "a sum of products below 2^13 in the pass pipeline");
+      Ls[i] = small_class(units[i].la, units[i].lb);
+      count[Ls[i]]++;
     } else {
       byL[Ls[i]].push_back((uint32_t)i);
+      n_large += units[i].la2 ? 2 : B.seg[i].L ? B.seg[i].S : 1;
     }
   }
-  // longest transforms first (a bucket pass by length, O(n))
-  {
-    std::vector<std::vector<uint32_t>> sb(SMALL_LOG_MAX + 1);
-    for (uint32_t i : B.small) sb[small_class(units[i].la, units[i].lb)].push_back(i);
-    B.small.clear();
-    for (int c = SMALL_LOG_MAX; c >= SMALL_TINY; c--) {
-      const uint32_t per = small_per_cta(c);
-      for (size_t k = 0; k < sb[c].size(); k += per)
-        B.chunks.push_back(SmallChunk{(uint32_t)(B.small.size() + k), (uint32_t)std::min<size_t>(per, sb[c].size() - k), c});
-      if (!sb[c].empty()) B.small_smem = std::max(B.small_smem, small_cta_smem(c));
-      B.small.insert(B.small.end(), sb[c].begin(), sb[c].end());
-    }
+  B.desc.reserve(n_large);
+  // longest transforms first
+  size_t total = 0;
+  for (int c = SMALL_LOG_MAX; c >= SMALL_TINY; c--) {
+    if (!count[c]) continue;
+    const uint32_t per = small_per_cta(c);
+    for (size_t k = 0; k < count[c]; k += per)
+      B.chunks.push_back(SmallChunk{(uint32_t)(total + k), (uint32_t)std::min<size_t>(per, count[c] - k), c});
+    B.small_smem = std::max(B.small_smem, small_cta_smem(c));
+    at[c] = total;
+    total += count[c];
   }
+  B.small.resize(total);
+  if (total)
+    for (size_t i = 0; i < n; i++)
+      if (Ls[i] >= 0 && Ls[i] <= SMALL_LOG_MAX) B.small[at[Ls[i]]++] = (uint32_t)i;
   // Groups of one length: at most 65535 descriptors (grid.y) whose scratch
   // fits BATCH_ARENA_CAP; groups run one after another on the stream, so
   // they all reuse the same arena.
@@ -2909,7 +2943,14 @@ static int layout_batch(const Unit* units, size_t n, BatchLayout& B, bool share,
       }
       // descriptors, those with carries first; the first of several with the
       // same b owns its spectrum, a product's first segment that of the others
-      std::unordered_map<const uint64_t*, std::vector<size_t>> by_b;
+      PairMap owner_of(share ? bk.nd : 0);  // by array and length
+      auto lend = [&](const uint64_t* b, uint64_t lb, size_t di) {
+        const size_t o = owner_of.at(b, lb, di);
+        if (o == di) return;
+        B.desc[di].flags |= JF_B_SHARED;
+        B.desc[di].owner = (int64_t)o;
+        B.desc[o].lent = true;
+      };
       bk.nc = e - s;
       for (size_t k = s; k < e; k++) {
         const Unit& u = units[byL[L][k]];
@@ -2919,8 +2960,8 @@ static int layout_batch(const Unit* units, size_t n, BatchLayout& B, bool share,
         d1.flags = 0;
         d1.lent = B.seg[d1.unit].S > 1;
         const bool sq1 = u.a == u.b && u.la == u.lb;
-        if (share && !sq1 && !B.seg[d1.unit].L) by_b[u.b].push_back(B.desc.size());
         B.desc.push_back(d1);
+        if (share && !sq1 && !B.seg[d1.unit].L) lend(u.b, u.lb, B.desc.size() - 1);
       }
       for (size_t k = s; k < e; k++) {
         const uint32_t ui = byL[L][k];
@@ -2932,8 +2973,8 @@ static int layout_batch(const Unit* units, size_t n, BatchLayout& B, bool share,
           d2.second = true;
           d2.flags = JF_ADDEND;
           B.desc[i1].addend = (int64_t)B.desc.size();
-          if (share) by_b[u.b2].push_back(B.desc.size());
           B.desc.push_back(d2);
+          if (share) lend(u.b2, u.lb2, B.desc.size() - 1);
         }
         for (uint32_t g = 1; g < B.seg[ui].S; g++) {
           BatchLayout::Desc d2;
@@ -2943,23 +2984,6 @@ static int layout_batch(const Unit* units, size_t n, BatchLayout& B, bool share,
           d2.flags = JF_SEGMENT | JF_B_SHARED;
           d2.owner = (int64_t)i1;
           B.desc.push_back(d2);
-        }
-      }
-      for (auto& kv : by_b) {
-        std::vector<size_t>& v = kv.second;
-        // same array and same length
-        std::unordered_map<uint64_t, size_t> owner_of;
-        for (size_t di : v) {
-          const BatchLayout::Desc& d = B.desc[di];
-          const uint64_t lb = d.second ? units[d.unit].lb2 : units[d.unit].lb;
-          auto it = owner_of.find(lb);
-          if (it == owner_of.end()) {
-            owner_of.emplace(lb, di);
-          } else {
-            B.desc[di].flags |= JF_B_SHARED;
-            B.desc[di].owner = (int64_t)it->second;
-            B.desc[it->second].lent = true;
-          }
         }
       }
       // scratch offsets
