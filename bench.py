@@ -47,12 +47,12 @@ def mul_metric():
 BITS_A = 1 << 30
 BITS_B = 1 << 30
 
-# DRAM traffic of the dominant kernel class (forward passes) per transform
-# word: dram__bytes_read.sum + dram__bytes_write.sum from one ncu capture of
-# each of k_col_mid<9,fwd> (15.60 bytes per word) and k_fwd_last<9> (15.53)
-# of a 2^30 x 2^30-bit product (N = 2^27); the class runs the first twice
-# and the second once per transform: 15.58 N bytes per launch.
-NCU_TRAFFIC_BYTES_PER_WORD = 15.58
+# DRAM traffic of the dominant kernel class (forward passes after the first) per
+# transform word: dram__bytes_read.sum + dram__bytes_write.sum from one ncu
+# capture of each of k_col_mid<8,fwd> (15.19 bytes per word) and k_fwd_last<9>
+# (15.07) of a 2^28 x 2^28-bit product (N = 2^25); the class runs each once per
+# transform.
+NCU_TRAFFIC_BYTES_PER_WORD = 15.13
 
 
 def b_mul(n, la, lb, square=False):
@@ -204,39 +204,42 @@ def stats(lib):
     return out
 
 
-# ALU-pipe warp instructions per transform word, per launch of each pass
-# kernel (smsp__inst_executed_pipe_alu.sum / N from one ncu capture per
-# kernel of a 2^30 x 2^30-bit product, N = 2^27, plan 2^9 x 2^9 x 2^9;
-# k_fwd_first<9> with the half-zero first round from a 2^28 x 2^28-bit
-# product, N = 2^25, the same kernel); "carry" is the three carry kernels
-# together.  Instruction counts do not depend on the clock or on timing.
+# ALU-pipe warp instructions per transform word of each pass kernel
+# (smsp__inst_executed_pipe_alu.sum / words from one ncu capture per kernel of a
+# 2^30 x 2^30-bit product, N = 2^27, plan 2^9 x 2^9 x 2^9).  Instruction counts
+# do not depend on the clock or on timing.
 NCU_ALU_PER_WORD = {
-    "k_fwd_first": 2.68, "k_col_mid_fwd": 2.82, "k_fwd_last": 2.22, "k_mid": 4.36,
-    "k_col_mid_inv": 2.66, "k_inv_first_carry": 3.04, "carry": 0.46,
+    "k_fwd_first": 1.88, "k_col_mid_fwd": 1.82, "k_fwd_last": 1.42, "k_inv_last": 1.75,
+    "k_col_mid_inv": 1.89, "k_inv_first_carry": 2.15, "k_carry": 0.48,
 }
 # The integer ALU pipe retires 16 lanes per clock per SM sub-partition:
 # half a warp instruction per clock, four sub-partitions per SM.
 ALU_WARP_INSTR_PER_CLK_PER_SM = 4 * 0.5
 
 
+def words_per_launch(kind, n):
+    """Transform words of one launch: the forward passes run both operands."""
+    return 2 * n if kind in ("pack", "pass_fwd") else n
+
+
 def alu_per_word(kind):
     """Mean ALU warp instructions per word of one launch of a kernel class."""
     a = NCU_ALU_PER_WORD
-    return {"pack": a["k_fwd_first"], "pass_fwd": (2 * a["k_col_mid_fwd"] + a["k_fwd_last"]) / 3,
-            "pass_inv": (a["k_col_mid_inv"] + a["k_inv_first_carry"]) / 2, "pointwise": a["k_mid"],
-            "carry": a["carry"] / 3}.get(kind, 0.0)
+    return {"pack": a["k_fwd_first"], "pass_fwd": (a["k_col_mid_fwd"] + a["k_fwd_last"]) / 2,
+            "pass_inv": (a["k_col_mid_inv"] + a["k_inv_first_carry"]) / 2, "pointwise": a["k_inv_last"],
+            "carry": a["k_carry"]}.get(kind, 0.0)
 
 
 def kernel_bytes_per_launch(kind, n, la, lb):
     """Algorithmic bytes of one launch of each kernel class."""
     if kind in ("pass_fwd", "pass_inv"):
-        return 16 * n              # read and write the N-word array once
+        return 16 * words_per_launch(kind, n)   # read and write each array once
     if kind == "pack":
-        return 8 * n + 8 * la      # read limbs, write N coefficients
+        return 16 * n + 8 * (la + lb)           # read limbs, write N coefficients per operand
     if kind == "pointwise":
-        return 24 * n              # read two arrays, write one
+        return 24 * n                           # read two arrays, write one
     if kind == "carry":
-        return 8 * n + 8 * (la + lb)
+        return 20 * (la + lb)                   # read 3 words per window of 2 limbs, write its limbs
     return 0
 
 
@@ -343,8 +346,8 @@ def run_gpu(args):
     n_sm = torch.cuda.get_device_properties(local).multi_processor_count
     f_sm = (clocks["sm_mhz"] or clocks["sm_max_mhz"] or 2070.0) * 1e6
     alu_cap = n_sm * ALU_WARP_INSTR_PER_CLK_PER_SM * f_sm  # warp instructions / s
-    int_frac = alu_per_word(dom) * N / (avg_ms * 1e-3) / alu_cap
-    step_alu = sum(alu_per_word(k) * N * ks[k]["launches"] / args.steps for k in ks)
+    int_frac = alu_per_word(dom) * words_per_launch(dom, N) / (avg_ms * 1e-3) / alu_cap
+    step_alu = sum(alu_per_word(k) * words_per_launch(k, N) * ks[k]["launches"] / args.steps for k in ks)
     int_frac_step = step_alu / (ms_step * 1e-3) / alu_cap
 
     cpu = None
@@ -383,7 +386,7 @@ def run_gpu(args):
                                  "the multiply; b's upload is hidden behind a's forward transform"},
             "roofline": {"bound": "hbm", "kernel": dom, "achieved": round(achieved, 1), "peak": peak,
                          "peak_source": peak_kind, "unit": "GB/s", "frac": round(achieved / peak, 4),
-                         "traffic": round(NCU_TRAFFIC_BYTES_PER_WORD * N) if dom == "pass_fwd" else None,
+                         "traffic": round(NCU_TRAFFIC_BYTES_PER_WORD * words_per_launch(dom, N)) if dom == "pass_fwd" else None,
                          "bytes_per_launch": per_launch, "avg_launch_ms": round(avg_ms, 4),
                          "step_achieved": round(step_achieved, 1),
                          "step_frac": round(step_achieved / peak, 4),
@@ -392,7 +395,7 @@ def run_gpu(args):
                                        "alu_warp_instr_per_step": round(step_alu),
                                        "peak_warp_instr_per_s": round(alu_cap),
                                        "sms": n_sm, "sm_mhz": f_sm / 1e6,
-                                       "model": "ALU-pipe warp instructions per word from ncu x N, over "
+                                       "model": "ALU-pipe warp instructions per word from ncu x words, over "
                                                 "SMs x 4 sub-partitions x 0.5 warp instr/clk x sampled SM clock"},
                          "binding_unit": "integer ALU pipe (int_frac), not HBM (frac)",
                          "io_effective_gbs": round(16 * (la + lb) / (ms_step * 1e-3) / 1e9, 1),
@@ -481,7 +484,8 @@ def sweep_measure(peak):
         del da, db, dout
     del flush
     torch.cuda.empty_cache()
-    return {"model": "B_mul(N) = 96N + 16(la+lb), B_sqr(N) = 64N + 24la bytes; hbm_frac of measured HBM GB/s",
+    return {"model": "B_mul(N) = 96N + 16(la+lb), B_sqr(N) = 64N + 24la bytes (N the power of two; products run in "
+                     "segments move less); hbm_frac of measured HBM GB/s",
             "timing": "each call alone: CUDA events around one pimul_mul_device after a 512 MiB L2 flush; median",
             "parity": "bit-exact vs the oracle in tests/test_mul_gpu.py (full sizes included)",
             "rows": rows}

@@ -102,8 +102,9 @@ typedef struct pimul_job {
 /*
  * Batched form: n independent products on device buffers in one call
  * (asynchronous on `stream`, NULL = the calling thread's stream).  Products
- * are grouped by transform length: up to 2^12 one CTA per product in a
- * persistent kernel, longer ones one launch per pass for the whole group;
+ * are grouped by transform length: up to 2^12 points whole products in
+ * shared memory by a persistent kernel, longer ones (2^k or 3 2^k points,
+ * long operands by short ones in segments) one launch per pass for the whole group;
  * products of one length whose operand b is the same array (same pointer
  * and length) compute b's transform once.  Each out[i] is written exactly
  * as pimul_mul_device would write it.
@@ -201,12 +202,11 @@ int pimul_batch_plan_destroy(pimul_batch_plan* plan);
 /*
  * Autotuner: times the candidate pass counts per transform for every
  * transform length 2^log_n_min .. 2^log_n_max on `reps` synthetic products
- * (each count split into radices 2^6 .. 2^9, the first at least 2^7, with
- * the fewest radix-8/4 rounds), and the one-CTA kernel's persistent grid
- * (CTAs per SM); keeps the fastest for later calls and writes a JSON
+ * (each count split into radices 2^6 .. 2^9, one of them at least 2^7), and
+ * the short products' persistent grid (CTAs per SM); keeps the fastest for later calls and writes a JSON
  * report.  pimul_tuning_set applies saved choices (passes = 0: default
  * count, ceil(log_n / 9) and at least 2; ctas <= 0: unchanged).
- * The transform length itself is the reference's rule and is not tuned.
+ * Transform lengths are not tuned.
  */
 int pimul_autotune(int log_n_min, int log_n_max, int reps, char* report, size_t report_cap);
 int pimul_tuning_set(int log_n, int passes, int small_ctas_per_sm);
@@ -214,11 +214,12 @@ int pimul_tuning_set(int log_n, int passes, int small_ctas_per_sm);
 /*
  * Twiddle-table cache.  The first and middle passes of a transform read
  * their twiddles from tables laid out like the data (one coalesced load per
- * element; the inverse first pass's table also carries the 1/N scaling),
+ * element; the inverse first pass's table also carries the 1/N scaling;
+ * transforms of 3 2^k points have theirs),
  * built on first use per transform shape and kept until pimul_shutdown.
  * First passes use tables up to transform length 2^28 (8 N bytes per
  * direction); longer transforms, and shapes past the cap, compute their
- * twiddles.  pimul_twiddle_cache sets the cap in bytes (default 8 GiB;
+ * twiddles (and take 2^k points).  pimul_twiddle_cache sets the cap in bytes (default 8 GiB;
  * 0: build no more tables) for tables built from then on and reports the
  * bytes already held in *held (may be NULL).  The cache is device memory
  * outside the served form's HBM budget.
@@ -434,8 +435,10 @@ int pimul_pi_gauss_legendre(uint64_t digits, char* out, size_t cap, pimul_mul_fn
 int pimul_pi_gauss_legendre_ex(uint64_t digits, char* out, size_t cap, pimul_mul_fn backend, uint64_t ntt_threshold,
                                uint32_t flags, double* phase_ms, uint64_t* ntt_products);
 
-/* Transform plan for a product: N and the number of HBM passes per transform.
- * Mirrors the sizing of crates/bignum/src/ntt.rs:810-813. */
+/* Transform plan for a product: the power of two N that holds it and the number
+ * of HBM passes per transform of that length.  Mirrors the sizing of
+ * crates/bignum/src/ntt.rs:810-813; a product that fills at most three quarters
+ * of N, or has a short operand, may run shorter transforms. */
 int pimul_plan(size_t la, size_t lb, uint64_t* n_transform, int* passes);
 
 /* Kernel launch statistics (this engine's own instrumentation; the
