@@ -229,7 +229,12 @@ constexpr uint32_t JF_SEGMENT = 16;
 
 // Every kernel of the pipeline starts with these two (see launch_pdl): the next
 // kernel on the stream may be scheduled as this one's CTAs leave, and nothing
-// is read or written before the kernels in front are done.
+// is read or written before the kernels in front are done.  What an earlier
+// kernel may have written (operands, spectra, windows) is read with plain
+// loads through pointers that promise nothing: the read-only path (__ldg, or
+// const __restrict__) wants words that stay the same from the kernel's start
+// on, which lies before the wait, and a load from it is not tied to the wait.
+// The root and twiddle tables, finished before any launch that reads them, keep it.
 __device__ __forceinline__ void pdl_wait() {
   asm volatile("griddepcontrol.launch_dependents;\n\tgriddepcontrol.wait;" ::: "memory");
 }
@@ -270,7 +275,7 @@ __global__ void __launch_bounds__(PASS_THREADS, pass_min_ctas(R)) k_fwd_first(co
   const Job J = job_of(jobs, one, L);
   const int which = w0 + (int)blockIdx.z;
   if (which == 1 && skips_b(J)) return;
-  const uint16_t* __restrict__ coef = reinterpret_cast<const uint16_t*>(which ? J.b : J.a);
+  const uint16_t* coef = reinterpret_cast<const uint16_t*>(which ? J.b : J.a);
   const int64_t c0 = which ? 0 : J.c0, nc = (int64_t)(4 * (which ? J.lb : J.la));
   uint64_t* __restrict__ data = which ? J.B : J.A;
   extern __shared__ uint64_t sm[];
@@ -283,7 +288,7 @@ __global__ void __launch_bounds__(PASS_THREADS, pass_min_ctas(R)) k_fwd_first(co
     // inputs ml <= m < mc exist (ml > 0: a first segment starts before a does)
     const uint32_t ml = n0 < 0 ? (uint32_t)((uint64_t)(-n0 + (int64_t)step - 1) >> (S + B2)) : 0;
     const uint32_t mc = n0 < nc ? (uint32_t)((uint64_t)(nc - n0 + (int64_t)step - 1) >> (S + B2)) - ml : 0;
-    const uint16_t* __restrict__ cn = coef + n0;
+    const uint16_t* cn = coef + n0;
     uint64_t v[1 << B1];
     gl::Lz x[1 << B1];
     bool done = false;
@@ -292,7 +297,7 @@ __global__ void __launch_bounds__(PASS_THREADS, pass_min_ctas(R)) k_fwd_first(co
       // (coefficients N/2 and up): those inputs are neither read nor added
       if (nc - c0 <= (int64_t)(1ull << (L - 1))) {
 #pragma unroll
-        for (int m = 0; m < (1 << (B1 - 1)); m++) x[m] = gl::Lz{m - ml < mc ? (uint32_t)__ldg(cn + m * step) : 0u, 0u, 0};
+        for (int m = 0; m < (1 << (B1 - 1)); m++) x[m] = gl::Lz{m - ml < mc ? (uint32_t)cn[m * step] : 0u, 0u, 0};
         x[0] = gl::lz_bias(x[0]);
         dft_lz<B1, false, true>(x, v);
         done = true;
@@ -300,7 +305,7 @@ __global__ void __launch_bounds__(PASS_THREADS, pass_min_ctas(R)) k_fwd_first(co
     }
     if (!done) {
 #pragma unroll
-      for (int m = 0; m < (1 << B1); m++) x[m] = gl::Lz{m - ml < mc ? (uint32_t)__ldg(cn + m * step) : 0u, 0u, 0};
+      for (int m = 0; m < (1 << B1); m++) x[m] = gl::Lz{m - ml < mc ? (uint32_t)cn[m * step] : 0u, 0u, 0};
       x[0] = gl::lz_bias(x[0]);
       dft_lz<B1, false>(x, v);
     }
@@ -490,7 +495,7 @@ __global__ void __launch_bounds__(PASS_THREADS, pass_min_ctas(R)) k_inv_last(con
   const uint64_t off = ((uint64_t)blockIdx.x << G::TILE) + warp * G::WWORDS;
   const bool sq = is_square(J);
   uint64_t* __restrict__ chunk = J.A + off;
-  const uint64_t* __restrict__ bspec = J.B + off;
+  const uint64_t* bspec = J.B + off;
   uint64_t* sw = sm + warp * G::XWORDS;
   constexpr uint32_t LINE = 16;  // words of 128 bytes
   for (uint32_t t = G::WWORDS / G::ITERS2 + LINE * lane; t < G::WWORDS; t += LINE * 32) {
@@ -513,8 +518,8 @@ __global__ void __launch_bounds__(PASS_THREADS, pass_min_ctas(R)) k_inv_last(con
       for (int k = 0; k < (1 << B2); k++) y[k] = bspec[at + (k << 5)];
     }
     if (J.X) {
-      const uint64_t* __restrict__ X = J.X + off;
-      const uint64_t* __restrict__ Y = J.Y + off;
+      const uint64_t* X = J.X + off;
+      const uint64_t* Y = J.Y + off;
 #pragma unroll
       for (int k = 0; k < (1 << B2); k++) x[k] = gl::lz(gl::add(gl::mul(v[k], y[k]), gl::mul(X[at + (k << 5)], Y[at + (k << 5)])));
     } else {
@@ -642,7 +647,7 @@ __global__ void __launch_bounds__(PASS_THREADS, pass_min_ctas(R)) k_inv_first_ca
   constexpr int B1 = G::B1, B2 = G::B2, T = G::T;
   const Job J = job_of(jobs, one, L);
   if (J.flags & JF_ADDEND) return;
-  const uint64_t* __restrict__ data = J.A;
+  const uint64_t* data = J.A;
   extern __shared__ uint64_t sm[];
   const int tid = threadIdx.x;
   const int S = L - R;
@@ -712,7 +717,7 @@ __global__ void __launch_bounds__(128, 5) k_fwd_first3(const Job* jobs, Job one,
   const Job J = job_of(jobs, one, 0);
   const int which = w0 + (int)blockIdx.z;
   if (which == 1 && skips_b(J)) return;
-  const uint16_t* __restrict__ coef = reinterpret_cast<const uint16_t*>(which ? J.b : J.a);
+  const uint16_t* coef = reinterpret_cast<const uint16_t*>(which ? J.b : J.a);
   const uint64_t nc = 4 * (which ? J.lb : J.la);
   uint64_t* __restrict__ data = which ? J.B : J.A;
   extern __shared__ uint64_t sm[];
@@ -725,12 +730,12 @@ __global__ void __launch_bounds__(128, 5) k_fwd_first3(const Job* jobs, Job one,
     gl::Lz x[16];
     if (nc <= 96ull << S) {  // the upper half of the rows is zero
 #pragma unroll
-      for (int m = 0; m < 8; m++) x[m] = gl::Lz{n0 + m * step < nc ? (uint32_t)__ldg(coef + n0 + m * step) : 0u, 0u, 0};
+      for (int m = 0; m < 8; m++) x[m] = gl::Lz{n0 + m * step < nc ? (uint32_t)coef[n0 + m * step] : 0u, 0u, 0};
       x[0] = gl::lz_bias(x[0]);
       dft_lz<4, false, true>(x, v);
     } else {
 #pragma unroll
-      for (int m = 0; m < 16; m++) x[m] = gl::Lz{n0 + m * step < nc ? (uint32_t)__ldg(coef + n0 + m * step) : 0u, 0u, 0};
+      for (int m = 0; m < 16; m++) x[m] = gl::Lz{n0 + m * step < nc ? (uint32_t)coef[n0 + m * step] : 0u, 0u, 0};
       x[0] = gl::lz_bias(x[0]);
       dft_lz<4, false>(x, v);
     }
@@ -756,7 +761,7 @@ __global__ void __launch_bounds__(128, 5) k_inv_first3_carry(const Job* jobs, Jo
   using G = ThreeGeom;
   const Job J = job_of(jobs, one, 0);
   if (J.flags & JF_ADDEND) return;
-  const uint64_t* __restrict__ data = J.A;
+  const uint64_t* data = J.A;
   extern __shared__ uint64_t sm[];
   const int tid = threadIdx.x;
   const uint64_t j0 = (uint64_t)blockIdx.x << G::T;
@@ -1372,7 +1377,7 @@ __global__ void __cluster_dims__(2 * ClusterGeom<L>::OP, 1, 1) __launch_bounds__
   constexpr uint64_t ninv = gl::P - ((1ull << (64 - L)) - (1ull << (32 - L)));  // 2^-L
   if (!(isb && square)) {
     // pass 1, round 1: coefficients row 2^R2 + column, rows (m << B2) + jp
-    const uint16_t* __restrict__ coef = reinterpret_cast<const uint16_t*>(isb ? job.b : job.a);
+    const uint16_t* coef = reinterpret_cast<const uint16_t*>(isb ? job.b : job.a);
     const uint32_t nc = 4 * (isb ? lb : la);
 #pragma unroll 1
     for (uint32_t w = t; w < (1u << (B2 + TC)); w += NT) {
@@ -1382,7 +1387,7 @@ __global__ void __cluster_dims__(2 * ClusterGeom<L>::OP, 1, 1) __launch_bounds__
 #pragma unroll
       for (int m = 0; m < (1 << B1); m++) {
         const uint32_t n = (((m << B2) + jp) << R2) + col0 + c;
-        x[m] = gl::Lz{n < nc ? (uint32_t)__ldg(coef + n) : 0u, 0u, 0};
+        x[m] = gl::Lz{n < nc ? (uint32_t)coef[n] : 0u, 0u, 0};
       }
       x[0] = gl::lz_bias(x[0]);
       dft_lz<B1, false>(x, v);
