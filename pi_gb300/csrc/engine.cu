@@ -2350,6 +2350,18 @@ static uint64_t scratch_bytes(uint64_t la, uint64_t lb, bool square) {
   if (sg.L) return ((uint64_t)(sg.S + 1) << sg.L) * 8 + round256(z.nwin * 16) + round256(carry_words(z.nwin) * 8);
   return round256(z.N * 8) + round256(square ? z.nwin * 16 : z.N * 8) + round256(carry_words(z.nwin) * 8);
 }
+// Device memory that a pipeline product of a batch takes at most, descriptors
+// included, whatever it is batched with: whole, or cut, which it is not where
+// another product of the batch has the same b.  (One that lends its spectrum
+// holds the windows' low parts, at most N/4 words, apart, and the one that
+// borrows it has N words less.)
+static uint64_t batch_bytes(uint64_t la, uint64_t lb) {
+  const Sizes z = sizes_for(la, lb);
+  const SegPlan sg = plan_segments(la, lb);
+  const uint64_t carry = round256(carry_words(z.nwin) * 8);
+  const uint64_t cut = sg.L ? ((uint64_t)(sg.S + 1) << sg.L) * 8 + round256(z.nwin * 16) + sg.S * sizeof(Job) : 0;
+  return std::max(2 * round256(z.N * 8) + sizeof(Job), cut) + carry;
+}
 static void carve_carry(Job& J, uint64_t* base, uint64_t nwin) {
   J.H = base;
   J.state = reinterpret_cast<uint32_t*>(base + nwin);
@@ -3873,7 +3885,7 @@ int pimul_submit(int op, uint64_t a, uint64_t b, uint64_t* out_handle, uint64_t*
   uint64_t outl = op == PIMUL_OP_ADD ? std::max(la, lb) + 1 : op == PIMUL_OP_SUB ? std::max(la, lb) : la + lb;
   uint64_t obytes = round256(std::max<uint64_t>(outl, 1) * 8);
   uint64_t scratch =
-      (!linear && la && lb && sizes_for(la, lb).L > SMALL_LOG_MAX) ? scratch_bytes(la, lb, false) : 0;
+      (!linear && la && lb && sizes_for(la, lb).L > SMALL_LOG_MAX) ? batch_bytes(la, lb) : 0;
   if (!linear && la && lb && sizes_for(la, lb).L > 32) return fail(PIMUL_EINVAL, "transform length above 2^32");
   if (obytes + scratch > g_svc.budget) return fail(PIMUL_ENOMEM, "request larger than the HBM budget");
   uint64_t* d = nullptr;
