@@ -2322,7 +2322,7 @@ static SegPlan plan_segments(uint64_t la, uint64_t lb) {
   SegPlan best;
   if (la < lb) std::swap(la, lb);
   const Sizes z = sizes_for(la, lb);
-  if (z.L <= SMALL_LOG_MAX + 1 || la < 2 * lb) return best;
+  if (z.L <= SMALL_LOG_MAX + 1 || z.L > 32 || la < 2 * lb) return best;
   double cost = 0.9 * 3 * transform_cost(z.L) * (three_holds(z.n_out, z.L) ? 0.8 : 1.0);
   const uint64_t wlo = (4 * lb - 1 + WIN_COEFFS - 1) / WIN_COEFFS;
   for (int L = SMALL_LOG_MAX + 1; L < z.L; L++) {
@@ -3884,9 +3884,9 @@ int pimul_submit(int op, uint64_t a, uint64_t b, uint64_t* out_handle, uint64_t*
   // a sum keeps every carry in max + 1 limbs; a difference (a >= b) fits in max
   uint64_t outl = op == PIMUL_OP_ADD ? std::max(la, lb) + 1 : op == PIMUL_OP_SUB ? std::max(la, lb) : la + lb;
   uint64_t obytes = round256(std::max<uint64_t>(outl, 1) * 8);
-  uint64_t scratch =
-      (!linear && la && lb && sizes_for(la, lb).L > SMALL_LOG_MAX) ? batch_bytes(la, lb) : 0;
-  if (!linear && la && lb && sizes_for(la, lb).L > 32) return fail(PIMUL_EINVAL, "transform length above 2^32");
+  const int L = !linear && la && lb ? sizes_for(la, lb).L : 0;
+  if (L > 32) return fail(PIMUL_EINVAL, "transform length above 2^32");
+  uint64_t scratch = L > SMALL_LOG_MAX ? batch_bytes(la, lb) : 0;
   if (obytes + scratch > g_svc.budget) return fail(PIMUL_ENOMEM, "request larger than the HBM budget");
   uint64_t* d = nullptr;
   cudaError_t e = cudaMallocFromPoolAsync((void**)&d, obytes, g_svc.pool, g_svc.streams[0]);
@@ -3907,7 +3907,7 @@ int pimul_submit(int op, uint64_t a, uint64_t b, uint64_t* out_handle, uint64_t*
   SvcRequest r;
   r.ticket = t;
   r.op = op;
-  r.L = (!linear && la && lb) ? log2_ceil(4 * la + 4 * lb - 1) : 0;
+  r.L = L;
   r.a = a;
   r.b = op == PIMUL_OP_SQR ? a : b;
   r.out = oid;

@@ -1,6 +1,6 @@
 """The service's HBM budget bounds what its requests really take: scratch of a
 group whose products share an operand (and are then not cut into segments)
-stays within the budget."""
+stays within the budget, and a length no transform holds is refused."""
 import ctypes
 
 import numpy as np
@@ -63,3 +63,17 @@ def test_products_that_share_an_operand_stay_within_the_budget(la, lb):
         pm.free(h)
     assert all(np.array_equal(g, want) for g in got)
     assert peak <= room, (peak, room)
+
+
+def test_a_length_above_2_32_is_refused():
+    import torch
+    x = torch.empty((1 << 30) + 1, dtype=torch.int64, device="cuda")  # 2^32 + 4 coefficients
+    long, short = pm.adopt(x.data_ptr(), x.numel()), pm.adopt(x.data_ptr(), 1000)
+    try:
+        for p, q in ((long, short), (short, long), (long, long)):
+            with pytest.raises(pm.PimulError) as e:
+                pm.submit(p, q, pm.OP_MUL)
+            assert e.value.code == 1
+    finally:
+        pm.free(long)
+        pm.free(short)
