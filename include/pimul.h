@@ -206,7 +206,9 @@ int pimul_batch_plan_destroy(pimul_batch_plan* plan);
  * the short products' persistent grid (CTAs per SM); keeps the fastest for later calls and writes a JSON
  * report.  pimul_tuning_set applies saved choices (passes = 0: default
  * count, ceil(log_n / 9) and at least 2; ctas <= 0: unchanged).
- * Transform lengths are not tuned.
+ * Transform lengths are not tuned, nor are transforms of 3 2^k points, nor
+ * few transforms of 2^17 or 2^18 points (up to 2^18 and 2^20 points in all),
+ * which run three short passes whatever the count.
  */
 int pimul_autotune(int log_n_min, int log_n_max, int reps, char* report, size_t report_cap);
 int pimul_tuning_set(int log_n, int passes, int small_ctas_per_sm);

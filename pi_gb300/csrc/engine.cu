@@ -2258,7 +2258,8 @@ static Plan make_plan_np(int L, int np) {
 // leave a warp or less per SM sub-partition with 32 elements a thread.  2^18
 // points: a lone product 31.0 us against 45.0, four 59.6 against 65.7, eight 90.8
 // against 82.3; 2^17 points: a lone one 26.7 against 35.9, two 39.1 against 45.3, four
-// 48.5 against 46.9.
+// 48.5 against 46.9.  A tuned count is for more than those: two passes are all it can
+// say at these lengths.
 static Plan make_plan(int L, uint64_t points = ~0ull) {
   if (is_three(L)) {
     // 192 rows, then 2^S points in one pass or two, the shorter first
@@ -2267,13 +2268,13 @@ static Plan make_plan(int L, uint64_t points = ~0ull) {
     const int r1 = S <= 14 ? 6 : S / 2;
     return Plan{L, 3, {0, r1, S - r1, 0, 0}};
   }
+  if (L == 17 && points <= 1ull << 18) return Plan{L, 3, {6, 6, 5, 0, 0}};
+  if (L == 18 && points <= 1ull << 20) return Plan{L, 3, {6, 6, 6, 0, 0}};
   int np = (L >= 0 && L <= 32) ? g_tuned_np[L].load(std::memory_order_relaxed) : 0;
   if (np) {
     Plan p = make_plan_np(L, np);
     if (plan_valid(p)) return p;
   }
-  if (L == 17 && points <= 1ull << 18) return Plan{L, 3, {6, 6, 5, 0, 0}};
-  if (L == 18 && points <= 1ull << 20) return Plan{L, 3, {6, 6, 6, 0, 0}};
   return make_plan_np(L, default_np(L));
 }
 
