@@ -1,6 +1,8 @@
 """Transforms of 2^L points where no shorter form takes the product over: more
 than three quarters full, and short operands whose spectrum two products share
-(which are not cut into segments).  Bit-exact against the CPU oracle."""
+(which are not cut into segments); and the longest transforms of 3 2^k points
+against the same product in a power of two.  Bit-exact against the CPU oracle
+where the case says nothing else."""
 import numpy as np
 import pytest
 
@@ -57,3 +59,25 @@ def test_random_product_through_two_middle_passes(passes):
     finally:
         pm.tuning_apply({"np_25": 0})
     assert np.array_equal(got, O.mul_mag(a, b))
+
+
+@pytest.mark.parametrize("k", [20, 21, 22, 23, 24])
+def test_three_times_a_power_of_two_against_a_power_of_two(k):
+    """Alone a product of at most 3 2^k coefficients runs at 3 2^k points; beside one that shares its b and needs
+    2^(k+2), at 2^(k+2)."""
+    import torch
+    q = 3 << (k - 2)  # limbs of 3 2^k coefficients
+    g = torch.Generator(device="cuda")
+    g.manual_seed(k)
+
+    def limbs(n):
+        return torch.randint(-(1 << 63), (1 << 63) - 1, (n,), generator=g, device="cuda", dtype=torch.int64)
+
+    a, long, b = limbs(q // 2 - 1), limbs(q // 2 + 3), limbs(q // 2 - 1)
+    alone = torch.full((a.numel() + b.numel(),), -1, dtype=torch.int64, device="cuda")
+    beside = torch.full_like(alone, -2)
+    other = torch.empty(long.numel() + b.numel(), dtype=torch.int64, device="cuda")
+    pm.mul_device(a, b, alone)
+    pm.mul_batch([(a, b, beside), (long, b, other)])
+    torch.cuda.synchronize()
+    assert torch.equal(alone, beside)
