@@ -1840,6 +1840,7 @@ static Roots roots_at(const uint64_t* d) {
 struct DeviceState {
   int device = -1;
   bool ready = false;
+  int lone_log = SMALL_LOG_MAX;  // longest transform (log2) of a lone product in one cluster
   uint64_t* d_roots = nullptr;
   Roots roots{};
   cudaMemPool_t pool = nullptr;
@@ -1869,6 +1870,33 @@ static cudaError_t set_smem_attrs() {
   return e;
 }
 
+// Longest transform (log2) that a lone product runs within a cluster here.  From
+// 2^13 points on that takes sixteen CTAs, more than every GPU or partition of one
+// need be able to place at once; where they cannot be (or PIMUL_WIDE_CLUSTERS=0
+// says so) those lengths take the passes.
+template <int L>
+static bool wide_cluster_fits() {
+  cudaLaunchConfig_t c = {};
+  c.gridDim = dim3(2 * ClusterGeom<L>::OP);
+  c.blockDim = dim3(ClusterGeom<L>::NT);
+  c.dynamicSmemBytes = ClusterGeom<L>::SMEM;
+  cudaLaunchAttribute at;
+  at.id = cudaLaunchAttributeClusterDimension;
+  at.val.clusterDim.x = 2 * ClusterGeom<L>::OP;
+  at.val.clusterDim.y = at.val.clusterDim.z = 1;
+  c.attrs = &at;
+  c.numAttrs = 1;
+  int n = 0;
+  if (cudaOccupancyMaxActiveClusters(&n, k_cluster_mul<L>, &c) == cudaSuccess) return n > 0;
+  cudaGetLastError();
+  return false;
+}
+static int lone_log_here() {
+  const char* e = getenv("PIMUL_WIDE_CLUSTERS");
+  if (e && atoi(e) == 0) return SMALL_LOG_MAX;
+  return !wide_cluster_fits<13>() ? SMALL_LOG_MAX : wide_cluster_fits<14>() ? CLUSTER_LOG_MAX : 13;
+}
+
 static int ensure_init(int device) {
   std::lock_guard<std::mutex> lk(g_mu);
   if (g_dev.ready) {
@@ -1887,6 +1915,7 @@ static int ensure_init(int device) {
   uint64_t thr = UINT64_MAX;  // keep freed blocks cached in the pool
   CU(cudaMemPoolSetAttribute(g_dev.pool, cudaMemPoolAttrReleaseThreshold, &thr));
   CU(set_smem_attrs());
+  g_dev.lone_log = lone_log_here();
   g_dev.device = device;
   g_dev.ready = true;
   return PIMUL_OK;
@@ -2705,7 +2734,7 @@ static int mul_device(const uint64_t* d_a, uint64_t la, const uint64_t* d_b, uin
   if (z.L > 32) return fail(PIMUL_EINVAL, "transform length above 2^32");
   const Roots& R = g_dev.roots;
   const bool square = d_a == d_b && la == lb;
-  if (z.L <= CLUSTER_LOG_MAX) {
+  if (z.L <= g_dev.lone_log) {
     if (b_ready) cudaStreamWaitEvent(st, b_ready, 0);
     SmallJob job{d_a, d_b, d_out, (uint32_t)la, (uint32_t)lb};
     {
@@ -4628,7 +4657,7 @@ static int mul_host_small(const uint64_t* a, size_t la, const uint64_t* b, size_
                           cudaStream_t st) {
   const size_t off_b = round256(la * 8), off_out = off_b + (square ? 0 : round256(lb * 8));
   const size_t off_s = off_out + round256((la + lb) * 8);
-  const size_t scratch = sizes_for(la, lb).L > CLUSTER_LOG_MAX ? scratch_bytes(la, lb, square) : 0;
+  const size_t scratch = sizes_for(la, lb).L > g_dev.lone_log ? scratch_bytes(la, lb, square) : 0;
   uint8_t* d = nullptr;
   cudaError_t e = cudaMallocAsync((void**)&d, off_s + scratch, g_dev.pool, st);
   if (e != cudaSuccess) {
@@ -4858,6 +4887,7 @@ static __device__ __align__(256) uint64_t g_noalloc_roots[ROOT_WORDS];
 
 struct NoAllocDev {
   bool ready = false;
+  int lone_log = SMALL_LOG_MAX;  // as DeviceState::lone_log
   uint64_t* scratch = nullptr;  // device address of g_noalloc_scratch on this device
   Roots roots{};
 };
@@ -4889,6 +4919,7 @@ static int noalloc_setup(NoAllocDev** out) {
     if (e != cudaSuccess) return fail(PIMUL_ECUDA, std::string("cudaGetSymbolAddress(roots): ") + cudaGetErrorString(e));
     CU(cudaMemcpyToSymbol(g_noalloc_roots, g_na_host_roots, sizeof(g_na_host_roots)));
     CU(set_smem_attrs());
+    d.lone_log = lone_log_here();
     d.scratch = scratch;
     d.roots = roots_at(roots);
     d.ready = true;
@@ -4904,7 +4935,7 @@ static int mul_device_noalloc(const uint64_t* d_a, uint64_t la, const uint64_t* 
   if (rc) return rc;
   const Sizes z = sizes_for(la, lb);
   const Roots& R = nd->roots;
-  if (z.L <= CLUSTER_LOG_MAX) {  // whole product in shared memory: no scratch
+  if (z.L <= nd->lone_log) {  // whole product in shared memory: no scratch
     SmallJob job{d_a, d_b, d_out, (uint32_t)la, (uint32_t)lb};
     if (z.L < CLUSTER_LOG_MIN) launch_small(job, R, st);
     else launch_cluster(z.L, job, R, st);
