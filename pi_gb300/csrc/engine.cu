@@ -1314,7 +1314,7 @@ __global__ void __launch_bounds__(small_threads(C, true), 1) k_small_one(SmallJo
     small_multiply<C, true>(job, R, sm, threadIdx.x, 0, sA, sBm);
 }
 
-// ---- whole multiply in one cluster (a lone product of 2^11 .. 2^14 points) --
+// ---- whole multiply in one cluster (a lone product of 2^11 .. 2^14 points, few of a batch) --
 // One SM takes 10.5 us for a lone product of 2^11 points and 18.7 for 2^12, and
 // the pass pipeline 17 us for 2^13 (five launches of mostly idle grids): eight
 // CTAs take 8.5 us for up to 2^12 points, sixteen 10.5 for 2^13 and 13.6 for
@@ -1323,11 +1323,21 @@ __global__ void __launch_bounds__(small_threads(C, true), 1) k_small_one(SmallJo
 // transposes between them (and the hand-over of b's spectrum, of the inverse's
 // columns and of the coefficients in natural order) as stores into the other
 // CTAs' shared memory.  Below 2^11 points one CTA is as fast.
+//
+// Few products of up to 2^11 points of a batch take four CTAs each: in
+// k_small_mul one of 2^11 points is 24 us of instructions, most of them fetched
+// for the first time (11 stall cycles per issue), and 8 of 250 x 250 limbs took
+// 32.4 us, 28.7 with the kernel before that one, 16 so; 100 of them 33.2 and 20.4,
+// 250 33.6 and 30.2, 300 33.7 and 33.5.  The batch's shorter products of 2^9
+// points and more go along (32 of 32 to 256 limbs 32.5 and 17.0 us), which saves
+// their turn in k_small_mul; without one of 2^11 points that is the faster
+// (14.9 against 15.3 us for 32 of 2^9 points, 17.2 and 29.2 for 250).
 constexpr int CLUSTER_LOG_MIN = 11, CLUSTER_LOG_MAX = 14;
+constexpr size_t CLUSTER_FEW = 256;
 
 template <int L>
 struct ClusterGeom {
-  static constexpr int LOP = L == 12 ? 2 : 3, OP = 1 << LOP;  // CTAs per operand
+  static constexpr int LOP = L == 11 ? 1 : L == 12 ? 2 : 3, OP = 1 << LOP;  // CTAs per operand
   static constexpr int R1 = (L + 1) / 2, R2 = L / 2;
   static constexpr int B1 = pass_b1(R1), B2 = pass_b2(R1), D1 = pass_b1(R2), D2 = pass_b2(R2);
   static constexpr int TC = R2 - LOP;                // log2 columns per CTA
@@ -1355,19 +1365,20 @@ __device__ __forceinline__ uint64_t* cluster_ptr(uint64_t* p, uint32_t rank) {
 }
 
 template <int L>
-__global__ void __cluster_dims__(2 * ClusterGeom<L>::OP, 1, 1) __launch_bounds__(ClusterGeom<L>::NT, 1) k_cluster_mul(SmallJob job, Roots R) {
+__global__ void __cluster_dims__(2 * ClusterGeom<L>::OP, 1, 1) __launch_bounds__(ClusterGeom<L>::NT, 1) k_cluster_mul(const SmallJob* jobs, SmallJob one, Roots R) {
   using G = ClusterGeom<L>;
   constexpr int R1 = G::R1, R2 = G::R2, B1 = G::B1, B2 = G::B2, D1 = G::D1, D2 = G::D2, TC = G::TC, RC = G::RC, NT = G::NT;
   constexpr uint32_t N = 1u << L, CM = (1u << TC) - 1;
   cluster_arrive();  // waited on before the first store into another CTA: all of them run by then
   pdl_wait();
+  const SmallJob job = jobs ? jobs[blockIdx.y] : one;
   extern __shared__ uint64_t sm[];
   uint64_t* X = sm;            // this CTA's columns: [row][column], stride CS
   uint64_t* Y = X + G::XW;     // its rows: [row][2^R2 words], stride YS; later its coefficients
   uint64_t* Z = Y + G::YW;     // b's spectrum; later the windows' high parts
   __shared__ uint32_t sA[NT / 32], sB[NT / 32];
   __shared__ uint64_t sF[G::OP];
-  const uint32_t rank = blockIdx.x & (G::OP - 1);  // the grid is one cluster
+  const uint32_t rank = blockIdx.x & (G::OP - 1);  // a cluster per blockIdx.y
   const bool isb = blockIdx.x >= G::OP;
   const uint32_t mine = isb ? G::OP : 0;           // first CTA of this operand
   const uint32_t la = job.la, lb = job.lb;
@@ -1857,6 +1868,7 @@ static cudaError_t set_smem_attrs() {
   cudaError_t e = cudaSuccess;
   if (e == cudaSuccess)
     e = cudaFuncSetAttribute(k_small_mul, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)small_cta_smem(SMALL_LOG_MAX));
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(k_cluster_mul<11>, cudaFuncAttributeMaxDynamicSharedMemorySize, ClusterGeom<11>::SMEM);
   if (e == cudaSuccess) e = cudaFuncSetAttribute(k_cluster_mul<12>, cudaFuncAttributeMaxDynamicSharedMemorySize, ClusterGeom<12>::SMEM);
   if (e == cudaSuccess) e = cudaFuncSetAttribute(k_cluster_mul<13>, cudaFuncAttributeMaxDynamicSharedMemorySize, ClusterGeom<13>::SMEM);
   if (e == cudaSuccess) e = cudaFuncSetAttribute(k_cluster_mul<13>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
@@ -2452,7 +2464,13 @@ static void launch_small_c(const SmallJob& job, const Roots& R, cudaStream_t st)
 // One product within a cluster.
 template <int L>
 static void launch_cluster_c(const SmallJob& job, const Roots& R, cudaStream_t st) {
-  launch_pdl(k_cluster_mul<L>, dim3(2 * ClusterGeom<L>::OP), ClusterGeom<L>::NT, ClusterGeom<L>::SMEM, st, job, R);
+  launch_pdl(k_cluster_mul<L>, dim3(2 * ClusterGeom<L>::OP), ClusterGeom<L>::NT, ClusterGeom<L>::SMEM, st,
+             (const SmallJob*)nullptr, job, R);
+}
+// n products of a batch, up to 2^11 points, a cluster each.
+static void launch_clusters(const SmallJob* d_jobs, unsigned n, const Roots& R, cudaStream_t st) {
+  using G = ClusterGeom<11>;
+  launch_pdl(k_cluster_mul<11>, dim3(2 * G::OP, n), G::NT, G::SMEM, st, d_jobs, SmallJob{}, R);
 }
 static void launch_cluster(int L, const SmallJob& job, const Roots& R, cudaStream_t st) {
   if (L <= 12) launch_cluster_c<12>(job, R, st);
@@ -2822,7 +2840,8 @@ struct BatchLayout {
   std::vector<Bucket> large;
   uint64_t arena_bytes = 0;
   std::vector<SegPlan> seg;  // per unit: how a product of a long by a short operand is cut
-  std::vector<SmallChunk> chunks;  // the small jobs in same-length chunks
+  size_t clusters = 0;             // of the small jobs the first ones that run in a cluster each
+  std::vector<SmallChunk> chunks;  // the others in same-length chunks
   size_t small_smem = 0;           // dynamic shared memory of their CTAs
 };
 
@@ -2950,14 +2969,18 @@ static int layout_batch(const Unit* units, size_t n, BatchLayout& B, bool share,
   }
   B.desc.reserve(n_large);
   // longest transforms first
-  size_t total = 0;
+  size_t total = 0, longer = 0;
+  for (int c = 9; c <= SMALL_LOG_MAX; c++) longer += count[c];
+  if (count[11] && !count[12] && longer <= CLUSTER_FEW) B.clusters = longer;
   for (int c = SMALL_LOG_MAX; c >= SMALL_TINY; c--) {
     if (!count[c]) continue;
-    const uint32_t per = small_per_cta(c);
-    for (size_t k = 0; k < count[c]; k += per)
-      B.chunks.push_back(SmallChunk{(uint32_t)(total + k), (uint32_t)std::min<size_t>(per, count[c] - k), c});
-    B.small_smem = std::max(B.small_smem, small_cta_smem(c));
     at[c] = total;
+    if (total >= B.clusters) {
+      const uint32_t per = small_per_cta(c);
+      for (size_t k = 0; k < count[c]; k += per)
+        B.chunks.push_back(SmallChunk{(uint32_t)(total + k), (uint32_t)std::min<size_t>(per, count[c] - k), c});
+      B.small_smem = std::max(B.small_smem, small_cta_smem(c));
+    }
     total += count[c];
   }
   B.small.resize(total);
@@ -3126,7 +3149,11 @@ static void fill_descriptors(const Unit* units, const BatchLayout& B, uint8_t* a
 }
 
 static void launch_batch(const Launcher& X, const BatchLayout& B, const SmallJob* d_small, const Job* d_large) {
-  if (!B.small.empty()) {
+  if (B.clusters) {
+    KTimer kt(K_SMALL, X.st, X.stats);
+    launch_clusters(d_small, (unsigned)B.clusters, X.R, X.st);
+  }
+  if (!B.chunks.empty()) {
     int sms = 152;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, g_dev.device);
     uint64_t grid = (uint64_t)sms * (uint64_t)g_small_ctas_per_sm.load();
@@ -4827,10 +4854,14 @@ int mul_batch_strided(const uint64_t* a, uint64_t sa, size_t la, const uint64_t*
   SmallChunk* dc = reinterpret_cast<SmallChunk*>(dev + jb);
   k_fill_small<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(dj, dc, SmallJob{a, b, out, (uint32_t)la, (uint32_t)lb},
                                                            sa, so, (uint32_t)n, per, c);
-  int sms = 152;
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, g_dev.device);
-  const uint64_t grid = std::min<uint64_t>((uint64_t)sms * (uint64_t)g_small_ctas_per_sm.load(), nch);
-  launch_pdl(k_small_mul, dim3((unsigned)grid), SMALL_THREADS, small_cta_smem(c), st, dj, dc, (uint32_t)nch, g_dev.roots);
+  if (c == 11 && n <= CLUSTER_FEW) {
+    launch_clusters(dj, (unsigned)n, g_dev.roots, st);
+  } else {
+    int sms = 152;
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, g_dev.device);
+    const uint64_t grid = std::min<uint64_t>((uint64_t)sms * (uint64_t)g_small_ctas_per_sm.load(), nch);
+    launch_pdl(k_small_mul, dim3((unsigned)grid), SMALL_THREADS, small_cta_smem(c), st, dj, dc, (uint32_t)nch, g_dev.roots);
+  }
   e = cudaGetLastError();
   cudaFreeAsync(dev, st);
   if (e != cudaSuccess) return fail(PIMUL_ECUDA, std::string("strided batch launch: ") + cudaGetErrorString(e));
