@@ -15,7 +15,6 @@
 #include <chrono>
 #include <condition_variable>
 #include <deque>
-#include <functional>
 #include <thread>
 #include <unordered_map>
 #include <atomic>
@@ -935,9 +934,9 @@ __global__ void __launch_bounds__(CARRY_THREADS) k_carry(const Job* jobs, Job on
 
 // ---- whole multiply in one CTA (N <= 2^SMALL_LOG_MAX) --------------------
 // Products of up to 64 limbs in all are schoolbook column sums by one warp
-// (class 7); longer ones take three transforms of 2^c points (class c = 8 ..
+// (class 7); longer ones take three transforms of 2^c points (class c = 9 ..
 // 12) as two or three rounds of radix 8 or 16 in registers.  A lone product
-// (and class 8, one warp) holds operands a and b side by side in the halves of
+// holds operands a and b side by side in the halves of
 // its threads: one SM is all it has, and a thread's instructions are its time.
 // In a batch a group of G threads transforms one operand after the other, two
 // CTAs per SM, so that no thread idles through the inverse and other groups
@@ -948,7 +947,8 @@ constexpr int SMALL_LOG_MAX = 12;
 constexpr int SMALL_TINY = 7;        // class of the one-warp products
 constexpr uint64_t TINY_LIMBS = 64;  // la + lb
 
-// Radix (log2) of round q of a class-c transform (0: no such round).
+// Radix (log2) of round q of a 2^c-point transform (0: no such round; 2^8 points come
+// in the merged splitting levels only).
 __host__ __device__ constexpr int small_b(int c, int q) {
   return c == 8 ? (q < 2 ? 4 : 0) : c == 9 ? 3 : c == 10 ? (q == 0 ? 4 : 3) : c == 11 ? (q < 2 ? 4 : 3) : 4;
 }
@@ -957,12 +957,11 @@ __host__ __device__ constexpr int small_op_threads(int c) { return c == 9 ? 64 :
 __host__ __device__ constexpr int small_threads(int c, bool split) {
   return c == SMALL_TINY ? 32 : (split ? 2 : 1) * small_op_threads(c);
 }
-__host__ __device__ constexpr bool small_split(int c) { return c <= 8; }  // in a batch
 // Class of a product of la + lb limbs.
 __host__ __device__ __forceinline__ int small_class(uint64_t la, uint64_t lb) {
   if (la + lb <= TINY_LIMBS) return SMALL_TINY;
   const uint32_t n = (uint32_t)(4 * (la + lb) - 1);
-  return n <= 256 ? 8 : n <= 512 ? 9 : n <= 1024 ? 10 : n <= 2048 ? 11 : 12;
+  return n <= 512 ? 9 : n <= 1024 ? 10 : n <= 2048 ? 11 : 12;
 }
 // Dynamic shared memory words of one product: a padded array per operand held
 // at a time, and the windows' high parts (a tiny product: its operands, 64 zero
@@ -971,9 +970,9 @@ __host__ __device__ constexpr uint32_t small_words(int c, bool split) {
   return c == SMALL_TINY ? 256 : split ? 2 * spad(1u << c) : spad(1u << c) + (1u << c) / 16;
 }
 // Products of one class side by side in a batch CTA, and its shared memory.
-__host__ __device__ __forceinline__ uint32_t small_per_cta(int c) { return SMALL_THREADS / small_threads(c, small_split(c)); }
+__host__ __device__ __forceinline__ uint32_t small_per_cta(int c) { return SMALL_THREADS / small_threads(c, false); }
 __host__ __device__ __forceinline__ size_t small_cta_smem(int c) {
-  return (size_t)small_per_cta(c) * small_words(c, small_split(c)) * 8;
+  return (size_t)small_per_cta(c) * small_words(c, false) * 8;
 }
 
 struct SmallJob {
@@ -1113,7 +1112,7 @@ __device__ __forceinline__ void small_multiply(const SmallJob& job, const Roots&
                                                uint32_t* sBm) {
   constexpr int B1 = small_b(C, 0), B2 = small_b(C, 1), B3 = small_b(C, 2);
   constexpr int G = small_op_threads(C), T = small_threads(C, SPLIT);
-  constexpr int S1 = C - B1, S2 = S1 - B2, BL = B3 ? B3 : B2, ITL = (1 << (C - BL)) / G;
+  constexpr int BL = B3 ? B3 : B2, ITL = (1 << (C - BL)) / G;
   constexpr uint32_t N = 1u << C;
   uint64_t* smB = smA + spad(N);  // b's array (SPLIT); the windows' high parts
   const uint32_t la = job.la, lb = job.lb;
@@ -1267,15 +1266,15 @@ __device__ void tiny_multiply(const SmallJob& job, uint64_t* sm, int lane) {
 template <int C>
 __device__ __noinline__ void small_chunk(const SmallJob* jobs, const SmallChunk& ch, const Roots& R, uint64_t* sm,
                                          uint32_t* sA, uint32_t* sBm) {
-  constexpr int T = small_threads(C, small_split(C));
+  constexpr int T = small_threads(C, false);
   const uint32_t grp = threadIdx.x / T;
   if (grp >= ch.count) return;
   const SmallJob job = jobs[ch.first + grp];
-  uint64_t* base = sm + (size_t)grp * small_words(C, small_split(C));
+  uint64_t* base = sm + (size_t)grp * small_words(C, false);
   if constexpr (C == SMALL_TINY)
     tiny_multiply(job, base, threadIdx.x & 31);
   else
-    small_multiply<C, small_split(C)>(job, R, base, (int)(threadIdx.x % T), (int)grp, sA, sBm);
+    small_multiply<C, false>(job, R, base, (int)(threadIdx.x % T), (int)grp, sA, sBm);
 }
 
 // Chunks of same-class products; the CTAs stride over the chunks (a
@@ -1292,7 +1291,6 @@ __global__ void __launch_bounds__(SMALL_THREADS, 2) k_small_mul(const SmallJob* 
     const SmallChunk ch = chunks[k];
     switch (ch.c) {
       case SMALL_TINY: small_chunk<SMALL_TINY>(jobs, ch, R, sm, sA, sBm); break;
-      case 8: small_chunk<8>(jobs, ch, R, sm, sA, sBm); break;
       case 9: small_chunk<9>(jobs, ch, R, sm, sA, sBm); break;
       case 10: small_chunk<10>(jobs, ch, R, sm, sA, sBm); break;
       case 11: small_chunk<11>(jobs, ch, R, sm, sA, sBm); break;
@@ -2481,7 +2479,6 @@ static void launch_cluster(int L, const SmallJob& job, const Roots& R, cudaStrea
 static void launch_small(const SmallJob& job, const Roots& R, cudaStream_t st) {
   switch (small_class(job.la, job.lb)) {
     case SMALL_TINY: launch_small_c<SMALL_TINY>(job, R, st); break;
-    case 8: launch_small_c<8>(job, R, st); break;
     case 9: launch_small_c<9>(job, R, st); break;
     default: launch_small_c<10>(job, R, st); break;  // longer ones: launch_cluster
   }

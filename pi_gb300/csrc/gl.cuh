@@ -2,7 +2,7 @@
 //
 // Same field as the reference's CPU code (crates/bignum/src/ntt.rs:159-284).
 // Inside the transforms values are kept "weak": any 64-bit word congruent to
-// the field element (so possibly in [p, 2^64)).  add / sub / mul accept weak
+// the field element (so possibly in [p, 2^64)).  add / mul accept weak
 // inputs and return weak outputs; canon() gives the canonical representative
 // in [0, p), which is what leaves the engine.  The reduction uses
 // 2^64 = 2^32 - 1 (mod p) and 2^96 = -1 (mod p), written as 32-bit carry
@@ -35,25 +35,6 @@ __device__ __forceinline__ uint64_t add(uint64_t a, uint64_t b) {
       "neg.s32 m, c;\n\t"
       "add.cc.u32 %0, %0, m;\n\t"
       "addc.u32 %1, %1, 0;\n\t"
-      "}"
-      : "=&r"(z0), "=&r"(z1)
-      : "r"(lo32(a)), "r"(hi32(a)), "r"(lo32(b)), "r"(hi32(b)));
-  return mk64(z0, z1);
-}
-
-// a - b (weak in, weak out).  A borrow is worth -2^64 = -EPS; subtracting
-// EPS can borrow once more, folded the same way.
-__device__ __forceinline__ uint64_t sub(uint64_t a, uint64_t b) {
-  uint32_t z0, z1;
-  asm("{\n\t.reg .u32 m;\n\t"
-      "sub.cc.u32 %0, %2, %4;\n\t"
-      "subc.cc.u32 %1, %3, %5;\n\t"
-      "subc.u32 m, 0, 0;\n\t"
-      "sub.cc.u32 %0, %0, m;\n\t"
-      "subc.cc.u32 %1, %1, 0;\n\t"
-      "subc.u32 m, 0, 0;\n\t"
-      "sub.cc.u32 %0, %0, m;\n\t"
-      "subc.u32 %1, %1, 0;\n\t"
       "}"
       : "=&r"(z0), "=&r"(z1)
       : "r"(lo32(a)), "r"(hi32(a)), "r"(lo32(b)), "r"(hi32(b)));
@@ -261,17 +242,6 @@ __device__ __forceinline__ Lz lz_shl24_wide(Lz x) {
   z.h = __funnelshift_l(x.l, x.h, 24);
   z.k = (int32_t)__funnelshift_l(x.h, (uint32_t)x.k, 24);
   return z;
-}
-
-// base^e mod p (canonical result).
-__device__ __forceinline__ uint64_t pow(uint64_t base, uint64_t e) {
-  uint64_t acc = 1;
-  while (e) {
-    if (e & 1) acc = mul(acc, base);
-    e >>= 1;
-    if (e) base = mul(base, base);
-  }
-  return canon(acc);
 }
 
 }  // namespace gl
