@@ -437,10 +437,12 @@ int pimul_pi_gauss_legendre(uint64_t digits, char* out, size_t cap, pimul_mul_fn
 int pimul_pi_gauss_legendre_ex(uint64_t digits, char* out, size_t cap, pimul_mul_fn backend, uint64_t ntt_threshold,
                                uint32_t flags, double* phase_ms, uint64_t* ntt_products);
 
-/* Transform plan for a product: the power of two N that holds it and the number
- * of HBM passes per transform of that length.  Mirrors the sizing of
- * crates/bignum/src/ntt.rs:810-813; a product that fills at most three quarters
- * of N, or has a short operand, may run shorter transforms. */
+/* The sizing rule for a product: the power of two N that holds it
+ * (crates/bignum/src/ntt.rs:810-813) and the default or tuned number of HBM
+ * passes per transform of N points, 0 up to 2^12.  It does not say which kernels
+ * a call launches: a product that fills at most three quarters of N, or has a
+ * short operand, may run shorter transforms; a lone one of 2^13 or 2^14 points
+ * runs in shared memory; few of 2^17 or 2^18 points run three passes. */
 int pimul_plan(size_t la, size_t lb, uint64_t* n_transform, int* passes);
 
 /* Kernel launch statistics (this engine's own instrumentation; the

@@ -544,8 +544,8 @@ __global__ void __launch_bounds__(PASS_THREADS, pass_min_ctas(R)) k_inv_last(con
 // V_w = sum_t c[8w+t] 2^(16t) = lo_w + hi_w 2^128 (hi_w < 2^49).  The
 // product is sum_w (lo_w + hi_(w-1)) 2^(128w); s_w = lo_w + hi_(w-1) may
 // carry one bit (g_w) into window w+1, which a run of all-ones windows (p_w)
-// propagates.  Carries are resolved with a carry-lookahead scan over (g, p)
-// bit vectors: with A = g|p and B = g, the carry into each window is bit w of
+// propagates.  Carries are resolved by lookahead over (g, p) bit vectors: with
+// A = g|p and B = g, the carry into each window of a warp is bit w of
 // (A + B + cin) ^ A ^ B.
 
 struct Win2 {
@@ -1860,8 +1860,9 @@ static DeviceState g_dev;
 static thread_local cudaStream_t t_stream = nullptr;
 static thread_local int t_stream_dev = -1;
 
-// Opt the one-CTA kernels into their dynamic shared memory (the pass kernels
-// stay below 48 KB).
+// Opt the short products', cluster and merge kernels into their dynamic shared
+// memory (the pass kernels stay below 48 KB) and the sixteen-CTA clusters into
+// their size.
 static cudaError_t set_smem_attrs() {
   cudaError_t e = cudaSuccess;
   if (e == cudaSuccess)
@@ -2263,7 +2264,7 @@ static uint64_t length_words(int L) { return is_three(L) ? 3ull << (L - THREE) :
 
 // Pass-count override per L chosen by the autotuner (0 = default).
 static std::atomic<int> g_tuned_np[33];
-// Persistent grid of the one-CTA kernel in a batch: CTAs per SM (autotuned).
+// Persistent grid of the short products' kernel in a batch: CTAs per SM (autotuned).
 static std::atomic<int> g_small_ctas_per_sm{4};
 
 static int default_np(int L) {
@@ -2279,7 +2280,8 @@ static bool plan_valid(const Plan& p) { return p.np != 0; }
 // 1285 as 8 + 8 + 9, 1301 as 9 + 8 + 8).  Two passes: even, the longer first (16
 // products of 2^15 points: 40.0 us as 8 + 7, 43.5 as 7 + 8, 45.3 as 6 + 9).  Four
 // and five: even, the longer last.  np passes must leave radices of 2^6 .. 2^9 and
-// one of at least 2^7; an invalid plan (np 0) for anything else.
+// one of at least 2^7; an invalid plan (np 0) for anything else.  (make_plan's
+// three passes for few transforms of 2^17 or 2^18 points are not among these.)
 static Plan make_plan_np(int L, int np) {
   Plan p{L, 0, {0, 0, 0, 0, 0}};
   if (np < 2 || np > 5 || L < 6 * np + 1 || L > 9 * np) return p;
@@ -2789,10 +2791,11 @@ static int mul_device(const uint64_t* d_a, uint64_t la, const uint64_t* d_b, uin
 
 // ------------------------------------------------------------------ batches
 // A batch of independent products (and sums of two products) on device
-// buffers.  Products are grouped by transform length: lengths up to 2^12
-// run as one CTA per product in a persistent kernel over a size-sorted list;
-// longer ones run the pass pipeline once per length with one grid row
-// (blockIdx.y) per descriptor.  Within a group of one length, products whose
+// buffers.  Products are grouped by transform length: those of up to 2^12
+// points run whole in shared memory, several of one class side by side in the
+// CTAs of a persistent kernel over a list sorted by class (few of up to 2^11
+// points in a cluster each); longer ones run the pass pipeline once per length
+// with one grid row (blockIdx.y) per descriptor.  Within a group of one length, products whose
 // operand b is the same array share b's spectrum (computed once), and a sum
 // a1 b1 + a2 b2 runs as two descriptors whose spectra are added before one
 // inverse transform and one carry pass.
@@ -3318,7 +3321,7 @@ static void plan_destroy(BatchPlan* P) {
 // ------------------------------------------------------------------ autotuner
 // Times the candidate pass counts for each length in [Lmin, Lmax] on a
 // batch of `reps` synthetic products (device-resident), keeps the fastest,
-// and tunes the one-CTA kernel's persistent grid on a batch of small
+// and tunes the short products' persistent grid on a batch of small
 // products.  The choice only changes the schedule; products are identical.
 static int autotune(int Lmin, int Lmax, int reps, char* report, size_t cap) {
   int rc = ensure_init(-1);
@@ -4133,11 +4136,13 @@ int pimul_service_reset_stats(void) {
 // ------------------------------------------------- batched add / subtract
 // out = x + y or x - y (x >= y) for many limb arrays at once, the additions
 // and subtractions of a binary-splitting level done where its products
-// live.  Same carry-lookahead structure as the product's carry pass: windows
-// of 4 limbs add with carry-in 0 and report (generate, propagate); a scan
-// over chunk summaries gives every window its carry; windows that receive
-// one ripple it (+1 / -1) through their limbs.  A carry or borrow out of the
-// top limb is reported (it means x < y for a subtraction).
+// live.  Windows of 4 limbs add with carry-in 0 and report (generate,
+// propagate) and chunks of 256 windows their carry function; a chunk's carry in
+// comes from the nearest chunk on its left that has a fixed carry out, or from a
+// scan where there are many chunks; windows that receive a carry ripple it (+1 /
+// -1) through their limbs.  An array of one chunk is finished by the first
+// kernel.  A carry or borrow out of the top limb is reported (it means x < y for
+// a subtraction).
 constexpr int AS_THREADS = 256;
 constexpr int AS_W = 4;
 
@@ -4785,7 +4790,7 @@ int pimul_mul(const uint64_t* a, size_t la, const uint64_t* b, size_t lb, uint64
 //
 // Limits and sharing rules:
 //  * scratch holds two transform arrays of at most 2^20 words plus the carry
-//    windows and scan flags: la + lb <= 262144 limbs (transform length
+//    windows and chunk states: la + lb <= 262144 limbs (transform length
 //    N <= 2^20); larger products are rejected with PIMUL_EINVAL.  The
 //    scratch (17 MiB) and this path's own root tables (18 MiB) stay
 //    resident on every GPU that loads this library, until the process exits.

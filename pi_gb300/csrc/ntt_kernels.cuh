@@ -13,9 +13,9 @@
 // (crates/bignum/src/ntt.rs:905-1105) without the transposes: strided tiles
 // are read as coalesced 64-byte (or wider) row segments.
 //
-// Inside a pass the R_p-point DFT runs as two rounds of radix 8, 16 or 32
-// held in registers (rounds of radix 8, 4 or 2 in shared memory in the
-// merged splitting levels).  2 is a 192nd root of unity mod p, and the root tables
+// Inside a pass the R_p-point DFT runs as two rounds of radix 4 to 32 held in
+// registers; the short products and the merged splitting levels run two or three
+// rounds of radix 8 or 16.  2 is a 192nd root of unity mod p, and the root tables
 // are built so that the 64th root of unity is 2^3: the butterflies' internal
 // twiddles are constant shifts.
 #pragma once
