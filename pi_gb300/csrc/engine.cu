@@ -1362,21 +1362,26 @@ __device__ __forceinline__ uint64_t* cluster_ptr(uint64_t* p, uint32_t rank) {
   return reinterpret_cast<uint64_t*>(r);
 }
 
-template <int L>
-__global__ void __cluster_dims__(2 * ClusterGeom<L>::OP, 1, 1) __launch_bounds__(ClusterGeom<L>::NT, 1) k_cluster_mul(const SmallJob* jobs, SmallJob one, Roots R) {
+// LIST: a cluster per blockIdx.y and its job from a device list; else one product
+// by value (read from either, a lone 2^13-point product took 10.7 us, not 10.5).
+template <int L, bool LIST = false>
+__global__ void __cluster_dims__(2 * ClusterGeom<L>::OP, 1, 1) __launch_bounds__(ClusterGeom<L>::NT, 1)
+    k_cluster_mul(std::conditional_t<LIST, const SmallJob*, SmallJob> from, Roots R) {
   using G = ClusterGeom<L>;
   constexpr int R1 = G::R1, R2 = G::R2, B1 = G::B1, B2 = G::B2, D1 = G::D1, D2 = G::D2, TC = G::TC, RC = G::RC, NT = G::NT;
   constexpr uint32_t N = 1u << L, CM = (1u << TC) - 1;
   cluster_arrive();  // waited on before the first store into another CTA: all of them run by then
   pdl_wait();
-  const SmallJob job = jobs ? jobs[blockIdx.y] : one;
+  SmallJob job;
+  if constexpr (LIST) job = from[blockIdx.y];
+  else job = from;
   extern __shared__ uint64_t sm[];
   uint64_t* X = sm;            // this CTA's columns: [row][column], stride CS
   uint64_t* Y = X + G::XW;     // its rows: [row][2^R2 words], stride YS; later its coefficients
   uint64_t* Z = Y + G::YW;     // b's spectrum; later the windows' high parts
   __shared__ uint32_t sA[NT / 32], sB[NT / 32];
   __shared__ uint64_t sF[G::OP];
-  const uint32_t rank = blockIdx.x & (G::OP - 1);  // a cluster per blockIdx.y
+  const uint32_t rank = blockIdx.x & (G::OP - 1);
   const bool isb = blockIdx.x >= G::OP;
   const uint32_t mine = isb ? G::OP : 0;           // first CTA of this operand
   const uint32_t la = job.la, lb = job.lb;
@@ -1867,7 +1872,7 @@ static cudaError_t set_smem_attrs() {
   cudaError_t e = cudaSuccess;
   if (e == cudaSuccess)
     e = cudaFuncSetAttribute(k_small_mul, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)small_cta_smem(SMALL_LOG_MAX));
-  if (e == cudaSuccess) e = cudaFuncSetAttribute(k_cluster_mul<11>, cudaFuncAttributeMaxDynamicSharedMemorySize, ClusterGeom<11>::SMEM);
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(k_cluster_mul<11, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, ClusterGeom<11>::SMEM);
   if (e == cudaSuccess) e = cudaFuncSetAttribute(k_cluster_mul<12>, cudaFuncAttributeMaxDynamicSharedMemorySize, ClusterGeom<12>::SMEM);
   if (e == cudaSuccess) e = cudaFuncSetAttribute(k_cluster_mul<13>, cudaFuncAttributeMaxDynamicSharedMemorySize, ClusterGeom<13>::SMEM);
   if (e == cudaSuccess) e = cudaFuncSetAttribute(k_cluster_mul<13>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
@@ -2464,13 +2469,12 @@ static void launch_small_c(const SmallJob& job, const Roots& R, cudaStream_t st)
 // One product within a cluster.
 template <int L>
 static void launch_cluster_c(const SmallJob& job, const Roots& R, cudaStream_t st) {
-  launch_pdl(k_cluster_mul<L>, dim3(2 * ClusterGeom<L>::OP), ClusterGeom<L>::NT, ClusterGeom<L>::SMEM, st,
-             (const SmallJob*)nullptr, job, R);
+  launch_pdl(k_cluster_mul<L>, dim3(2 * ClusterGeom<L>::OP), ClusterGeom<L>::NT, ClusterGeom<L>::SMEM, st, job, R);
 }
 // n products of a batch, up to 2^11 points, a cluster each.
 static void launch_clusters(const SmallJob* d_jobs, unsigned n, const Roots& R, cudaStream_t st) {
   using G = ClusterGeom<11>;
-  launch_pdl(k_cluster_mul<11>, dim3(2 * G::OP, n), G::NT, G::SMEM, st, d_jobs, SmallJob{}, R);
+  launch_pdl(k_cluster_mul<11, true>, dim3(2 * G::OP, n), G::NT, G::SMEM, st, d_jobs, R);
 }
 static void launch_cluster(int L, const SmallJob& job, const Roots& R, cudaStream_t st) {
   if (L <= 12) launch_cluster_c<12>(job, R, st);
