@@ -49,10 +49,10 @@ BITS_B = 1 << 30
 
 # DRAM traffic of the dominant kernel class (forward passes after the first) per
 # transform word: dram__bytes_read.sum + dram__bytes_write.sum from one ncu
-# capture of each of k_col_mid<8,fwd> (15.19 bytes per word) and k_fwd_last<9>
-# (15.07) of a 2^28 x 2^28-bit product (N = 2^25); the class runs each once per
+# capture of each of k_col_mid<9,fwd> (15.79 bytes per word) and k_fwd_last<9>
+# (15.76) of a 2^30 x 2^30-bit product (N = 2^27); the class runs each once per
 # transform.
-NCU_TRAFFIC_BYTES_PER_WORD = 15.13
+NCU_TRAFFIC_BYTES_PER_WORD = 15.78
 
 
 def b_mul(n, la, lb, square=False):
@@ -209,8 +209,8 @@ def stats(lib):
 # 2^30 x 2^30-bit product, N = 2^27, plan 2^9 x 2^9 x 2^9).  Instruction counts
 # do not depend on the clock or on timing.
 NCU_ALU_PER_WORD = {
-    "k_fwd_first": 1.88, "k_col_mid_fwd": 1.82, "k_fwd_last": 1.42, "k_inv_last": 1.75,
-    "k_col_mid_inv": 1.89, "k_inv_first_carry": 2.15, "k_carry": 0.48,
+    "k_fwd_first": 1.88, "k_col_mid_fwd": 1.82, "k_fwd_last": 1.42, "k_inv_last": 1.61,
+    "k_col_mid_inv": 1.89, "k_inv_first_carry": 2.20, "k_carry": 0.48,
 }
 # The integer ALU pipe retires 16 lanes per clock per SM sub-partition:
 # half a warp instruction per clock, four sub-partitions per SM.
